@@ -9,19 +9,15 @@
  * not below eps, which is the same predicate. Orientation: rows are the query when the
  * candidate is at least as long, else the candidate (Grid.cpp:1234-1247).
  *
- * Mapping: a warp works on row tiles of 32*R rows. Lane L owns R consecutive rows of the tile
- * and handles column j = s - L at step s, so a step advances 32*R cells of one anti-diagonal
- * band. The value below a lane's last row moves to the next lane with one shuffle per step;
- * columns are staged 32 at a time in per-warp shared memory that every lane reads; a tile hands
- * its bottom row to the next tile through a carry row in global memory (L2-resident).
- * Everything is int32 arithmetic plus two float subtractions and two compares per cell.
- *
- * Two kernels: k_edr (one warp per pair, its tiles in sequence; used by the allocation-free
- * entry point) and k_edr_tiles (row tiles as work items, longest pairs first, consecutive
- * tiles of a pair pipelined across warps; every other caller).
+ * Three kernels: k_edr_rows (row tiles as work items, longest pairs first, consecutive tiles of a
+ * pair pipelined across warps, two cells per 32-bit word; every caller but the next two),
+ * k_edr_cols (column tiles, one cell per word; GAT_TUNE_EDR_FORM = 2) and k_edr (one warp per pair,
+ * its tiles in sequence; the allocation-free entry point). Everything is integer arithmetic plus
+ * float subtractions and compares for the match test.
  */
 #pragma once
 #include <algorithm>
+#include <type_traits>
 
 #include "internal.h"
 #include "launch.cuh"
@@ -30,7 +26,8 @@ namespace gat {
 namespace edr {
 
 constexpr int kWarps = 8; /* k_edr (one warp per pair) */
-constexpr int kTileWarps = 8; /* k_edr_tiles (2-warp CTAs measured no better on small launches) */
+constexpr int kRowWarps = 16; /* k_edr_rows: one CTA per SM, 128 registers per thread */
+constexpr int kColWarps = 8;  /* k_edr_cols */
 constexpr int kBig = 1 << 29; /* above any distance; up + 1 never overflows against it */
 
 /* Pair source over (a_off, a_len, b_off, b_len) arrays; results to out[p]. A pair with a side
@@ -226,7 +223,7 @@ constexpr int kCtrEpoch = 4 + 2 * kClasses;
 constexpr int kCtrWords = kCtrEpoch + 2;
 typedef unsigned long long carry_t;
 
-constexpr int kEdrCarveoutPct = 100; /* preferred shared-memory share of the SM for k_edr_tiles (launch_tiles) */
+constexpr int kEdrCarveoutPct = 100; /* preferred shared-memory share of the SM for the tile kernels (launch_tiles) */
 
 struct TileCtl {
     const int4* items; /* (pair, tile or -1 for a whole pair on one warp, cooperative slot, tiles) */
@@ -238,6 +235,7 @@ struct TileCtl {
     int32_t* flag;
     int spin_limit;  /* polls before a carry wait gives up (kSpinLimit) */
     int stall_pair;  /* tests of the bounded wait: this pair's first pipelined tile writes no carries (-1: none) */
+    unsigned one;    /* 1, unknown to the compiler: x * one + c is a multiply-add on the FMA pipe (row_step) */
 };
 
 /* The carry word is the only datum exchanged, so neither access needs to order other memory
@@ -260,6 +258,13 @@ __device__ __forceinline__ int duration_class(long long d) {
     return min(2 * e + half, kClasses - 1);
 }
 
+/* How a pair is cut: column tiles of 32 R columns, row tiles of 32 R rows (2H = R rows per lane),
+ * the last row tile of the smallest height 64 h, h a power of two, that holds the rest. */
+template <int R>
+__device__ __forceinline__ int tile_count(int nlane) {
+    return nlane <= 0 ? 1 : (nlane + 32 * R - 1) / (32 * R);
+}
+
 template <int R, bool COL, class Src>
 __global__ void k_sched_count(Src src, int cap, int coop_cap, int* __restrict__ ctr, int2* __restrict__ meta) {
     dep_wait();
@@ -274,7 +279,7 @@ __global__ void k_sched_count(Src src, int cap, int coop_cap, int* __restrict__ 
         src.get(p, a, la, b, lb, o);
         const int len1 = min(la, lb), len2 = max(la, lb);
         const int nlane = COL ? len2 : len1, nstep = COL ? len1 : len2;
-        const int T = nlane <= 0 ? 1 : (nlane + 32 * R - 1) / (32 * R);
+        const int T = tile_count<R>(nlane);
         int slot = -1, items = 1;
         if (T >= 2) {
             const int sl = atomicAdd(&ctr[1], 1);
@@ -283,7 +288,10 @@ __global__ void k_sched_count(Src src, int cap, int coop_cap, int* __restrict__ 
                 items = T;
             }
         }
-        const long long dur = slot >= 0 ? (long long)nstep + 32LL * (T - 1) : (long long)T * (nstep + 31);
+        /* steps of the critical path: a row tile starts 96 steps behind its predecessor, a column
+         * tile 32 */
+        constexpr int kLag = COL ? 32 : 96, kRamp = COL ? 31 : 63;
+        const long long dur = slot >= 0 ? (long long)nstep + (long long)kLag * (T - 1) : (long long)T * (nstep + kRamp);
         const int c = duration_class(dur);
         atomicAdd(&hist[c], items);
         meta[p] = make_int2(slot, (c << 16) | items);
@@ -356,29 +364,365 @@ __device__ __forceinline__ int match_mask(float ax, float ay, float2 b, float u)
     return m;
 }
 
-/* One wavefront step of a lane's R rows at column c (DP column index). Values are held shifted
- * by their column: E[r][c] = D[r][c] - c. The reference's three operands at (r, c) become, in
- * column c's shift, m = E[r-1][c-1] + (match ? -1 : 0), l = E[r][c-1] and u = E[r-1][c] + 1;
- * a common shift keeps every comparison, so the choice min(u, mml), mml = min(m, l) or +inf
- * when m == l, is taken on shifted values unchanged. State per row i: Lp[i] = E[r0+i+1][c-1];
- * diag0 = E[r0][c-1]; up0 = E[r0][c] (the value above the lane's first row). */
-template <int R>
-__device__ __forceinline__ int wf_step(const float (&ax)[R], const float (&ay)[R], int (&Lp)[R], int& diag0, float2 b,
-                                       int up0, float u) {
-    int mml[R];
-#pragma unroll
-    for (int i = 0; i < R; i++) {
-        const int m = (i == 0 ? diag0 : Lp[i - 1]) + match_mask(ax[i], ay[i], b, u);
-        mml[i] = (m == Lp[i]) ? kBig : min(m, Lp[i]);
+/* ---------------------------------------------------------------- row tiles, two cells per word
+ * The row form works on column-shifted distances E[r][c] = D[r][c] - c: in column c's shift the
+ * reference's three operands at (r, c) become m = E[r-1][c-1] + (match ? -1 : 0), l = E[r][c-1]
+ * and u = E[r-1][c] + 1; a common shift keeps every comparison, so the choice min(u, mml), with
+ * mml = min(m, l) or +inf when m == l, is taken on shifted values unchanged.
+ *
+ * |E[r][c]| <= r (D <= c + r along the column boundary; D >= |r - c|), so with a bias of 16384 every
+ * value of a supported pair lies in [0, 0x8000] and two of them share a 32-bit word. A lane owns
+ * 2H consecutive rows: word i holds row i of the lane (low half) and row H + i (high half). The
+ * high half runs one column behind the low half, and the next lane's low half one column behind
+ * that, so the value above a half's first row is always one step old: the lane's own low bottom
+ * row for the high half, the lane above's high bottom row (one shuffle) for the low half. At step
+ * s lane L handles columns s - 2L (low) and s - 2L - 1 (high).
+ *
+ * What bounds it: the ALU pipe, at half the issue rate (16-bit min / add, min.f32, lop3 and prmt all
+ * ran at 62 lanes per clock and SM on a B200, float adds at 117 and multiply-adds at 62 beside
+ * them). Two cells take 8 ALU and 7 FMA-pipe instructions where a match is possible and 4 + 1 where
+ * it is not, against 14 ALU and 4 FMA for two cells held one per word. Measured on 4,096 pairs of
+ * log-uniform [16, 4096] lengths: 0.87 ms, 2.5 Tcell/s; one cell per word: 1.62 ms, 1.34 Tcell/s. */
+constexpr int kBias = 16384;
+constexpr unsigned kHalfOnes = 0x00010001u, kHalfTops = 0x80008000u, kHalfRest = 0x7fff7fffu;
+
+__device__ __forceinline__ unsigned add_u16x2(unsigned a, unsigned b) {
+    unsigned d;
+    asm("add.u16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned min_u16x2(unsigned a, unsigned b) {
+    unsigned d;
+    asm("min.u16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+/* Negative exactly when |dx| < u and |dy| < u: max propagates a NaN (no match, as the compares
+ * have it), and a difference of unequal floats is never zero. */
+__device__ __forceinline__ float match_sign(float dx, float dy, float u) {
+    float t;
+    asm("{\n\t.reg .f32 a, b;\n\tabs.f32 a, %1;\n\tabs.f32 b, %2;\n\tmax.NaN.f32 %0, a, b;\n\t}" : "=f"(t) : "f"(dx), "f"(dy));
+    return __fsub_rn(t, u);
+}
+/* 0xffff in each half whose float is negative (prmt with replicated sign bits) */
+__device__ __forceinline__ unsigned sign_halves(float lo, float hi) {
+    unsigned d;
+    asm("prmt.b32 %0, %1, %2, 0xffbb;" : "=r"(d) : "r"(__float_as_uint(lo)), "r"(__float_as_uint(hi)));
+    return d;
+}
+
+/* E of row r at column c when no point of the first r rows matches any of the first c columns.
+ * Let k be the highest bit set in r and clear in c: E = (r mod 2^(k+1)) - (c mod 2^(k+1)), and 0
+ * when there is no such bit. (The recurrence without matches depends on r and c alone. Row r has
+ * period 2^(k+1) in c for 2^k <= r < 2^(k+1): over a period E falls r, r - 1, ..., r - 2^k + 1,
+ * then repeats row r - 2^k from its start, where E = r - 2^k; by induction on r the rule m == l ->
+ * u restarts the fall at each period, as m and l meet there.) */
+__device__ __forceinline__ int unmatched_e(int r, int c) {
+    const int x = r & ~c;
+    if (x == 0) return 0;
+    const int mask = (2 << (31 - __clz(x))) - 1;
+    return (r & mask) - (c & mask);
+}
+__device__ __forceinline__ unsigned unmatched_pair(int rlo, int rhi, int c) {
+    return (unsigned)(kBias + unmatched_e(rlo, c)) | (unsigned)(kBias + unmatched_e(rhi, c)) << 16;
+}
+
+/* A box of row points. near() is true when a column point may match one of them: rounding is
+ * monotone, so a difference to the box's edge of at least u bounds the difference to every row
+ * from below. NaN rows widen nothing (they match nothing), a NaN point is near nothing. */
+struct RowBox {
+    float x0, y0, x1, y1;
+    __device__ __forceinline__ void clear() {
+        x0 = y0 = __int_as_float(0x7f800000);
+        x1 = y1 = __int_as_float(0xff800000);
     }
-    int up = up0;
-#pragma unroll
-    for (int i = 0; i < R; i++) {
-        up = __viaddmin_s32(up, 1, mml[i]);
-        Lp[i] = up;
+    __device__ __forceinline__ void add(float x, float y) {
+        x0 = fminf(x0, x);
+        y0 = fminf(y0, y);
+        x1 = fmaxf(x1, x);
+        y1 = fmaxf(y1, y);
     }
-    diag0 = up0;
-    return up;
+    __device__ __forceinline__ void add(const RowBox& o) {
+        x0 = fminf(x0, o.x0);
+        y0 = fminf(y0, o.y0);
+        x1 = fmaxf(x1, o.x1);
+        y1 = fmaxf(y1, o.y1);
+    }
+    __device__ __forceinline__ void warp_union() {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            x0 = fminf(x0, __shfl_xor_sync(0xffffffffu, x0, o));
+            y0 = fminf(y0, __shfl_xor_sync(0xffffffffu, y0, o));
+            x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, o));
+            y1 = fmaxf(y1, __shfl_xor_sync(0xffffffffu, y1, o));
+        }
+    }
+    __device__ __forceinline__ bool near(float2 p, float u) const {
+        return (__fsub_rn(p.x, x1) < u) & (__fsub_rn(x0, p.x) < u) & (__fsub_rn(p.y, y1) < u) & (__fsub_rn(y0, p.y) < u);
+    }
+};
+
+/* Where the distances of a row tile stop being unmatched_e: `mine` is the first column (rounded
+ * down to 32) that may match one of the rows [0, r1), `above` the same for the rows [0, r0) above
+ * the tile; both are kNever when there is none. Every value left of the first match of the rows
+ * so far is known without any work, so a tile starts at `mine`, takes the values above its first
+ * row from its predecessor from column `above` on and by formula before it, and a pair without a
+ * possible match (most candidates of a top-k walk) costs one pass over its points. The tile above
+ * evaluates the same rows and columns, so its `mine` is this tile's `above`. Called by a warp. */
+constexpr int kNever = 1 << 30;
+struct Front {
+    int above, mine;
+};
+__device__ __forceinline__ Front row_front(const float2* __restrict__ rows, const float2* __restrict__ cols, int len2, int r0,
+                                           int r1, float u) {
+    const int lane = threadIdx.x & 31;
+    RowBox up, all;
+    up.clear();
+#pragma unroll 4
+    for (int i = lane; i < r0; i += 32) {
+        const float2 v = rows[i];
+        up.add(v.x, v.y);
+    }
+    all = up;
+#pragma unroll 4
+    for (int i = r0 + lane; i < r1; i += 32) {
+        const float2 v = rows[i];
+        all.add(v.x, v.y);
+    }
+    if (r0 > 0) up.warp_union();
+    all.warp_union();
+    Front f{kNever, kNever};
+    for (int c0 = 0; c0 < len2; c0 += 128) {
+        /* four loads in flight per lane */
+        float2 p[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int c = c0 + 32 * q + lane;
+            p[q] = c < len2 ? cols[c] : make_float2(__int_as_float(0x7fffffff), 0.f);
+        }
+        bool done = false;
+#pragma unroll
+        for (int q = 3; q >= 0; q--)
+            if (__any_sync(0xffffffffu, all.near(p[q], u))) done = true;
+        if (!done) continue;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (f.mine == kNever && __any_sync(0xffffffffu, all.near(p[q], u))) f.mine = c0 + 32 * q;
+            if (r0 > 0 && f.above == kNever && __any_sync(0xffffffffu, up.near(p[q], u))) f.above = c0 + 32 * q;
+        }
+        if (r0 == 0 || f.above != kNever) break;
+    }
+    return f;
+}
+
+/* One step of a lane: up0 holds the values above its two halves' first rows, d0 the same one
+ * column earlier. L[i] goes from column c - 1 to column c of its half, where `keep` (MASKED: the
+ * halves whose column lies inside the pair) allows it. m == l is found by (m ^ l) + 0x7fff, whose
+ * top bit is clear only for zero; it then sets the top bit of min(m, l), which no value below
+ * exceeds. */
+template <int H, bool MATCH, bool MASKED>
+__device__ __forceinline__ void row_step(const float (&ax)[2 * H], const float (&ay)[2 * H], unsigned (&L)[H], unsigned& d0,
+                                         float2 blo, float2 bhi, unsigned up0, float u, unsigned one, unsigned keep) {
+    unsigned mml[H];
+#pragma unroll
+    for (int i = 0; i < H; i++) {
+        unsigned m = i == 0 ? d0 : L[i - 1];
+        if (MATCH) {
+            const float slo = match_sign(__fsub_rn(ax[i], blo.x), __fsub_rn(ay[i], blo.y), u);
+            const float shi = match_sign(__fsub_rn(ax[H + i], bhi.x), __fsub_rn(ay[H + i], bhi.y), u);
+            m = add_u16x2(m, sign_halves(slo, shi));
+        }
+        const unsigned y = (m ^ L[i]) * one + kHalfRest;
+        mml[i] = min_u16x2(m, L[i]) | (~y & kHalfTops);
+    }
+    unsigned up = up0;
+#pragma unroll
+    for (int i = 0; i < H; i++) {
+        up = __viaddmin_u16x2(up, kHalfOnes, mml[i]);
+        if (MASKED)
+            L[i] = (up & keep) | (L[i] & ~keep);
+        else
+            L[i] = up;
+    }
+    d0 = MASKED ? (up0 & keep) | (d0 & ~keep) : up0;
+}
+
+/* Per-warp shared memory of a row tile: the window of 96 column points (at the start of the chunk of
+ * steps [s0, s0 + 32): columns s0 - 64 .. s0 + 31), the chunk's carry values (in the high half) and
+ * the bottom-row words lane 31 leaves during the chunk. */
+struct RowShared {
+    float4 pts[48]; /* two points each */
+    uint4 in[8], out[8];
+};
+
+/* Stores four words to shared memory where `on` is set: predicated, and without a memory clobber, so
+ * that the compiler neither branches around it nor orders the next loads of the window behind it
+ * (they never touch these words; a warp barrier follows the last store of a chunk). */
+__device__ __forceinline__ void put_words(unsigned addr, const unsigned (&v)[4], bool on) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %0, 0;\n\t@p st.shared.v4.u32 [%1], {%2, %3, %4, %5};\n\t}" ::"r"((int)on),
+                 "r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]));
+}
+
+/* The first `kend` steps (rounded up to 4) of one chunk. Four steps at a time: their points and
+ * carry values come in 128-bit shared loads, their bottom-row words leave in one store. UN groups of
+ * four are unrolled: two where the kernel holds the loops of one or two tile heights, one where it
+ * holds three, since warps in loops that do not fit the instruction cache together wait for
+ * instructions (4,096 pairs of log-uniform [16, 4096] lengths, 8 rows per lane: 0.86 ms with one
+ * group, 1.15 ms with two; 4 rows: 0.96 and 0.92 ms). */
+template <int H, int UN, bool MATCH, bool MASKED>
+__device__ __forceinline__ void row_chunk(const float (&ax)[2 * H], const float (&ay)[2 * H], unsigned (&L)[H], unsigned& d0,
+                                          RowShared& sh, int s0, int kend, int c0, int len2, bool writer, float u,
+                                          unsigned one) {
+    const int lane = threadIdx.x & 31;
+    const float4* pb = sh.pts + 32 - lane; /* the lane's low column of step k: point k of pb */
+    float2 bhi = make_float2(0.f, 0.f);
+    if (MATCH) bhi = reinterpret_cast<const float2*>(pb)[-1];
+    const int groups = MASKED ? (kend + 3) >> 2 : 8;
+    const unsigned out = (unsigned)__cvta_generic_to_shared(sh.out);
+    constexpr int kUnroll = MASKED ? 1 : UN;
+#pragma unroll(kUnroll)
+    for (int g = 0; g < groups; g++) {
+        float4 p0 = make_float4(0.f, 0.f, 0.f, 0.f), p1 = p0;
+        if (MATCH) {
+            p0 = pb[2 * g];
+            p1 = pb[2 * g + 1];
+        }
+        const uint4 in = sh.in[g];
+        const float2 b[4] = {make_float2(p0.x, p0.y), make_float2(p0.z, p0.w), make_float2(p1.x, p1.y), make_float2(p1.z, p1.w)};
+        const unsigned cv[4] = {in.x, in.y, in.z, in.w};
+        unsigned o[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const unsigned above = __shfl_up_sync(0xffffffffu, L[H - 1], 1);
+            const unsigned up0 = __byte_perm(lane == 0 ? cv[k] : above, L[H - 1], 0x5432);
+            unsigned keep = 0xffffffffu;
+            if (MASKED) {
+                const int j = s0 + 4 * g + k - 2 * lane;
+                keep = (j >= c0 && j < len2 ? 0xffffu : 0u) | (j > c0 && j <= len2 ? 0xffff0000u : 0u);
+            }
+            row_step<H, MATCH, MASKED>(ax, ay, L, d0, b[k], bhi, up0, u, one, keep);
+            bhi = b[k];
+            o[k] = L[H - 1];
+        }
+        put_words(out + 16 * g, o, writer);
+    }
+}
+
+/* One row tile of one pair: the 64H rows of the shorter side from t0 on, steps over the columns from the
+ * tile's front on. cin: the carry words of tile t-1's bottom row (used from column fr.above on),
+ * accepted with tag tag_in; cout: this tile's bottom row for tile t+1 (nullptr for the last tile),
+ * written with tag tag_out. Returns false when a wait gave up. The owner lane of the pair's last
+ * row leaves the distance in `result`. The next chunk's points and carry words are loaded one
+ * chunk early. A chunk none of whose columns is near the tile's rows (their box) takes the steps
+ * without the match test: 29% of the chunks over pairs of log-uniform [16, 4096] lengths that follow
+ * one another, nearly all over a top-k walk's candidates. */
+template <int H, int UN>
+__device__ __forceinline__ bool row_tile(const float2* __restrict__ rows, const float2* __restrict__ cols, int len1, int len2,
+                                      int t0, Front fr, const carry_t* cin, carry_t* cout, carry_t tag_in, carry_t tag_out,
+                                      float u, RowShared& sh, int& result, int spin_limit, unsigned one) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const bool writer = cout != nullptr && lane == 31;
+    const int r0 = t0 + lane * 2 * H; /* the lane's first row */
+    const int c0 = fr.mine;
+    float ax[2 * H], ay[2 * H];
+    RowBox box;
+    box.clear();
+#pragma unroll
+    for (int i = 0; i < 2 * H; i++) {
+        ax[i] = ay[i] = __int_as_float(0x7f800000); /* +inf never matches */
+        if (r0 + i < len1) {
+            const float2 v = rows[r0 + i];
+            ax[i] = v.x;
+            ay[i] = v.y;
+            box.add(v.x, v.y);
+        }
+    }
+    box.warp_union();
+    unsigned L[H];
+#pragma unroll
+    for (int i = 0; i < H; i++) L[i] = unmatched_pair(r0 + i + 1, r0 + H + i + 1, c0);
+    unsigned d0 = unmatched_pair(r0, r0 + H, c0);
+    const int steps = len2 + 63;
+    const carry_t tag_hi = tag_out << 16;
+    const int from = cin ? fr.above : kNever; /* first column whose value above comes from cin */
+    float2 nb = make_float2(0.f, 0.f);
+    carry_t nw = 0;
+    bool nw_ok = false;
+    if (c0 + lane < len2) {
+        nb = cols[c0 + lane];
+        if (c0 + lane >= from) {
+            nw = ld_carry(cin + c0 + lane + 1);
+            nw_ok = (nw >> 16) == tag_in;
+        }
+    }
+    float2* pts = reinterpret_cast<float2*>(sh.pts);
+    unsigned near = 0; /* bit 0: this chunk holds a near column, bits 1 and 2: the two before */
+    for (int s0 = c0; s0 < steps; s0 += 32) {
+        const int c = s0 + lane;
+        near = (near << 1) & 7u;
+        if (s0 < len2) {
+            unsigned cv = s0 < from ? (unsigned)(kBias + unmatched_e(t0, c + 1)) : 0u;
+            if (s0 + 31 >= from) {
+                const bool want = c >= from && c < len2;
+                bool ok = !want || nw_ok;
+                for (int polls = 0;; polls++) {
+                    if (!ok) {
+                        nw = ld_carry(cin + c + 1);
+                        ok = (nw >> 16) == tag_in;
+                    }
+                    if (__all_sync(FULL, ok)) break;
+                    if (polls >= spin_limit) return false;
+                    if (polls >= 16) __nanosleep(64); /* each poll is an L2 round trip already */
+                }
+                if (want) cv = (unsigned)nw & 0xffffu;
+            }
+            near |= __any_sync(FULL, c < len2 && box.near(nb, u)) ? 1u : 0u;
+            __syncwarp();
+            pts[lane] = pts[32 + lane];
+            pts[32 + lane] = pts[64 + lane];
+            pts[64 + lane] = nb;
+            reinterpret_cast<unsigned*>(sh.in)[lane] = cv << 16;
+            __syncwarp();
+            const int cn = c + 32;
+            nw_ok = false;
+            if (cn < len2) {
+                nb = cols[cn];
+                if (cn >= from) {
+                    nw = ld_carry(cin + cn + 1);
+                    nw_ok = (nw >> 16) == tag_in;
+                }
+            }
+        } else {
+            __syncwarp();
+            pts[lane] = pts[32 + lane];
+            pts[32 + lane] = pts[64 + lane];
+            __syncwarp();
+        }
+        if (s0 >= c0 + 64 && s0 + 32 <= len2) {
+            /* both columns of every lane lie in [c0, len2) throughout */
+            if (near)
+                row_chunk<H, UN, true, false>(ax, ay, L, d0, sh, s0, 32, c0, len2, writer, u, one);
+            else
+                row_chunk<H, UN, false, false>(ax, ay, L, d0, sh, s0, 32, c0, len2, writer, u, one);
+        } else {
+            const int kend = min(32, steps - s0);
+            row_chunk<H, UN, true, true>(ax, ay, L, d0, sh, s0, kend, c0, len2, writer, u, one);
+        }
+        if (cout) {
+            /* lane 31's high half was at column s0 + k - 63 in step k */
+            __syncwarp();
+            const int j = s0 + lane - 63;
+            if (j >= c0 && j < len2) st_carry(cout + (j + 1), tag_hi | (carry_t)(reinterpret_cast<const unsigned*>(sh.out)[lane] >> 16));
+        }
+    }
+    const int last = len1 - 1 - r0;
+    if (last >= 0 && last < 2 * H) {
+#pragma unroll
+        for (int i = 0; i < 2 * H; i++)
+            if (i == last) result = (int)(i < H ? L[i] & 0xffffu : L[i - H] >> 16) - kBias + len2; /* D = E + column */
+    }
+    __syncwarp();
+    return true;
 }
 
 /* Column-tile form of the same recurrence: a lane owns R consecutive DP columns and a step
@@ -388,7 +732,7 @@ __device__ __forceinline__ int wf_step(const float (&ax)[R], const float (&ay)[R
  * prev = F[r][c-1], m == l exactly when mm1 == prev, min(m, l) = min(mm1, prev) + 1, and the
  * cell is u when they are equal, else min(u, min(m, l)). State per column j: F[j] =
  * F[r-1][c_j] on entry, F[r][c_j] on exit; diag0 = F[r-1][c_0 - 1]; left = F[r][c_0 - 1] (the
- * value to the left of the lane's first column). Same interface as wf_step. */
+ * value to the left of the lane's first column). Returns the value in the last column. */
 template <int R>
 __device__ __forceinline__ int cf_step(const float (&bx)[R], const float (&by)[R], int (&F)[R], int& diag0, float2 a,
                                        int left, float u) {
@@ -408,21 +752,19 @@ __device__ __forceinline__ int cf_step(const float (&bx)[R], const float (&by)[R
     return prev;
 }
 
-/* One row tile of one pair (rows r0 = t * 32R ...). cin: the carry words of tile t-1's bottom
- * row (nullptr for t == 0), accepted with tag tag_in; cout: this tile's bottom row for tile t+1
- * (nullptr for the last tile), written with tag tag_out. Returns false when a wait gave up.
- * The owner lane of the pair's last row leaves the distance in `result`.
+/* One column tile of one pair: lanes own the columns lpts[t * 32R ..], steps walk the rows spts. cin:
+ * the carry words of tile t-1's last column (nullptr for t == 0), accepted with tag tag_in; cout:
+ * this tile's last column for tile t+1 (nullptr for the last tile), written with tag tag_out.
+ * Returns false when a wait gave up. The owner lane of the pair's last column leaves the distance
+ * in `result`.
  *
- * Columns move through a per-warp window of 64 points in shared memory: at the start of the
- * chunk of columns [s0, s0 + 32) the window holds columns s0 - 32 .. s0 + 31, so lane L reads
- * column s0 + k - L of step k at window index 32 + k - L (a per-lane base plus a constant).
- * The next chunk's points and carry words are loaded one chunk early. Chunks where every
- * lane's column is inside the pair skip the bounds test. */
-/* COL: the column-tile form (cf_step); rows / cols / len1 / len2 then name the lane side
- * (columns) and the step side (rows), the carry runs along the tile's last column, and the
- * result is F + len2 (the step side's length), exactly as the row form's E + len2. */
-template <int R, bool COL = false>
-__device__ __forceinline__ bool edr_tile(const float2* __restrict__ rows, const float2* __restrict__ cols, int len1,
+ * Step points move through a per-warp window of 64 points in shared memory: at the start of the
+ * chunk of steps [s0, s0 + 32) the window holds points s0 - 32 .. s0 + 31, so lane L reads point
+ * s0 + k - L of step k at window index 32 + k - L (a per-lane base plus a constant). The next
+ * chunk's points and carry words are loaded one chunk early. Chunks where every lane's point is
+ * inside the pair skip the bounds test. */
+template <int R>
+__device__ __forceinline__ bool col_tile(const float2* __restrict__ rows, const float2* __restrict__ cols, int len1,
                                          int len2, int t, const carry_t* cin, carry_t* cout, carry_t tag_in,
                                          carry_t tag_out, float u, float2* sb, int* sc, int& result,
                                          int spin_limit) {
@@ -506,7 +848,7 @@ __device__ __forceinline__ bool edr_tile(const float2* __restrict__ rows, const 
             for (int k = 0; k < 32; k++) {
                 const int from_above = __shfl_up_sync(FULL, bottom, 1);
                 const int up0 = lane0 ? sc[k] : from_above;
-                bottom = COL ? cf_step<R>(ax, ay, Lp, diag0, pb[k], up0, u) : wf_step<R>(ax, ay, Lp, diag0, pb[k], up0, u);
+                bottom = cf_step<R>(ax, ay, Lp, diag0, pb[k], up0, u);
                 if (writer) st_carry(cout + (s0 + k - 30), tag_hi | (carry_t)(unsigned short)bottom);
             }
         } else {
@@ -516,8 +858,7 @@ __device__ __forceinline__ bool edr_tile(const float2* __restrict__ rows, const 
                 const int j = s0 + k - lane;
                 if (j >= 0 && j < len2) {
                     const int up0 = lane0 ? sc[k] : from_above;
-                    bottom = COL ? cf_step<R>(ax, ay, Lp, diag0, pb[k], up0, u)
-                                 : wf_step<R>(ax, ay, Lp, diag0, pb[k], up0, u);
+                    bottom = cf_step<R>(ax, ay, Lp, diag0, pb[k], up0, u);
                     if (writer) st_carry(cout + (j + 1), tag_hi | (carry_t)(unsigned short)bottom);
                 }
             }
@@ -533,18 +874,15 @@ __device__ __forceinline__ bool edr_tile(const float2* __restrict__ rows, const 
     return true;
 }
 
-template <int R, bool COL, class Src>
-__global__ void __launch_bounds__(kTileWarps * 32, R == 2 ? 4 : 3) k_edr_tiles(Src src, float u, TileCtl ctl, unsigned* __restrict__ work,
-                                                           unsigned long long* __restrict__ cells) {
-    dep_wait();
-    __shared__ float2 bring[kTileWarps][64];
-    __shared__ int cring[kTileWarps][32];
+/* The work items of one warp: orients each pair (rows are the query when the candidate is at least
+ * as long, else the candidate, Grid.cpp:1234-1247) and hands the tile to `run`, which returns
+ * whether its waits succeeded and leaves the distance in the owner lane's `result` (owner < 0: in
+ * every lane) when it finished the pair. */
+template <class Src, class Run>
+__device__ __forceinline__ void walk_tiles(const Src& src, const TileCtl& ctl, unsigned* work, unsigned long long* cells,
+                                           Run run) {
     const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int gw = blockIdx.x * kTileWarps + wib;
-    carry_t* wc0 = ctl.warp_carry + (size_t)gw * 2 * ctl.stride;
-    carry_t* wc1 = wc0 + ctl.stride;
-    const carry_t ep = *ctl.epoch << 8;
+    const int lane = threadIdx.x & 31;
     const unsigned total = (unsigned)*ctl.total;
     for (;;) {
         unsigned idx = 0;
@@ -552,51 +890,20 @@ __global__ void __launch_bounds__(kTileWarps * 32, R == 2 ? 4 : 3) k_edr_tiles(S
         idx = __shfl_sync(FULL, idx, 0);
         if (idx >= total) break;
         const int4 it = ctl.items[idx];
-        const int p = it.x, t = it.y;
         const float2 *pa, *pb;
         int la, lb;
         int32_t* outp;
-        src.get(p, pa, la, pb, lb, outp);
-        const float2 *rows, *cols;
-        int len1, len2;
-        if (lb >= la) {
-            rows = pa;
-            cols = pb;
-            len1 = la;
-            len2 = lb;
-        } else {
-            rows = pb;
-            cols = pa;
-            len1 = lb;
-            len2 = la;
-        }
-        if (len1 == 0 || len2 == 0) {
-            if (lane == 0) *outp = len1 + len2;
+        src.get(it.x, pa, la, pb, lb, outp);
+        const bool swap = lb < la;
+        const float2 *rows = swap ? pb : pa, *cols = swap ? pa : pb;
+        const int len1 = swap ? lb : la, len2 = swap ? la : lb;
+        if (len1 == 0) {
+            if (lane == 0) *outp = len2;
             continue;
         }
-        /* lane side and step side: rows / columns for row tiles, columns / rows for column tiles */
-        const float2* lpts = COL ? cols : rows;
-        const float2* spts = COL ? rows : cols;
-        const int nlane = COL ? len2 : len1, nstep = COL ? len1 : len2;
-        constexpr int kTile = 32 * R;
-        const int T = (nlane + kTile - 1) / kTile;
-        int result = 0;
-        bool ok = true, finished = false;
-        if (t < 0) {
-            for (int tt = 0; tt < T && ok; tt++)
-                ok = edr_tile<R, COL>(lpts, spts, nlane, nstep, tt, tt > 0 ? ((tt - 1) & 1 ? wc1 : wc0) : nullptr,
-                                      tt + 1 < T ? ((tt & 1) ? wc1 : wc0) : nullptr, ep | ((tt - 1) & 0xff),
-                                      ep | (tt & 0xff), u, bring[wib], cring[wib], result, ctl.spin_limit);
-            finished = true;
-        } else {
-            carry_t* pc = ctl.pair_carry + (size_t)it.z * 2 * ctl.stride;
-            const bool stalled = p == ctl.stall_pair && t == 0;
-            ok = edr_tile<R, COL>(lpts, spts, nlane, nstep, t, t > 0 ? pc + ((t - 1) & 1) * ctl.stride : nullptr,
-                                  t + 1 < T && !stalled ? pc + (t & 1) * ctl.stride : nullptr, ep | ((t - 1) & 0xff),
-                                  ep | (t & 0xff), u, bring[wib], cring[wib], result, ctl.spin_limit);
-            finished = t == T - 1;
-        }
-        if (!ok) {
+        int result = 0, owner = -1;
+        bool finished = false;
+        if (!run(it, rows, cols, len1, len2, result, owner, finished)) {
             if (lane == 0) {
                 atomicCAS(ctl.flag, 0, GAT_ERR_TIMEOUT);
                 *outp = -1;
@@ -604,8 +911,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, R == 2 ? 4 : 3) k_edr_tiles(S
             continue;
         }
         if (finished) {
-            const int owner = ((nlane - 1) % kTile) / R;
-            result = __shfl_sync(FULL, result, owner);
+            if (owner >= 0) result = __shfl_sync(FULL, result, owner);
             if (lane == 0) {
                 *outp = result;
                 if (cells) atomicAdd(cells, (unsigned long long)len1 * (unsigned long long)len2);
@@ -613,6 +919,105 @@ __global__ void __launch_bounds__(kTileWarps * 32, R == 2 ? 4 : 3) k_edr_tiles(S
         }
     }
 }
+
+/* Row tiles of at most 32 R rows (R = 2, 4 or 8 rows per lane). */
+constexpr int kSpread = 500; /* cycles between the first items of a CTA's warps (below) */
+
+template <int R, class Src>
+__global__ void __launch_bounds__(kRowWarps * 32, 1) k_edr_rows(Src src, float u, TileCtl ctl, unsigned* __restrict__ work,
+                                                                unsigned long long* __restrict__ cells) {
+    dep_wait();
+    __shared__ RowShared shared[kRowWarps];
+    const int wib = threadIdx.x >> 5;
+    RowShared& sh = shared[wib];
+    carry_t* wc0 = ctl.warp_carry + (size_t)(blockIdx.x * kRowWarps + wib) * 2 * ctl.stride;
+    const carry_t ep = *ctl.epoch << 8;
+    /* Warp w of every CTA asks for its first item about w * kSpread cycles after the start, so the
+     * first items go to the first warps of all SMs, the next to the second warps, and a launch with
+     * fewer items than warps (a few long pairs) spreads over the SMs and their four schedulers
+     * instead of filling the SMs that start first. A delay, not a rule: whichever warp comes takes
+     * the next item, so a tile's predecessor has always been taken before it. */
+    for (const long long start = clock64(); clock64() - start < (long long)wib * kSpread;) __nanosleep(20);
+    walk_tiles(src, ctl, work, cells, [&](const int4& it, const float2* rows, const float2* cols, int len1, int len2,
+                                          int& result, int& owner, bool& finished) {
+        constexpr int kHeight = 32 * R;
+        constexpr int kGroups = R == 8 ? 1 : 2; /* row_chunk's unrolled groups */
+        const int T = tile_count<R>(len1);
+        const bool pipelined = it.y >= 0;
+        carry_t* buf = pipelined ? ctl.pair_carry + (size_t)it.z * 2 * ctl.stride : wc0;
+        finished = !pipelined || it.y == T - 1;
+        for (int t = pipelined ? it.y : 0; t < (pipelined ? it.y + 1 : T); t++) {
+            const int t0 = t * kHeight, left = len1 - t0;
+            const Front fr = row_front(rows, cols, len2, t0, min(len1, t0 + kHeight), u);
+            if (fr.mine == kNever) {
+                /* no match so far: known values below this tile too */
+                result = len2 + unmatched_e(len1, len2);
+                owner = -1;
+                continue;
+            }
+            const carry_t* cin = t > 0 ? buf + (size_t)((t - 1) & 1) * ctl.stride : nullptr;
+            const bool stalled = pipelined && it.x == ctl.stall_pair && t == 0;
+            carry_t* cout = t + 1 < T && !stalled ? buf + (size_t)(t & 1) * ctl.stride : nullptr;
+            const carry_t tin = ep | ((t - 1) & 0xff), tout = ep | (t & 0xff);
+            bool ok = false;
+            auto tile = [&](auto half) {
+                constexpr int H = decltype(half)::value;
+                if constexpr (2 * H <= R) {
+                    ok = row_tile<H, kGroups>(rows, cols, len1, len2, t0, fr, cin, cout, tin, tout, u, sh, result, ctl.spin_limit, ctl.one);
+                    owner = (left - 1) / (2 * H); /* the last tile's */
+                }
+            };
+            if (left <= 64 || R == 2)
+                tile(std::integral_constant<int, 1>{});
+            else if (left <= 128 || R == 4)
+                tile(std::integral_constant<int, 2>{});
+            else
+                tile(std::integral_constant<int, 4>{});
+            if (!ok) return false;
+        }
+        return true;
+    });
+}
+
+/* Column tiles of 32 R columns. */
+template <int R, class Src>
+__global__ void __launch_bounds__(kColWarps * 32, R == 2 ? 4 : 3) k_edr_cols(Src src, float u, TileCtl ctl,
+                                                                              unsigned* __restrict__ work,
+                                                                              unsigned long long* __restrict__ cells) {
+    dep_wait();
+    __shared__ float2 bring[kColWarps][64];
+    __shared__ int cring[kColWarps][32];
+    const int wib = threadIdx.x >> 5;
+    carry_t* wc0 = ctl.warp_carry + (size_t)(blockIdx.x * kColWarps + wib) * 2 * ctl.stride;
+    const carry_t ep = *ctl.epoch << 8;
+    walk_tiles(src, ctl, work, cells, [&](const int4& it, const float2* rows, const float2* cols, int len1, int len2,
+                                          int& result, int& owner, bool& finished) {
+        const int T = tile_count<R>(len2);
+        const bool pipelined = it.y >= 0;
+        carry_t* buf = pipelined ? ctl.pair_carry + (size_t)it.z * 2 * ctl.stride : wc0;
+        finished = !pipelined || it.y == T - 1;
+        owner = ((len2 - 1) % (32 * R)) / R;
+        for (int t = pipelined ? it.y : 0; t < (pipelined ? it.y + 1 : T); t++) {
+            const bool stalled = pipelined && it.x == ctl.stall_pair && t == 0;
+            if (!col_tile<R>(cols, rows, len2, len1, t, t > 0 ? buf + (size_t)((t - 1) & 1) * ctl.stride : nullptr,
+                             t + 1 < T && !stalled ? buf + (size_t)(t & 1) * ctl.stride : nullptr, ep | ((t - 1) & 0xff),
+                             ep | (t & 0xff), u, bring[wib], cring[wib], result, ctl.spin_limit))
+                return false;
+        }
+        return true;
+    });
+}
+
+template <int R, bool COL, class Src>
+struct TileKernel {
+    static constexpr int kWarps = kRowWarps;
+    static constexpr auto get() { return k_edr_rows<R, Src>; }
+};
+template <int R, class Src>
+struct TileKernel<R, true, Src> {
+    static constexpr int kWarps = kColWarps;
+    static constexpr auto get() { return k_edr_cols<R, Src>; }
+};
 
 /* Host side: schedule (count, write) -> tiled kernel. cap is the number of pairs (exact for
  * host-known lists, an upper bound for device-counted ones); max_rows / max_cols bound the
@@ -624,14 +1029,16 @@ int launch_tiles(gat_ctx* ctx, const Src& src, int64_t cap, int max_rows, int ma
     cudaStream_t s = ctx->stream;
     int per_sm = 0;
     /* An SM's split between L1 and shared memory changes only while no block is resident on it.
-     * With the default (no preference) the persistent grid's blocks, which need 5 KB, leave their
+     * With the default (no preference) the persistent grid's blocks, which need 5 to 8 KB, leave their
      * SMs at a small shared-memory split for the whole launch, and a kernel of another stream that
      * needs more (the range scan's 48 KB blocks) could not start on any of them until the grid
      * ended: range batches beside a long top-k round waited for it (16 rectangles, 1.1 ms alone:
      * 10.5 ms median beside 18 ms EDR launches that left half the SMs free; 2.5 ms with the
      * largest split). The tile kernel reads its points once and uses little L1. */
-    prefer_split(reinterpret_cast<const void*>(k_edr_tiles<R, COL, Src>), ctx->device, kEdrCarveoutPct);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_edr_tiles<R, COL, Src>, kTileWarps * 32, 0);
+    constexpr auto kernel = TileKernel<R, COL, Src>::get();
+    constexpr int kWarps = TileKernel<R, COL, Src>::kWarps;
+    prefer_split(reinterpret_cast<const void*>(kernel), ctx->device, kEdrCarveoutPct);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kWarps * 32, 0);
     /* a serving lane leaves sm_reserve SMs free of this persistent grid for other streams */
     const int grid = std::max(1, ctx->sm_count - ctx->sm_reserve) * (per_sm > 0 ? per_sm : 1);
     /* carry rows run along the step side; tiles are cut along the lane side */
@@ -649,7 +1056,7 @@ int launch_tiles(gat_ctx* ctx, const Src& src, int64_t cap, int max_rows, int ma
     int4* items = (int4*)scratch(ctx, S_EDR_ITEMS, (size_t)item_cap * sizeof(int4), &st);
     carry_t* pcarry =
         coop > 0 ? (carry_t*)scratch_zeroed(ctx, S_EDR_PCARRY, (size_t)coop * 2 * stride * sizeof(carry_t), &st) : nullptr;
-    carry_t* wcarry = (carry_t*)scratch_zeroed(ctx, S_EDR_CARRY, (size_t)grid * kTileWarps * 2 * stride * sizeof(carry_t), &st);
+    carry_t* wcarry = (carry_t*)scratch_zeroed(ctx, S_EDR_CARRY, (size_t)grid * kWarps * 2 * stride * sizeof(carry_t), &st);
     if (!ctr || !meta || !items || !wcarry || (coop > 0 && !pcarry)) return st;
     (void)launch_dep(ctx, k_zero_words, dim3(1), dim3(256), 0, s, ctr, (int)kCtrWords);
     const int pgrid = (int)std::max<int64_t>(1, std::min<int64_t>((cap + 255) / 256, (int64_t)ctx->sm_count * 8));
@@ -660,7 +1067,7 @@ int launch_tiles(gat_ctx* ctx, const Src& src, int64_t cap, int max_rows, int ma
     /* the stall knob (tests of the bounded wait) also shortens the wait to ~2^12 polls */
     const int stall = ctx->test_stall_pair - 1;
     TileCtl ctl{items, ctr + 2, pcarry, wcarry, stride, reinterpret_cast<const unsigned long long*>(ctr + kCtrEpoch),
-                ctx->d_flag, stall >= 0 ? (1 << 12) : kSpinLimit, stall};
+                ctx->d_flag, stall >= 0 ? (1 << 12) : kSpinLimit, stall, 1u};
     /* serving lanes: after the previous EDR grid of any sibling lane (not inside a capture, whose
      * graph cannot wait on an event recorded outside it) */
     std::unique_lock<std::mutex> chain;
@@ -674,7 +1081,7 @@ int launch_tiles(gat_ctx* ctx, const Src& src, int64_t cap, int max_rows, int ma
     }
     timed_begin(ctx, GAT_KERNEL_EDR);
     if (ev0) cudaEventRecord(ev0, s);
-    (void)launch_dep(ctx, k_edr_tiles<R, COL, Src>, dim3(grid), dim3(kTileWarps * 32), 0, s, src, u, ctl, reinterpret_cast<unsigned*>(ctr), cells);
+    (void)launch_dep(ctx, kernel, dim3(grid), dim3(kWarps * 32), 0, s, src, u, ctl, reinterpret_cast<unsigned*>(ctr), cells);
     if (ev1) cudaEventRecord(ev1, s);
     timed_end(ctx, GAT_KERNEL_EDR, 0.0);
     if (chain.owns_lock()) GAT_CUDA_TRY(ctx, cudaEventRecord(ctx->edr_chain->ev, s), "edr chain");
@@ -716,8 +1123,8 @@ int edr_launch(gat_ctx* ctx, const Src& src, int64_t cap, int max_rows, int max_
     if (cap <= 0) return GAT_OK;
     int cand[6], nc = 0;
     for (int form = 0; form < 2; form++) {
-        if (ctx->edr_form && ctx->edr_form != form + 1) continue;
-        for (int r : {4, 8, 2}) {
+        if ((ctx->edr_form ? ctx->edr_form : 1) != form + 1) continue; /* column tiles only when asked for */
+        for (int r : {8, 4, 2}) {
             if (ctx->edr_rows && ctx->edr_rows != r) continue;
             cand[nc++] = r | (form ? kShapeCol : 0);
         }

@@ -1022,7 +1022,7 @@ void lone_graph_free(void* p) {
 
 constexpr int kLoneGraphCache = 2;
 constexpr int kLoneRows = 4; /* 128-point tiles: the best of 2/4/8 on one query's pairs (a few hundred points) */
-constexpr int kLoneForm = 1; /* row tiles: column tiles measured slower on one query's pairs (many short tiles) */
+constexpr int kLoneForm = 1; /* row tiles */
 
 int lone_graph_get(gat_ctx* ctx, const gat_index* g, int max_q_len, int k, float u, LoneGraph** out) {
     for (auto& o : ctx->owned)

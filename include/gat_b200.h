@@ -95,16 +95,17 @@ enum { GAT_KERNEL_EDR = 0, GAT_KERNEL_BOUNDS = 1, GAT_KERNEL_RANGE_SCAN = 2, GAT
 int gat_ctx_set_timing(gat_ctx* ctx, int on);
 int gat_ctx_kernel_stats(gat_ctx* ctx, int kernel_class, double* ms, int64_t* launches, double* work);
 /* Tuning knobs (no counterpart in the reference, which has fixed launch shapes).
- * GAT_TUNE_EDR_ROWS: rows each lane of the EDR wavefront owns (tile height = 32 x rows).
- *   0 (default) = autotune: the first launch of each shape class (pair count, longest shorter
- *   side and longest longer side, each rounded up to a power of two) times 2, 4 and 8 rows
- *   per lane on the caller's own data and keeps the fastest for that class; results are the
- *   same for every choice. 2, 4 or 8 fixes the value. Setting the knob clears the tuned table.
+ * GAT_TUNE_EDR_ROWS: rows each lane of the EDR wavefront owns (tile height = 32 x rows; the last
+ *   tile of a pair may be lower). 0 (default) = autotune: the first launch of each shape class
+ *   (pair count, longest shorter side and longest longer side, each rounded up to a power of two)
+ *   times 2, 4 and 8 rows per lane on the caller's own data and keeps the fastest for that class;
+ *   results are the same for every choice. 2, 4 or 8 fixes the value. Setting the knob clears the
+ *   tuned table.
  * gat_ctx_get_tuning(GAT_TUNE_EDR_ROWS) returns the knob; GAT_TUNE_EDR_TUNED returns the
  * number of tuned shape classes.
- * GAT_TUNE_EDR_FORM: 0 (default) = autotune, 1 = row tiles (lanes own rows of the shorter
- *   side, steps walk the longer side), 2 = column tiles (lanes own columns, steps walk the
- *   shorter side: a shorter critical path for pairs of uneven length). Same results.
+ * GAT_TUNE_EDR_FORM: 0 (default) and 1 = row tiles (lanes own rows of the shorter side, steps walk
+ *   the longer side), 2 = column tiles (lanes own columns, steps walk the shorter side: a shorter
+ *   critical path for pairs of uneven length, at a fraction of the row tiles' rate). Same results.
  * GAT_TUNE_TOPK_CHUNK / GAT_TUNE_TOPK_GROWTH: candidates a query evaluates in the first round
  *   of the top-k walk, and the factor each later round grows by (0 = defaults: a first round of
  *   1280 for up to 4 queries per batch and 128 for larger batches, never below 8k or 4k;
