@@ -535,6 +535,7 @@ void gat_index_destroy(gat_index* ix) {
     for (void* p : ix->allocs) cudaFree(p);
     if (ix->d_pidx) cudaFree(ix->d_pidx);
     if (ix->d_pbox) cudaFree(ix->d_pbox);
+    index_groups_free(ix);
     delete ix;
 }
 

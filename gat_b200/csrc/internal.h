@@ -73,6 +73,29 @@ struct MortonDev {
     const int32_t* cbeg;
 };
 
+/* Point groups (groups.cu): the runs of one trajectory inside one leaf (Grid) or cell (FSG). Group g
+ * is trajectory ids[g], positions [gbeg[g], gbeg[g + 1]), box gbox[g]. */
+struct NodeRec {
+    float4 mbb;  /* the node's box */
+    float4 pbox; /* exact box of its points */
+    int child;   /* first child, -1 for a leaf */
+    int ib, ie;  /* a leaf's groups, or an inner node's distinct trajectories in ids (ib -1: no list) */
+    int pad;
+};
+constexpr int kNodeIds = 4096; /* distinct trajectories of a node that keeps a list */
+struct GroupsDev {
+    int n = 0;
+    const int32_t* gbeg = nullptr;   /* [n + 1] */
+    const int32_t* ids = nullptr;    /* [n] group trajectories, then the node lists */
+    const float4* gbox = nullptr;    /* [n] */
+    const NodeRec* rec = nullptr;    /* Grid: per node */
+    const int32_t* cell_g = nullptr; /* FSG: first group of every cell, [cellnum + 1] */
+    /* Grid: the node covering each of the 2^jump_level x 2^jump_level equal squares (row-major from
+     * the upper left): the node of level jump_level there, or the leaf above it */
+    const int32_t* jump = nullptr;
+    int jump_level = 0;
+};
+
 /* One EDR problem: query side (a) and candidate side (b), offsets into two point arrays. */
 struct EdrPair {
     int64_t a_off;
@@ -176,6 +199,9 @@ struct gat_index {
     std::mutex host_mu;
     int32_t* d_pidx = nullptr; /* device-placed index whose point index does not fit the key */
     float4* d_pbox = nullptr;  /* derived, not saved in snapshots: GridDev::node_pbox / StigDev::pbox */
+    gat::GroupsDev groups{};         /* derived, not saved (index_groups); n == 0: none */
+    std::vector<void*> group_allocs;
+    size_t group_bytes = 0;
     int64_t leaves = 0, nodes = 0;
     gat::GridDev grid{};
     gat::StigDev stig{};
@@ -222,6 +248,16 @@ void* host_stage(gat_ctx* ctx, size_t bytes, int* status);
  * range walks can mark candidate ranges whose every point is a hit (pbox.cu). Called after a
  * Grid or STIG is built or loaded on a device context; a no-op for other kinds. */
 int index_point_boxes(gat_index* ix);
+/* Derives the point groups of a Grid (with its nodes' point boxes) or FSG for the id range scan
+ * (groups.cu); called after a build or load on a device context. Leaves the index without groups
+ * when there is no memory for them. */
+int index_groups(gat_index* ix);
+void index_groups_free(gat_index* ix);
+/* Batched id-set queries over an index with groups (range_groups.cu): per-query segments of `arena`
+ * (cap entries) in segbase / segcnt, the counters in ctr[0..8) (device, 8 words): [0] arena entries
+ * used, [1] work bytes when `timed`, [3] queries left in ovf_list for the bitmap scan. */
+int range_groups_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, uint32_t* arena, int64_t cap,
+                        unsigned long long* ctr, int64_t* segbase, int64_t* segcnt, int* ovf_list, bool timed);
 /* reads and clears the device status word; returns GAT_OK or the code a kernel stored */
 int check_device_flag(gat_ctx* ctx, const char* what);
 inline void count_launch(gat_ctx* ctx, int n = 1) { ctx->launches += n; }
@@ -275,6 +311,7 @@ enum Slot {
     S_RANGE_ORDER,
     S_RANGE_TPOS,
     S_RANGE_TASK,
+    S_RANGE_SPLIT,
     S_EDR_PAIRS,
     S_EDR_CARRY,
     S_EDR_COUNTERS,

@@ -104,6 +104,7 @@ int blocks_for(const gat_ctx* ctx, int64_t threads) {
 int index_point_boxes(gat_index* ix) {
     gat_ctx* ctx = ix->ctx;
     if (ctx->device < 0 || (ix->kind != GAT_INDEX_GRID && ix->kind != GAT_INDEX_STIG)) return GAT_OK;
+    if (ix->groups.n > 0) return GAT_OK; /* a Grid's boxes came with its groups */
     const int nn = ix->kind == GAT_INDEX_GRID ? ix->grid.nnodes : ix->stig.nnodes;
     if (nn <= 0) return GAT_OK;
     cudaStream_t s = ctx->stream;

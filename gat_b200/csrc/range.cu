@@ -18,6 +18,8 @@
  *                  de-duplicates.
  *   3. offsets     scan of per-query result counts; one CTA per query copies its segment.
  * Plain execution runs the same pipeline once per query.
+ * Batched id sets of an index with point groups (a Grid or FSG) take range_groups.cu instead; this
+ * pipeline serves point lists, STIG, the MortonGrid and the queries that outgrow that kernel's sets.
  */
 #include <algorithm>
 #include <climits>
@@ -25,6 +27,7 @@
 #include "cells.cuh"
 #include "internal.h"
 #include "launch.cuh"
+#include "range_common.cuh"
 
 namespace gat {
 namespace {
@@ -34,47 +37,6 @@ constexpr int kStack = 96;
 constexpr int kChunk = 1024;       /* candidate points per scan item */
 constexpr int kChunkAllHit = 4096; /* points per item whose every point is a hit (ids only) */
 constexpr int kAllHit = (int)0x80000000; /* item start flag: every point of the item is a hit */
-
-struct Box {
-    float xmin, ymin, xmax, ymax;
-};
-
-__device__ __forceinline__ bool in_box(const Box& q, float x, float y) {
-    /* MBB::pInBox (MBB.cpp:21-26) */
-    return x <= q.xmax && x >= q.xmin && y <= q.ymax && y >= q.ymin;
-}
-
-/* BoxIntersect (MBB.cpp:28-73) reduced to its zero / non-zero outcome, the only use the
- * traversals make of it. */
-__device__ __forceinline__ bool box_intersect(const Box& a1, const Box& b1) {
-    Box a, b;
-    if (a1.xmin < b1.xmin) {
-        a = a1;
-        b = b1;
-    } else if (a1.xmin == b1.xmin) {
-        if (a1.xmax > b1.xmax) {
-            a = a1;
-            b = b1;
-        } else {
-            b = a1;
-            a = b1;
-        }
-    } else {
-        b = a1;
-        a = b1;
-    }
-    if (b.xmin >= a.xmax) return false;
-    if (b.ymax <= a.ymin) return false;
-    if (b.ymin >= a.ymax) return false;
-    return true;
-}
-
-__device__ __forceinline__ Box load_box(const gat_mbb* q, int i) {
-    gat_mbb m = q[i];
-    return Box{m.xmin, m.ymin, m.xmax, m.ymax};
-}
-
-__device__ __forceinline__ void set_flag(int32_t* flag, int code) { atomicCAS(flag, 0, code); }
 
 /* ---------------------------------------------------------------- candidates */
 /* Whole subtrees. Quadtree node boxes (the Grid's and the MortonGrid's) are made from the first
@@ -86,10 +48,6 @@ __device__ __forceinline__ void set_flag(int32_t* flag, int code) { atomicCAS(fl
  * one range: the range joiner of walk_ranges turns the leaves' ranges into exactly the same
  * joined range, so the items are unchanged and the walk visits only the nodes that straddle the
  * query's border. */
-__device__ __forceinline__ bool box_inside(const Box& q, const float4& m) {
-    return q.xmin < m.x && m.z < q.xmax && q.ymin < m.y && m.w < q.ymax;
-}
-
 /* All points hit. A range the walk takes (a leaf, or a whole subtree as above) whose exact point
  * box (pbox.cu) lies inside the query under MBB::pInBox's inclusive comparisons has every point
  * in the query: the scan takes its ids without testing coordinates. False without point boxes. */
@@ -854,48 +812,7 @@ __global__ void k_split_scatter(int nq, const int* __restrict__ order, const int
  * run_batch picks one per batch-size class by timing both on the first batch. */
 /* A set of 2^HB slots holds up to 2^(HB-1) ids (load factor <= 1/2): 48 KB of shared memory per
  * CTA for HB = 13 (256 threads), 24 KB for HB = 12 (128 threads). */
-constexpr int kRankSortMax = 512; /* lists up to this length are sorted by run ranks */
 constexpr int kSmallItems = 16;   /* shape 3: queries with at most this many items are scanned one per warp */
-
-template <int HB>
-__device__ __forceinline__ unsigned hs_slot(int t) { return ((unsigned)t * 2654435761u) >> (32 - HB); }
-
-/* inserts t; a new id is appended to list (count: ids inserted; ovf: the list or a probe ran out) */
-template <int HB>
-__device__ __forceinline__ void hs_insert(int* tab, int* list, int t, int* count, int* ovf) {
-    unsigned h = hs_slot<HB>(t);
-    for (int p = 0; p < 64; p++) {
-        int v = tab[h];
-        if (v == t) return;
-        if (v == -1) {
-            v = atomicCAS(&tab[h], -1, t);
-            if (v == -1) {
-                const int pos = atomicAdd(count, 1);
-                if (pos < (1 << (HB - 1)))
-                    list[pos] = t;
-                else
-                    *ovf = 1;
-                return;
-            }
-            if (v == t) return;
-        }
-        h = (h + 1) & ((1u << HB) - 1);
-    }
-    *ovf = 1;
-}
-
-/* empties the slot holding t (t is in the set) */
-template <int HB>
-__device__ __forceinline__ void hs_erase(int* tab, int t) {
-    unsigned h = hs_slot<HB>(t);
-    for (int p = 0; p < (1 << HB); p++) {
-        if (tab[h] == t) {
-            tab[h] = -1;
-            return;
-        }
-        h = (h + 1) & ((1u << HB) - 1);
-    }
-}
 
 /* Inserts those of a lane's 4 ids that start a run (differ from the previous point's id; -1 =
  * not a hit). Most steps start no run (a trajectory's points in a cell are consecutive), so the
@@ -911,31 +828,6 @@ __device__ __forceinline__ void insert_runs(int* tab, int* list, int prev, int t
     if (n1) hs_insert<HB>(tab, list, t1, count, ovf);
     if (n2) hs_insert<HB>(tab, list, t2, count, ovf);
     if (n3) hs_insert<HB>(tab, list, t3, count, ovf);
-}
-
-/* ascending sort of the 32 values of a warp (one per lane), bitonic network over shuffles */
-__device__ __forceinline__ int warp_sort32(int v) {
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int k = 2; k <= 32; k <<= 1)
-#pragma unroll
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            const int o = __shfl_xor_sync(0xffffffffu, v, j);
-            const bool up = (lane & k) == 0;
-            const bool lower = (lane & j) == 0;
-            v = (lower == up) ? min(v, o) : max(v, o);
-        }
-    return v;
-}
-
-/* number of the 32 ascending values run[0..32) below x: a binary search over the first 31
- * (it leaves lo = how many of them are below x), then the last */
-__device__ __forceinline__ int lower_bound32(const int* run, int x) {
-    int lo = 0;
-#pragma unroll
-    for (int step = 16; step > 0; step >>= 1)
-        if (run[lo + step - 1] < x) lo += step;
-    return lo + (run[31] < x ? 1 : 0);
 }
 
 /* One candidate item scanned by one warp: the ids of its points in q that start a run of equal
@@ -1561,7 +1453,7 @@ int run_batch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, int
     int st = GAT_OK;
     int64_t* segbase = (int64_t*)scratch(ctx, S_RANGE_SEGBASE, (nq + 1) * sizeof(int64_t), &st);
     int64_t* segcnt = (int64_t*)scratch(ctx, S_RANGE_SEGCNT, (nq + 1) * sizeof(int64_t), &st);
-    unsigned long long* cursor = (unsigned long long*)scratch(ctx, S_RANGE_CURSOR, 64, &st);
+    unsigned long long* cursor = (unsigned long long*)scratch(ctx, S_RANGE_CURSOR, 128, &st);
     int* ovf_list = (int*)scratch(ctx, S_RANGE_OVF, (size_t)(nq + 1) * sizeof(int), &st);
     if (!segbase || !segcnt || !cursor || !ovf_list) return st;
     const int words = (ix->db->n + 1 + 31) / 32;
@@ -1744,6 +1636,128 @@ int run_batch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, int
     return GAT_OK;
 }
 
+/* Offsets and gather of an id-set batch whose counts are known on the device only: nothing is copied
+ * when the ids do not fit the caller's capacity or the arena, or when queries are left for the bitmap
+ * scan (ctr as in range_groups_launch); the host then learns it from ctr and off[nq].
+ * Up to kGatherScan queries the CTAs sum the counts themselves, so a small batch needs no scan
+ * launches; ctr[8] receives the total. */
+constexpr int kGatherScan = 1024;
+
+__global__ void __launch_bounds__(kThreads) k_gather_ids(int nq, const int64_t* __restrict__ segbase,
+                                                         const int64_t* __restrict__ segcnt, int64_t* off,
+                                                         const uint32_t* __restrict__ arena, int64_t arena_cap, int32_t* out,
+                                                         int64_t capacity, unsigned long long* ctr, bool scan) {
+    __shared__ int64_t wsum[2][kThreads / 32];
+    int64_t total = scan ? 0 : off[nq];
+    for (int qi = blockIdx.x; qi < nq; qi += gridDim.x) {
+        int64_t o = 0;
+        if (scan) {
+            int64_t before = 0, all = 0;
+            for (int j = threadIdx.x; j < nq; j += kThreads) {
+                const int64_t c = segcnt[j];
+                all += c;
+                if (j < qi) before += c;
+            }
+            for (int s = 16; s > 0; s >>= 1) {
+                before += __shfl_xor_sync(0xffffffffu, before, s);
+                all += __shfl_xor_sync(0xffffffffu, all, s);
+            }
+            __syncthreads();
+            if ((threadIdx.x & 31) == 0) {
+                wsum[0][threadIdx.x >> 5] = before;
+                wsum[1][threadIdx.x >> 5] = all;
+            }
+            __syncthreads();
+            total = 0;
+            for (int w = 0; w < kThreads / 32; w++) {
+                o += wsum[0][w];
+                total += wsum[1][w];
+            }
+            if (threadIdx.x == 0) {
+                off[qi] = o;
+                if (qi == nq - 1) off[nq] = total;
+            }
+        } else {
+            o = off[qi];
+        }
+        if (qi == 0 && threadIdx.x == 0) ctr[8] = (unsigned long long)total;
+        if (total > capacity || (int64_t)ctr[0] > arena_cap || ctr[3] != 0) continue;
+        const int64_t b = segbase[qi], n = segcnt[qi];
+        for (int64_t i = threadIdx.x; i < n; i += kThreads) out[o + i] = (int32_t)arena[b + i];
+    }
+}
+
+/* Batched id sets over an index with point groups (range_groups.cu), offsets and ids in the caller's
+ * device arrays. Queries whose ids outgrow the kernel's set get their items built and take the bitmap
+ * kernel. The host waits once, after the gather. */
+int run_groups(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, int64_t* d_off, int32_t* d_tid, int64_t capacity,
+               int64_t* total) {
+    cudaStream_t s = ctx->stream;
+    int st = GAT_OK;
+    int64_t* segbase = (int64_t*)scratch(ctx, S_RANGE_SEGBASE, (nq + 1) * sizeof(int64_t), &st);
+    int64_t* segcnt = (int64_t*)scratch(ctx, S_RANGE_SEGCNT, (nq + 1) * sizeof(int64_t), &st);
+    unsigned long long* ctr = (unsigned long long*)scratch(ctx, S_RANGE_CURSOR, 128, &st);
+    int* ovf_list = (int*)scratch(ctx, S_RANGE_OVF, (size_t)(nq + 1) * sizeof(int), &st);
+    if (!segbase || !segcnt || !ctr || !ovf_list) return st;
+    int64_t cap = std::max<int64_t>(1 << 20, (int64_t)nq * 256);
+    uint32_t* arena = nullptr;
+    /* offsets, gather, and the counters on the host */
+    auto finish = [&]() -> int {
+        const bool scan = nq <= kGatherScan;
+        int rc = GAT_OK;
+        if (!scan && (rc = scan_i64(ctx, segcnt, d_off, nq)) != GAT_OK) return rc;
+        k_gather_ids<<<std::max(1, std::min(nq, ctx->sm_count * 8)), kThreads, 0, s>>>(nq, segbase, segcnt, d_off, arena, cap,
+                                                                                    d_tid, capacity, ctr, scan);
+        count_launch(ctx);
+        GAT_CUDA_TRY(ctx, cudaGetLastError(), "range gather launch");
+        GAT_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_pinned, ctr, 9 * sizeof(int64_t), cudaMemcpyDeviceToHost, s), "range");
+        GAT_CUDA_TRY(ctx, cudaStreamSynchronize(s), "range scan");
+        return GAT_OK;
+    };
+    for (int attempt = 0; attempt < 2; attempt++) {
+        arena = (uint32_t*)scratch(ctx, S_RANGE_ARENA, (size_t)cap * 4, &st);
+        if (!arena) return st;
+        cap = (int64_t)(ctx->slot_bytes[S_RANGE_ARENA] / 4);
+        timed_begin(ctx, GAT_KERNEL_RANGE_SCAN);
+        st = range_groups_launch(ctx, ix, d_q, nq, arena, cap, ctr, segbase, segcnt, ovf_list, ctx->timing);
+        timed_end(ctx, GAT_KERNEL_RANGE_SCAN, 0.0);
+        if (st != GAT_OK || (st = finish()) != GAT_OK) return st;
+        const int64_t n_ovf = ctx->h_pinned[3];
+        if (n_ovf > 0) {
+            int64_t* ioff = nullptr;
+            int2* items = nullptr;
+            if ((st = build_items(ctx, ix, d_q, (int)n_ovf, ovf_list, &ioff, &items)) != GAT_OK) return st;
+            if ((st = check_device_flag(ctx, "range candidates")) != GAT_OK) return st;
+            const int words = (ix->db->n + 1 + 31) / 32;
+            const size_t smem_bm = (size_t)words * 4;
+            const bool in_smem = smem_bm <= 200 * 1024;
+            int per_sm = 0;
+            if (in_smem) allow_smem(k_range_ids, smem_bm);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_range_ids, kThreads, in_smem ? smem_bm : 0);
+            const int g = (int)std::max<int64_t>(1, std::min<int64_t>(n_ovf, (int64_t)std::max(1, per_sm) * ctx->sm_count));
+            uint32_t* gbm = in_smem ? nullptr : (uint32_t*)scratch(ctx, S_RANGE_ARENA2, (size_t)g * words * 4, &st);
+            if (!in_smem && !gbm) return st;
+            timed_begin(ctx, GAT_KERNEL_RANGE_SCAN);
+            k_range_ids<<<g, kThreads, in_smem ? smem_bm : 0, s>>>(d_q, (int)n_ovf, ioff, items, ix->d_x, ix->d_y, ix->d_tid,
+                                                                  words, gbm, arena, cap, ctr, segbase, segcnt,
+                                                                  ctx->timing ? ctr + 1 : nullptr, ovf_list, 1);
+            timed_end(ctx, GAT_KERNEL_RANGE_SCAN, 0.0);
+            count_launch(ctx);
+            GAT_CUDA_TRY(ctx, cudaGetLastError(), "range scan launch");
+            GAT_CUDA_TRY(ctx, cudaMemsetAsync(ctr + 3, 0, sizeof(int64_t), s), "range");
+            if ((st = finish()) != GAT_OK) return st;
+        }
+        const int64_t used = ctx->h_pinned[0];
+        if (used <= cap) {
+            if (ctx->timing) timed_add_work(ctx, GAT_KERNEL_RANGE_SCAN, (double)ctx->h_pinned[1]);
+            *total = ctx->h_pinned[8];
+            return GAT_OK;
+        }
+        cap = used;
+    }
+    return fail(ctx, GAT_ERR_OOM, "range: result arena overflow");
+}
+
 int run_gather(gat_ctx* ctx, const gat_index* ix, int nq, int mode, const int64_t* d_off, int32_t* d_tid,
                int32_t* d_pidx) {
     int st = GAT_OK;
@@ -1775,7 +1789,7 @@ int run_plain_ids(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq,
     int2* items = (int2*)scratch(ctx, S_RANGE_ITEMS, (size_t)(item_cap + 1) * sizeof(int2), &st);
     uint32_t* bitmap = (uint32_t*)scratch(ctx, S_RANGE_ARENA2, (size_t)words * 4, &st);
     /* cursor: [0] truncation word, [1] work of the whole call */
-    unsigned long long* cursor = (unsigned long long*)scratch(ctx, S_RANGE_CURSOR, 64, &st);
+    unsigned long long* cursor = (unsigned long long*)scratch(ctx, S_RANGE_CURSOR, 128, &st);
     if (!ioff || !items || !bitmap || !cursor) return st;
     GAT_CUDA_TRY(ctx, cudaMemsetAsync(bitmap, 0, (size_t)words * 4, s), "range");
     GAT_CUDA_TRY(ctx, cudaMemsetAsync(cursor, 0, 64, s), "range");
@@ -1824,6 +1838,13 @@ int range_dev(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, int
     int st;
     if (exec == GAT_EXEC_BATCHED) {
         int64_t total = 0;
+        /* id sets of an index with point groups; a shape fixed by GAT_TUNE_RANGE_SHAPE is the point scan's */
+        if (mode == GAT_RESULT_IDS && ix->groups.n > 0 && ctx->range_shape == 0) {
+            if ((st = run_groups(ctx, ix, d_q, nq, d_off, d_tid, capacity, &total)) != GAT_OK) return st;
+            *needed = total;
+            if (total > capacity) return fail(ctx, GAT_ERR_TRUNCATED, "range: output capacity too small");
+            return GAT_OK;
+        }
         if ((st = run_batch(ctx, ix, d_q, nq, mode, d_off, &total)) != GAT_OK) return st;
         *needed = total;
         if (total > capacity) return fail(ctx, GAT_ERR_TRUNCATED, "range: output capacity too small");

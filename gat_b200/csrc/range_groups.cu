@@ -1,0 +1,788 @@
+/* Batched trajectory-id range queries over point groups (groups.cu), Grid and FSG.
+ *
+ * A query's candidates are the reference's: the leaves the quadtree walk takes (BoxIntersect,
+ * Grid.cpp:428-446), or the cells of the candidate rectangle (FSG.cpp:183-262). Their points are not
+ * scanned one by one:
+ *   - a node inside the query (by its box and the exact box of its points), or the FSG cells strictly
+ *     inside the candidate rectangle, have every point in the query: their ids are taken as they
+ *     are, a node's from its list of distinct trajectories;
+ *   - of the other candidate leaves and cells each group is taken or left by its box; only a group
+ *     that straddles the query's border, of a trajectory not yet found, has its points tested
+ *     (MBB::pInBox, MBB.cpp:21-26) until one is inside.
+ * On 100k rectangles of log-U[0.001, 0.05] degree sides over 1M walks (200M points) that reads about
+ * 1/20 of the candidates' bytes, and the walk, the scan, the sort and the output of a query run in
+ * one kernel without items in global memory.
+ *
+ * One kernel, three kinds of team by the ids a query is expected to hold (k_order_class): a warp, a
+ * pair of warps, or the CTA of 256 threads, each with its share of the CTA's shared memory (an eighth,
+ * a quarter, all). Small teams keep more queries in flight and wait less at barriers: 15k rectangles
+ * of 0.02 to 0.05 degrees over 1M walks took 2.07 ms by CTAs alone, 1.86 ms with pairs for those of
+ * 400 to 1,100 expected ids (1.16 ms less on 100k of 0.001 to 0.05). A query that outgrows its team
+ * runs again on the CTA, one that outgrows that goes to the bitmap scan (range.cu).
+ */
+#include <algorithm>
+#include <climits>
+#include <cmath>
+
+#include "launch.cuh"
+#include "range_common.cuh"
+
+namespace gat {
+namespace {
+
+constexpr int kNT = 256, kW = kNT / 32;
+/* id set slots (log2), ids, walk frontier and candidate ranges of a team in each mode */
+constexpr int kBlockBits = 13, kBlockIds = 4096, kBlockFront = 512, kBlockItems = 2048;
+constexpr int kMidBits = 11, kMidIds = 1408, kMidFront = 128, kMidItems = 320;
+constexpr int kSmallBits = 10, kSmallIds = 512, kSmallFront = 64, kSmallItems = 256;
+constexpr int kMidTeams = kW / 2; /* pairs of warps */
+constexpr int kCtl = 24; /* control words of a team */
+/* expected ids up to which a query is small or mid: short of the set, since the estimate is not exact */
+constexpr float kSmallMax = 400.f, kMidMax = 1100.f;
+constexpr int kFarCell = 1 << 20; /* FSG cell coordinates beyond this take the general scan */
+constexpr int kBorder = (int)0x80000000; /* item end flag: groups to be tested by box */
+constexpr int kDirectMax = 444; /* batches up to this size: every query in block mode */
+
+/* shared memory of one query's team */
+template <int HB_, int IDS_, int FRONT_, int ITEMS_, int NTHREADS_>
+struct Team {
+    static constexpr int HB = HB_, IDS = IDS_, FRONT = FRONT_, ITEMS = ITEMS_, NTHREADS = NTHREADS_;
+    static constexpr int kInts = (1 << HB) + IDS + 2 * FRONT + 2 * ITEMS;
+    static_assert((1 << HB) / 8 + IDS <= (1 << HB), "sort_ids keeps buckets and ids in the set's slots");
+    int* tab;    /* 2^HB slots, -1 = empty */
+    int* list;   /* IDS ids in insertion order */
+    int* front;  /* 2 x FRONT first children of the nodes to open */
+    int2* items; /* ITEMS ranges of ids / groups */
+    int* nitems;
+    int* nfront; /* [2] */
+    int* cnt;
+    int* ovf;
+    int* next;                /* items handed out */
+    unsigned long long* base; /* the answer's place in the arena */
+    int* sort;                /* sort_ids: [0] least id, [1] greatest, [2] largest bucket, [4 + w] bucket totals per warp */
+    int* query;               /* the query being answered */
+    int id;                   /* which of the CTA's teams */
+    __device__ Team(int* mem, int* ctl, int id_)
+        : tab(mem), list(mem + (1 << HB)), front(list + IDS), items(reinterpret_cast<int2*>(front + 2 * FRONT)), nitems(ctl),
+          nfront(ctl + 1), cnt(ctl + 3), ovf(ctl + 4), next(ctl + 5), base(reinterpret_cast<unsigned long long*>(ctl + 6)),
+          sort(ctl + 8), query(ctl + 20), id(id_) {}
+    __device__ __forceinline__ void sync() const {
+        if (NTHREADS == 32)
+            __syncwarp();
+        else if (NTHREADS == kNT)
+            __syncthreads();
+        else
+            asm volatile("bar.sync %0, %1;" ::"r"(id + 1), "n"(NTHREADS) : "memory");
+    }
+    /* hs_insert with this team's list length */
+    __device__ __forceinline__ void insert(int t) {
+        unsigned h = hs_slot<HB>(t);
+        for (int p = 0; p < 64; p++) {
+            int v = tab[h];
+            if (v == t) return;
+            if (v == -1) {
+                v = atomicCAS(&tab[h], -1, t);
+                if (v == -1) {
+                    const int pos = atomicAdd(cnt, 1);
+                    if (pos < IDS)
+                        list[pos] = t;
+                    else
+                        *ovf = 1;
+                    return;
+                }
+                if (v == t) return;
+            }
+            h = (h + 1) & ((1u << HB) - 1);
+        }
+        *ovf = 1;
+    }
+    __device__ __forceinline__ bool has(int t) const {
+        unsigned h = hs_slot<HB>(t);
+        for (int p = 0; p < 64; p++) {
+            const int v = *(const volatile int*)(tab + h);
+            if (v == t) return true;
+            if (v == -1) return false;
+            h = (h + 1) & ((1u << HB) - 1);
+        }
+        return false;
+    }
+};
+using BlockTeam = Team<kBlockBits, kBlockIds, kBlockFront, kBlockItems, kNT>;
+using MidTeam = Team<kMidBits, kMidIds, kMidFront, kMidItems, 64>;
+using SmallTeam = Team<kSmallBits, kSmallIds, kSmallFront, kSmallItems, 32>;
+constexpr int kInts = BlockTeam::kInts;
+static_assert(kW * SmallTeam::kInts <= kInts && kMidTeams * MidTeam::kInts <= kInts, "the warps share the CTA's memory");
+constexpr size_t kSmem = (size_t)kInts * sizeof(int);
+
+__device__ __forceinline__ bool pbox_inside(const Box& q, const float4& b) {
+    return b.x >= q.xmin && b.z <= q.xmax && b.y >= q.ymin && b.w <= q.ymax;
+}
+
+template <class T>
+__device__ __forceinline__ void put_item(T& t, int b, int e, bool border) {
+    if (b >= e) return;
+    const int k = atomicAdd(t.nitems, 1);
+    if (k < T::ITEMS)
+        t.items[k] = make_int2(b, border ? e | kBorder : e);
+    else
+        *t.ovf = 1;
+}
+
+/* The quadtree walk, one level of the frontier at a time, by thread `me` of the team. The root is
+ * taken without a test (Grid.cpp:428-433), every other node when BoxIntersect holds for it and all its
+ * ancestors. A node's box lies within its ancestors' and has a width, and then BoxIntersect with the
+ * node implies BoxIntersect with them (both ask for open overlap in y, and in x for the larger xmin
+ * below the other's xmax, which a wider box keeps), so a query smaller than a few squares of the jump
+ * table starts at the nodes of its squares (one more on every side, for the rounding of the division)
+ * and skips the levels above. */
+constexpr int kJumpMax = 64; /* squares a walk starts from at most */
+
+template <class T>
+__device__ void walk_grid(const GroupsDev& g, const GridDev& tree, const Box& q, T& t, int me) {
+    constexpr int FRONT = T::FRONT;
+    const NodeRec* __restrict__ rec = g.rec;
+    auto classify = [&](const NodeRec& r, int* out, int* nout) {
+        const bool in = pbox_inside(q, r.pbox);
+        if (r.child < 0)
+            put_item(t, r.ib, r.ie, !in);
+        else if (in && r.ib >= 0 && box_inside(q, r.mbb))
+            put_item(t, r.ib, r.ie, false);
+        else {
+            const int k = atomicAdd(nout, 1);
+            if (k < FRONT)
+                out[k] = r.child;
+            else
+                *t.ovf = 1;
+        }
+    };
+    bool jumped = false;
+    if (g.jump) {
+        const int n = 1 << g.jump_level;
+        const float inv = 1.f / (tree.cell * (float)(tree.axis >> g.jump_level));
+        auto square = [&](float d, int off) { return min(n - 1, max(0, (int)fminf(fmaxf(d * inv, -4.f), 1e6f) + off)); };
+        const int x0 = square(q.xmin - tree.rxmin, -1), x1 = square(q.xmax - tree.rxmin, 1);
+        const int y0 = square(tree.rymax - q.ymax, -1), y1 = square(tree.rymax - q.ymin, 1);
+        const int w = x1 - x0 + 1, h = y1 - y0 + 1;
+        jumped = w > 0 && h > 0 && w * h <= kJumpMax;
+        if (jumped)
+            for (int k = me; k < w * h; k += T::NTHREADS) {
+                const int x = x0 + k % w, y = y0 + k / w;
+                const int nd = g.jump[y * n + x];
+                /* a leaf above the table's level covers several squares: the first of the query's takes it */
+                if ((x > x0 && g.jump[y * n + x - 1] == nd) || (y > y0 && g.jump[(y - 1) * n + x] == nd)) continue;
+                const NodeRec r = rec[nd];
+                if (nd == 0 || box_intersect(q, Box{r.mbb.x, r.mbb.y, r.mbb.z, r.mbb.w})) classify(r, t.front, t.nfront);
+            }
+    }
+    if (!jumped && me == 0) {
+        const NodeRec r = rec[0];
+        classify(r, t.front, t.nfront);
+    }
+    t.sync();
+    for (int cur = 0;; cur ^= 1) {
+        /* read by all before any thread opens nodes (and may flag an overflow) again */
+        const int n = min(t.nfront[cur], FRONT);
+        const bool lost = *(volatile int*)t.ovf != 0;
+        t.sync();
+        if (n == 0 || lost) break;
+        for (int k = me; k < 4 * n; k += T::NTHREADS) {
+            const NodeRec r = rec[t.front[cur * FRONT + (k >> 2)] + (k & 3)];
+            if (box_intersect(q, Box{r.mbb.x, r.mbb.y, r.mbb.z, r.mbb.w}))
+                classify(r, t.front + (cur ^ 1) * FRONT, t.nfront + (cur ^ 1));
+        }
+        t.sync();
+        if (me == 0) t.nfront[cur] = 0;
+    }
+}
+
+/* The FSG's candidate cells row by row (fsg_walk in range.cu): row r covers the cells g1 + r nx ..
+ * g2 + r nx, unclamped as in the reference. f(v) = (int)((v - origin) / cell) is monotone in float
+ * arithmetic, so a point in a column strictly between g1 and g2 and a row strictly between g3 and g4
+ * lies inside the query: those cells are taken whole, the rest by their groups' boxes. (A NaN
+ * coordinate would break the ordering: no cell is then taken whole.) */
+template <class T>
+__device__ void walk_fsg(const FsgDev& f, const int32_t* __restrict__ cell_g, const Box& q, T& t, int me) {
+    const int g1 = (int)__fdiv_rn(__fsub_rn(q.xmin, f.rxmin), f.cell), g2 = (int)__fdiv_rn(__fsub_rn(q.xmax, f.rxmin), f.cell);
+    const int g3 = (int)__fdiv_rn(__fsub_rn(f.rymax, q.ymax), f.cell), g4 = (int)__fdiv_rn(__fsub_rn(f.rymax, q.ymin), f.cell);
+    if (max(max(g1, g2), max(g3, g4)) > kFarCell || min(min(g1, g2), min(g3, g4)) < -kFarCell || g4 - g3 > 4 * T::ITEMS) {
+        if (me == 0) *t.ovf = 1;
+        t.sync();
+        return;
+    }
+    const bool ordered = q.xmin <= q.xmax && q.ymin <= q.ymax;
+    for (int r = g3 + me; r <= g4; r += T::NTHREADS) {
+        const long long row = (long long)r * f.nx;
+        const long long lo_ = max(0ll, row + g1), hi_ = min((long long)f.cellnum - 1, row + g2);
+        if (lo_ > hi_) continue;
+        const int lo = (int)lo_, hi = (int)hi_;
+        int a = hi + 1, b = hi + 1; /* cells [a, b) taken whole */
+        if (ordered && r > g3 && r < g4 && r >= 0 && r < f.ny) {
+            const int c0 = max(g1 + 1, 0), c1 = min(g2 - 1, f.nx - 1);
+            if (c0 <= c1) {
+                a = (int)row + c0;
+                b = (int)row + c1 + 1;
+            }
+        }
+        put_item(t, cell_g[lo], cell_g[a], true);
+        put_item(t, cell_g[a], cell_g[b], false);
+        put_item(t, cell_g[b], cell_g[hi + 1], true);
+    }
+    t.sync();
+}
+
+/* groups a warp has found to straddle the query's border, tested kOpen / 2 or more at a time */
+constexpr int kOpen = 64;
+struct OpenGroups {
+    int beg[kOpen], end[kOpen], id[kOpen];
+};
+
+/* Tests the points of `n` open groups whose trajectory is not in the set yet, four groups at a time
+ * with eight lanes each, until one lies in the query. */
+template <class T>
+__device__ __forceinline__ void test_open(const OpenGroups& og, int n, const Box& q, const float* __restrict__ X,
+                                          const float* __restrict__ Y, T& t, unsigned& bytes) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    for (int k0 = 0; k0 < n; k0 += 32) {
+        const bool on = k0 + lane < n;
+        int b = 0, e = 0, id = -1;
+        if (on) {
+            b = og.beg[k0 + lane];
+            e = og.end[k0 + lane];
+            id = og.id[k0 + lane];
+        }
+        unsigned m = __ballot_sync(FULL, on && !t.has(id));
+        while (m) {
+            int src = -1;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if (k == (lane >> 3) && m) src = __ffs(m) - 1;
+                m &= m - 1;
+            }
+            const int b0 = __shfl_sync(FULL, b, src & 31), e0 = __shfl_sync(FULL, e, src & 31);
+            const int tid = __shfl_sync(FULL, id, src & 31);
+            bool found = false;
+            if (src >= 0)
+                for (int i = b0 + (lane & 7); i < e0 && !found; i += 16) {
+                    /* two steps of the eight lanes in flight */
+                    const int i2 = min(i + 8, e0 - 1);
+                    const float x = __ldg(X + i), y = __ldg(Y + i), x2 = __ldg(X + i2), y2 = __ldg(Y + i2);
+                    found = in_box(q, x, y) || in_box(q, x2, y2);
+                    bytes += 16;
+                }
+            const unsigned hits = __ballot_sync(FULL, found);
+            if (src >= 0 && (lane & 7) == 0 && ((hits >> (lane & 24)) & 0xffu)) t.insert(tid);
+        }
+    }
+    __syncwarp();
+}
+
+/* One warp takes the `n` <= 32 ranges from items[0]: their ids are dealt to the lanes as one sequence
+ * (an owner search over the running lengths), so that short ranges fill the warp. The ids, boxes and
+ * extents of the next 32 are loaded before the current 32 are looked at: with a load after each test
+ * a step waited for three trips to L2 (100k rectangles over 1M walks 4.6 ms). Groups that straddle
+ * the border gather in `og`. */
+template <class T>
+__device__ __forceinline__ void take_items(const int2* items, int n, const Box& q, const int32_t* __restrict__ ids,
+                                           const int32_t* __restrict__ gbeg, const float4* __restrict__ gbox,
+                                           const float* __restrict__ X, const float* __restrict__ Y, T& t, OpenGroups& og,
+                                           unsigned long long& work) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int2 it = lane < n ? items[lane] : make_int2(0, 0);
+    const int len = (it.y & ~kBorder) - it.x;
+    int incl = len;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(FULL, incl, o);
+        if (lane >= o) incl += y;
+    }
+    const int total = __shfl_sync(FULL, incl, 31);
+    const int shift = it.x - (incl - len); /* position = shift + sequence index */
+    unsigned bytes = 0;
+    int nopen = 0;
+    struct Next {
+        int id, beg, end;
+        float4 box;
+        bool border;
+    };
+    auto load = [&](int e0) {
+        Next x;
+        const int e = e0 + lane;
+        int l = 0; /* the owner: the first lane whose running length exceeds e */
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1)
+            if (__shfl_sync(FULL, incl, l + s - 1) <= e) l += s;
+        const int pos = __shfl_sync(FULL, shift, l) + e;
+        x.border = __shfl_sync(FULL, it.y, l) < 0;
+        x.id = -1;
+        x.beg = x.end = 0;
+        x.box = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (e < total) {
+            x.id = __ldg(ids + pos);
+            bytes += 4;
+            if (x.border) {
+                x.box = __ldg(gbox + pos);
+                x.beg = __ldg(gbeg + pos);
+                x.end = __ldg(gbeg + pos + 1);
+                bytes += 24;
+            }
+        }
+        return x;
+    };
+    Next nx = load(0);
+    for (int e0 = 0; e0 < total; e0 += 32) {
+        const Next x = nx;
+        if (e0 + 32 < total) nx = load(e0 + 32);
+        const bool in = pbox_inside(q, x.box);
+        const bool out = x.box.x > q.xmax || x.box.z < q.xmin || x.box.y > q.ymax || x.box.w < q.ymin;
+        if (__shfl_sync(FULL, *(volatile int*)t.ovf, 0)) break;
+        if (x.id >= 0 && (!x.border || in)) t.insert(x.id);
+        const bool open = x.id >= 0 && x.border && !in && !out;
+        const unsigned m = __ballot_sync(FULL, open);
+        if (open) {
+            const int k = nopen + __popc(m & ((1u << lane) - 1u));
+            og.beg[k] = x.beg;
+            og.end[k] = x.end;
+            og.id[k] = x.id;
+        }
+        nopen += __popc(m);
+        __syncwarp();
+        if (nopen > kOpen - 32) {
+            test_open(og, nopen, q, X, Y, t, bytes);
+            nopen = 0;
+        }
+    }
+    if (nopen) test_open(og, nopen, q, X, Y, t, bytes);
+    work += bytes;
+}
+
+/* The team's m ids, ascending, to out (nothing when `write` is false); leaves the set empty. Ids are
+ * counted into buckets of equal width between the least and the greatest (about two to a bucket),
+ * scattered to their buckets, and placed by the number of smaller ids in their own bucket. When ids
+ * crowd in a few buckets the list is sorted in runs of 32 that are merged in pairs instead. (Sorting
+ * runs and searching every id in every run took half of a query's instructions.) */
+constexpr int kCrowd = 32;
+
+template <class T>
+__device__ void sort_ids(T& t, int m, uint32_t* out, bool write, int me) {
+    constexpr int HB = T::HB, NTHREADS = T::NTHREADS;
+    int *const tab = t.tab, *const list = t.list;
+    constexpr int B = 1 << (HB - 3); /* buckets, counted in tab[0..B); the scattered ids follow */
+    constexpr int kPer = B / NTHREADS;
+    const unsigned FULL = 0xffffffffu;
+    const int lane = me & 31, warp = me >> 5;
+    int* lo_hi = t.sort;
+    /* the list is complete and the set no longer needed */
+    int lo = INT_MAX, hi = 0;
+    for (int i = me; i < m; i += NTHREADS) {
+        lo = min(lo, list[i]);
+        hi = max(hi, list[i]);
+    }
+    for (int b = me; b < B; b += NTHREADS) tab[b] = 0;
+    if (NTHREADS > 32 && me == 0) {
+        lo_hi[0] = INT_MAX;
+        lo_hi[1] = lo_hi[2] = 0;
+    }
+    t.sync();
+    lo = __reduce_min_sync(FULL, lo);
+    hi = __reduce_max_sync(FULL, hi);
+    if (NTHREADS > 32) {
+        if (lane == 0) {
+            atomicMin(&lo_hi[0], lo);
+            atomicMax(&lo_hi[1], hi);
+        }
+        t.sync();
+        lo = lo_hi[0];
+        hi = lo_hi[1];
+    }
+    /* bucket of t: (t - lo) B / width by a rounded-down 0.32 reciprocal, monotone in t, which is all
+     * that the placement needs */
+    const unsigned scale = (unsigned)min(0xffffffffull, ((unsigned long long)B << 32) / (unsigned long long)max(1, hi - lo + 1));
+    auto bucket = [&](int x) -> int {
+        const unsigned long long p = (unsigned long long)(unsigned)(x - lo) * scale;
+        return min(B - 1, (int)(p >> 32));
+    };
+    for (int i = me; i < m; i += NTHREADS) atomicAdd(&tab[bucket(list[i])], 1);
+    t.sync();
+    /* exclusive scan of the counts, kPer consecutive buckets per thread */
+    int c[kPer], sum = 0, most = 0;
+#pragma unroll
+    for (int k = 0; k < kPer; k++) {
+        c[k] = tab[me * kPer + k];
+        most = max(most, c[k]);
+        sum += c[k];
+    }
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(FULL, incl, o);
+        if (lane >= o) incl += y;
+    }
+    most = __reduce_max_sync(FULL, most);
+    int start = incl - sum;
+    if (NTHREADS > 32) {
+        if (lane == 31) lo_hi[4 + warp] = incl;
+        if (lane == 0) atomicMax(&lo_hi[2], most);
+        t.sync();
+        most = lo_hi[2];
+        for (int w = 0; w < warp; w++) start += lo_hi[4 + w];
+    }
+    if (most <= kCrowd) {
+#pragma unroll
+        for (int k = 0; k < kPer; k++) {
+            tab[me * kPer + k] = start;
+            start += c[k];
+        }
+        t.sync();
+        int* dst = tab + B;
+        for (int i = me; i < m; i += NTHREADS) {
+            const int x = list[i];
+            dst[atomicAdd(&tab[bucket(x)], 1)] = x;
+        }
+        t.sync();
+        /* tab[b] is now the end of bucket b */
+        if (write)
+            for (int i = me; i < m; i += NTHREADS) {
+                const int x = dst[i], b = bucket(x), first = b ? tab[b - 1] : 0, end = tab[b];
+                int rank = first;
+                for (int k = first; k < end; k++) rank += dst[k] < x ? 1 : 0;
+                out[rank] = (uint32_t)x;
+            }
+    } else {
+        /* runs of 32 sorted by the warps, then merged in pairs: an id's place in the merged run is its
+         * place in its own run plus the ids below it in the partner run */
+        t.sync();
+        const int runs = (m + 31) >> 5;
+        for (int r = warp; r < runs; r += NTHREADS / 32) {
+            const int i = 32 * r + lane;
+            const int v = warp_sort32(i < m ? list[i] : INT_MAX);
+            __syncwarp();
+            if (i < m) list[i] = v;
+        }
+        t.sync();
+        int* src = list;
+        int* dst = tab;
+        for (int L = 32; L < m; L <<= 1) {
+            for (int i = me; i < m; i += NTHREADS) {
+                const int x = src[i];
+                const int begin = i & ~(2 * L - 1);
+                const int mid = min(begin + L, m), end = min(begin + 2 * L, m);
+                const bool in_a = i < mid;
+                const int first = in_a ? mid : begin;
+                int at = first, len = in_a ? end - mid : mid - begin;
+                while (len > 0) {
+                    const int half = len >> 1;
+                    if (src[at + half] < x) {
+                        at += half + 1;
+                        len -= half + 1;
+                    } else {
+                        len = half;
+                    }
+                }
+                dst[begin + (i - (in_a ? begin : mid)) + (at - first)] = x;
+            }
+            t.sync();
+            int* s = src;
+            src = dst;
+            dst = s;
+        }
+        if (write)
+            for (int i = me; i < m; i += NTHREADS) out[i] = (uint32_t)src[i];
+    }
+    t.sync();
+    int4* slots = reinterpret_cast<int4*>(tab);
+    for (int i = me; i < (1 << HB) / 4; i += NTHREADS) slots[i] = make_int4(-1, -1, -1, -1);
+}
+
+struct GroupQuery {
+    const gat_mbb* queries;
+    GridDev grid;
+    FsgDev fsg;
+    GroupsDev g;
+    const float* X;
+    const float* Y;
+    uint32_t* arena;
+    int64_t cap;
+    /* [0] arena cursor, [1] work bytes, [2] big queries taken, [3] queries for the bitmap scan, [4] small
+     * queries taken, [5] queries that outgrew their team, [7] mid queries taken */
+    unsigned long long* ctr;
+    int64_t* segbase;
+    int64_t* segcnt;
+    int2* retry;   /* queries that outgrew their team, chained per CTA: (query, next or -1) */
+    int* ovf_list; /* queries for the bitmap scan */
+    unsigned long long* work;
+};
+
+/* one query of a team: walk, scan, sort, write; false when it outgrew the team's memory (which is
+ * then empty again) */
+template <int KIND, class T>
+__device__ bool answer(const GroupQuery& a, int qi, T& t, OpenGroups& og, int me, unsigned long long& bytes) {
+    const Box q = load_box(a.queries, qi);
+    if (KIND == GAT_INDEX_GRID)
+        walk_grid(a.g, a.grid, q, t, me);
+    else
+        walk_fsg(a.fsg, a.g.cell_g, q, t, me);
+    const int n = min(*t.nitems, T::ITEMS);
+    if (!__shfl_sync(0xffffffffu, *(volatile int*)t.ovf, 0)) {
+        /* ranges per turn: enough turns for every warp, up to 32 a turn */
+        constexpr int kWarps = T::NTHREADS / 32;
+        const int per = kWarps == 1 ? 32 : max(1, min(32, (n + kWarps - 1) / kWarps));
+        for (;;) {
+            int k = 0;
+            if ((me & 31) == 0) k = atomicAdd(t.next, per);
+            k = __shfl_sync(0xffffffffu, k, 0);
+            if (k >= n) break;
+            take_items(t.items + k, min(per, n - k), q, a.g.ids, a.g.gbeg, a.g.gbox, a.X, a.Y, t, og, bytes);
+        }
+    }
+    t.sync();
+    const int m = *t.cnt;
+    const bool lost = *(volatile int*)t.ovf != 0;
+    if (me == 0 && !lost) {
+        *t.base = atomicAdd(&a.ctr[0], (unsigned long long)m);
+        a.segcnt[qi] = m;
+        a.segbase[qi] = (int64_t)*t.base;
+    }
+    t.sync();
+    if (lost) {
+        for (int i = me; i < (1 << T::HB); i += T::NTHREADS) t.tab[i] = -1;
+    } else {
+        const int64_t at = (int64_t)*t.base;
+        sort_ids(t, m, a.arena + at, at + m <= a.cap, me);
+    }
+    t.sync();
+    if (me == 0) *t.nitems = t.nfront[0] = t.nfront[1] = *t.cnt = *t.ovf = *t.next = 0;
+    return !lost;
+}
+
+/* A team's share of the queries list[0..n), taken from *ctr; the ones that outgrow it go on the CTA's chain. */
+template <int KIND, class T>
+__device__ void answer_list(const GroupQuery& a, const int* __restrict__ list, int n, unsigned long long* ctr, T t,
+                            OpenGroups& og, int* chain, unsigned long long& bytes) {
+    const int me = threadIdx.x % T::NTHREADS;
+    for (;;) {
+        if (me == 0) *t.query = (int)atomicAdd(ctr, 1ull);
+        t.sync(); /* also: the set and the counters are clear */
+        const int j = *t.query;
+        t.sync();
+        if (j >= n) break;
+        const int qi = list[j];
+        if (!answer<KIND>(a, qi, t, og, me, bytes) && me == 0) {
+            const int k = (int)atomicAdd(&a.ctr[5], 1ull);
+            a.retry[k] = make_int2(qi, atomicExch(chain, k));
+        }
+    }
+}
+
+/* Big queries by the CTA, then mid and small ones by its teams, then those that outgrew their team.
+ * list: the queries by class, small, mid, big (k_order), *counts how many of them (ends of the small and
+ * the mid part, then nq); list null: queries 0..nq-1, all big. */
+template <int KIND>
+__global__ void __launch_bounds__(kNT, 3) k_range_groups(GroupQuery a, const int* __restrict__ list, const int* counts, int nq) {
+    dep_wait();
+    extern __shared__ int4 smem4[];
+    int* mem = reinterpret_cast<int*>(smem4);
+    __shared__ __align__(8) int ctl[kW][kCtl];
+    __shared__ int q_sh, chain;
+    __shared__ OpenGroups open[kW];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    auto empty = [&] {
+        int4* m = smem4;
+        for (int i = threadIdx.x; i < kInts / 4; i += kNT) m[i] = make_int4(-1, -1, -1, -1);
+    };
+    empty();
+    if (lane < kCtl) ctl[warp][lane] = 0;
+    if (threadIdx.x == 0) chain = -1;
+    __syncthreads();
+    unsigned long long bytes = 0;
+    int first_big = 0;
+    BlockTeam t(mem, ctl[0], 0);
+    auto block_query = [&](int qi) {
+        if (!answer<KIND>(a, qi, t, open[warp], threadIdx.x, bytes) && threadIdx.x == 0) {
+            a.ovf_list[atomicAdd(&a.ctr[3], 1ull)] = qi;
+            a.segcnt[qi] = 0;
+            a.segbase[qi] = 0;
+        }
+    };
+    if (counts) first_big = counts[1];
+    for (const int nbig = nq - first_big;;) {
+        if (threadIdx.x == 0) q_sh = nbig > 0 ? (int)atomicAdd(&a.ctr[2], 1ull) : 0;
+        __syncthreads(); /* also: the set and the counters are clear */
+        const int j = q_sh;
+        __syncthreads();
+        if (j >= nbig) break;
+        block_query(list ? list[first_big + j] : j);
+    }
+    if (counts) {
+        const int nsmall = counts[0], nmid = counts[1] - nsmall;
+        empty();
+        __syncthreads();
+        const int pair = warp >> 1;
+        answer_list<KIND>(a, list + nsmall, nmid, &a.ctr[7], MidTeam(mem + pair * MidTeam::kInts, ctl[2 * pair], pair), open[warp],
+                          &chain, bytes);
+        __syncthreads();
+        empty();
+        __syncthreads();
+        answer_list<KIND>(a, list, nsmall, &a.ctr[4], SmallTeam(mem + warp * SmallTeam::kInts, ctl[warp], warp), open[warp],
+                          &chain, bytes);
+        __syncthreads();
+        if (chain >= 0) {
+            empty();
+            __syncthreads();
+            for (int k = chain; k >= 0;) {
+                const int2 r = a.retry[k];
+                block_query(r.x);
+                __syncthreads();
+                k = r.y;
+            }
+        }
+    }
+    if (a.work) {
+        for (int o = 16; o > 0; o >>= 1) bytes += __shfl_down_sync(0xffffffffu, bytes, o);
+        if (lane == 0 && bytes) atomicAdd(a.work, bytes);
+    }
+}
+
+/* ---------------------------------------------------------------- order and class of a batch */
+/* The queries of a batch in one counting sort: by class (small, mid, big), then by where they start in
+ * the index's point order, bucketed: queries that run at one time then read overlapping groups, which
+ * stay in L2. The order changes no result. */
+constexpr int kBuckets = 8192;
+constexpr int kBins = 3 * kBuckets;
+
+/* The class: by the distinct ids a query is expected to hold. A box of sides w, h meets about
+ * D (w + e)(h + e) walks, D the density of walks there and e how far a walk reaches (from the mean
+ * number of cells a walk has groups in, range_groups_launch). Grid: D from the list of the smallest
+ * node around the query's centre that is no smaller than it, or the largest one with a list; the
+ * bucket from the last node of that descent. FSG: D from the groups in the query's middle row of
+ * cells, the bucket from its first cell. */
+template <int KIND>
+__global__ void k_order_class(const gat_mbb* queries, int nq, GroupsDev g, FsgDev f, float reach, int* __restrict__ hist,
+                              int* __restrict__ bin) {
+    const int qi = blockIdx.x * blockDim.x + threadIdx.x;
+    if (qi >= nq) return;
+    const Box q = load_box(queries, qi);
+    const float w = q.xmax - q.xmin, h = q.ymax - q.ymin;
+    float density = 0.f; /* walks per unit area */
+    int at = 0;          /* a group near the query's first one */
+    if (KIND == GAT_INDEX_GRID) {
+        const float cx = q.xmin + 0.5f * w, cy = q.ymin + 0.5f * h;
+        NodeRec r = g.rec[0];
+        bool set = false;
+        for (int guard = 0; guard < 32; guard++) {
+            const float nw = r.mbb.z - r.mbb.x, nh = r.mbb.w - r.mbb.y;
+            if (!set && (r.child < 0 || (r.ib >= 0 && (0.5f * nw < w || 0.5f * nh < h)))) {
+                density = (float)(r.ie - r.ib) / ((nw + reach) * (nh + reach));
+                set = true;
+            }
+            if (r.child < 0) break;
+            /* children UL, UR, DL, DR around the middle */
+            const int c = (cx >= r.mbb.x + 0.5f * nw ? 1 : 0) + (cy < r.mbb.y + 0.5f * nh ? 2 : 0);
+            r = g.rec[r.child + c];
+        }
+        at = max(r.ib, 0);
+    } else {
+        const int g1 = max((int)__fdiv_rn(__fsub_rn(q.xmin, f.rxmin), f.cell), 0);
+        const int g2 = min((int)__fdiv_rn(__fsub_rn(q.xmax, f.rxmin), f.cell), f.nx - 1);
+        const int g3 = max((int)__fdiv_rn(__fsub_rn(f.rymax, q.ymax), f.cell), 0);
+        const int g4 = min((int)__fdiv_rn(__fsub_rn(f.rymax, q.ymin), f.cell), f.ny - 1);
+        if (g1 <= g2 && g3 <= g4) {
+            const int row = ((g3 + g4) >> 1) * f.nx;
+            const float c = f.cell + reach;
+            at = g.cell_g[row + g1];
+            density = (float)(g.cell_g[row + g2 + 1] - at) / ((float)(g2 - g1 + 1) * c * c);
+        }
+    }
+    const float est = density * (w + reach) * (h + reach);
+    const int cls = est <= kSmallMax ? 0 : est <= kMidMax ? 1 : 2; /* NaN: big */
+    const int b = cls * kBuckets + (int)min((long long)kBuckets - 1, (long long)at * kBuckets / (g.n + 1));
+    bin[qi] = b;
+    atomicAdd(&hist[b], 1);
+}
+
+/* one CTA: exclusive scan of the bins in place; counts: queries below the mid and the big class */
+__global__ void __launch_bounds__(1024) k_order_scan(int* hist, int* counts) {
+    constexpr int kPer = kBins / 1024;
+    __shared__ int warp_sum[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int c[kPer], sum = 0;
+    int4* mine = reinterpret_cast<int4*>(hist + threadIdx.x * kPer);
+#pragma unroll
+    for (int k = 0; k < kPer / 4; k++) {
+        const int4 v = mine[k];
+        c[4 * k] = v.x, c[4 * k + 1] = v.y, c[4 * k + 2] = v.z, c[4 * k + 3] = v.w;
+        sum += v.x + v.y + v.z + v.w;
+    }
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) warp_sum[warp] = incl;
+    __syncthreads();
+    int run = incl - sum;
+    for (int w = 0; w < warp; w++) run += warp_sum[w];
+#pragma unroll
+    for (int k = 0; k < kPer; k++) {
+        const int b = threadIdx.x * kPer + k, n = c[k];
+        if (b == kBuckets) counts[0] = run;
+        if (b == 2 * kBuckets) counts[1] = run;
+        c[k] = run;
+        run += n;
+    }
+#pragma unroll
+    for (int k = 0; k < kPer / 4; k++) mine[k] = make_int4(c[4 * k], c[4 * k + 1], c[4 * k + 2], c[4 * k + 3]);
+}
+
+__global__ void k_order(int nq, const int* __restrict__ bin, int* __restrict__ base, int* __restrict__ list) {
+    const int qi = blockIdx.x * blockDim.x + threadIdx.x;
+    if (qi < nq) list[atomicAdd(&base[bin[qi]], 1)] = qi;
+}
+
+}  // namespace
+
+int range_groups_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, uint32_t* arena, int64_t cap,
+                        unsigned long long* ctr, int64_t* segbase, int64_t* segcnt, int* ovf_list, bool timed) {
+    cudaStream_t s = ctx->stream;
+    const bool grid = ix->kind == GAT_INDEX_GRID;
+    auto kernel = grid ? k_range_groups<GAT_INDEX_GRID> : k_range_groups<GAT_INDEX_FSG>;
+    allow_smem(kernel, kSmem);
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kNT, kSmem);
+    const int full = std::max(1, per_sm) * ctx->sm_count;
+    GAT_CUDA_TRY(ctx, cudaMemsetAsync(ctr, 0, 8 * sizeof(unsigned long long), s), "range");
+    GroupQuery a{d_q, ix->grid, ix->fsg, ix->groups, ix->d_x, ix->d_y, arena, cap, ctr, segbase, segcnt, nullptr, ovf_list,
+                 timed ? ctr + 1 : nullptr};
+    if (nq <= std::min(full, kDirectMax)) {
+        /* no more queries than resident CTAs: one each */
+        kernel<<<nq, kNT, kSmem, s>>>(a, nullptr, nullptr, nq);
+        count_launch(ctx);
+        GAT_CUDA_TRY(ctx, cudaGetLastError(), "range scan launch");
+        return GAT_OK;
+    }
+    /* [retry nq int2 | bins | counts 4 | bin nq | list nq] */
+    int st = GAT_OK;
+    char* p = (char*)scratch(ctx, S_RANGE_SPLIT, (size_t)nq * 16 + (size_t)(kBins + 4) * 4, &st);
+    if (!p) return st;
+    int* hist = reinterpret_cast<int*>(p);
+    int* counts = hist + kBins;
+    a.retry = reinterpret_cast<int2*>(counts + 4);
+    int* bin = reinterpret_cast<int*>(a.retry + nq);
+    int* list = bin + nq;
+    const int tb = (nq + 255) / 256;
+    GAT_CUDA_TRY(ctx, cudaMemsetAsync(hist, 0, kBins * 4, s), "range");
+    const float cell = grid ? ix->grid.cell : ix->fsg.cell;
+    const float reach = cell * (std::sqrt(std::max(1.f, (float)ix->groups.n / (float)std::max(1, ix->db->n))) - 1.f);
+    (grid ? k_order_class<GAT_INDEX_GRID> : k_order_class<GAT_INDEX_FSG>)<<<tb, 256, 0, s>>>(d_q, nq, ix->groups, ix->fsg, reach,
+                                                                                          hist, bin);
+    k_order_scan<<<1, 1024, 0, s>>>(hist, counts);
+    k_order<<<tb, 256, 0, s>>>(nq, bin, hist, list);
+    kernel<<<full, kNT, kSmem, s>>>(a, list, counts, nq);
+    count_launch(ctx, 4);
+    GAT_CUDA_TRY(ctx, cudaGetLastError(), "range scan launch");
+    return GAT_OK;
+}
+
+}  // namespace gat

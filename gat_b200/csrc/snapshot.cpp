@@ -258,7 +258,9 @@ int gat_index_load(gat_ctx* ctx, const gat_db* db, const char* path, gat_index**
             }
             *fl[i] = p;
         }
-        if (int st = index_point_boxes(ix)) {
+        int st = index_groups(ix);
+        if (st == GAT_OK) st = index_point_boxes(ix);
+        if (st != GAT_OK) {
             gat_index_destroy(ix);
             return st;
         }

@@ -1,0 +1,116 @@
+"""Id-set range queries over point groups against the point scan (GAT_TUNE_RANGE_SHAPE = 1, the general
+path) and the oracle, over the forms a query and a set can take: rectangles on cell borders, of no size,
+inverted, beyond the grid, infinite or NaN; clustered sets that outgrow a team's set; trees that are one
+leaf or as deep as the grid; batch sizes on both sides of every switch."""
+import numpy as np
+import pytest
+
+import gat_b200 as G
+from gat_b200 import _lib as L
+from gat_b200 import data as D
+from gat_b200.api import Index
+from oracle import pyoracle as po
+
+pytestmark = pytest.mark.gpu
+
+
+def _general(ctx, ix, q):
+    ctx.set_tuning(L.GAT_TUNE_RANGE_SHAPE, 1)
+    try:
+        return ix.range_query(q, capacity=4_000_000)
+    finally:
+        ctx.set_tuning(L.GAT_TUNE_RANGE_SHAPE, 0)
+
+
+def _same(ctx, ix, q):
+    a, b = _general(ctx, ix, q), ix.range_query(q, capacity=4_000_000)
+    assert np.array_equal(a.offsets, b.offsets) and np.array_equal(a.tids, b.tids)
+    return b
+
+
+def _odd_rectangles(t, cell, seed):
+    """Rectangles whose edges lie on cell borders, on points, or nowhere sensible."""
+    rng = np.random.default_rng(seed)
+    x0, y0, x1, y1 = D.BOX
+    c = np.float32(cell)
+    k = rng.integers(0, int(1 / cell), (300, 4))
+    gx = np.float32(x0) + c * np.minimum(k[:, 0], k[:, 1]).astype(np.float32)
+    hx = np.float32(x0) + c * (np.maximum(k[:, 0], k[:, 1]) + rng.integers(0, 2, 300)).astype(np.float32)
+    gy = np.float32(y1) - c * np.maximum(k[:, 2], k[:, 3]).astype(np.float32)
+    hy = np.float32(y1) - c * np.minimum(k[:, 2], k[:, 3]).astype(np.float32)
+    p = rng.integers(0, t.lon.size, (300, 2))
+    ax, ay = t.lon[p], t.lat[p]
+    point = np.stack([ax[:, 0], ay[:, 0], ax[:, 0], ay[:, 0]], 1)
+    span = np.stack([ax.min(1), ay.min(1), ax.max(1), ay.max(1)], 1)
+    inf, nan = np.inf, np.nan
+    wild = np.array([[x0, y0, x1, y1], [x0 - 5, y0 - 5, x1 + 5, y1 + 5], [x1, y1, x0, y0], [-inf, -inf, inf, inf],
+                     [121.4, 31.0, inf, inf], [-inf, 31.0, 121.2, 31.1], [nan, y0, x1, y1], [x0, nan, x1, y1], [x0, y0, nan, y1],
+                     [x0, y0, x1, nan], [nan] * 4, [121.5, 31.2, 121.4, 31.3], [10, 10, 11, 11], [121.999, 30.69, 122.5, 30.71],
+                     [120.9, 31.69, 121.001, 31.8], [121.3, 30.0, 121.31, 33.0]], np.float32)
+    return np.concatenate([np.stack([gx, gy, hx, hy], 1), point, span, wild]).astype(np.float32)
+
+
+@pytest.mark.parametrize("cell,cap", [(0.01, 512), (0.01, 1), (0.02, 10_000_000), (0.003, 64)])
+def test_odd_rectangles(gpu_ctx, cell, cap):
+    t = D.walks(D.lengths(3000, 0, 0, 0, 1, 200, 31), 31)
+    db = G.TrajectorySet(gpu_ctx, t)
+    q = _odd_rectangles(t, cell, 5)
+    finite = np.isfinite(q).all(1)
+    g, f = G.Grid(gpu_ctx, db, D.BOX, cell, 2, cap), G.FSG(gpu_ctx, db, D.BOX, cell)
+    for ix, o in ((g, po.OracleGrid(t, D.BOX, cell, 2, cap)), (f, po.OracleFSG(t, D.BOX, cell))):
+        r = _same(gpu_ctx, ix, q[finite])
+        off, ids = o.range(q[finite], 0)
+        assert np.array_equal(r.offsets, off) and np.array_equal(r.tids, ids)
+    _same(gpu_ctx, g, q)  # NaN and infinite rectangles too: the two paths agree
+    _same(gpu_ctx, f, q[~np.isinf(q).any(1)])
+
+
+@pytest.mark.parametrize("nq", [1, 31, 444, 445, 1024, 1025, 3001])
+def test_batch_sizes(gpu_ctx, nq):
+    t = D.walks(D.lengths(20_000, 0, 0, 0, 20, 200, 32), 32)
+    db = G.TrajectorySet(gpu_ctx, t)
+    q = D.boxes(nq, 1, 0.001, 0.3, 33)
+    _same(gpu_ctx, G.Grid(gpu_ctx, db, D.BOX, 0.005, 2, 512), q)
+    _same(gpu_ctx, G.FSG(gpu_ctx, db, D.BOX, 0.005), q)
+
+
+def test_clustered_set(gpu_ctx):
+    """Most walks in one corner, ids in two far ranges: the expected sizes are wrong, so queries outgrow
+    every team in turn, and a result's ids crowd in few buckets."""
+    t = D.walks(D.lengths(12_000, 0, 0, 0, 20, 120, 34), 34)
+    off = t.offsets
+    for i in range(t.n):
+        s, e = off[i], off[i + 1]
+        if i < 2500 or i >= 9000:  # pulled into a 0.02 degree square
+            t.lon[s:e] = np.float32(121.3) + (t.lon[s:e] - np.float32(121.0)) * np.float32(0.02)
+            t.lat[s:e] = np.float32(31.1) + (t.lat[s:e] - np.float32(30.7)) * np.float32(0.02)
+    db = G.TrajectorySet(gpu_ctx, t)
+    rng = np.random.default_rng(6)
+    c = rng.uniform([121.295, 31.095], [121.325, 31.125], (900, 2))
+    h = np.exp(rng.uniform(np.log(0.0005), np.log(0.02), (900, 2)))
+    q = np.concatenate([np.concatenate([c - h, c + h], 1), D.boxes(600, 1, 0.001, 0.05, 35)]).astype(np.float32)
+    for ix in (G.Grid(gpu_ctx, db, D.BOX, 0.002, 2, 512), G.FSG(gpu_ctx, db, D.BOX, 0.002)):
+        r = _same(gpu_ctx, ix, q)
+        assert int(np.diff(r.offsets).max()) > 4096  # beyond the largest set
+        _same(gpu_ctx, ix, q[:200])
+
+
+def test_tiny_sets_and_fine_cells(gpu_ctx):
+    for n, lo, hi, cell in ((1, 1, 1, 0.01), (2, 300, 300, 0.5), (40, 2000, 4000, 0.0005)):
+        t = D.walks(D.lengths(n, 0, 0, 0, lo, hi, 36), 36)
+        db = G.TrajectorySet(gpu_ctx, t)
+        q = np.concatenate([D.boxes(500, 1, 0.0005, 0.5, 37), _odd_rectangles(t, 0.01, 38)[:600]])
+        _same(gpu_ctx, G.Grid(gpu_ctx, db, D.BOX, cell, 2, 512), q)
+        _same(gpu_ctx, G.FSG(gpu_ctx, db, D.BOX, cell), q)
+
+
+def test_snapshot_keeps_groups(gpu_ctx, tmp_path):
+    t = D.walks(D.lengths(4000, 0, 0, 0, 20, 200, 39), 39)
+    db = G.TrajectorySet(gpu_ctx, t)
+    q = D.boxes(700, 1, 0.001, 0.1, 40)
+    for ix in (G.Grid(gpu_ctx, db, D.BOX, 0.005, 2, 512), G.FSG(gpu_ctx, db, D.BOX, 0.005)):
+        ix.save(str(tmp_path / "i.bin"))
+        back = Index.load(gpu_ctx, db, str(tmp_path / "i.bin"))
+        assert back.info()["device_bytes"] == ix.info()["device_bytes"]
+        a, b = ix.range_query(q), back.range_query(q)
+        assert np.array_equal(a.offsets, b.offsets) and np.array_equal(a.tids, b.tids)
