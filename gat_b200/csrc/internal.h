@@ -16,6 +16,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <functional>
 #include <map>
@@ -177,7 +178,15 @@ struct gat_db {
     float2* d_xy = nullptr;
 };
 
+/* Never the same for two indexes of a process: what a cache keys an index by (a new index can get the
+ * address of a destroyed one). */
+inline uint64_t next_index_uid() {
+    static std::atomic<uint64_t> n{0};
+    return ++n;
+}
+
 struct gat_index {
+    const uint64_t uid = next_index_uid();
     gat_ctx* ctx = nullptr;
     const gat_db* db = nullptr;
     int kind = 0;

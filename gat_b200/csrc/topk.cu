@@ -994,6 +994,7 @@ __global__ void k_loop_cond(const int32_t* ws, int* iter, int maxit, int32_t* fl
 
 struct LoneGraph {
     const gat_index* g = nullptr;
+    uint64_t uid = 0; /* the index's, which tells it from a later one at its address */
     int max_q_len = 0, k = 0;
     float u = 0.f;
     int chunk = 0, growth = 0, rows = 0, form = 0, dep = 1; /* the context's knobs when the graph was built */
@@ -1028,7 +1029,7 @@ int lone_graph_get(gat_ctx* ctx, const gat_index* g, int max_q_len, int k, float
     for (auto& o : ctx->owned)
         if (o.second == lone_graph_free) {
             auto* L = static_cast<LoneGraph*>(o.first);
-            if (L->g == g && L->max_q_len == max_q_len && L->k == k && L->u == u && L->chunk == ctx->topk_chunk &&
+            if (L->uid == g->uid && L->max_q_len == max_q_len && L->k == k && L->u == u && L->chunk == ctx->topk_chunk &&
                 L->growth == ctx->topk_growth && L->rows == ctx->edr_rows && L->form == ctx->edr_form &&
                 L->dep == ctx->dep_launch) {
                 *out = L;
@@ -1047,6 +1048,7 @@ int lone_graph_get(gat_ctx* ctx, const gat_index* g, int max_q_len, int k, float
     }
     auto* L = new LoneGraph();
     L->g = g;
+    L->uid = g->uid;
     L->max_q_len = max_q_len;
     L->k = k;
     L->u = u;
