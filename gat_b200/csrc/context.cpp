@@ -487,13 +487,16 @@ int gat_db_create(gat_ctx* ctx, int n, const int32_t* lengths, const float* lon,
     if ((e = cudaMalloc(&db->d_len, (n + 1) * sizeof(int32_t))) != cudaSuccess ||
         (e = cudaMalloc(&db->d_off, (n + 2) * sizeof(int64_t))) != cudaSuccess ||
         (e = cudaMalloc(&db->d_xy, (db->npoints + 1) * sizeof(float2))) != cudaSuccess ||
+        (e = cudaMalloc(&db->d_box, (n + 1) * sizeof(float4))) != cudaSuccess ||
         (e = cudaMemcpy(db->d_len, db->h_len.data(), (n + 1) * sizeof(int32_t), cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = cudaMemcpy(db->d_off, db->h_off.data(), (n + 2) * sizeof(int64_t), cudaMemcpyHostToDevice)) != cudaSuccess) {
         int rc = cuda_fail(ctx, e, "gat_db_create");
         gat_db_destroy(db);
         return rc;
     }
-    if (int rc = upload_set_points(ctx, lon, lat, db->npoints, db->d_xy)) {
+    int rc = upload_set_points(ctx, lon, lat, db->npoints, db->d_xy);
+    if (rc == GAT_OK) rc = set_boxes(ctx, db);
+    if (rc != GAT_OK) {
         gat_db_destroy(db);
         return rc;
     }
@@ -512,6 +515,7 @@ void gat_db_destroy(gat_db* db) {
     cudaFree(db->d_len);
     cudaFree(db->d_off);
     cudaFree(db->d_xy);
+    cudaFree(db->d_box);
     delete db;
 }
 

@@ -47,6 +47,8 @@ struct SoaPairs {
     int32_t* flag;
     static constexpr int kKind = 0;
     __device__ int count() const { return d_npairs ? *d_npairs : npairs; }
+    /* whether the pair is known to share no match (the arrays carry no boxes) */
+    __device__ bool apart(int, float) const { return false; }
     __device__ void get(int p, const float2*& a, int& la, const float2*& b, int& lb, int32_t*& o) const {
         la = a_len[p];
         lb = b_len[p];
@@ -258,6 +260,25 @@ __device__ __forceinline__ int duration_class(long long d) {
     return min(2 * e + half, kClasses - 1);
 }
 
+/* E of row r at column c when no point of the first r rows matches any of the first c columns.
+ * Let k be the highest bit set in r and clear in c: E = (r mod 2^(k+1)) - (c mod 2^(k+1)), and 0
+ * when there is no such bit. (The recurrence without matches depends on r and c alone. Row r has
+ * period 2^(k+1) in c for 2^k <= r < 2^(k+1): over a period E falls r, r - 1, ..., r - 2^k + 1,
+ * then repeats row r - 2^k from its start, where E = r - 2^k; by induction on r the rule m == l ->
+ * u restarts the fall at each period, as m and l meet there.) */
+__device__ __forceinline__ int unmatched_e(int r, int c) {
+    const int x = r & ~c;
+    if (x == 0) return 0;
+    const int mask = (2 << (31 - __clz(x))) - 1;
+    return (r & mask) - (c & mask);
+}
+/* Whether boxes a and b (x0, y0, x1, y1 of the points) are too far apart for any match: rounding is
+ * monotone, so a difference of edges of at least u bounds every difference of points from below. False
+ * when an edge is NaN. */
+__device__ __forceinline__ bool boxes_apart(const float4& a, const float4& b, float u) {
+    return __fsub_rn(b.x, a.z) >= u || __fsub_rn(a.x, b.z) >= u || __fsub_rn(b.y, a.w) >= u || __fsub_rn(a.y, b.w) >= u;
+}
+
 /* How a pair is cut: column tiles of 32 R columns, row tiles of 32 R rows (2H = R rows per lane),
  * the last row tile of the smallest height 64 h, h a power of two, that holds the rest. */
 template <int R>
@@ -265,9 +286,13 @@ __device__ __forceinline__ int tile_count(int nlane) {
     return nlane <= 0 ? 1 : (nlane + 32 * R - 1) / (32 * R);
 }
 
+/* The count pass also answers the pairs whose boxes are apart (most candidates of a top-k walk are far
+ * from the query): their distance is the lengths' alone (unmatched_e) and they take no item. */
 template <int R, bool COL, class Src>
-__global__ void k_sched_count(Src src, int cap, int coop_cap, int* __restrict__ ctr, int2* __restrict__ meta) {
+__global__ void k_sched_count(Src src, int cap, int coop_cap, int* __restrict__ ctr, int2* __restrict__ meta, float u,
+                              unsigned long long* __restrict__ cells) {
     dep_wait();
+    unsigned long long done = 0; /* cells of the pairs answered here */
     __shared__ int hist[kClasses];
     for (int i = threadIdx.x; i < kClasses; i += blockDim.x) hist[i] = 0;
     __syncthreads();
@@ -278,6 +303,12 @@ __global__ void k_sched_count(Src src, int cap, int coop_cap, int* __restrict__ 
         int32_t* o;
         src.get(p, a, la, b, lb, o);
         const int len1 = min(la, lb), len2 = max(la, lb);
+        if (src.apart(p, u)) {
+            *o = len2 + unmatched_e(len1, len2);
+            done += (unsigned long long)len1 * (unsigned long long)len2;
+            meta[p] = make_int2(-1, 0);
+            continue;
+        }
         const int nlane = COL ? len2 : len1, nstep = COL ? len1 : len2;
         const int T = tile_count<R>(nlane);
         int slot = -1, items = 1;
@@ -295,6 +326,10 @@ __global__ void k_sched_count(Src src, int cap, int coop_cap, int* __restrict__ 
         const int c = duration_class(dur);
         atomicAdd(&hist[c], items);
         meta[p] = make_int2(slot, (c << 16) | items);
+    }
+    if (cells) {
+        for (int o = 16; o > 0; o >>= 1) done += __shfl_xor_sync(0xffffffffu, done, o);
+        if ((threadIdx.x & 31) == 0 && done) atomicAdd(cells, done);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < kClasses; i += blockDim.x)
@@ -341,7 +376,9 @@ __global__ void k_sched_write(Src src, int cap, int* __restrict__ ctr, const int
         __syncthreads();
         if (p < n) {
             const int pos = off[c] + lbase[c] + loc;
-            if (slot < 0)
+            if (nit == 0)
+                ; /* answered by the count pass */
+            else if (slot < 0)
                 items[pos] = make_int4(p, -1, -1, 1);
             else
                 for (int t = 0; t < nit; t++) items[pos + t] = make_int4(p, t, slot, nit);
@@ -410,18 +447,6 @@ __device__ __forceinline__ unsigned sign_halves(float lo, float hi) {
     return d;
 }
 
-/* E of row r at column c when no point of the first r rows matches any of the first c columns.
- * Let k be the highest bit set in r and clear in c: E = (r mod 2^(k+1)) - (c mod 2^(k+1)), and 0
- * when there is no such bit. (The recurrence without matches depends on r and c alone. Row r has
- * period 2^(k+1) in c for 2^k <= r < 2^(k+1): over a period E falls r, r - 1, ..., r - 2^k + 1,
- * then repeats row r - 2^k from its start, where E = r - 2^k; by induction on r the rule m == l ->
- * u restarts the fall at each period, as m and l meet there.) */
-__device__ __forceinline__ int unmatched_e(int r, int c) {
-    const int x = r & ~c;
-    if (x == 0) return 0;
-    const int mask = (2 << (31 - __clz(x))) - 1;
-    return (r & mask) - (c & mask);
-}
 __device__ __forceinline__ unsigned unmatched_pair(int rlo, int rhi, int c) {
     return (unsigned)(kBias + unmatched_e(rlo, c)) | (unsigned)(kBias + unmatched_e(rhi, c)) << 16;
 }
@@ -1060,7 +1085,8 @@ int launch_tiles(gat_ctx* ctx, const Src& src, int64_t cap, int max_rows, int ma
     if (!ctr || !meta || !items || !wcarry || (coop > 0 && !pcarry)) return st;
     (void)launch_dep(ctx, k_zero_words, dim3(1), dim3(256), 0, s, ctr, (int)kCtrWords);
     const int pgrid = (int)std::max<int64_t>(1, std::min<int64_t>((cap + 255) / 256, (int64_t)ctx->sm_count * 8));
-    (void)launch_dep(ctx, k_sched_count<R, COL, Src>, dim3(pgrid), dim3(256), 0, s, src, (int)cap, (int)coop, ctr, meta);
+    (void)launch_dep(ctx, k_sched_count<R, COL, Src>, dim3(pgrid), dim3(256), 0, s, src, (int)cap, (int)coop, ctr, meta, u,
+                     cells);
     count_launch(ctx);
     (void)launch_dep(ctx, k_sched_write<Src>, dim3(pgrid), dim3(256), 0, s, src, (int)cap, ctr, meta, items, edr_epochs(ctx));
     count_launch(ctx);

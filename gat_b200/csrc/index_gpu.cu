@@ -792,7 +792,37 @@ __global__ void k_interleave(int64_t P, const float* __restrict__ lon, const flo
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < P; i += (int64_t)gridDim.x * blockDim.x)
         xy[i] = make_float2(lon[i], lat[i]);
 }
+
+/* a warp per trajectory */
+__global__ void k_set_boxes(int n, const int64_t* __restrict__ off, const float2* __restrict__ xy, float4* box) {
+    const int lane = threadIdx.x & 31;
+    for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t <= n; t += (gridDim.x * blockDim.x) >> 5) {
+        const int64_t b = t ? off[t] : 0, e = t ? off[t + 1] : 0;
+        float4 v = make_float4(__int_as_float(0x7f800000), __int_as_float(0x7f800000), __int_as_float(0xff800000),
+                               __int_as_float(0xff800000));
+#pragma unroll 4
+        for (int64_t i = b + lane; i < e; i += 32) {
+            const float2 p = xy[i];
+            v = make_float4(fminf(v.x, p.x), fminf(v.y, p.y), fmaxf(v.z, p.x), fmaxf(v.w, p.y));
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            v.x = fminf(v.x, __shfl_xor_sync(0xffffffffu, v.x, o));
+            v.y = fminf(v.y, __shfl_xor_sync(0xffffffffu, v.y, o));
+            v.z = fmaxf(v.z, __shfl_xor_sync(0xffffffffu, v.z, o));
+            v.w = fmaxf(v.w, __shfl_xor_sync(0xffffffffu, v.w, o));
+        }
+        if (lane == 0) box[t] = v;
+    }
+}
 }  // namespace
+
+int set_boxes(gat_ctx* ctx, gat_db* db) {
+    k_set_boxes<<<grid_size(ctx, (int64_t)(db->n + 1) * 32), 256, 0, ctx->stream>>>(db->n, db->d_off, db->d_xy, db->d_box);
+    count_launch(ctx);
+    GAT_CUDA_TRY(ctx, cudaGetLastError(), "gat_db_create");
+    GAT_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream), "gat_db_create");
+    return GAT_OK;
+}
 
 int upload_set_points(gat_ctx* ctx, const float* lon, const float* lat, int64_t P, float2* d_xy) {
     if (P == 0) return GAT_OK;

@@ -176,6 +176,7 @@ struct gat_db {
     int32_t* d_len = nullptr;
     int64_t* d_off = nullptr;
     float2* d_xy = nullptr;
+    float4* d_box = nullptr; /* [n + 1] box of each trajectory's points (+inf .. -inf without points) */
 };
 
 /* Never the same for two indexes of a process: what a cache keys an index by (a new index can get the
@@ -364,6 +365,8 @@ int device_build_grid(gat_index* ix, const DevicePlaceArgs& a, int total_level, 
 int device_build_fsg(gat_index* ix, const DevicePlaceArgs& a);
 /* uploads lon / lat (host, trajectory order) into d_xy as interleaved (lon, lat) pairs */
 int upload_set_points(gat_ctx* ctx, const float* lon, const float* lat, int64_t P, float2* d_xy);
+/* the box of every trajectory's points (NaN coordinates left out: they match nothing) */
+int set_boxes(gat_ctx* ctx, gat_db* db);
 /* downloads the host copies (h_x, h_y) of a device trajectory set (no-op when present) */
 int db_host_copies(const gat_db* db);
 /* downloads the host copies of a device-placed index (no-op otherwise) */

@@ -68,17 +68,37 @@ __device__ __forceinline__ int cell_of(const GridDev& g, float lon, float lat) {
  * (a trajectory stays in a cell for many points), then the few runs sorted and merged.
  * qfv rows have stride `stride` (>= longest query); nnz in qfv_n. */
 __global__ void k_query_fv(GridDev g, int nq, const int32_t* q_len, const int64_t* q_off, const float2* Q,
-                           int stride, int pow2, int32_t* qfv_cell, int32_t* qfv_cnt, int32_t* qfv_n) {
+                           int stride, int pow2, int32_t* qfv_cell, int32_t* qfv_cnt, int32_t* qfv_n, float4* q_box) {
     dep_wait();
     extern __shared__ unsigned long long rkey[]; /* pow2 run keys (cell << 32 | count), then pow2 cells */
     int* sk = reinterpret_cast<int*>(rkey + pow2);
     __shared__ int wsum[32];
+    __shared__ float4 wbox[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int qi = blockIdx.x; qi < nq; qi += gridDim.x) {
         const int L = q_len[qi];
         const int64_t o = q_off[qi];
-        for (int i = threadIdx.x; i < L; i += blockDim.x) sk[i] = cell_of(g, Q[o + i].x, Q[o + i].y) >> g.vparam;
+        float4 box = make_float4(__int_as_float(0x7f800000), __int_as_float(0x7f800000), __int_as_float(0xff800000),
+                                 __int_as_float(0xff800000));
+        for (int i = threadIdx.x; i < L; i += blockDim.x) {
+            const float2 p = Q[o + i];
+            sk[i] = cell_of(g, p.x, p.y) >> g.vparam;
+            box = make_float4(fminf(box.x, p.x), fminf(box.y, p.y), fmaxf(box.z, p.x), fmaxf(box.w, p.y));
+        }
+        for (int s = 16; s > 0; s >>= 1) {
+            box.x = fminf(box.x, __shfl_xor_sync(0xffffffffu, box.x, s));
+            box.y = fminf(box.y, __shfl_xor_sync(0xffffffffu, box.y, s));
+            box.z = fmaxf(box.z, __shfl_xor_sync(0xffffffffu, box.z, s));
+            box.w = fmaxf(box.w, __shfl_xor_sync(0xffffffffu, box.w, s));
+        }
+        if (lane == 0) wbox[warp] = box;
         __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < nw; w++)
+                box = make_float4(fminf(box.x, wbox[w].x), fminf(box.y, wbox[w].y), fmaxf(box.z, wbox[w].z),
+                                  fmaxf(box.w, wbox[w].w));
+            q_box[qi] = box;
+        }
         /* run heads, compacted in order (L <= pow2 <= blockDim.x * chunks) */
         int base = 0;
         for (int c0 = 0; c0 < L; c0 += blockDim.x) {
@@ -94,18 +114,25 @@ __global__ void k_query_fv(GridDev g, int nq, const int32_t* q_len, const int64_
             }
             unsigned lt;
             asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
-            if (head) {
-                int r = base + wb + __popc(bal & lt);
-                int e = i + 1;
-                while (e < L && sk[e] == sk[i]) e++;
-                rkey[r] = ((unsigned long long)(unsigned)sk[i] << 32) | (unsigned)(e - i);
-            }
+            if (head) rkey[base + wb + __popc(bal & lt)] = ((unsigned long long)(unsigned)sk[i] << 32) | (unsigned)i;
             base += tot;
             __syncthreads();
         }
         /* sort the runs by cell (bitonic over 64-bit (cell, count) keys in the run area),
          * then one thread merges equal cells; runs are few, the sort is short */
         const int R = base;
+        /* a run ends where the next begins */
+        for (int c0 = 0; c0 < R; c0 += blockDim.x) {
+            const int r = c0 + threadIdx.x;
+            unsigned long long k = 0;
+            if (r < R) {
+                k = rkey[r];
+                const int end = r + 1 < R ? (int)(rkey[r + 1] & 0xffffffffu) : L;
+                k = (k & 0xffffffff00000000ull) | (unsigned)(end - (int)(k & 0xffffffffu));
+            }
+            __syncthreads(); /* the run after this chunk's last is read before it is rewritten */
+            if (r < R) rkey[r] = k;
+        }
         int p2 = 1;
         while (p2 < R) p2 <<= 1;
         for (int a = R + threadIdx.x; a < p2; a += blockDim.x) rkey[a] = ~0ull;
@@ -125,18 +152,27 @@ __global__ void k_query_fv(GridDev g, int nq, const int32_t* q_len, const int64_
                 __syncthreads();
             }
         if (threadIdx.x == 0) {
+            /* the open cell and its count stay in registers */
             int w = 0;
             int32_t* oc = qfv_cell + (size_t)qi * stride;
             int32_t* on = qfv_cnt + (size_t)qi * stride;
+            int open = 0, sum = 0;
             for (int a = 0; a < R; a++) {
-                int cell = (int)(rkey[a] >> 32), cnt = (int)(rkey[a] & 0xffffffffu);
-                if (w > 0 && oc[w - 1] == cell) {
-                    on[w - 1] += cnt;
-                } else {
-                    oc[w] = cell;
-                    on[w] = cnt;
-                    w++;
+                const int cell = (int)(rkey[a] >> 32), cnt = (int)(rkey[a] & 0xffffffffu);
+                if (a > 0 && cell == open) {
+                    sum += cnt;
+                    continue;
                 }
+                if (a > 0) {
+                    oc[w] = open;
+                    on[w++] = sum;
+                }
+                open = cell;
+                sum = cnt;
+            }
+            if (R > 0) {
+                oc[w] = open;
+                on[w++] = sum;
             }
             qfv_n[qi] = w;
         }
@@ -157,32 +193,32 @@ __global__ void k_near_bitmap(int nq, int vbits, const int32_t* qfv_cell, const 
 /* ---------------------------------------------------------------- 2b. bound kernel */
 /* FVTable::findNeighbor (FVTable.cpp:53-75): x from even bits, y from odd bits of the
  * virtual cell id over log2(vcells) bits, neighbours in order xx = x-1..x+1, yy = y-1..y+1. */
+__device__ __forceinline__ uint32_t compact16(uint32_t v) {
+    v &= 0x55555555;
+    v = (v | (v >> 1)) & 0x33333333;
+    v = (v | (v >> 2)) & 0x0F0F0F0F;
+    v = (v | (v >> 4)) & 0x00FF00FF;
+    return (v | (v >> 8)) & 0x0000FFFF;
+}
 __device__ __forceinline__ void fv_neighbors(int cell, int bits, int nb[8]) {
-    int x = 0, y = 0;
-    for (int bit = 0; bit < bits; bit++) {
-        if ((bit & 1) == 0)
-            x += ((cell >> bit) & 1) << (bit >> 1);
-        else
-            y += ((cell >> bit) & 1) << (bit >> 1);
+    const uint32_t low = bits >= 32 ? (uint32_t)cell : (uint32_t)cell & ((1u << bits) - 1u);
+    const int x = (int)compact16(low), y = (int)compact16(low >> 1);
+    if (x > 0 && y > 0 && x < 0xFFFF && y < 0xFFFF) {
+        /* no negative coordinate: the keys are the plain interleaving of the three columns and rows */
+        const uint32_t sx[3] = {spread16(x - 1), spread16(x), spread16(x + 1)};
+        const uint32_t sy[3] = {spread16(y - 1) << 1, spread16(y) << 1, spread16(y + 1) << 1};
+        int c = 0;
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+#pragma unroll
+            for (int j = 0; j < 3; j++)
+                if (i != 1 || j != 1) nb[c++] = (int)(sx[i] | sy[j]);
+        return;
     }
     int c = 0;
     for (int xx = x - 1; xx <= x + 1; xx++)
         for (int yy = y - 1; yy <= y + 1; yy++)
             if (xx != x || yy != y) nb[c++] = ref_morton(xx, yy);
-}
-
-__device__ __forceinline__ int find_key(const int* key, int n, int k) {
-    int lo = 0, hi = n - 1;
-    while (lo <= hi) {
-        int mid = (lo + hi) >> 1;
-        int v = key[mid];
-        if (v == k) return mid;
-        if (v < k)
-            lo = mid + 1;
-        else
-            hi = mid - 1;
-    }
-    return -1;
 }
 
 __device__ __forceinline__ bool in_qfv(const int32_t* qc, int qn, int c) {
@@ -211,6 +247,12 @@ __global__ void k_near_bitmap(int nq, int vbits, const int32_t* qfv_cell, const 
     __syncthreads();
     const int qn = qfv_n[qi];
     const int32_t* qc = qfv_cell + (size_t)qi * stride;
+    __shared__ int32_t qs[1024]; /* the query's cells, when they fit: every border cell searches them */
+    if (qn <= 1024) {
+        for (int i = threadIdx.x; i < qn; i += blockDim.x) qs[i] = qc[i];
+        qc = qs;
+        __syncthreads();
+    }
     int nb[8];
     for (int i = threadIdx.x; i < qn; i += blockDim.x) {
         set_bit(bm, words, qc[i]);
@@ -236,130 +278,177 @@ __global__ void k_near_bitmap(int nq, int vbits, const int32_t* qfv_cell, const 
     }
 }
 
-/* one thread per (query, trajectory). The merged vector holds every cell of either vector
- * with value db - query (0 = absent). Pass 1 visits the positive cells in ascending order,
- * pass 2 the negative ones (FVTable.cpp:129-187); the reference increments a map iterator
- * after erasing its node, this visits each key present when the pass starts once. */
-__global__ void __launch_bounds__(kT) k_lower_bounds(int n, int nq, const int64_t* __restrict__ fv_off,
-                                                     const int32_t* __restrict__ fv_cell,
-                                                     const int32_t* __restrict__ fv_cnt, const int32_t* qfv_cell,
-                                                     const int32_t* qfv_cnt, const int32_t* qfv_n, int stride,
-                                                     int vbits, const uint32_t* __restrict__ near, int words,
-                                                     const int32_t* __restrict__ q_len, int32_t* lb, int32_t* flag) {
-    dep_wait();
-    extern __shared__ int sq[];
-    int qi = blockIdx.y;
-    int qn = qfv_n[qi];
-    const int qlen = q_len[qi];
-    int* qc = sq;
-    int* qv = sq + stride;
-    for (int i = threadIdx.x; i < qn; i += blockDim.x) {
-        qc[i] = qfv_cell[(size_t)qi * stride + i];
-        qv[i] = qfv_cnt[(size_t)qi * stride + i];
-    }
-    __syncthreads();
-    int t = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    if (t > n) return;
-    int64_t b = fv_off[t], e = fv_off[t + 1];
-    {
-        const uint32_t* bm = near + (size_t)qi * words;
-        bool touches = false;
-        int tlen = 0;
-        for (int64_t j = b; j < e; j++) {
-            int c = fv_cell[j];
-            tlen += fv_cnt[j];
-            if ((c >> 5) < words && ((__ldg(bm + (c >> 5)) >> (c & 31)) & 1u)) touches = true;
-        }
-        if (!touches) {
-            lb[(size_t)qi * (n + 1) + t] = max(tlen, qlen);
-            return;
-        }
-    }
+/* The bound of one (query, trajectory) pair whose vectors touch, by one warp. The merged vector holds
+ * every cell of either vector with value db - query (0 = absent), in ascending order: an entry's place
+ * is its own index plus the smaller cells of the other vector less the cells both hold below it. Pass 1
+ * visits the positive cells in ascending order, pass 2 the negative ones (FVTable.cpp:129-187); the
+ * reference increments a map iterator after erasing its node, this visits each key present when the
+ * pass starts once. The lanes find all eight neighbours of a cell at once by comparing their keys (one
+ * thread with its vector in local memory took 20 us over a pair, and a lone query waited for it). */
+struct Merged {
     int key[kMaxFv], val[kMaxFv];
-    int m = 0, i = 0;
-    int64_t j = b;
-    bool overflow = false;
-    /* merge (both sorted by cell): db - query */
-    while (i < qn || j < e) {
-        int kc, kv;
-        if (j < e && (i >= qn || fv_cell[j] < qc[i])) {
-            kc = fv_cell[j];
-            kv = fv_cnt[j];
-            j++;
-        } else if (i < qn && (j >= e || qc[i] < fv_cell[j])) {
-            kc = qc[i];
-            kv = -qv[i];
-            i++;
-        } else {
-            kc = qc[i];
-            kv = fv_cnt[j] - qv[i];
-            i++;
-            j++;
-        }
-        if (m >= kMaxFv) {
-            overflow = true;
-            break;
-        }
-        key[m] = kc;
-        val[m] = kv;
-        m++;
+};
+
+__device__ __forceinline__ int count_below(const int32_t* __restrict__ a, int n, int c) {
+    int lo = 0, hi = n;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (a[mid] < c)
+            lo = mid + 1;
+        else
+            hi = mid;
     }
-    if (overflow) {
-        atomicCAS(flag, 0, GAT_ERR_ARG);
-        lb[(size_t)qi * (n + 1) + t] = 0;
-        return;
+    return lo;
+}
+
+__device__ int touching_bound(const int32_t* __restrict__ dc, const int32_t* __restrict__ dv, int dn,
+                              const int32_t* __restrict__ qc, const int32_t* __restrict__ qv, int qn, int vbits, Merged& g,
+                              int32_t* flag) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    int both = 0;
+    for (int i0 = 0; i0 < dn; i0 += 32) {
+        const int i = i0 + lane;
+        int c = 0, v = 0, at = 0;
+        bool dup = false;
+        if (i < dn) {
+            c = dc[i];
+            v = dv[i];
+            at = count_below(qc, qn, c);
+            dup = at < qn && qc[at] == c;
+            if (dup) v -= qv[at];
+        }
+        const unsigned m = __ballot_sync(FULL, dup);
+        const int pos = i + at - both - __popc(m & below);
+        if (i < dn && pos < kMaxFv) {
+            g.key[pos] = c;
+            g.val[pos] = v;
+        }
+        both += __popc(m);
     }
-    int nb[8];
-    for (int a = 0; a < m; a++) {
-        int pv = val[a];
-        if (pv <= 0) continue;
-        fv_neighbors(key[a], vbits, nb);
-        for (int s = 0; s < 8; s++) {
-            int f = find_key(key, m, nb[s]);
-            if (f < 0 || val[f] >= 0) continue;
-            int nv = -val[f];
-            if (pv > nv) {
-                val[a] = pv - nv;
-                val[f] = 0;
-            } else if (pv == nv) {
-                val[a] = 0;
-                val[f] = 0;
-                break;
-            } else {
-                val[f] = -(nv - pv);
-                val[a] = 0;
-                break;
+    const int m = dn + qn - both;
+    if (m > kMaxFv) {
+        if (lane == 0) atomicCAS(flag, 0, GAT_ERR_ARG);
+        return 0;
+    }
+    int seen = 0;
+    for (int j0 = 0; j0 < qn; j0 += 32) {
+        const int j = j0 + lane;
+        int c = 0, at = 0;
+        bool dup = false;
+        if (j < qn) {
+            c = qc[j];
+            at = count_below(dc, dn, c);
+            dup = at < dn && dc[at] == c;
+        }
+        const unsigned d = __ballot_sync(FULL, dup);
+        if (j < qn && !dup) {
+            const int pos = j + at - seen - __popc(d & below);
+            g.key[pos] = c;
+            g.val[pos] = -qv[j];
+        }
+        seen += __popc(d);
+    }
+    __syncwarp();
+    constexpr int kPer = kMaxFv / 32;
+    int key[kPer];
+#pragma unroll
+    for (int k = 0; k < kPer; k++) key[k] = 32 * k + lane < m ? g.key[32 * k + lane] : INT_MIN;
+    /* sign +1: pass 1 (positive cells against negative neighbours), -1: pass 2 */
+    for (int sign = 1; sign >= -1; sign -= 2) {
+        for (int a = 0; a < m; a++) {
+            const int pv = sign * g.val[a];
+            if (pv <= 0) continue; /* the same for all lanes */
+            int left = pv;
+            int nb[8], f[8];
+            fv_neighbors(g.key[a], vbits, nb);
+#pragma unroll
+            for (int s = 0; s < 8; s++) {
+                f[s] = -1;
+#pragma unroll
+                for (int k = 0; k < kPer; k++) {
+                    if (32 * k >= m) break;
+                    const unsigned hit = __ballot_sync(FULL, key[k] == nb[s] && 32 * k + lane < m);
+                    if (hit) f[s] = 32 * k + __ffs(hit) - 1;
+                }
             }
-        }
-    }
-    for (int a = 0; a < m; a++) {
-        if (val[a] >= 0) continue;
-        int nv = -val[a];
-        fv_neighbors(key[a], vbits, nb);
-        for (int s = 0; s < 8; s++) {
-            int f = find_key(key, m, nb[s]);
-            if (f < 0 || val[f] <= 0) continue;
-            int pv = val[f];
-            if (nv > pv) {
-                val[a] = -(nv - pv);
-                val[f] = 0;
-            } else if (pv == nv) {
-                val[a] = 0;
-                val[f] = 0;
-                break;
-            } else {
-                val[f] = pv - nv;
-                val[a] = 0;
-                break;
+#pragma unroll
+            for (int s = 0; s < 8; s++) {
+                if (f[s] < 0 || left == 0) continue;
+                const int nv = -sign * g.val[f[s]];
+                if (nv <= 0) continue;
+                /* against every neighbour the cell stands with its full value, as in the reference */
+                left = max(pv - nv, 0);
+                __syncwarp();
+                if (lane == 0) g.val[f[s]] = -sign * max(nv - pv, 0);
+                __syncwarp();
             }
+            __syncwarp();
+            if (lane == 0) g.val[a] = sign * left;
+            __syncwarp();
         }
     }
     int sp = 0, sn = 0;
-    for (int a = 0; a < m; a++) {
-        if (val[a] > 0) sp += val[a];
-        if (val[a] < 0) sn -= val[a];
+    for (int a = lane; a < m; a += 32) {
+        const int v = g.val[a];
+        sp += max(v, 0);
+        sn += max(-v, 0);
     }
-    lb[(size_t)qi * (n + 1) + t] = max(sp, sn);
+    sp = __reduce_add_sync(FULL, sp);
+    sn = __reduce_add_sync(FULL, sn);
+    __syncwarp();
+    return max(sp, sn);
+}
+
+/* Bounds of 256 trajectories against kBoundQ queries per CTA. A trajectory none of whose cells is in
+ * the query's near set has bound max(its length, query length); its vector is read once for all the
+ * queries. The pairs that touch are listed and dealt to the warps (64 queries over 100k walks: 112 us
+ * with one query per CTA and one thread per pair). */
+constexpr int kBoundQ = 4;
+
+__global__ void __launch_bounds__(kT) k_lower_bounds(int n, int nq, const int64_t* __restrict__ fv_off,
+                                                     const int32_t* __restrict__ fv_cell,
+                                                     const int32_t* __restrict__ fv_cnt, const int32_t* __restrict__ qfv_cell,
+                                                     const int32_t* __restrict__ qfv_cnt, const int32_t* __restrict__ qfv_n,
+                                                     int stride, int vbits, const uint32_t* __restrict__ near, int words,
+                                                     const int32_t* __restrict__ q_len, int32_t* lb, int32_t* flag) {
+    dep_wait();
+    __shared__ int list[kT * kBoundQ], count;
+    if (threadIdx.x == 0) count = 0;
+    __syncthreads();
+    const int q0 = blockIdx.y * kBoundQ, qs = min(kBoundQ, nq - q0);
+    const int t = blockIdx.x * kT + threadIdx.x + 1;
+    if (t <= n) {
+        const int64_t b = fv_off[t], e = fv_off[t + 1];
+        const uint32_t* bm = near + (size_t)q0 * words;
+        unsigned touches = 0;
+        int tlen = 0;
+        for (int64_t j = b; j < e; j++) {
+            const int c = fv_cell[j];
+            tlen += fv_cnt[j];
+            if ((c >> 5) < words)
+#pragma unroll
+                for (int k = 0; k < kBoundQ; k++)
+                    if (k < qs) touches |= ((__ldg(bm + (size_t)k * words + (c >> 5)) >> (c & 31)) & 1u) << k;
+        }
+        for (int k = 0; k < qs; k++) {
+            if ((touches >> k) & 1u)
+                list[atomicAdd(&count, 1)] = threadIdx.x * kBoundQ + k;
+            else
+                lb[(size_t)(q0 + k) * (n + 1) + t] = max(tlen, q_len[q0 + k]);
+        }
+    }
+    __syncthreads();
+    __shared__ Merged merged[kT / 32];
+    const int warp = threadIdx.x >> 5;
+    for (int i = warp; i < count; i += kT / 32) {
+        const int tt = blockIdx.x * kT + list[i] / kBoundQ + 1, qi = q0 + list[i] % kBoundQ;
+        const int64_t b = fv_off[tt];
+        const int v = touching_bound(fv_cell + b, fv_cnt + b, (int)(fv_off[tt + 1] - b), qfv_cell + (size_t)qi * stride,
+                                     qfv_cnt + (size_t)qi * stride, qfv_n[qi], vbits, merged[warp], flag);
+        if ((threadIdx.x & 31) == 0) lb[(size_t)qi * (n + 1) + tt] = v;
+    }
 }
 
 /* ---------------------------------------------------------------- 3. candidate order */
@@ -367,7 +456,8 @@ __global__ void __launch_bounds__(kT) k_lower_bounds(int n, int nq, const int64_
  * their bounds (per-tile histograms laid out bound-major, tile-minor), one exclusive scan over
  * all queries turns them into output positions, and one warp per tile scatters its ids in id
  * order, so equal bounds keep ascending ids: the order is (bound, id). */
-constexpr int kSortTile = 2048;
+constexpr int kSortTile = 4096;
+constexpr int kSortThreads = 512;
 
 __global__ void k_sort_hist(int n, const int32_t* lb, int bins, int ntile, int64_t* H) {
     dep_wait();
@@ -382,19 +472,35 @@ __global__ void k_sort_hist(int n, const int32_t* lb, int bins, int ntile, int64
     for (int v = threadIdx.x; v < bins; v += blockDim.x) H[((size_t)qi * bins + v) * ntile + tile] = hist[v];
 }
 
-/* one warp per (tile, query); the tile's running output offset per bound lives in shared
- * memory (loaded from the scanned histograms), the warp walks its ids in order 32 at a time */
-__global__ void __launch_bounds__(32) k_sort_scatter(int n, const int32_t* lb, int bins, int ntile, const int64_t* H,
-                                                     int32_t* cand, int32_t* slb) {
+/* One CTA per (tile, query), its warps taking consecutive parts of the tile: each warp counts its part's
+ * bounds, a prefix over the warps on top of the scanned histogram gives every warp its first position
+ * per bound, and the warp walks its ids in order 32 at a time. (One warp per tile walked 64 steps of
+ * ballots in sequence: 129 us for 64 queries over 100k walks, 50 us for one.) */
+__global__ void __launch_bounds__(kSortThreads) k_sort_scatter(int n, const int32_t* __restrict__ lb, int bins, int ntile,
+                                                     const int64_t* __restrict__ H, int32_t* cand) {
     dep_wait();
-    extern __shared__ long long run[];
+    extern __shared__ int run[]; /* [warps][bins] */
     const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int tile = blockIdx.x, qi = blockIdx.y;
-    for (int v = lane; v < bins; v += 32) run[v] = H[((size_t)qi * bins + v) * ntile + tile];
-    __syncwarp();
+    for (int i = threadIdx.x; i < nw * bins; i += blockDim.x) run[i] = 0;
+    __syncthreads();
     const int32_t* row = lb + (size_t)qi * (n + 1);
-    const int t0 = 1 + tile * kSortTile, t1 = min(n, (tile + 1) * kSortTile);
+    const int part = (kSortTile / nw + 31) & ~31;
+    const int t0 = 1 + tile * kSortTile + warp * part, t1 = min(min(n, (tile + 1) * kSortTile), t0 + part - 1);
+    int* mine = run + warp * bins;
+    for (int t = t0 + lane; t <= t1; t += 32) atomicAdd(&mine[min(row[t], bins - 1)], 1);
+    __syncthreads();
+    for (int v = threadIdx.x; v < bins; v += blockDim.x) {
+        /* positions fit 32 bits: a batch holds under 2^30 (query, trajectory) pairs (topk_dev) */
+        int at = (int)H[((size_t)qi * bins + v) * ntile + tile];
+        for (int w = 0; w < nw; w++) {
+            const int c = run[w * bins + v];
+            run[w * bins + v] = at;
+            at += c;
+        }
+    }
+    __syncthreads();
     unsigned lt;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
     for (int b = t0; b <= t1; b += 32) {
@@ -403,17 +509,15 @@ __global__ void __launch_bounds__(32) k_sort_scatter(int n, const int32_t* lb, i
         const int v = raw < 0 ? -1 : min(raw, bins - 1);
         const unsigned peers = __match_any_sync(FULL, v);
         const int leader = __ffs(peers) - 1;
-        const int rank = __popc(peers & lt);
-        long long base = 0;
+        int base = 0;
         if (v >= 0 && lane == leader) {
-            base = run[v];
-            run[v] = base + __popc(peers);
+            base = mine[v];
+            mine[v] = base + __popc(peers);
         }
         base = __shfl_sync(FULL, base, leader);
         if (v >= 0) {
-            const int64_t pos = base + rank; /* global position; query qi's slice starts at qi * n */
+            const int64_t pos = base + __popc(peers & lt); /* global position; query qi's slice starts at qi * n */
             cand[pos] = t;
-            slb[pos] = raw;
         }
         __syncwarp();
     }
@@ -438,7 +542,7 @@ __global__ void k_walk_init(int nq, int chunk, int32_t* ws) {
 /* One CTA: each unfinished query extends its evaluated prefix [0, end) of the (bound, id)
  * order by up to `chunk` candidates whose bound is at most W; the new slices are numbered
  * consecutively over the queries (wprefix) for the EDR kernel. */
-__global__ void k_walk_plan(int n, int nq, const int32_t* slb, int32_t* ws, int* wprefix) {
+__global__ void k_walk_plan(int n, int nq, const int32_t* __restrict__ lb, const int32_t* __restrict__ cand, int32_t* ws, int* wprefix) {
     dep_wait();
     __shared__ int warp_sum[32];
     __shared__ int carry;
@@ -456,12 +560,12 @@ __global__ void k_walk_plan(int n, int nq, const int32_t* slb, int32_t* ws, int*
                 int e = (int)min((long long)n, (long long)end + s[WS_CHUNK]);
                 /* candidates with a bound above W can never be needed */
                 int W = s[WS_W];
-                const int32_t* row = slb + (size_t)qi * n;
-                if (e > end && row[e - 1] > W) {
+                const int32_t *row = lb + (size_t)qi * (n + 1), *ids = cand + (size_t)qi * n;
+                if (e > end && row[ids[e - 1]] > W) {
                     int lo = end, hi = e - 1; /* first index in [end, e) with bound > W */
                     while (lo < hi) {
                         int mid = (lo + hi) >> 1;
-                        if (row[mid] > W)
+                        if (row[ids[mid]] > W)
                             hi = mid;
                         else
                             lo = mid + 1;
@@ -509,10 +613,12 @@ struct WalkPairs {
     const int32_t* db_len;
     const int64_t* db_off;
     const float2* DB;
+    const float4* q_box;  /* boxes of the queries' points (k_query_fv) and of the set's */
+    const float4* db_box;
     int32_t* sdist;
     static constexpr int kKind = 1;
     __device__ int count() const { return wprefix[nq]; }
-    __device__ void get(int w, const float2*& a, int& la, const float2*& b, int& lb, int32_t*& o) const {
+    __device__ int query_of(int w) const {
         int lo = 0, hi = nq - 1; /* last q with wprefix[q] <= w */
         while (lo < hi) {
             int mid = (lo + hi + 1) >> 1;
@@ -521,8 +627,18 @@ struct WalkPairs {
             else
                 hi = mid - 1;
         }
-        int q = lo;
-        size_t idx = (size_t)q * n + ws[(size_t)q * WS_WORDS + WS_START] + (w - wprefix[q]);
+        return lo;
+    }
+    __device__ size_t index_of(int w, int q) const {
+        return (size_t)q * n + ws[(size_t)q * WS_WORDS + WS_START] + (w - wprefix[q]);
+    }
+    __device__ bool apart(int w, float u) const {
+        const int q = query_of(w);
+        return edr::boxes_apart(q_box[q], db_box[cand[index_of(w, q)]], u);
+    }
+    __device__ void get(int w, const float2*& a, int& la, const float2*& b, int& lb, int32_t*& o) const {
+        const int q = query_of(w);
+        const size_t idx = index_of(w, q);
         int t = cand[idx];
         a = Q + q_off[q];
         la = q_len[q];
@@ -536,7 +652,7 @@ struct WalkPairs {
  * (nlb, nid) the next candidate: done at the end of the order, when nlb > W, or when nlb == W
  * and k evaluated pairs already sort before (W, nid). While nlb < W the walk goes on: a
  * candidate with a smaller bound may still be closer. */
-__global__ void k_walk_kth(int n, int k, int bins, int growth, const int32_t* slb, const int32_t* cand,
+__global__ void k_walk_kth(int n, int k, int bins, int growth, const int32_t* lb, const int32_t* cand,
                            const int32_t* sdist, int32_t* ws) {
     dep_wait();
     extern __shared__ int hist[];
@@ -602,7 +718,7 @@ __global__ void k_walk_kth(int n, int k, int bins, int growth, const int32_t* sl
     if (end >= n) {
         done = true;
     } else {
-        int nlb = slb[(size_t)qi * n + end];
+        int nlb = lb[(size_t)qi * (n + 1) + cand[(size_t)qi * n + end]];
         if (nlb < W) {
             done = false;
         } else if (nlb > W) {
@@ -649,8 +765,9 @@ __global__ void k_final(int n, int k, int words, uint32_t* gbitmap, const int32_
     for (int w = threadIdx.x; w < words; w += blockDim.x) bm[w] = 0;
     if (threadIdx.x == 0) lt_n = 0;
     __syncthreads();
+#pragma unroll 4
     for (int i = threadIdx.x; i < end; i += blockDim.x) {
-        int d = dist[i], id = ids[i];
+        const int d = dist[i], id = ids[i];
         if (d < W) {
             int slot = atomicAdd(&lt_n, 1);
             if (slot < 1024) lt_keys[slot] = ((unsigned long long)(unsigned)d << 32) | (unsigned)id;
@@ -727,10 +844,10 @@ __global__ void k_final(int n, int k, int words, uint32_t* gbitmap, const int32_
     }
 }
 
-/* device bytes topk_batch needs per query (sorted candidates, bounds, distances, histograms) */
+/* device bytes topk_batch needs per query (bounds, sorted candidates, distances, histograms) */
 size_t topk_bytes_per_query(int n, int bins) {
     int ntile = (n + kSortTile - 1) / kSortTile;
-    return (size_t)(n + 1) * 4 + (size_t)n * 12 + (size_t)bins * ntile * 8 + 64;
+    return (size_t)(n + 1) * 4 + (size_t)n * 8 + (size_t)bins * ntile * 8 + 64;
 }
 
 /* State of one batch between its phases (pointers into the context's scratch). */
@@ -739,7 +856,7 @@ struct TopkRun {
     int nq = 0, n = 0, k = 0, max_q_len = 0;
     float u = 0.f;
     int32_t* lb = nullptr;
-    int32_t *cand = nullptr, *slb = nullptr, *sdist = nullptr, *ws = nullptr;
+    int32_t *cand = nullptr, *sdist = nullptr, *ws = nullptr;
     int* wprefix = nullptr;
     bool lone = false;
     int chunk0 = 0, growth = 0, rounds = 0;
@@ -767,15 +884,17 @@ int topk_pre(gat_ctx* ctx, const gat_index* g, int nq, const int32_t* d_q_len, c
     while (pow2 < max_q_len) pow2 <<= 1;
     /* query FVs */
     size_t fvb = (size_t)nq * stride * 4;
-    char* qfv = (char*)scratch(ctx, S_TOPK_QFV, fvb * 2 + (size_t)nq * 4 + 1024, &st);
+    char* qfv = (char*)scratch(ctx, S_TOPK_QFV, (size_t)nq * 16 + fvb * 2 + (size_t)nq * 4 + 1024, &st);
     if (!qfv) return st;
+    float4* q_box = (float4*)qfv;
+    qfv += (size_t)nq * 16;
     int32_t* qfv_cell = (int32_t*)qfv;
     int32_t* qfv_cnt = (int32_t*)(qfv + fvb);
     int32_t* qfv_n = (int32_t*)(qfv + 2 * fvb);
     size_t smem_fv = (size_t)pow2 * 12;
     allow_smem(k_query_fv, smem_fv);
     (void)launch_dep(ctx, k_query_fv, dim3(std::min(nq, ctx->sm_count * 4)), dim3(512), smem_fv, s, g->grid, nq, d_q_len, d_q_off, d_q_xy, stride, pow2,
-                                                                      qfv_cell, qfv_cnt, qfv_n);
+                                                                      qfv_cell, qfv_cnt, qfv_n, q_box);
     count_launch(ctx);
     /* lower bounds */
     int32_t* lb = (int32_t*)scratch(ctx, S_TOPK_LB, (size_t)nq * (n + 1) * 4, &st);
@@ -785,13 +904,11 @@ int topk_pre(gat_ctx* ctx, const gat_index* g, int nq, const int32_t* d_q_len, c
     int nwords = ((1 << vbits) + 31) / 32;
     uint32_t* near = (uint32_t*)scratch(ctx, S_TOPK_NEAR, (size_t)nq * nwords * 4 + 64, &st);
     if (!near) return st;
-    (void)launch_dep(ctx, k_near_bitmap, dim3(nq), dim3(kT), 0, s, nq, vbits, qfv_cell, qfv_n, stride, nwords, near);
+    (void)launch_dep(ctx, k_near_bitmap, dim3(nq), dim3(1024), 0, s, nq, vbits, qfv_cell, qfv_n, stride, nwords, near);
     count_launch(ctx);
-    size_t smem_lb = (size_t)stride * 8;
-    allow_smem(k_lower_bounds, smem_lb);
-    dim3 lgrid((n + kT - 1) / kT, nq);
+    dim3 lgrid((n + kT - 1) / kT, (nq + kBoundQ - 1) / kBoundQ);
     timed_begin(ctx, GAT_KERNEL_BOUNDS);
-    (void)launch_dep(ctx, k_lower_bounds, dim3(lgrid), dim3(kT), smem_lb, s, n, nq, g->d_fv_off, g->d_fv_cell, g->d_fv_cnt, qfv_cell, qfv_cnt, qfv_n, stride,
+    (void)launch_dep(ctx, k_lower_bounds, dim3(lgrid), dim3(kT), 0, s, n, nq, g->d_fv_off, g->d_fv_cell, g->d_fv_cnt, qfv_cell, qfv_cnt, qfv_n, stride,
                                              vbits, near, nwords, d_q_len, lb, ctx->d_flag);
     /* algorithmic bytes: every trajectory's FV (8 B per entry + 8 B offset) and its bound (4 B)
      * per query */
@@ -802,12 +919,11 @@ int topk_pre(gat_ctx* ctx, const gat_index* g, int nq, const int32_t* d_q_len, c
     int bins_lb = std::max(max_q_len, db->maxlen) + 2;
     int ntile = (n + kSortTile - 1) / kSortTile;
     int64_t* H = (int64_t*)scratch(ctx, S_TOPK_SEG, (size_t)nq * bins_lb * ntile * 8 + 64, &st);
-    char* sorted = (char*)scratch(ctx, S_TOPK_PAIRS, (size_t)nq * n * 12 + 1024, &st);
+    char* sorted = (char*)scratch(ctx, S_TOPK_PAIRS, (size_t)nq * n * 8 + 1024, &st);
     int32_t* ws = (int32_t*)scratch(ctx, S_TOPK_QSTATE, (size_t)nq * WS_WORDS * 4 + (size_t)(nq + 1) * 4 + 256, &st);
     if (!H || !sorted || !ws) return st;
     R.cand = (int32_t*)sorted;
-    R.slb = R.cand + (size_t)nq * n;
-    R.sdist = R.slb + (size_t)nq * n;
+    R.sdist = R.cand + (size_t)nq * n;
     R.ws = ws;
     R.wprefix = (int*)(ws + (size_t)nq * WS_WORDS);
     size_t smem_h = (size_t)bins_lb * 4;
@@ -815,18 +931,20 @@ int topk_pre(gat_ctx* ctx, const gat_index* g, int nq, const int32_t* d_q_len, c
     (void)launch_dep(ctx, k_sort_hist, dim3(dim3(ntile, nq)), dim3(kT), smem_h, s, n, lb, bins_lb, ntile, H);
     count_launch(ctx);
     if ((st = scan_i64(ctx, H, H, (int64_t)nq * bins_lb * ntile)) != GAT_OK) return st;
-    size_t smem_run = (size_t)bins_lb * 8;
+    const int sort_warps = std::max(1, std::min(kSortThreads / 32, (int)((size_t)(160 << 10) / ((size_t)bins_lb * 4))));
+    size_t smem_run = (size_t)sort_warps * bins_lb * 4;
     allow_smem(k_sort_scatter, smem_run);
-    (void)launch_dep(ctx, k_sort_scatter, dim3(dim3(ntile, nq)), dim3(32), smem_run, s, n, lb, bins_lb, ntile, H, R.cand, R.slb);
+    (void)launch_dep(ctx, k_sort_scatter, dim3(dim3(ntile, nq)), dim3(32 * sort_warps), smem_run, s, n, lb, bins_lb, ntile, H, R.cand);
     count_launch(ctx);
     /* the walk: a finished query costs nothing in later rounds and `rounds` covers the whole
      * order with growing chunks. A lone query leaves most of the GPU idle in a small round, so
      * it starts with a larger chunk; every walk doubles its chunk per round, which keeps the
-     * surplus evaluations of the last round small. On the C2 set (100k walks, k = 32), first
-     * rounds of 768 / 1024 / 1280 / 1536 candidates with doubling ran 3.21k / 3.29k / 3.40k /
-     * 3.28k queries per second, quadrupling from 1024 2.9k. */
+     * surplus evaluations of the last round small. Candidates far from the query cost next to nothing
+     * (edr::boxes_apart), so a batch starts with 1024 too: on a set of 100k walks (k = 32), 64 queries
+     * took 945 / 709 / 664 / 626 us with first rounds of 128 / 256 / 512 / 1024 candidates; lone queries
+     * are within 3% of each other from 512 to 2048. */
     R.lone = nq <= 4;
-    R.chunk0 = ctx->topk_chunk ? ctx->topk_chunk : (R.lone ? 1280 : 128);
+    R.chunk0 = ctx->topk_chunk ? ctx->topk_chunk : (R.lone ? 1280 : 1024);
     R.chunk0 = std::max(R.chunk0, R.lone ? 8 * k : 4 * k);
     R.growth = ctx->topk_growth ? ctx->topk_growth : 2;
     R.rounds = 1;
@@ -842,13 +960,13 @@ int topk_pre(gat_ctx* ctx, const gat_index* g, int nq, const int32_t* d_q_len, c
     allow_smem(k_walk_kth, R.smem_d);
     R.rows_hint = std::min(max_q_len, db->maxlen);
     R.max_cols = std::max(max_q_len, db->maxlen);
-    R.src = WalkPairs{n, nq, R.wprefix, ws, R.cand, d_q_len, d_q_off, d_q_xy, db->d_len, db->d_off, db->d_xy, R.sdist};
+    R.src = WalkPairs{n, nq, R.wprefix, ws, R.cand, d_q_len, d_q_off, d_q_xy, db->d_len, db->d_off, db->d_xy, q_box, db->d_box, R.sdist};
     return GAT_OK;
 }
 
 /* Phase 2a: each unfinished query extends its evaluated prefix (pair numbering in wprefix). */
 void topk_plan(gat_ctx* ctx, const TopkRun& R) {
-    (void)launch_dep(ctx, k_walk_plan, dim3(1), dim3(1024), 0, ctx->stream, R.n, R.nq, R.slb, R.ws, R.wprefix);
+    (void)launch_dep(ctx, k_walk_plan, dim3(1), dim3(1024), 0, ctx->stream, R.n, R.nq, R.lb, R.cand, R.ws, R.wprefix);
     count_launch(ctx);
 }
 
@@ -856,7 +974,7 @@ void topk_plan(gat_ctx* ctx, const TopkRun& R) {
 int topk_round(gat_ctx* ctx, const TopkRun& R, int64_t npairs, unsigned long long* cells) {
     int st = edr::edr_launch(ctx, R.src, npairs, R.rows_hint, R.max_cols, R.u, cells);
     if (st != GAT_OK) return st;
-    (void)launch_dep(ctx, k_walk_kth, dim3(R.nq), dim3(kT), R.smem_d, ctx->stream, R.n, R.k, R.bins_d, R.growth, R.slb, R.cand, R.sdist, R.ws);
+    (void)launch_dep(ctx, k_walk_kth, dim3(R.nq), dim3(kT), R.smem_d, ctx->stream, R.n, R.k, R.bins_d, R.growth, R.lb, R.cand, R.sdist, R.ws);
     count_launch(ctx);
     return GAT_OK;
 }
