@@ -1,4 +1,4 @@
-/* Point groups of a Grid or FSG: the structure the trajectory-id range scan reads (range_groups.cu).
+/* Point groups of an index: the structure the trajectory-id range scan reads (range_groups.cu).
  *
  * A group is a maximal run of index positions with one trajectory inside one leaf (Grid) or cell
  * (FSG). Both layouts keep a cell's points sorted by trajectory (Grid::addDatasetToGrid,
@@ -13,9 +13,17 @@
  * list, so that a node inside a query costs its distinct walks instead of its points. The lists
  * follow the groups' trajectories in one array. FSG: the first group of every cell.
  *
+ * STIG: a leaf keeps its points in the order std::sort left them, so its groups are made on a copy of
+ * the coordinates sorted by (leaf, trajectory); a leaf of 10,240 points then is about a hundred boxes.
+ * The index's own arrays stay as the reference lays them out. MortonGrid: its Grid's groups and the
+ * first group of every Morton cell.
+ *
  * Derived like the point boxes (pbox.cu), after a build or a snapshot load, and not part of the
- * snapshot format. On 200M points: about 360 MB (the points take 3.2 GB). When the memory for it
- * is not there the index is left without groups and queries take the point scan. */
+ * snapshot format. A Grid of 200M points: 270 MB beside 3.3 GB, and 2 ms of a 16 ms build (its point
+ * boxes come from the groups, so the pass over the points that made them is gone). When the memory
+ * for it is not there the index is left without groups and queries take the point scan. */
+#include <cub/device/device_radix_sort.cuh>
+
 #include <algorithm>
 
 #include "range_common.cuh"
@@ -38,19 +46,26 @@ __global__ void __launch_bounds__(256) k_heads(int64_t P, const int32_t* __restr
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t w0 = (int64_t)blockIdx.x * (kTile / 32) + warp * kWordsPerWarp;
     int c = 0;
-#pragma unroll 4
+    /* all of the warp's loads in flight at once */
+    int t[kWordsPerWarp];
+#pragma unroll
     for (int w = 0; w < kWordsPerWarp; w++) {
         const int64_t i = (w0 + w) * 32 + lane;
-        const int t = i < P ? __ldg(tid + i) : -1;
-        int prev = __shfl_up_sync(0xffffffffu, t, 1);
-        if (lane == 0) prev = i > 0 && i < P ? __ldg(tid + i - 1) : -1;
-        unsigned word = __ballot_sync(0xffffffffu, i < P && t != prev);
-        if ((w0 + w) * 32 >= P) break;
-        word |= bits[w0 + w];
-        __syncwarp();
-        if (lane == 0) bits[w0 + w] = word;
+        t[w] = i < P ? __ldg(tid + i) : -1;
+    }
+    const unsigned starts = lane < kWordsPerWarp && (w0 + lane) * 32 < P ? bits[w0 + lane] : 0u;
+    int before = w0 > 0 && w0 * 32 <= P ? __ldg(tid + w0 * 32 - 1) : -1; /* the point before the word */
+    unsigned mine = 0;
+#pragma unroll
+    for (int w = 0; w < kWordsPerWarp; w++) {
+        int prev = __shfl_up_sync(0xffffffffu, t[w], 1);
+        if (lane == 0) prev = before;
+        before = __shfl_sync(0xffffffffu, t[w], 31);
+        const unsigned word = __ballot_sync(0xffffffffu, (w0 + w) * 32 + lane < P && t[w] != prev) | __shfl_sync(0xffffffffu, starts, w);
+        if (lane == w) mine = word;
         c += __popc(word);
     }
+    if (lane < kWordsPerWarp && (w0 + lane) * 32 < P) bits[w0 + lane] = mine;
     if (lane == 0) warp_cnt[warp] = c;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -107,10 +122,20 @@ __global__ void __launch_bounds__(128) k_group_boxes(int G, const int32_t* __res
         for (int s = lo; s < hi; s += kStage) {
             const int n = min(kStage, hi - s);
             __syncwarp();
-#pragma unroll 4
-            for (int k = lane; k < n; k += 32) {
-                sx[warp][k] = X[s + k];
-                sy[warp][k] = Y[s + k];
+#pragma unroll
+            for (int k0 = 0; k0 < kStage; k0 += 256) {
+                float x[8], y[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) {
+                    const int k = k0 + 32 * u + lane;
+                    x[u] = k < n ? X[s + k] : 0.f;
+                    y[u] = k < n ? Y[s + k] : 0.f;
+                }
+#pragma unroll
+                for (int u = 0; u < 8; u++) {
+                    sx[warp][k0 + 32 * u + lane] = x[u];
+                    sy[warp][k0 + 32 * u + lane] = y[u];
+                }
             }
             __syncwarp();
             for (int k = max(b, s) - s; k < min(e, s + n) - s; k++) {
@@ -164,7 +189,7 @@ __global__ void k_node_records(GridDev t, int G, const int32_t* __restrict__ gbe
         r.child = t.node_child[j];
         r.ib = r.ie = 0;
         r.pbox = no_points();
-        r.pad = 0;
+        r.aux = 0;
         if (r.child < 0 && t.node_pbeg[j] < t.node_pend[j]) {
             r.ib = group_at(gbeg, G, t.node_pbeg[j]);
             r.ie = group_at(gbeg, G, t.node_pend[j]);
@@ -309,6 +334,60 @@ __global__ void __launch_bounds__(256) k_big_lists(NodeRec* rec, int32_t* ids, u
     }
 }
 
+/* ---------------------------------------------------------------- STIG */
+__global__ void k_leaf_sizes(StigDev t, int64_t* size) {
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < t.nnodes; j += gridDim.x * blockDim.x)
+        size[j] = t.kind[j] ? t.hi[j] - t.lo[j] + 1 : 0;
+}
+
+/* entry e of leaf j: key (j, trajectory) and the point's position; neighbouring leaves share a point, so
+ * there are more entries than points. The leaf's first entry is marked in `bits`. */
+__global__ void k_leaf_entries(StigDev t, const int64_t* __restrict__ off, const int32_t* __restrict__ tid,
+                               unsigned long long* key, int32_t* at, uint32_t* bits) {
+    const int lane = threadIdx.x & 31;
+    for (int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < t.nnodes; j += (gridDim.x * blockDim.x) >> 5) {
+        const int64_t b = off[j], n = off[j + 1] - b;
+        if (n <= 0) continue;
+        if (lane == 0) atomicOr(bits + (b >> 5), 1u << (b & 31));
+        for (int64_t k = lane; k < n; k += 32) {
+            const int p = t.lo[j] + (int)k;
+            key[b + k] = (unsigned long long)j << 32 | (unsigned)tid[p];
+            at[b + k] = p;
+        }
+    }
+}
+
+__global__ void k_regroup(int64_t E, const unsigned long long* __restrict__ key, const int32_t* __restrict__ at,
+                          const float* __restrict__ X, const float* __restrict__ Y, int32_t* tid, float* gx, float* gy) {
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E; e += (int64_t)gridDim.x * blockDim.x) {
+        tid[e] = (int32_t)(key[e] & 0xffffffffull);
+        gx[e] = X[at[e]];
+        gy[e] = Y[at[e]];
+    }
+}
+
+__global__ void k_stig_records(StigDev t, const int64_t* __restrict__ off, int G, const int32_t* __restrict__ gbeg, NodeRec* rec) {
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < t.nnodes; j += gridDim.x * blockDim.x) {
+        NodeRec r;
+        r.mbb = make_float4(t.median[j], 0.f, 0.f, 0.f);
+        r.pbox = make_float4(0.f, 0.f, 0.f, 0.f);
+        r.child = t.left[j];
+        r.ib = r.ie = 0;
+        r.aux = t.right[j] * 2 + t.dim[j];
+        if (t.kind[j]) {
+            r.mbb = t.mbb[j];
+            r.pbox = t.pbox[j];
+            r.child = -1;
+            r.aux = 0;
+            if (off[j] < off[j + 1]) {
+                r.ib = group_at(gbeg, G, (int)off[j]);
+                r.ie = group_at(gbeg, G, (int)off[j + 1]);
+            }
+        }
+        rec[j] = r;
+    }
+}
+
 int blocks_for(const gat_ctx* ctx, int64_t threads, int per = 256) {
     return (int)std::max<int64_t>(1, std::min<int64_t>((threads + per - 1) / per, (int64_t)ctx->sm_count * 16));
 }
@@ -348,9 +427,9 @@ void index_groups_free(gat_index* ix) {
 
 int index_groups(gat_index* ix) {
     gat_ctx* ctx = ix->ctx;
-    const int64_t P = ix->npoints;
-    const bool grid = ix->kind == GAT_INDEX_GRID;
-    if (ctx->device < 0 || P <= 0 || P >= (int64_t)1 << 31 || (!grid && ix->kind != GAT_INDEX_FSG)) return GAT_OK;
+    const bool grid = ix->kind == GAT_INDEX_GRID, stig = ix->kind == GAT_INDEX_STIG, morton = ix->kind == GAT_INDEX_MORTON;
+    if (ctx->device < 0 || ix->npoints <= 0) return GAT_OK;
+    if (morton && ix->base->groups.n == 0) return GAT_OK;
     cudaStream_t s = ctx->stream;
     auto dev = [&](size_t bytes) -> void* {
         void* p = nullptr;
@@ -368,48 +447,107 @@ int index_groups(gat_index* ix) {
         index_groups_free(ix);
         return GAT_OK;
     };
+    if (morton) {
+        GroupsDev g = ix->base->groups;
+        const int ncells = ix->grid.cellnum;
+        int32_t* cell_g = (int32_t*)dev((size_t)(ncells + 1) * 4);
+        if (!cell_g) return without();
+        k_cell_groups<<<blocks_for(ctx, ncells + 1), 256, 0, s>>>(ncells, ix->morton.cbeg, nullptr, g.n, g.gbeg, cell_g);
+        count_launch(ctx);
+        GAT_CUDA_TRY(ctx, cudaGetLastError(), "point groups");
+        GAT_CUDA_TRY(ctx, cudaStreamSynchronize(s), "point groups");
+        g.cell_g = cell_g;
+        ix->groups = g;
+        return GAT_OK;
+    }
     Temp tmp(ctx);
+    GroupsDev g;
+    int64_t P = ix->npoints; /* entries to group */
+    const int32_t* tid = ix->d_tid;
+    int64_t* leaf_off = nullptr;
+    g.X = ix->d_x;
+    g.Y = ix->d_y;
+    if (stig) {
+        if (int st = index_point_boxes(ix)) return st;
+        const int n = ix->stig.nnodes;
+        leaf_off = tmp.get<int64_t>((size_t)n + 1);
+        if (!leaf_off) return without();
+        k_leaf_sizes<<<blocks_for(ctx, n), 256, 0, s>>>(ix->stig, leaf_off);
+        if (int st = scan_i64(ctx, leaf_off, leaf_off, n)) return st;
+        GAT_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_pinned, leaf_off + n, 8, cudaMemcpyDeviceToHost, s), "point groups");
+        GAT_CUDA_TRY(ctx, cudaStreamSynchronize(s), "point groups");
+        P = ctx->h_pinned[0];
+    }
+    if (P >= (int64_t)1 << 31) return without();
     const int64_t words = (P + 31) / 32, tiles = (P + kTile - 1) / kTile;
     uint32_t* bits = tmp.get<uint32_t>(words);
     int64_t* off = tmp.get<int64_t>(tiles + 1);
     if (!bits || !off) return without();
     GAT_CUDA_TRY(ctx, cudaMemsetAsync(bits, 0, words * 4, s), "point groups");
-    if (grid)
+    if (stig) {
+        const int n = ix->stig.nnodes;
+        auto* key = tmp.get<unsigned long long>(P);
+        auto* key_s = tmp.get<unsigned long long>(P);
+        int32_t* at = tmp.get<int32_t>(P);
+        int32_t* at_s = tmp.get<int32_t>(P);
+        int32_t* etid = tmp.get<int32_t>(P);
+        float* gx = (float*)dev((size_t)P * 4);
+        float* gy = gx ? (float*)dev((size_t)P * 4) : nullptr;
+        if (!key || !key_s || !at || !at_s || !etid || !gy) return without();
+        k_leaf_entries<<<blocks_for(ctx, (int64_t)n * 32), 256, 0, s>>>(ix->stig, leaf_off, ix->d_tid, key, at, bits);
+        int nbits = 32;
+        while (nbits < 63 && ((int64_t)n >> (nbits - 32))) nbits++;
+        size_t need = 0;
+        GAT_CUDA_TRY(ctx, cub::DeviceRadixSort::SortPairs(nullptr, need, key, key_s, at, at_s, P, 0, nbits, s), "point groups");
+        void* t = tmp.get<char>(need);
+        if (!t) return without();
+        GAT_CUDA_TRY(ctx, cub::DeviceRadixSort::SortPairs(t, need, key, key_s, at, at_s, P, 0, nbits, s), "point groups");
+        k_regroup<<<blocks_for(ctx, P), 256, 0, s>>>(P, key_s, at_s, ix->d_x, ix->d_y, etid, gx, gy);
+        count_launch(ctx, 3 + 2 * ((nbits + 7) / 8));
+        tid = etid;
+        g.X = gx;
+        g.Y = gy;
+    } else if (grid) {
         k_leaf_starts<<<blocks_for(ctx, ix->grid.nnodes), 256, 0, s>>>(ix->grid.nnodes, ix->grid.node_child, ix->grid.node_pbeg,
                                                                        ix->grid.node_pend, bits);
-    else
+    } else {
         k_leaf_starts<<<blocks_for(ctx, ix->fsg.cellnum), 256, 0, s>>>(ix->fsg.cellnum, nullptr, ix->fsg.cbeg, ix->fsg.cend, bits);
-    k_heads<<<(unsigned)tiles, 256, 0, s>>>(P, ix->d_tid, bits, off);
+    }
+    k_heads<<<(unsigned)tiles, 256, 0, s>>>(P, tid, bits, off);
     if (int st = scan_i64(ctx, off, off, tiles)) return st;
-    int64_t total = 0;
     GAT_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_pinned, off + tiles, 8, cudaMemcpyDeviceToHost, s), "point groups");
     GAT_CUDA_TRY(ctx, cudaStreamSynchronize(s), "point groups");
-    total = ctx->h_pinned[0];
+    const int64_t total = ctx->h_pinned[0];
     const int G = (int)total;
-    /* room for the node lists: each level holds at most as many ids as the one below, in practice
+    /* room for a Grid's node lists: each level holds at most as many ids as the one below, in practice
      * half as many until the nodes outgrow the walks; a node that does not fit goes without */
     const int64_t cap = std::min<int64_t>(grid ? total + total * 3 / 2 + 4096 : total, ((int64_t)1 << 31) - 2);
     int32_t* gbeg = (int32_t*)dev((size_t)(total + 1) * 4);
     int32_t* ids = gbeg ? (int32_t*)dev((size_t)cap * 4) : nullptr;
     float4* gbox = ids ? (float4*)dev((size_t)total * 16) : nullptr;
     if (!gbox) return without();
-    k_groups<<<(unsigned)tiles, 256, 0, s>>>(P, ix->d_tid, bits, off, gbeg, ids);
-    const int32_t end = (int32_t)P;
-    GAT_CUDA_TRY(ctx, cudaMemcpyAsync(gbeg + total, &end, 4, cudaMemcpyHostToDevice, s), "point groups");
-    k_group_boxes<<<blocks_for(ctx, total, 128), 128, 0, s>>>(G, gbeg, ix->d_x, ix->d_y, gbox);
+    k_groups<<<(unsigned)tiles, 256, 0, s>>>(P, tid, bits, off, gbeg, ids);
+    ctx->h_pinned[2] = P; /* the low word closes gbeg */
+    GAT_CUDA_TRY(ctx, cudaMemcpyAsync(gbeg + total, ctx->h_pinned + 2, 4, cudaMemcpyHostToDevice, s), "point groups");
+    k_group_boxes<<<blocks_for(ctx, total, 128), 128, 0, s>>>(G, gbeg, g.X, g.Y, gbox);
     count_launch(ctx, 4);
-    GroupsDev g;
     g.n = G;
     g.gbeg = gbeg;
     g.ids = ids;
     g.gbox = gbox;
-    if (!grid) {
+    if (ix->kind == GAT_INDEX_FSG) {
         int32_t* cell_g = (int32_t*)dev((size_t)(ix->fsg.cellnum + 1) * 4);
         if (!cell_g) return without();
         k_cell_groups<<<blocks_for(ctx, ix->fsg.cellnum + 1), 256, 0, s>>>(ix->fsg.cellnum, ix->fsg.cbeg, ix->fsg.cend, G, gbeg,
                                                                           cell_g);
         count_launch(ctx);
         g.cell_g = cell_g;
+    } else if (stig) {
+        NodeRec* rec = (NodeRec*)dev((size_t)ix->stig.nnodes * sizeof(NodeRec));
+        if (!rec) return without();
+        k_stig_records<<<blocks_for(ctx, ix->stig.nnodes), 256, 0, s>>>(ix->stig, leaf_off, G, gbeg, rec);
+        count_launch(ctx);
+        g.rec = rec;
     } else {
         const int n = ix->grid.nnodes, levels = ix->grid.total_level + 1;
         NodeRec* rec = (NodeRec*)dev((size_t)n * sizeof(NodeRec));
@@ -423,11 +561,11 @@ int index_groups(gat_index* ix) {
         }
         k_node_records<<<blocks_for(ctx, n), 256, 0, s>>>(ix->grid, G, gbeg, gbox, rec, ix->d_pbox);
         /* level l is [level[l], level[l + 1]); the root is level 0 */
-        ctx->h_pinned[2] = total;
+        ctx->h_pinned[3] = 1;
+        ctx->h_pinned[4] = total;
         GAT_CUDA_TRY(ctx, cudaMemsetAsync(level, 0, (size_t)(levels + 3) * 4, s), "point groups");
-        const int one = 1;
-        GAT_CUDA_TRY(ctx, cudaMemcpyAsync(level + 1, &one, 4, cudaMemcpyHostToDevice, s), "point groups");
-        GAT_CUDA_TRY(ctx, cudaMemcpyAsync(cursor, ctx->h_pinned + 2, 8, cudaMemcpyHostToDevice, s), "point groups");
+        GAT_CUDA_TRY(ctx, cudaMemcpyAsync(level + 1, ctx->h_pinned + 3, 4, cudaMemcpyHostToDevice, s), "point groups");
+        GAT_CUDA_TRY(ctx, cudaMemcpyAsync(cursor, ctx->h_pinned + 4, 8, cudaMemcpyHostToDevice, s), "point groups");
         for (int l = 0; l + 1 < levels; l++)
             k_next_level<<<blocks_for(ctx, n, 1024), 256, 0, s>>>(l, ix->grid.node_child, level);
         constexpr size_t kBigSmem = (size_t)(2 * kNodeIds + kNodeIds) * 4;
@@ -445,9 +583,9 @@ int index_groups(gat_index* ix) {
         if (!jump) return without();
         GAT_CUDA_TRY(ctx, cudaMemsetAsync(big + n, 0, 4, s), "point groups");
         k_jump<<<16, 256, 0, s>>>(g.jump_level, rec, jump, big + n);
-        GAT_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_pinned + 3, big + n, 4, cudaMemcpyDeviceToHost, s), "point groups");
+        GAT_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_pinned + 5, big + n, 4, cudaMemcpyDeviceToHost, s), "point groups");
         GAT_CUDA_TRY(ctx, cudaStreamSynchronize(s), "point groups");
-        if ((int32_t)ctx->h_pinned[3] == 0) g.jump = jump;
+        if (*reinterpret_cast<int32_t*>(ctx->h_pinned + 5) == 0) g.jump = jump;
         count_launch(ctx, 2 + levels * 3);
         ix->grid.node_pbox = ix->d_pbox;
         g.rec = rec;

@@ -74,14 +74,14 @@ struct MortonDev {
     const int32_t* cbeg;
 };
 
-/* Point groups (groups.cu): the runs of one trajectory inside one leaf (Grid) or cell (FSG). Group g
- * is trajectory ids[g], positions [gbeg[g], gbeg[g + 1]), box gbox[g]. */
+/* Point groups (groups.cu): the runs of one trajectory inside one leaf (Grid, STIG) or cell (FSG). Group
+ * g is trajectory ids[g], positions [gbeg[g], gbeg[g + 1]) of X / Y, box gbox[g]. */
 struct NodeRec {
-    float4 mbb;  /* the node's box */
+    float4 mbb;  /* the node's box (STIG inner node: x = the median) */
     float4 pbox; /* exact box of its points */
-    int child;   /* first child, -1 for a leaf */
+    int child;   /* first child (STIG: the left one), -1 for a leaf */
     int ib, ie;  /* a leaf's groups, or an inner node's distinct trajectories in ids (ib -1: no list) */
-    int pad;
+    int aux;     /* STIG inner node: (right child << 1) | split dimension */
 };
 constexpr int kNodeIds = 4096; /* distinct trajectories of a node that keeps a list */
 struct GroupsDev {
@@ -89,8 +89,10 @@ struct GroupsDev {
     const int32_t* gbeg = nullptr;   /* [n + 1] */
     const int32_t* ids = nullptr;    /* [n] group trajectories, then the node lists */
     const float4* gbox = nullptr;    /* [n] */
-    const NodeRec* rec = nullptr;    /* Grid: per node */
-    const int32_t* cell_g = nullptr; /* FSG: first group of every cell, [cellnum + 1] */
+    const float* X = nullptr;        /* the groups' points: the index's own, or a STIG's regrouped copy */
+    const float* Y = nullptr;
+    const NodeRec* rec = nullptr;    /* Grid, STIG: per node */
+    const int32_t* cell_g = nullptr; /* FSG, MortonGrid: first group at or after every cell, [cells + 1] */
     /* Grid: the node covering each of the 2^jump_level x 2^jump_level equal squares (row-major from
      * the upper left): the node of level jump_level there, or the leaf above it */
     const int32_t* jump = nullptr;
@@ -258,9 +260,9 @@ void* host_stage(gat_ctx* ctx, size_t bytes, int* status);
  * range walks can mark candidate ranges whose every point is a hit (pbox.cu). Called after a
  * Grid or STIG is built or loaded on a device context; a no-op for other kinds. */
 int index_point_boxes(gat_index* ix);
-/* Derives the point groups of a Grid (with its nodes' point boxes) or FSG for the id range scan
- * (groups.cu); called after a build or load on a device context. Leaves the index without groups
- * when there is no memory for them. */
+/* Derives the point groups of a Grid (with its nodes' point boxes), STIG or FSG for the id range scan
+ * (groups.cu), or points a MortonGrid at its Grid's; called after a build or load on a device context.
+ * Leaves the index without groups when there is no memory for them. */
 int index_groups(gat_index* ix);
 void index_groups_free(gat_index* ix);
 /* Batched id-set queries over an index with groups (range_groups.cu): per-query segments of `arena`

@@ -130,6 +130,10 @@ int gat_morton_grid_build(gat_ctx* ctx, const gat_index* grid, gat_index** out) 
         gat_index_destroy(ix);
         return st;
     }
+    if ((st = index_groups(ix)) != GAT_OK) {
+        gat_index_destroy(ix);
+        return st;
+    }
     *out = ix;
     return GAT_OK;
 }

@@ -18,8 +18,8 @@
  *                  de-duplicates.
  *   3. offsets     scan of per-query result counts; one CTA per query copies its segment.
  * Plain execution runs the same pipeline once per query.
- * Batched id sets of an index with point groups (a Grid or FSG) take range_groups.cu instead; this
- * pipeline serves point lists, STIG, the MortonGrid and the queries that outgrow that kernel's sets.
+ * Batched id sets of an index with point groups take range_groups.cu instead; this pipeline serves
+ * point lists, indexes without groups and the queries that outgrow that kernel's sets.
  */
 #include <algorithm>
 #include <climits>

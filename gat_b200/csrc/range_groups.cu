@@ -1,8 +1,8 @@
-/* Batched trajectory-id range queries over point groups (groups.cu), Grid and FSG.
+/* Batched trajectory-id range queries over point groups (groups.cu).
  *
  * A query's candidates are the reference's: the leaves the quadtree walk takes (BoxIntersect,
- * Grid.cpp:428-446), or the cells of the candidate rectangle (FSG.cpp:183-262). Their points are not
- * scanned one by one:
+ * Grid.cpp:428-446, MortonGrid.cpp:356-393) or the median slabs and leaf boxes select (STIG.cpp:179-252),
+ * or the cells of the candidate rectangle (FSG.cpp:183-262). Their points are not scanned one by one:
  *   - a node inside the query (by its box and the exact box of its points), or the FSG cells strictly
  *     inside the candidate rectangle, have every point in the query: their ids are taken as they
  *     are, a node's from its list of distinct trajectories;
@@ -24,6 +24,7 @@
 #include <climits>
 #include <cmath>
 
+#include "cells.cuh"
 #include "launch.cuh"
 #include "range_common.cuh"
 
@@ -189,6 +190,91 @@ __device__ void walk_grid(const GroupsDev& g, const GridDev& tree, const Box& q,
             const NodeRec r = rec[t.front[cur * FRONT + (k >> 2)] + (k & 3)];
             if (box_intersect(q, Box{r.mbb.x, r.mbb.y, r.mbb.z, r.mbb.w}))
                 classify(r, t.front + (cur ^ 1) * FRONT, t.nfront + (cur ^ 1));
+        }
+        t.sync();
+        if (me == 0) t.nfront[cur] = 0;
+    }
+}
+
+/* STIG::searchNode (STIG.cpp:201-252), one level at a time: an inner node sends the walk left and right
+ * by its median (intersectBlock, STIG.cpp:340-347), a leaf is taken when BoxIntersect(its box, query). */
+template <class T>
+__device__ void walk_stig(const NodeRec* __restrict__ rec, const Box& q, T& t, int me) {
+    if (me == 0) {
+        t.front[0] = 0;
+        t.nfront[0] = 1;
+    }
+    t.sync();
+    for (int cur = 0;; cur ^= 1) {
+        const int n = min(t.nfront[cur], T::FRONT);
+        const bool lost = *(volatile int*)t.ovf != 0;
+        t.sync();
+        if (n == 0 || lost) break;
+        int* out = t.front + (cur ^ 1) * T::FRONT;
+        auto push = [&](int nd) {
+            const int k = atomicAdd(t.nfront + (cur ^ 1), 1);
+            if (k < T::FRONT)
+                out[k] = nd;
+            else
+                *t.ovf = 1;
+        };
+        for (int k = me; k < n; k += T::NTHREADS) {
+            const NodeRec r = rec[t.front[cur * T::FRONT + k]];
+            if (r.child < 0) {
+                if (box_intersect(Box{r.mbb.x, r.mbb.y, r.mbb.z, r.mbb.w}, q)) put_item(t, r.ib, r.ie, !pbox_inside(q, r.pbox));
+                continue;
+            }
+            const float lo = r.aux & 1 ? q.ymin : q.xmin, hi = r.aux & 1 ? q.ymax : q.xmax, med = r.mbb.x;
+            if (!(hi < 0.0f) && !(lo > med)) push(r.child);
+            if (!(hi < med) && !(lo > 180.0f)) push(r.aux >> 1);
+        }
+        t.sync();
+        if (me == 0) t.nfront[cur] = 0;
+    }
+}
+
+/* The implicit quadtree of the MortonGrid (morton_walk in range.cu): frontier entries pack
+ * (id << 4) | level. The groups of what it takes are tested by their boxes, whole subtrees included
+ * (their points may lie a rounding outside the computed boxes). */
+template <class T>
+__device__ void walk_morton(const MortonDev& m, const int32_t* __restrict__ cell_g, const Box& q, T& t, int me) {
+    auto emit = [&](int level, uint32_t id) {
+        const uint32_t span = 1u << (2 * (m.total_level - level));
+        put_item(t, cell_g[id * span], cell_g[id * span + span], true);
+    };
+    auto leaf = [&](int level, uint32_t id) {
+        const uint64_t idx = (((uint64_t)1 << (2 * level)) - 1) / 3 + id;
+        return (__ldg(m.leaf + (idx >> 5)) >> (idx & 31)) & 1u;
+    };
+    if (me == 0) {
+        if (leaf(0, 0))
+            emit(0, 0);
+        else
+            t.nfront[0] = 1, t.front[0] = 0;
+    }
+    t.sync();
+    for (int cur = 0;; cur ^= 1) {
+        const int n = min(t.nfront[cur], T::FRONT);
+        const bool lost = *(volatile int*)t.ovf != 0;
+        t.sync();
+        if (n == 0 || lost) break;
+        for (int k = me; k < 4 * n; k += T::NTHREADS) {
+            const uint32_t e = (uint32_t)t.front[cur * T::FRONT + (k >> 2)];
+            const int level = (int)(e & 15u) + 1;
+            const uint32_t id = ((e >> 4) << 2) + (k & 3), span = 1u << (2 * (m.total_level - level));
+            const float4 a = morton_cell_box(m.rxmin, m.rymax, m.cell, (int)(id * span));
+            const float4 b = morton_cell_box(m.rxmin, m.rymax, m.cell, (int)(id * span + span - 1));
+            const float4 box = make_float4(a.x, b.y, b.z, a.w);
+            if (!box_intersect(q, Box{box.x, box.y, box.z, box.w})) continue;
+            if (leaf(level, id) || box_inside(q, box)) {
+                emit(level, id);
+                continue;
+            }
+            const int o = atomicAdd(t.nfront + (cur ^ 1), 1);
+            if (o < T::FRONT)
+                t.front[(cur ^ 1) * T::FRONT + o] = (int)((id << 4) | (uint32_t)level);
+            else
+                *t.ovf = 1;
         }
         t.sync();
         if (me == 0) t.nfront[cur] = 0;
@@ -499,9 +585,8 @@ struct GroupQuery {
     const gat_mbb* queries;
     GridDev grid;
     FsgDev fsg;
+    MortonDev morton;
     GroupsDev g;
-    const float* X;
-    const float* Y;
     uint32_t* arena;
     int64_t cap;
     /* [0] arena cursor, [1] work bytes, [2] big queries taken, [3] queries for the bitmap scan, [4] small
@@ -521,6 +606,10 @@ __device__ bool answer(const GroupQuery& a, int qi, T& t, OpenGroups& og, int me
     const Box q = load_box(a.queries, qi);
     if (KIND == GAT_INDEX_GRID)
         walk_grid(a.g, a.grid, q, t, me);
+    else if (KIND == GAT_INDEX_STIG)
+        walk_stig(a.g.rec, q, t, me);
+    else if (KIND == GAT_INDEX_MORTON)
+        walk_morton(a.morton, a.g.cell_g, q, t, me);
     else
         walk_fsg(a.fsg, a.g.cell_g, q, t, me);
     const int n = min(*t.nitems, T::ITEMS);
@@ -533,7 +622,7 @@ __device__ bool answer(const GroupQuery& a, int qi, T& t, OpenGroups& og, int me
             if ((me & 31) == 0) k = atomicAdd(t.next, per);
             k = __shfl_sync(0xffffffffu, k, 0);
             if (k >= n) break;
-            take_items(t.items + k, min(per, n - k), q, a.g.ids, a.g.gbeg, a.g.gbox, a.X, a.Y, t, og, bytes);
+            take_items(t.items + k, min(per, n - k), q, a.g.ids, a.g.gbeg, a.g.gbox, a.g.X, a.g.Y, t, og, bytes);
         }
     }
     t.sync();
@@ -656,15 +745,18 @@ constexpr int kBins = 3 * kBuckets;
  * number of cells a walk has groups in, range_groups_launch). Grid: D from the list of the smallest
  * node around the query's centre that is no smaller than it, or the largest one with a list; the
  * bucket from the last node of that descent. FSG: D from the groups in the query's middle row of
- * cells, the bucket from its first cell. */
+ * cells, the bucket from its first cell. MortonGrid: D from the groups of the cells of a square about
+ * as large as the query around its centre. STIG: the groups of the leaf at the query's lower corner,
+ * times how often the query covers that leaf's sides. */
 template <int KIND>
-__global__ void k_order_class(const gat_mbb* queries, int nq, GroupsDev g, FsgDev f, float reach, int* __restrict__ hist,
+__global__ void k_order_class(const gat_mbb* queries, int nq, GroupsDev g, GridDev tree, FsgDev f, float reach, int* __restrict__ hist,
                               int* __restrict__ bin) {
     const int qi = blockIdx.x * blockDim.x + threadIdx.x;
     if (qi >= nq) return;
     const Box q = load_box(queries, qi);
     const float w = q.xmax - q.xmin, h = q.ymax - q.ymin;
     float density = 0.f; /* walks per unit area */
+    float est = -1.f;
     int at = 0;          /* a group near the query's first one */
     if (KIND == GAT_INDEX_GRID) {
         const float cx = q.xmin + 0.5f * w, cy = q.ymin + 0.5f * h;
@@ -682,6 +774,28 @@ __global__ void k_order_class(const gat_mbb* queries, int nq, GroupsDev g, FsgDe
             r = g.rec[r.child + c];
         }
         at = max(r.ib, 0);
+    } else if (KIND == GAT_INDEX_STIG) {
+        NodeRec r = g.rec[0];
+        for (int guard = 0; guard < 64 && r.child >= 0; guard++) {
+            const float lo = r.aux & 1 ? q.ymin : q.xmin;
+            r = g.rec[!(lo > r.mbb.x) ? r.child : r.aux >> 1];
+        }
+        at = max(r.ib, 0);
+        const float kw = w / fmaxf(r.mbb.z - r.mbb.x, 1e-30f), kh = h / fmaxf(r.mbb.w - r.mbb.y, 1e-30f);
+        est = (float)(r.ie - r.ib) * fmaxf(kw, 1.f) * fmaxf(kh, 1.f);
+    } else if (KIND == GAT_INDEX_MORTON) {
+        /* level whose squares are just larger than the query */
+        const float side = fmaxf(fmaxf(w, h), tree.cell);
+        int l = tree.total_level;
+        while (l > 0 && tree.cell * (float)(1 << (tree.total_level - l)) < side) l--;
+        const int cells = 1 << (tree.total_level - l), n = 1 << l;
+        const float inv = 1.f / (tree.cell * (float)cells);
+        const int x = min(n - 1, max(0, (int)fminf((q.xmin + 0.5f * w - tree.rxmin) * inv, 1e6f)));
+        const int y = min(n - 1, max(0, (int)fminf((tree.rymax - q.ymin - 0.5f * h) * inv, 1e6f)));
+        const uint32_t id = spread_bits((uint32_t)x) | (spread_bits((uint32_t)y) << 1), span = (uint32_t)cells * (uint32_t)cells;
+        const float c = tree.cell + reach;
+        at = g.cell_g[id * span];
+        density = (float)(g.cell_g[id * span + span] - at) / ((float)span * c * c);
     } else {
         const int g1 = max((int)__fdiv_rn(__fsub_rn(q.xmin, f.rxmin), f.cell), 0);
         const int g2 = min((int)__fdiv_rn(__fsub_rn(q.xmax, f.rxmin), f.cell), f.nx - 1);
@@ -694,7 +808,7 @@ __global__ void k_order_class(const gat_mbb* queries, int nq, GroupsDev g, FsgDe
             density = (float)(g.cell_g[row + g2 + 1] - at) / ((float)(g2 - g1 + 1) * c * c);
         }
     }
-    const float est = density * (w + reach) * (h + reach);
+    if (KIND != GAT_INDEX_STIG) est = density * (w + reach) * (h + reach);
     const int cls = est <= kSmallMax ? 0 : est <= kMidMax ? 1 : 2; /* NaN: big */
     const int b = cls * kBuckets + (int)min((long long)kBuckets - 1, (long long)at * kBuckets / (g.n + 1));
     bin[qi] = b;
@@ -746,14 +860,20 @@ __global__ void k_order(int nq, const int* __restrict__ bin, int* __restrict__ b
 int range_groups_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, uint32_t* arena, int64_t cap,
                         unsigned long long* ctr, int64_t* segbase, int64_t* segcnt, int* ovf_list, bool timed) {
     cudaStream_t s = ctx->stream;
-    const bool grid = ix->kind == GAT_INDEX_GRID;
-    auto kernel = grid ? k_range_groups<GAT_INDEX_GRID> : k_range_groups<GAT_INDEX_FSG>;
+    auto kernel = ix->kind == GAT_INDEX_GRID     ? k_range_groups<GAT_INDEX_GRID>
+                  : ix->kind == GAT_INDEX_STIG   ? k_range_groups<GAT_INDEX_STIG>
+                  : ix->kind == GAT_INDEX_MORTON ? k_range_groups<GAT_INDEX_MORTON>
+                                                 : k_range_groups<GAT_INDEX_FSG>;
+    auto classify = ix->kind == GAT_INDEX_GRID     ? k_order_class<GAT_INDEX_GRID>
+                    : ix->kind == GAT_INDEX_STIG   ? k_order_class<GAT_INDEX_STIG>
+                    : ix->kind == GAT_INDEX_MORTON ? k_order_class<GAT_INDEX_MORTON>
+                                                   : k_order_class<GAT_INDEX_FSG>;
     allow_smem(kernel, kSmem);
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kNT, kSmem);
     const int full = std::max(1, per_sm) * ctx->sm_count;
     GAT_CUDA_TRY(ctx, cudaMemsetAsync(ctr, 0, 8 * sizeof(unsigned long long), s), "range");
-    GroupQuery a{d_q, ix->grid, ix->fsg, ix->groups, ix->d_x, ix->d_y, arena, cap, ctr, segbase, segcnt, nullptr, ovf_list,
+    GroupQuery a{d_q, ix->grid, ix->fsg, ix->morton, ix->groups, arena, cap, ctr, segbase, segcnt, nullptr, ovf_list,
                  timed ? ctr + 1 : nullptr};
     if (nq <= std::min(full, kDirectMax)) {
         /* no more queries than resident CTAs: one each */
@@ -773,10 +893,9 @@ int range_groups_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, i
     int* list = bin + nq;
     const int tb = (nq + 255) / 256;
     GAT_CUDA_TRY(ctx, cudaMemsetAsync(hist, 0, kBins * 4, s), "range");
-    const float cell = grid ? ix->grid.cell : ix->fsg.cell;
+    const float cell = ix->kind == GAT_INDEX_STIG ? 0.f : ix->kind == GAT_INDEX_FSG ? ix->fsg.cell : ix->grid.cell;
     const float reach = cell * (std::sqrt(std::max(1.f, (float)ix->groups.n / (float)std::max(1, ix->db->n))) - 1.f);
-    (grid ? k_order_class<GAT_INDEX_GRID> : k_order_class<GAT_INDEX_FSG>)<<<tb, 256, 0, s>>>(d_q, nq, ix->groups, ix->fsg, reach,
-                                                                                          hist, bin);
+    classify<<<tb, 256, 0, s>>>(d_q, nq, ix->groups, ix->grid, ix->fsg, reach, hist, bin);
     k_order_scan<<<1, 1024, 0, s>>>(hist, counts);
     k_order<<<tb, 256, 0, s>>>(nq, bin, hist, list);
     kernel<<<full, kNT, kSmem, s>>>(a, list, counts, nq);

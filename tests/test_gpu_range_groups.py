@@ -63,6 +63,13 @@ def test_odd_rectangles(gpu_ctx, cell, cap):
         assert np.array_equal(r.offsets, off) and np.array_equal(r.tids, ids)
     _same(gpu_ctx, g, q)  # NaN and infinite rectangles too: the two paths agree
     _same(gpu_ctx, f, q[~np.isinf(q).any(1)])
+    _same(gpu_ctx, G.MortonGrid(g), q)
+    for block in (2, 64, 5000):
+        s = G.STIG(gpu_ctx, db, block)
+        _same(gpu_ctx, s, q)
+        off, ids = po.OracleSTIG(t, block).range(q[finite], 0)
+        r = s.range_query(q[finite])
+        assert np.array_equal(r.offsets, off) and np.array_equal(r.tids, ids)
 
 
 @pytest.mark.parametrize("nq", [1, 31, 444, 445, 1024, 1025, 3001])
@@ -70,8 +77,9 @@ def test_batch_sizes(gpu_ctx, nq):
     t = D.walks(D.lengths(20_000, 0, 0, 0, 20, 200, 32), 32)
     db = G.TrajectorySet(gpu_ctx, t)
     q = D.boxes(nq, 1, 0.001, 0.3, 33)
-    _same(gpu_ctx, G.Grid(gpu_ctx, db, D.BOX, 0.005, 2, 512), q)
-    _same(gpu_ctx, G.FSG(gpu_ctx, db, D.BOX, 0.005), q)
+    g = G.Grid(gpu_ctx, db, D.BOX, 0.005, 2, 512)
+    for ix in (g, G.FSG(gpu_ctx, db, D.BOX, 0.005), G.MortonGrid(g), G.STIG(gpu_ctx, db, 1000)):
+        _same(gpu_ctx, ix, q)
 
 
 def test_clustered_set(gpu_ctx):
@@ -89,7 +97,8 @@ def test_clustered_set(gpu_ctx):
     c = rng.uniform([121.295, 31.095], [121.325, 31.125], (900, 2))
     h = np.exp(rng.uniform(np.log(0.0005), np.log(0.02), (900, 2)))
     q = np.concatenate([np.concatenate([c - h, c + h], 1), D.boxes(600, 1, 0.001, 0.05, 35)]).astype(np.float32)
-    for ix in (G.Grid(gpu_ctx, db, D.BOX, 0.002, 2, 512), G.FSG(gpu_ctx, db, D.BOX, 0.002)):
+    g = G.Grid(gpu_ctx, db, D.BOX, 0.002, 2, 512)
+    for ix in (g, G.FSG(gpu_ctx, db, D.BOX, 0.002), G.MortonGrid(g), G.STIG(gpu_ctx, db, 1024)):
         r = _same(gpu_ctx, ix, q)
         assert int(np.diff(r.offsets).max()) > 4096  # beyond the largest set
         _same(gpu_ctx, ix, q[:200])
@@ -100,15 +109,16 @@ def test_tiny_sets_and_fine_cells(gpu_ctx):
         t = D.walks(D.lengths(n, 0, 0, 0, lo, hi, 36), 36)
         db = G.TrajectorySet(gpu_ctx, t)
         q = np.concatenate([D.boxes(500, 1, 0.0005, 0.5, 37), _odd_rectangles(t, 0.01, 38)[:600]])
-        _same(gpu_ctx, G.Grid(gpu_ctx, db, D.BOX, cell, 2, 512), q)
-        _same(gpu_ctx, G.FSG(gpu_ctx, db, D.BOX, cell), q)
+        g = G.Grid(gpu_ctx, db, D.BOX, cell, 2, 512)
+        for ix in (g, G.FSG(gpu_ctx, db, D.BOX, cell), G.MortonGrid(g), G.STIG(gpu_ctx, db, 16)):
+            _same(gpu_ctx, ix, q)
 
 
 def test_snapshot_keeps_groups(gpu_ctx, tmp_path):
     t = D.walks(D.lengths(4000, 0, 0, 0, 20, 200, 39), 39)
     db = G.TrajectorySet(gpu_ctx, t)
     q = D.boxes(700, 1, 0.001, 0.1, 40)
-    for ix in (G.Grid(gpu_ctx, db, D.BOX, 0.005, 2, 512), G.FSG(gpu_ctx, db, D.BOX, 0.005)):
+    for ix in (G.Grid(gpu_ctx, db, D.BOX, 0.005, 2, 512), G.FSG(gpu_ctx, db, D.BOX, 0.005), G.STIG(gpu_ctx, db, 500)):
         ix.save(str(tmp_path / "i.bin"))
         back = Index.load(gpu_ctx, db, str(tmp_path / "i.bin"))
         assert back.info()["device_bytes"] == ix.info()["device_bytes"]
