@@ -270,6 +270,15 @@ void index_groups_free(gat_index* ix);
  * used, [1] work bytes when `timed`, [3] queries left in ovf_list for the bitmap scan. */
 int range_groups_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, uint32_t* arena, int64_t cap,
                         unsigned long long* ctr, int64_t* segbase, int64_t* segcnt, int* ovf_list, bool timed);
+/* Point lists likewise (Grid, FSG, MortonGrid; keys in the arena), queries of more than 4,096 points left
+ * in ovf_list. */
+int group_points_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, uint32_t* arena, int64_t cap,
+                        unsigned long long* ctr, int64_t* segbase, int64_t* segcnt, int* ovf_list);
+/* Plain execution of id-set query qi over an index with groups, launched in the order of qi: writes
+ * off[qi + 1] (and off[0]) and the ids at off[qi]; state: [0] set when they do not fit, [1] = 1 + the first
+ * query that outgrew the kernel (later ones then write nothing), [2..3] the end so far (64-bit). */
+int plain_groups_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int qi, int64_t* off, int32_t* out, int64_t capacity,
+                        int* state, unsigned long long* work);
 /* reads and clears the device status word; returns GAT_OK or the code a kernel stored */
 int check_device_flag(gat_ctx* ctx, const char* what);
 inline void count_launch(gat_ctx* ctx, int n = 1) { ctx->launches += n; }

@@ -1152,7 +1152,8 @@ __global__ void __launch_bounds__(kThreads) k_range_points(const gat_mbb* querie
                                                            const int2* items, const float* X, const float* Y,
                                                            const uint32_t* key, int key_bits, uint32_t* arena,
                                                            int64_t cap, unsigned long long* cursor,
-                                                           int64_t* segbase, int64_t* segcnt) {
+                                                           int64_t* segbase, int64_t* segcnt,
+                                                           const int* __restrict__ qlist) {
     __shared__ int sh[kThreads / 32 + 1];
     __shared__ int hist[256];
     __shared__ int wcount[kThreads / 32][257];
@@ -1160,11 +1161,13 @@ __global__ void __launch_bounds__(kThreads) k_range_points(const gat_mbb* querie
     __shared__ unsigned long long base_sh;
     __shared__ int wtot[kThreads / 32];
     int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int qi = blockIdx.x; qi < nq; qi += gridDim.x) {
+    /* queries 0..nq-1, or the nq queries of qlist (items by list position) */
+    for (int j = blockIdx.x; j < nq; j += gridDim.x) {
+        const int qi = qlist ? qlist[j] : j;
         Box q = load_box(queries, qi);
         /* pass 1: count */
         int c = 0;
-        for (int64_t it = ioff[(int64_t)qi * kSub]; it < ioff[(int64_t)(qi + 1) * kSub]; it++) {
+        for (int64_t it = ioff[(int64_t)j * kSub]; it < ioff[(int64_t)(j + 1) * kSub]; it++) {
             int2 r = items[it];
             r.x &= ~kAllHit; /* every point is tested here, all-hit items included */
             scan_range(X, Y, r.x, r.y, q, [&](int) { c++; });
@@ -1186,7 +1189,7 @@ __global__ void __launch_bounds__(kThreads) k_range_points(const gat_mbb* querie
         uint32_t* B = A + total;
         /* pass 2: compact keys in item order, tile by tile (kThreads points per tile) */
         int written = 0;
-        for (int64_t it = ioff[(int64_t)qi * kSub]; it < ioff[(int64_t)(qi + 1) * kSub]; it++) {
+        for (int64_t it = ioff[(int64_t)j * kSub]; it < ioff[(int64_t)(j + 1) * kSub]; it++) {
             int2 r = items[it];
             r.x &= ~kAllHit;
             for (int t0 = r.x; t0 < r.y; t0 += kThreads) {
@@ -1610,7 +1613,7 @@ int run_batch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, int
         } else {
             GAT_CUDA_TRY(ctx, cudaMemsetAsync(cursor, 0, 4 * sizeof(unsigned long long), s), "range");
             k_range_points<<<grid, kThreads, 0, s>>>(d_q, nq, ioff, items, ix->d_x, ix->d_y, ix->d_key, key_bits, arena,
-                                                     cap, cursor, segbase, segcnt);
+                                                     cap, cursor, segbase, segcnt, nullptr);
             count_launch(ctx);
         }
         timed_end(ctx, GAT_KERNEL_RANGE_SCAN, 0.0);
@@ -1636,17 +1639,18 @@ int run_batch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, int
     return GAT_OK;
 }
 
-/* Offsets and gather of an id-set batch whose counts are known on the device only: nothing is copied
+/* Offsets and gather of a batch (ids, or point keys when pidx_bits >= 0) whose counts are known on the device only: nothing is copied
  * when the ids do not fit the caller's capacity or the arena, or when queries are left for the bitmap
  * scan (ctr as in range_groups_launch); the host then learns it from ctr and off[nq].
  * Up to kGatherScan queries the CTAs sum the counts themselves, so a small batch needs no scan
  * launches; ctr[8] receives the total. */
 constexpr int kGatherScan = 1024;
 
-__global__ void __launch_bounds__(kThreads) k_gather_ids(int nq, const int64_t* __restrict__ segbase,
+__global__ void __launch_bounds__(kThreads) k_gather_groups(int nq, const int64_t* __restrict__ segbase,
                                                          const int64_t* __restrict__ segcnt, int64_t* off,
                                                          const uint32_t* __restrict__ arena, int64_t arena_cap, int32_t* out,
-                                                         int64_t capacity, unsigned long long* ctr, bool scan) {
+                                                         int64_t capacity, unsigned long long* ctr, bool scan, int pidx_bits,
+                                                         int32_t* out_pidx) {
     __shared__ int64_t wsum[2][kThreads / 32];
     int64_t total = scan ? 0 : off[nq];
     for (int qi = blockIdx.x; qi < nq; qi += gridDim.x) {
@@ -1683,15 +1687,24 @@ __global__ void __launch_bounds__(kThreads) k_gather_ids(int nq, const int64_t* 
         if (qi == 0 && threadIdx.x == 0) ctr[8] = (unsigned long long)total;
         if (total > capacity || (int64_t)ctr[0] > arena_cap || ctr[3] != 0) continue;
         const int64_t b = segbase[qi], n = segcnt[qi];
-        for (int64_t i = threadIdx.x; i < n; i += kThreads) out[o + i] = (int32_t)arena[b + i];
+        for (int64_t i = threadIdx.x; i < n; i += kThreads) {
+            const uint32_t k = arena[b + i];
+            if (pidx_bits < 0) {
+                out[o + i] = (int32_t)k;
+            } else {
+                out[o + i] = (int32_t)(k >> pidx_bits);
+                if (out_pidx) out_pidx[o + i] = (int32_t)(k & ((1u << pidx_bits) - 1u));
+            }
+        }
     }
 }
 
-/* Batched id sets over an index with point groups (range_groups.cu), offsets and ids in the caller's
- * device arrays. Queries whose ids outgrow the kernel's set get their items built and take the bitmap
- * kernel. The host waits once, after the gather. */
-int run_groups(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, int64_t* d_off, int32_t* d_tid, int64_t capacity,
-               int64_t* total) {
+/* A batch over an index with point groups (range_groups.cu), offsets and results in the caller's device
+ * arrays. Queries whose results outgrow the kernel's memory get their items built and take the bitmap
+ * or the point-list kernel. The host waits once, after the gather. */
+int run_groups(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, int mode, int64_t* d_off, int32_t* d_tid,
+               int32_t* d_pidx, int64_t capacity, int64_t* total) {
+    const bool ids = mode == GAT_RESULT_IDS;
     cudaStream_t s = ctx->stream;
     int st = GAT_OK;
     int64_t* segbase = (int64_t*)scratch(ctx, S_RANGE_SEGBASE, (nq + 1) * sizeof(int64_t), &st);
@@ -1706,8 +1719,8 @@ int run_groups(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, in
         const bool scan = nq <= kGatherScan;
         int rc = GAT_OK;
         if (!scan && (rc = scan_i64(ctx, segcnt, d_off, nq)) != GAT_OK) return rc;
-        k_gather_ids<<<std::max(1, std::min(nq, ctx->sm_count * 8)), kThreads, 0, s>>>(nq, segbase, segcnt, d_off, arena, cap,
-                                                                                    d_tid, capacity, ctr, scan);
+        k_gather_groups<<<std::max(1, std::min(nq, ctx->sm_count * 8)), kThreads, 0, s>>>(nq, segbase, segcnt, d_off, arena, cap,
+                                                                                    d_tid, capacity, ctr, scan, ids ? -1 : ix->pidx_bits, d_pidx);
         count_launch(ctx);
         GAT_CUDA_TRY(ctx, cudaGetLastError(), "range gather launch");
         GAT_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_pinned, ctr, 9 * sizeof(int64_t), cudaMemcpyDeviceToHost, s), "range");
@@ -1719,7 +1732,8 @@ int run_groups(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, in
         if (!arena) return st;
         cap = (int64_t)(ctx->slot_bytes[S_RANGE_ARENA] / 4);
         timed_begin(ctx, GAT_KERNEL_RANGE_SCAN);
-        st = range_groups_launch(ctx, ix, d_q, nq, arena, cap, ctr, segbase, segcnt, ovf_list, ctx->timing);
+        st = ids ? range_groups_launch(ctx, ix, d_q, nq, arena, cap, ctr, segbase, segcnt, ovf_list, ctx->timing)
+                 : group_points_launch(ctx, ix, d_q, nq, arena, cap, ctr, segbase, segcnt, ovf_list);
         timed_end(ctx, GAT_KERNEL_RANGE_SCAN, 0.0);
         if (st != GAT_OK || (st = finish()) != GAT_OK) return st;
         const int64_t n_ovf = ctx->h_pinned[3];
@@ -1732,15 +1746,22 @@ int run_groups(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, in
             const size_t smem_bm = (size_t)words * 4;
             const bool in_smem = smem_bm <= 200 * 1024;
             int per_sm = 0;
-            if (in_smem) allow_smem(k_range_ids, smem_bm);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_range_ids, kThreads, in_smem ? smem_bm : 0);
+            if (ids && in_smem) allow_smem(k_range_ids, smem_bm);
+            if (ids)
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_range_ids, kThreads, in_smem ? smem_bm : 0);
+            else
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_range_points, kThreads, 0);
             const int g = (int)std::max<int64_t>(1, std::min<int64_t>(n_ovf, (int64_t)std::max(1, per_sm) * ctx->sm_count));
-            uint32_t* gbm = in_smem ? nullptr : (uint32_t*)scratch(ctx, S_RANGE_ARENA2, (size_t)g * words * 4, &st);
-            if (!in_smem && !gbm) return st;
+            uint32_t* gbm = !ids || in_smem ? nullptr : (uint32_t*)scratch(ctx, S_RANGE_ARENA2, (size_t)g * words * 4, &st);
+            if (ids && !in_smem && !gbm) return st;
             timed_begin(ctx, GAT_KERNEL_RANGE_SCAN);
-            k_range_ids<<<g, kThreads, in_smem ? smem_bm : 0, s>>>(d_q, (int)n_ovf, ioff, items, ix->d_x, ix->d_y, ix->d_tid,
-                                                                  words, gbm, arena, cap, ctr, segbase, segcnt,
-                                                                  ctx->timing ? ctr + 1 : nullptr, ovf_list, 1);
+            if (ids)
+                k_range_ids<<<g, kThreads, in_smem ? smem_bm : 0, s>>>(d_q, (int)n_ovf, ioff, items, ix->d_x, ix->d_y, ix->d_tid,
+                                                                      words, gbm, arena, cap, ctr, segbase, segcnt,
+                                                                      ctx->timing ? ctr + 1 : nullptr, ovf_list, 1);
+            else
+                k_range_points<<<g, kThreads, 0, s>>>(d_q, (int)n_ovf, ioff, items, ix->d_x, ix->d_y, ix->d_key, key_bits_of(ix),
+                                                      arena, cap, ctr, segbase, segcnt, ovf_list);
             timed_end(ctx, GAT_KERNEL_RANGE_SCAN, 0.0);
             count_launch(ctx);
             GAT_CUDA_TRY(ctx, cudaGetLastError(), "range scan launch");
@@ -1772,11 +1793,48 @@ int run_gather(gat_ctx* ctx, const gat_index* ix, int nq, int mode, const int64_
 }
 
 
+/* Plain execution over point groups: one launch per query, until one outgrows the kernel (*first = that
+ * query, whose offset is known; nq when all are done). A query of over 4,096 ids is rare in a plain call
+ * and so are calls that hold several, so the rest of the call then takes the three-launch form. The
+ * first query's launches come in small lots: a call that must change over has wasted few. */
+int run_plain_groups(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, int64_t* d_off, int32_t* d_tid,
+                     int64_t capacity, int64_t* needed, int* first) {
+    cudaStream_t s = ctx->stream;
+    int st = GAT_OK;
+    unsigned long long* ctr = (unsigned long long*)scratch(ctx, S_RANGE_CURSOR, 128, &st);
+    if (!ctr) return st;
+    int* state = reinterpret_cast<int*>(ctr); /* set by the first query */
+    if (ctx->timing) GAT_CUDA_TRY(ctx, cudaMemsetAsync(ctr + 2, 0, sizeof(int64_t), s), "range");
+    int done = 0;
+    bool truncated = false;
+    for (int lot = 16; done < nq; lot = std::min(4 * lot, 1024)) {
+        const int end = std::min(nq, done + lot);
+        timed_begin(ctx, GAT_KERNEL_RANGE_SCAN);
+        for (int qi = done; qi < end; qi++)
+            if ((st = plain_groups_launch(ctx, ix, d_q, qi, d_off, d_tid, capacity, state, ctx->timing ? ctr + 2 : nullptr)) != GAT_OK)
+                return st;
+        timed_end(ctx, GAT_KERNEL_RANGE_SCAN, 0.0);
+        GAT_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_pinned, ctr, 3 * sizeof(int64_t), cudaMemcpyDeviceToHost, s), "range");
+        GAT_CUDA_TRY(ctx, cudaStreamSynchronize(s), "range scan");
+        const int32_t* h = reinterpret_cast<const int32_t*>(ctx->h_pinned);
+        truncated = h[0] != 0;
+        if (h[1] != 0) {
+            *first = h[1] - 1;
+            break;
+        }
+        done = *first = end;
+    }
+    if (ctx->timing) timed_add_work(ctx, GAT_KERNEL_RANGE_SCAN, (double)ctx->h_pinned[2]);
+    if (*first < nq) return GAT_OK; /* the rest decides about the capacity: its total includes these */
+    *needed = ctx->h_pinned[1];
+    return truncated ? fail(ctx, GAT_ERR_TRUNCATED, "range: output capacity too small") : GAT_OK;
+}
+
 /* Plain execution of id-set queries: per query three dependent launches (items, scan, emit),
  * every buffer sized for any single query before the first launch (items by the index's
  * candidate-range bound, the id bitmap by the set's trajectory count), so nothing waits on the
  * host between queries; one synchronisation at the end reads the total and the status. */
-int run_plain_ids(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, int64_t* d_off, int32_t* d_tid,
+int run_plain_ids(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int first, int nq, int64_t* d_off, int32_t* d_tid,
                   int64_t capacity, int64_t* needed) {
     cudaStream_t s = ctx->stream;
     int st = GAT_OK;
@@ -1800,7 +1858,7 @@ int run_plain_ids(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq,
                         : ix->kind == GAT_INDEX_MORTON ? k_plain_items<GAT_INDEX_MORTON>
                                                        : k_plain_items<GAT_INDEX_FSG>;
     const int scan_grid = ctx->sm_count;
-    for (int qi = 0; qi < nq; qi++) {
+    for (int qi = first; qi < nq; qi++) {
         cudaError_t e = launch_dep(ctx, items_kernel, dim3(1), dim3(kPlainSub), 0, s, ix->grid, ix->stig, ix->fsg,
                                    ix->morton, d_q, qi, ioff, items, item_cap, ctx->d_flag);
         timed_begin(ctx, GAT_KERNEL_RANGE_SCAN);
@@ -1836,11 +1894,14 @@ int range_dev(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, int
         return gat_ctx_sync(ctx);
     }
     int st;
+    /* through the point groups, unless GAT_TUNE_RANGE_SHAPE asks for the point scan; a STIG's groups are on
+     * an order of their own, so its point lists (with points shared by two leaves) are not among them */
+    const bool by_groups =
+        ix->groups.n > 0 && ctx->range_shape == 0 && (mode == GAT_RESULT_IDS || ix->kind != GAT_INDEX_STIG);
     if (exec == GAT_EXEC_BATCHED) {
         int64_t total = 0;
-        /* id sets of an index with point groups; a shape fixed by GAT_TUNE_RANGE_SHAPE is the point scan's */
-        if (mode == GAT_RESULT_IDS && ix->groups.n > 0 && ctx->range_shape == 0) {
-            if ((st = run_groups(ctx, ix, d_q, nq, d_off, d_tid, capacity, &total)) != GAT_OK) return st;
+        if (by_groups) {
+            if ((st = run_groups(ctx, ix, d_q, nq, mode, d_off, d_tid, d_pidx, capacity, &total)) != GAT_OK) return st;
             *needed = total;
             if (total > capacity) return fail(ctx, GAT_ERR_TRUNCATED, "range: output capacity too small");
             return GAT_OK;
@@ -1851,7 +1912,12 @@ int range_dev(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, int
         if ((st = run_gather(ctx, ix, nq, mode, d_off, d_tid, d_pidx)) != GAT_OK) return st;
         return gat_ctx_sync(ctx);
     }
-    if (mode == GAT_RESULT_IDS) return run_plain_ids(ctx, ix, d_q, nq, d_off, d_tid, capacity, needed);
+    if (mode == GAT_RESULT_IDS) {
+        int first = 0;
+        if (by_groups && ((st = run_plain_groups(ctx, ix, d_q, nq, d_off, d_tid, capacity, needed, &first)) != GAT_OK || first == nq))
+            return st;
+        return run_plain_ids(ctx, ix, d_q, first, nq, d_off, d_tid, capacity, needed);
+    }
     /* plain point lists: one query per pipeline run */
     int64_t done = 0;
     int64_t* off1 = (int64_t*)scratch(ctx, S_RANGE_OFF, 2 * sizeof(int64_t), &st);
@@ -1860,18 +1926,28 @@ int range_dev(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, int
     bool truncated = false;
     for (int qi = 0; qi < nq; qi++) {
         int64_t total = 0;
-        if ((st = run_batch(ctx, ix, d_q + qi, 1, mode, off1, &total)) != GAT_OK) return st;
-        if (!truncated && done + total <= capacity) {
-            if ((st = run_gather(ctx, ix, 1, mode, off1, d_tid + done, d_pidx ? d_pidx + done : nullptr)) != GAT_OK)
+        if (by_groups) {
+            const int64_t room = truncated ? 0 : std::max<int64_t>(0, capacity - done);
+            if ((st = run_groups(ctx, ix, d_q + qi, 1, mode, off1, d_tid + (truncated ? 0 : done),
+                                 d_pidx ? d_pidx + (truncated ? 0 : done) : nullptr, room, &total)) != GAT_OK)
                 return st;
+            if (total > room) truncated = true;
         } else {
-            truncated = true;
+            if ((st = run_batch(ctx, ix, d_q + qi, 1, mode, off1, &total)) != GAT_OK) return st;
+            if (!truncated && done + total <= capacity) {
+                if ((st = run_gather(ctx, ix, 1, mode, off1, d_tid + done, d_pidx ? d_pidx + done : nullptr)) != GAT_OK)
+                    return st;
+            } else {
+                truncated = true;
+            }
         }
         done += total;
-        ctx->h_pinned[1] = done;
-        GAT_CUDA_TRY(ctx, cudaMemcpyAsync(d_off + qi + 1, ctx->h_pinned + 1, sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream), "range");
-        GAT_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream), "range");
+        /* the pinned word is free again: the query above waited for the stream */
+        ctx->h_pinned[16] = done;
+        GAT_CUDA_TRY(ctx, cudaMemcpyAsync(d_off + qi + 1, ctx->h_pinned + 16, sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream),
+                     "range");
     }
+    if ((st = gat_ctx_sync(ctx)) != GAT_OK) return st;
     *needed = done;
     if (truncated) return fail(ctx, GAT_ERR_TRUNCATED, "range: output capacity too small");
     return GAT_OK;

@@ -19,6 +19,13 @@
  * of 0.02 to 0.05 degrees over 1M walks took 2.07 ms by CTAs alone, 1.86 ms with pairs for those of
  * 400 to 1,100 expected ids (1.16 ms less on 100k of 0.001 to 0.05). A query that outgrows its team
  * runs again on the CTA, one that outgrows that goes to the bitmap scan (range.cu).
+ *
+ * Plain execution (one query per launch): the CTA answers one query and writes it where the query before
+ * it ended. Each launch lets the next start at once; a query waits for the one before only to read its
+ * end, so the walks, scans and sorts of neighbouring launches overlap.
+ *
+ * Point lists (Grid, FSG, MortonGrid): the same walk gives ranges of points, the CTA collects the keys of
+ * those inside, sorts and writes them.
  */
 #include <algorithm>
 #include <climits>
@@ -138,16 +145,23 @@ __device__ __forceinline__ void put_item(T& t, int b, int e, bool border) {
  * and skips the levels above. */
 constexpr int kJumpMax = 64; /* squares a walk starts from at most */
 
-template <class T>
+template <bool PTS, class T>
 __device__ void walk_grid(const GroupsDev& g, const GridDev& tree, const Box& q, T& t, int me) {
     constexpr int FRONT = T::FRONT;
     const NodeRec* __restrict__ rec = g.rec;
-    auto classify = [&](const NodeRec& r, int* out, int* nout) {
+    /* PTS: ranges of points instead of ids and groups */
+    auto take = [&](int nd, const NodeRec& r, bool border) {
+        if (PTS)
+            put_item(t, tree.node_pbeg[nd], tree.node_pend[nd], border);
+        else
+            put_item(t, r.ib, r.ie, border);
+    };
+    auto classify = [&](int nd, const NodeRec& r, int* out, int* nout) {
         const bool in = pbox_inside(q, r.pbox);
         if (r.child < 0)
-            put_item(t, r.ib, r.ie, !in);
-        else if (in && r.ib >= 0 && box_inside(q, r.mbb))
-            put_item(t, r.ib, r.ie, false);
+            take(nd, r, !in);
+        else if (in && (PTS || r.ib >= 0) && box_inside(q, r.mbb))
+            take(nd, r, false);
         else {
             const int k = atomicAdd(nout, 1);
             if (k < FRONT)
@@ -172,12 +186,12 @@ __device__ void walk_grid(const GroupsDev& g, const GridDev& tree, const Box& q,
                 /* a leaf above the table's level covers several squares: the first of the query's takes it */
                 if ((x > x0 && g.jump[y * n + x - 1] == nd) || (y > y0 && g.jump[(y - 1) * n + x] == nd)) continue;
                 const NodeRec r = rec[nd];
-                if (nd == 0 || box_intersect(q, Box{r.mbb.x, r.mbb.y, r.mbb.z, r.mbb.w})) classify(r, t.front, t.nfront);
+                if (nd == 0 || box_intersect(q, Box{r.mbb.x, r.mbb.y, r.mbb.z, r.mbb.w})) classify(nd, r, t.front, t.nfront);
             }
     }
     if (!jumped && me == 0) {
         const NodeRec r = rec[0];
-        classify(r, t.front, t.nfront);
+        classify(0, r, t.front, t.nfront);
     }
     t.sync();
     for (int cur = 0;; cur ^= 1) {
@@ -187,9 +201,10 @@ __device__ void walk_grid(const GroupsDev& g, const GridDev& tree, const Box& q,
         t.sync();
         if (n == 0 || lost) break;
         for (int k = me; k < 4 * n; k += T::NTHREADS) {
-            const NodeRec r = rec[t.front[cur * FRONT + (k >> 2)] + (k & 3)];
+            const int nd = t.front[cur * FRONT + (k >> 2)] + (k & 3);
+            const NodeRec r = rec[nd];
             if (box_intersect(q, Box{r.mbb.x, r.mbb.y, r.mbb.z, r.mbb.w}))
-                classify(r, t.front + (cur ^ 1) * FRONT, t.nfront + (cur ^ 1));
+                classify(nd, r, t.front + (cur ^ 1) * FRONT, t.nfront + (cur ^ 1));
         }
         t.sync();
         if (me == 0) t.nfront[cur] = 0;
@@ -286,8 +301,10 @@ __device__ void walk_morton(const MortonDev& m, const int32_t* __restrict__ cell
  * arithmetic, so a point in a column strictly between g1 and g2 and a row strictly between g3 and g4
  * lies inside the query: those cells are taken whole, the rest by their groups' boxes. (A NaN
  * coordinate would break the ordering: no cell is then taken whole.) */
-template <class T>
+template <bool PTS, class T>
 __device__ void walk_fsg(const FsgDev& f, const int32_t* __restrict__ cell_g, const Box& q, T& t, int me) {
+    /* where cell c begins: its first group, or PTS its first point */
+    auto begin = [&](int c) { return PTS ? (c < f.cellnum ? f.cbeg[c] : f.cend[f.cellnum - 1]) : cell_g[c]; };
     const int g1 = (int)__fdiv_rn(__fsub_rn(q.xmin, f.rxmin), f.cell), g2 = (int)__fdiv_rn(__fsub_rn(q.xmax, f.rxmin), f.cell);
     const int g3 = (int)__fdiv_rn(__fsub_rn(f.rymax, q.ymax), f.cell), g4 = (int)__fdiv_rn(__fsub_rn(f.rymax, q.ymin), f.cell);
     if (max(max(g1, g2), max(g3, g4)) > kFarCell || min(min(g1, g2), min(g3, g4)) < -kFarCell || g4 - g3 > 4 * T::ITEMS) {
@@ -309,9 +326,10 @@ __device__ void walk_fsg(const FsgDev& f, const int32_t* __restrict__ cell_g, co
                 b = (int)row + c1 + 1;
             }
         }
-        put_item(t, cell_g[lo], cell_g[a], true);
-        put_item(t, cell_g[a], cell_g[b], false);
-        put_item(t, cell_g[b], cell_g[hi + 1], true);
+        const int ga = begin(a), gb = begin(b);
+        put_item(t, begin(lo), ga, true);
+        put_item(t, ga, gb, false);
+        put_item(t, gb, begin(hi + 1), true);
     }
     t.sync();
 }
@@ -447,10 +465,11 @@ __device__ __forceinline__ void take_items(const int2* items, int n, const Box& 
  * counted into buckets of equal width between the least and the greatest (about two to a bucket),
  * scattered to their buckets, and placed by the number of smaller ids in their own bucket. When ids
  * crowd in a few buckets the list is sorted in runs of 32 that are merged in pairs instead. (Sorting
- * runs and searching every id in every run took half of a query's instructions.) */
+ * runs and searching every id in every run took half of a query's instructions.) `out` may be the list
+ * itself. FLIP is xored into what is written (point keys are held with their top bit flipped). */
 constexpr int kCrowd = 32;
 
-template <class T>
+template <class T, unsigned FLIP = 0>
 __device__ void sort_ids(T& t, int m, uint32_t* out, bool write, int me) {
     constexpr int HB = T::HB, NTHREADS = T::NTHREADS;
     int *const tab = t.tab, *const list = t.list;
@@ -460,7 +479,7 @@ __device__ void sort_ids(T& t, int m, uint32_t* out, bool write, int me) {
     const int lane = me & 31, warp = me >> 5;
     int* lo_hi = t.sort;
     /* the list is complete and the set no longer needed */
-    int lo = INT_MAX, hi = 0;
+    int lo = INT_MAX, hi = INT_MIN;
     for (int i = me; i < m; i += NTHREADS) {
         lo = min(lo, list[i]);
         hi = max(hi, list[i]);
@@ -468,7 +487,8 @@ __device__ void sort_ids(T& t, int m, uint32_t* out, bool write, int me) {
     for (int b = me; b < B; b += NTHREADS) tab[b] = 0;
     if (NTHREADS > 32 && me == 0) {
         lo_hi[0] = INT_MAX;
-        lo_hi[1] = lo_hi[2] = 0;
+        lo_hi[1] = INT_MIN;
+        lo_hi[2] = 0;
     }
     t.sync();
     lo = __reduce_min_sync(FULL, lo);
@@ -484,9 +504,9 @@ __device__ void sort_ids(T& t, int m, uint32_t* out, bool write, int me) {
     }
     /* bucket of t: (t - lo) B / width by a rounded-down 0.32 reciprocal, monotone in t, which is all
      * that the placement needs */
-    const unsigned scale = (unsigned)min(0xffffffffull, ((unsigned long long)B << 32) / (unsigned long long)max(1, hi - lo + 1));
+    const unsigned scale = (unsigned)min(0xffffffffull, ((unsigned long long)B << 32) / ((unsigned long long)((unsigned)hi - (unsigned)lo) + 1ull));
     auto bucket = [&](int x) -> int {
-        const unsigned long long p = (unsigned long long)(unsigned)(x - lo) * scale;
+        const unsigned long long p = (unsigned long long)((unsigned)x - (unsigned)lo) * scale;
         return min(B - 1, (int)(p >> 32));
     };
     for (int i = me; i < m; i += NTHREADS) atomicAdd(&tab[bucket(list[i])], 1);
@@ -533,7 +553,7 @@ __device__ void sort_ids(T& t, int m, uint32_t* out, bool write, int me) {
                 const int x = dst[i], b = bucket(x), first = b ? tab[b - 1] : 0, end = tab[b];
                 int rank = first;
                 for (int k = first; k < end; k++) rank += dst[k] < x ? 1 : 0;
-                out[rank] = (uint32_t)x;
+                out[rank] = (uint32_t)x ^ FLIP;
             }
     } else {
         /* runs of 32 sorted by the warps, then merged in pairs: an id's place in the merged run is its
@@ -574,7 +594,7 @@ __device__ void sort_ids(T& t, int m, uint32_t* out, bool write, int me) {
             dst = s;
         }
         if (write)
-            for (int i = me; i < m; i += NTHREADS) out[i] = (uint32_t)src[i];
+            for (int i = me; i < m; i += NTHREADS) out[i] = (uint32_t)src[i] ^ FLIP;
     }
     t.sync();
     int4* slots = reinterpret_cast<int4*>(tab);
@@ -594,6 +614,11 @@ struct GroupQuery {
     unsigned long long* ctr;
     int64_t* segbase;
     int64_t* segcnt;
+    /* plain execution: offsets, ids, their capacity, and the state of the call (answer) */
+    int64_t* p_off;
+    int32_t* p_out;
+    int64_t p_cap;
+    int* p_state;
     int2* retry;   /* queries that outgrew their team, chained per CTA: (query, next or -1) */
     int* ovf_list; /* queries for the bitmap scan */
     unsigned long long* work;
@@ -601,17 +626,17 @@ struct GroupQuery {
 
 /* one query of a team: walk, scan, sort, write; false when it outgrew the team's memory (which is
  * then empty again) */
-template <int KIND, class T>
+template <int KIND, bool PLAIN = false, class T>
 __device__ bool answer(const GroupQuery& a, int qi, T& t, OpenGroups& og, int me, unsigned long long& bytes) {
     const Box q = load_box(a.queries, qi);
     if (KIND == GAT_INDEX_GRID)
-        walk_grid(a.g, a.grid, q, t, me);
+        walk_grid<false>(a.g, a.grid, q, t, me);
     else if (KIND == GAT_INDEX_STIG)
         walk_stig(a.g.rec, q, t, me);
     else if (KIND == GAT_INDEX_MORTON)
         walk_morton(a.morton, a.g.cell_g, q, t, me);
     else
-        walk_fsg(a.fsg, a.g.cell_g, q, t, me);
+        walk_fsg<false>(a.fsg, a.g.cell_g, q, t, me);
     const int n = min(*t.nitems, T::ITEMS);
     if (!__shfl_sync(0xffffffffu, *(volatile int*)t.ovf, 0)) {
         /* ranges per turn: enough turns for every warp, up to 32 a turn */
@@ -628,6 +653,31 @@ __device__ bool answer(const GroupQuery& a, int qi, T& t, OpenGroups& og, int me
     t.sync();
     const int m = *t.cnt;
     const bool lost = *(volatile int*)t.ovf != 0;
+    if (PLAIN) {
+        if (!lost) sort_ids(t, m, reinterpret_cast<uint32_t*>(t.list), true, me);
+        dep_wait(); /* the query before has written its end */
+        /* state: [0] ids that do not fit, [1] 1 + the first query that outgrew the CTA, [2..3] the end */
+        const int stop = qi > 0 ? a.p_state[1] : 0;
+        const bool go = stop == 0 && !lost;
+        const int64_t at = go && qi > 0 ? a.p_off[qi] : 0;
+        t.sync();
+        if (me == 0) {
+            if (qi == 0) {
+                a.p_off[0] = 0;
+                a.p_state[0] = a.p_state[1] = 0;
+            }
+            if (go) {
+                a.p_off[qi + 1] = at + m;
+                *reinterpret_cast<int64_t*>(a.p_state + 2) = at + m;
+                if (at + m > a.p_cap) a.p_state[0] = 1;
+            } else if (stop == 0) {
+                a.p_state[1] = qi + 1;
+            }
+        }
+        if (go && at + m <= a.p_cap)
+            for (int i = me; i < m; i += T::NTHREADS) a.p_out[at + i] = t.list[i];
+        return go;
+    }
     if (me == 0 && !lost) {
         *t.base = atomicAdd(&a.ctr[0], (unsigned long long)m);
         a.segcnt[qi] = m;
@@ -730,6 +780,114 @@ __global__ void __launch_bounds__(kNT, 3) k_range_groups(GroupQuery a, const int
     if (a.work) {
         for (int o = 16; o > 0; o >>= 1) bytes += __shfl_down_sync(0xffffffffu, bytes, o);
         if (lane == 0 && bytes) atomicAdd(a.work, bytes);
+    }
+}
+
+/* Plain execution: query qi of the call. */
+template <int KIND>
+__global__ void __launch_bounds__(kNT, 2) k_plain_groups(GroupQuery a, int qi) {
+    asm volatile("griddepcontrol.launch_dependents;");
+    extern __shared__ int4 smem4[];
+    int* mem = reinterpret_cast<int*>(smem4);
+    __shared__ __align__(8) int ctl[kCtl];
+    __shared__ OpenGroups open[kW];
+    for (int i = threadIdx.x; i < (1 << kBlockBits) / 4; i += kNT) smem4[i] = make_int4(-1, -1, -1, -1);
+    if (threadIdx.x < kCtl) ctl[threadIdx.x] = 0;
+    __syncthreads();
+    BlockTeam t(mem, ctl, 0);
+    unsigned long long bytes = 0;
+    answer<KIND, true>(a, qi, t, open[threadIdx.x >> 5], threadIdx.x, bytes);
+    if (a.work) {
+        for (int o = 16; o > 0; o >>= 1) bytes += __shfl_down_sync(0xffffffffu, bytes, o);
+        if ((threadIdx.x & 31) == 0 && bytes) atomicAdd(a.work, bytes);
+    }
+}
+
+/* Point lists: the keys (trajectory << bits | point index) of the points inside, ascending. A query of
+ * more than kBlockIds points, or one that outgrows the walk's memory, goes on the overflow list for
+ * k_range_points. Keys are held with the top bit flipped, so that signed compares order them. */
+template <int KIND>
+__global__ void __launch_bounds__(kNT, 3) k_group_points(GroupQuery a, const uint32_t* __restrict__ key, int nq) {
+    extern __shared__ int4 smem4[];
+    int* mem = reinterpret_cast<int*>(smem4);
+    __shared__ __align__(8) int ctl[kCtl];
+    __shared__ int q_sh;
+    const int lane = threadIdx.x & 31, me = threadIdx.x;
+    const unsigned FULL = 0xffffffffu;
+    if (me < kCtl) ctl[me] = 0;
+    BlockTeam t(mem, ctl, 0);
+    const float *X = a.g.X, *Y = a.g.Y;
+    for (;;) {
+        if (me == 0) q_sh = (int)atomicAdd(&a.ctr[2], 1ull);
+        __syncthreads();
+        const int qi = q_sh;
+        __syncthreads();
+        if (qi >= nq) break;
+        const Box q = load_box(a.queries, qi);
+        if (KIND == GAT_INDEX_GRID)
+            walk_grid<true>(a.g, a.grid, q, t, me);
+        else if (KIND == GAT_INDEX_MORTON)
+            walk_morton(a.morton, a.morton.cbeg, q, t, me);
+        else
+            walk_fsg<true>(a.fsg, nullptr, q, t, me);
+        const int n = min(*t.nitems, BlockTeam::ITEMS);
+        if (!__shfl_sync(FULL, *(volatile int*)t.ovf, 0)) {
+            for (;;) {
+                int k = 0;
+                if (lane == 0) k = atomicAdd(t.next, 1);
+                k = __shfl_sync(FULL, k, 0);
+                if (k >= n) break;
+                const int2 r = t.items[k];
+                const int end = r.y & ~kBorder;
+                const bool test = r.y < 0;
+                for (int i0 = r.x; i0 < end; i0 += 128) {
+                    /* four points per lane in flight */
+                    float x[4], y[4];
+                    uint32_t kk[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        const int i = i0 + 32 * u + lane;
+                        const bool on = i < end;
+                        x[u] = on && test ? __ldg(X + i) : 0.f;
+                        y[u] = on && test ? __ldg(Y + i) : 0.f;
+                        kk[u] = on ? __ldg(key + i) : 0u;
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        const bool hit = i0 + 32 * u + lane < end && (!test || in_box(q, x[u], y[u]));
+                        const unsigned m = __ballot_sync(FULL, hit);
+                        if (m == 0) continue;
+                        int at = 0;
+                        if (lane == 0) at = atomicAdd(t.cnt, __popc(m));
+                        at = __shfl_sync(FULL, at, 0) + __popc(m & ((1u << lane) - 1u));
+                        if (hit && at < kBlockIds) t.list[at] = (int)(kk[u] ^ 0x80000000u);
+                    }
+                }
+                if (__shfl_sync(FULL, *(volatile int*)t.cnt, 0) > kBlockIds) break;
+            }
+        }
+        __syncthreads();
+        const int m = *t.cnt;
+        const bool lost = *(volatile int*)t.ovf != 0 || m > kBlockIds;
+        if (me == 0) {
+            if (lost) {
+                a.ovf_list[atomicAdd(&a.ctr[3], 1ull)] = qi;
+                a.segcnt[qi] = 0;
+                a.segbase[qi] = 0;
+            } else {
+                *t.base = atomicAdd(&a.ctr[0], (unsigned long long)m);
+                a.segcnt[qi] = m;
+                a.segbase[qi] = (int64_t)*t.base;
+            }
+        }
+        __syncthreads();
+        if (!lost) {
+            const int64_t at = (int64_t)*t.base;
+            sort_ids<BlockTeam, 0x80000000u>(t, m, a.arena + at, at + m <= a.cap, me);
+        }
+        __syncthreads();
+        if (me == 0) *t.nitems = t.nfront[0] = t.nfront[1] = *t.cnt = *t.ovf = *t.next = 0;
+        __syncthreads();
     }
 }
 
@@ -873,8 +1031,8 @@ int range_groups_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, i
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kNT, kSmem);
     const int full = std::max(1, per_sm) * ctx->sm_count;
     GAT_CUDA_TRY(ctx, cudaMemsetAsync(ctr, 0, 8 * sizeof(unsigned long long), s), "range");
-    GroupQuery a{d_q, ix->grid, ix->fsg, ix->morton, ix->groups, arena, cap, ctr, segbase, segcnt, nullptr, ovf_list,
-                 timed ? ctr + 1 : nullptr};
+    GroupQuery a{d_q, ix->grid, ix->fsg, ix->morton, ix->groups, arena, cap, ctr, segbase, segcnt, nullptr, nullptr, 0, nullptr, nullptr,
+                 ovf_list, timed ? ctr + 1 : nullptr};
     if (nq <= std::min(full, kDirectMax)) {
         /* no more queries than resident CTAs: one each */
         kernel<<<nq, kNT, kSmem, s>>>(a, nullptr, nullptr, nq);
@@ -900,6 +1058,43 @@ int range_groups_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, i
     k_order<<<tb, 256, 0, s>>>(nq, bin, hist, list);
     kernel<<<full, kNT, kSmem, s>>>(a, list, counts, nq);
     count_launch(ctx, 4);
+    GAT_CUDA_TRY(ctx, cudaGetLastError(), "range scan launch");
+    return GAT_OK;
+}
+
+int plain_groups_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int qi, int64_t* off, int32_t* out, int64_t capacity,
+                        int* state, unsigned long long* work) {
+    auto kernel = ix->kind == GAT_INDEX_GRID     ? k_plain_groups<GAT_INDEX_GRID>
+                  : ix->kind == GAT_INDEX_STIG   ? k_plain_groups<GAT_INDEX_STIG>
+                  : ix->kind == GAT_INDEX_MORTON ? k_plain_groups<GAT_INDEX_MORTON>
+                                                 : k_plain_groups<GAT_INDEX_FSG>;
+    if (qi == 0) allow_smem(kernel, kSmem);
+    GroupQuery a{d_q, ix->grid, ix->fsg, ix->morton, ix->groups, nullptr, 0, nullptr, nullptr, nullptr, off, out, capacity, state,
+                 nullptr, nullptr, work};
+    /* the first launch of a call waits for all before it: the queries may come from a kernel */
+    if (qi == 0)
+        kernel<<<1, kNT, kSmem, ctx->stream>>>(a, qi);
+    else
+        (void)launch_dep(ctx, kernel, dim3(1), dim3(kNT), kSmem, ctx->stream, a, qi);
+    count_launch(ctx);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? GAT_OK : cuda_fail(ctx, e, "range plain launch");
+}
+
+int group_points_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, uint32_t* arena, int64_t cap,
+                        unsigned long long* ctr, int64_t* segbase, int64_t* segcnt, int* ovf_list) {
+    cudaStream_t s = ctx->stream;
+    auto kernel = ix->kind == GAT_INDEX_GRID     ? k_group_points<GAT_INDEX_GRID>
+                  : ix->kind == GAT_INDEX_MORTON ? k_group_points<GAT_INDEX_MORTON>
+                                                 : k_group_points<GAT_INDEX_FSG>;
+    allow_smem(kernel, kSmem);
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kNT, kSmem);
+    GAT_CUDA_TRY(ctx, cudaMemsetAsync(ctr, 0, 8 * sizeof(unsigned long long), s), "range");
+    GroupQuery a{d_q, ix->grid, ix->fsg, ix->morton, ix->groups, arena, cap, ctr, segbase, segcnt, nullptr, nullptr, 0, nullptr,
+                 nullptr, ovf_list, nullptr};
+    kernel<<<std::min(nq, std::max(1, per_sm) * ctx->sm_count), kNT, kSmem, s>>>(a, ix->d_key, nq);
+    count_launch(ctx);
     GAT_CUDA_TRY(ctx, cudaGetLastError(), "range scan launch");
     return GAT_OK;
 }

@@ -14,12 +14,24 @@ from oracle import pyoracle as po
 pytestmark = pytest.mark.gpu
 
 
-def _general(ctx, ix, q):
+def _general(ctx, ix, q, result="ids"):
     ctx.set_tuning(L.GAT_TUNE_RANGE_SHAPE, 1)
     try:
-        return ix.range_query(q, capacity=4_000_000)
+        return ix.range_query(q, result, capacity=4_000_000)
     finally:
         ctx.set_tuning(L.GAT_TUNE_RANGE_SHAPE, 0)
+
+
+def _same_plain_and_points(ctx, ix, q):
+    """Plain id sets, batched and plain point lists of few queries."""
+    a, b = _general(ctx, ix, q), ix.range_query(q, "ids", "plain", capacity=4_000_000)
+    assert np.array_equal(a.offsets, b.offsets) and np.array_equal(a.tids, b.tids)
+    a = _general(ctx, ix, q, "points")
+    for execution, part in (("batched", len(q)), ("plain", min(len(q), 12))):
+        b = ix.range_query(q[:part], "points", execution, capacity=4_000_000)
+        e = a.offsets[part]
+        assert np.array_equal(a.offsets[:part + 1], b.offsets)
+        assert np.array_equal(a.tids[:e], b.tids) and np.array_equal(a.pidx[:e], b.pidx)
 
 
 def _same(ctx, ix, q):
@@ -61,6 +73,9 @@ def test_odd_rectangles(gpu_ctx, cell, cap):
         r = _same(gpu_ctx, ix, q[finite])
         off, ids = o.range(q[finite], 0)
         assert np.array_equal(r.offsets, off) and np.array_equal(r.tids, ids)
+    few = np.concatenate([q[:20], q[300:320], q[600:620], q[900:903], q[-5:]])
+    for ix in (g, f, G.MortonGrid(g), G.STIG(gpu_ctx, db, 64)):
+        _same_plain_and_points(gpu_ctx, ix, few)
     _same(gpu_ctx, g, q)  # NaN and infinite rectangles too: the two paths agree
     _same(gpu_ctx, f, q[~np.isinf(q).any(1)])
     _same(gpu_ctx, G.MortonGrid(g), q)
@@ -80,6 +95,7 @@ def test_batch_sizes(gpu_ctx, nq):
     g = G.Grid(gpu_ctx, db, D.BOX, 0.005, 2, 512)
     for ix in (g, G.FSG(gpu_ctx, db, D.BOX, 0.005), G.MortonGrid(g), G.STIG(gpu_ctx, db, 1000)):
         _same(gpu_ctx, ix, q)
+        _same_plain_and_points(gpu_ctx, ix, q[:100])
 
 
 def test_clustered_set(gpu_ctx):
@@ -102,6 +118,7 @@ def test_clustered_set(gpu_ctx):
         r = _same(gpu_ctx, ix, q)
         assert int(np.diff(r.offsets).max()) > 4096  # beyond the largest set
         _same(gpu_ctx, ix, q[:200])
+        _same_plain_and_points(gpu_ctx, ix, np.concatenate([q[900:930], q[:8], q[930:940]]))
 
 
 def test_tiny_sets_and_fine_cells(gpu_ctx):
