@@ -340,8 +340,12 @@ struct OpenGroups {
     int beg[kOpen], end[kOpen], id[kOpen];
 };
 
-/* Tests the points of `n` open groups whose trajectory is not in the set yet, four groups at a time
- * with eight lanes each, until one lies in the query. */
+/* Tests the points of `n` open groups whose trajectory is not in the set yet, eight groups at a time with
+ * four lanes each and kFly points per lane in flight (24 points: most groups in one trip to L2), until
+ * one lies in the query. (Four groups with two points per lane in flight took two trips each: 100k
+ * rectangles over 1M walks 2.24 ms, 2.05 ms now.) */
+constexpr int kFly = 6;
+
 template <class T>
 __device__ __forceinline__ void test_open(const OpenGroups& og, int n, const Box& q, const float* __restrict__ X,
                                           const float* __restrict__ Y, T& t, unsigned& bytes) {
@@ -355,27 +359,33 @@ __device__ __forceinline__ void test_open(const OpenGroups& og, int n, const Box
             e = og.end[k0 + lane];
             id = og.id[k0 + lane];
         }
-        unsigned m = __ballot_sync(FULL, on && !t.has(id));
-        while (m) {
-            int src = -1;
+        const unsigned m = __ballot_sync(FULL, on && !t.has(id));
+        const int total = __popc(m);
+        /* the lanes of the open groups, in order: lane i holds the i-th */
+        int nth = 0;
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                if (k == (lane >> 3) && m) src = __ffs(m) - 1;
-                m &= m - 1;
-            }
-            const int b0 = __shfl_sync(FULL, b, src & 31), e0 = __shfl_sync(FULL, e, src & 31);
-            const int tid = __shfl_sync(FULL, id, src & 31);
+        for (int s = 16; s > 0; s >>= 1)
+            if (__popc(m & ((1u << (nth + s)) - 1u)) <= lane) nth += s;
+        for (int k = 0; k < total; k += 8) {
+            const int g = k + (lane >> 2);
+            const int src = __shfl_sync(FULL, nth, g & 31);
+            const int b0 = __shfl_sync(FULL, b, src), e1 = __shfl_sync(FULL, e, src), e0 = g < total ? e1 : b0;
+            const int tid = __shfl_sync(FULL, id, src);
             bool found = false;
-            if (src >= 0)
-                for (int i = b0 + (lane & 7); i < e0 && !found; i += 16) {
-                    /* two steps of the eight lanes in flight */
-                    const int i2 = min(i + 8, e0 - 1);
-                    const float x = __ldg(X + i), y = __ldg(Y + i), x2 = __ldg(X + i2), y2 = __ldg(Y + i2);
-                    found = in_box(q, x, y) || in_box(q, x2, y2);
-                    bytes += 16;
+            for (int i = b0 + (lane & 3); i < e0 && !found; i += 4 * kFly) {
+                float x[kFly], y[kFly];
+#pragma unroll
+                for (int u = 0; u < kFly; u++) {
+                    const int p = min(i + 4 * u, e0 - 1);
+                    x[u] = __ldg(X + p);
+                    y[u] = __ldg(Y + p);
                 }
+#pragma unroll
+                for (int u = 0; u < kFly; u++) found |= in_box(q, x[u], y[u]);
+                bytes += 8 * kFly;
+            }
             const unsigned hits = __ballot_sync(FULL, found);
-            if (src >= 0 && (lane & 7) == 0 && ((hits >> (lane & 24)) & 0xffu)) t.insert(tid);
+            if ((lane & 3) == 0 && ((hits >> lane) & 0xfu)) t.insert(tid);
         }
     }
     __syncwarp();
