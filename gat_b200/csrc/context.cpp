@@ -88,13 +88,16 @@ void free_slots(gat_ctx* ctx) {
     cudaStreamSynchronize(ctx->stream);
 }
 
+/* one pinned allocation per context holds the words for small reads and the first staging area */
+constexpr size_t kPinnedWords = 64, kFirstStage = (size_t)64 << 10;
+
 void* host_stage(gat_ctx* ctx, size_t bytes, int* status) {
     if (bytes <= ctx->h_stage_bytes) return ctx->h_stage;
     const size_t had = ctx->h_stage_bytes;
     if (ctx->h_stage) {
         /* an earlier copy may still read it */
         cudaStreamSynchronize(ctx->stream);
-        cudaFreeHost(ctx->h_stage);
+        if (ctx->h_stage != ctx->h_pinned + kPinnedWords) cudaFreeHost(ctx->h_stage);
         ctx->h_stage = nullptr;
         ctx->h_stage_bytes = 0;
     }
@@ -136,12 +139,21 @@ void* index_alloc(gat_index* ix, size_t bytes, int* status) {
     return p;
 }
 
-int check_device_flag(gat_ctx* ctx, const char* what) {
+int queue_device_flag(gat_ctx* ctx, const char* what) {
     /* read into the context's pinned words: a copy to pageable memory goes through the driver's
      * shared staging buffer and can wait behind other streams' pageable copies */
-    int32_t* hf = reinterpret_cast<int32_t*>(ctx->h_pinned + 63);
-    GAT_CUDA_TRY(ctx, cudaMemcpyAsync(hf, ctx->d_flag, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream), what);
+    GAT_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_pinned + 63, ctx->d_flag, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream), what);
+    return GAT_OK;
+}
+
+int check_device_flag(gat_ctx* ctx, const char* what) {
+    if (int st = queue_device_flag(ctx, what)) return st;
     GAT_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream), what);
+    return judge_device_flag(ctx, what);
+}
+
+int judge_device_flag(gat_ctx* ctx, const char* what) {
+    const int32_t* hf = reinterpret_cast<const int32_t*>(ctx->h_pinned + 63);
     const int32_t flag = *hf;
     if (flag == 0) return GAT_OK;
     cudaMemsetAsync(ctx->d_flag, 0, sizeof(int32_t), ctx->stream);
@@ -259,11 +271,13 @@ int gat_ctx_create(int device, gat_ctx** out) {
         (e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaMalloc(&c->d_flag, 16 * sizeof(int32_t))) != cudaSuccess ||
         (e = cudaMemset(c->d_flag, 0, 16 * sizeof(int32_t))) != cudaSuccess ||
-        (e = cudaMallocHost(&c->h_pinned, 64 * sizeof(int64_t))) != cudaSuccess) {
+        (e = cudaMallocHost(&c->h_pinned, kPinnedWords * sizeof(int64_t) + kFirstStage)) != cudaSuccess) {
         cudaGetLastError();
         gat_ctx_destroy(c);
         return e == cudaErrorMemoryAllocation ? GAT_ERR_OOM : GAT_ERR_CUDA;
     }
+    c->h_stage = c->h_pinned + kPinnedWords;
+    c->h_stage_bytes = kFirstStage;
     *out = c;
     return GAT_OK;
 }
@@ -302,8 +316,8 @@ void gat_ctx_destroy(gat_ctx* ctx) {
     free_slots(ctx);
     if (ctx->build_pool) cudaMemPoolDestroy(ctx->build_pool);
     if (ctx->d_flag) cudaFree(ctx->d_flag);
+    if (ctx->h_stage && ctx->h_stage != ctx->h_pinned + kPinnedWords) cudaFreeHost(ctx->h_stage);
     if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
-    if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
 }

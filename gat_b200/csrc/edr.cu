@@ -1,6 +1,7 @@
 /* EDR of (query, candidate) pair lists: the C ABI entry points over the wavefront kernel of
  * edr_kernel.cuh. */
 #include <algorithm>
+#include <cstring>
 
 #include "edr_kernel.cuh"
 #include "internal.h"
@@ -70,21 +71,40 @@ int gat_edr_pairs(gat_ctx* ctx, int npairs, const int32_t* q_len, const int64_t*
     int32_t* d_out = (int32_t*)p; p += up(n4);
     float2* d_a = (float2*)p; p += up(a_bytes);
     float2* d_b = (float2*)p;
-    GAT_CUDA_TRY(ctx, cudaMemcpyAsync(d_aoff, q_off, n8, cudaMemcpyHostToDevice, s), "edr H2D");
-    GAT_CUDA_TRY(ctx, cudaMemcpyAsync(d_boff, c_off, n8, cudaMemcpyHostToDevice, s), "edr H2D");
-    GAT_CUDA_TRY(ctx, cudaMemcpyAsync(d_alen, q_len, n4, cudaMemcpyHostToDevice, s), "edr H2D");
-    GAT_CUDA_TRY(ctx, cudaMemcpyAsync(d_blen, c_len, n4, cudaMemcpyHostToDevice, s), "edr H2D");
-    if (a_bytes) GAT_CUDA_TRY(ctx, cudaMemcpyAsync(d_a, q_xy, a_bytes, cudaMemcpyHostToDevice, s), "edr H2D");
-    if (b_bytes) GAT_CUDA_TRY(ctx, cudaMemcpyAsync(d_b, c_xy, b_bytes, cudaMemcpyHostToDevice, s), "edr H2D");
+    /* host arrays in the order of the device buffer */
+    const struct {
+        void* d;
+        const void* h;
+        size_t bytes;
+    } in[6] = {{d_aoff, q_off, n8}, {d_boff, c_off, n8}, {d_alen, q_len, n4}, {d_blen, c_len, n4}, {d_a, q_xy, a_bytes},
+               {d_b, c_xy, b_bytes}};
+    if (total <= kStageIn) {
+        char* stage = (char*)host_stage(ctx, total, &st);
+        if (!stage) return st;
+        for (const auto& c : in)
+            if (c.bytes) memcpy(stage + ((char*)c.d - buf), c.h, c.bytes);
+        GAT_CUDA_TRY(ctx, cudaMemcpyAsync(buf, stage, total, cudaMemcpyHostToDevice, s), "edr H2D");
+    } else {
+        for (const auto& c : in)
+            if (c.bytes) GAT_CUDA_TRY(ctx, cudaMemcpyAsync(c.d, c.h, c.bytes, cudaMemcpyHostToDevice, s), "edr H2D");
+    }
     if ((st = edr_launch_soa(ctx, npairs, nullptr, d_aoff, d_alen, d_boff, d_blen, mr, mc, d_a, d_b,
                              match_threshold(eps), d_out, nullptr)) != GAT_OK)
         return st;
+    /* the distances come back with the status word, in one wait; they are handed over when it is clear */
+    int32_t* back = n4 <= kStageOut ? (int32_t*)host_stage(ctx, n4, &st) : nullptr;
+    if (n4 <= kStageOut && !back) return st;
+    if (back) GAT_CUDA_TRY(ctx, cudaMemcpyAsync(back, d_out, n4, cudaMemcpyDeviceToHost, s), "edr D2H");
     if ((st = check_device_flag(ctx, "edr")) != GAT_OK) return st;
+    if (back) {
+        memcpy(out, back, n4);
+    } else {
+        GAT_CUDA_TRY(ctx, cudaMemcpyAsync(out, d_out, n4, cudaMemcpyDeviceToHost, s), "edr D2H");
+        GAT_CUDA_TRY(ctx, cudaStreamSynchronize(s), "edr");
+    }
     double cells = 0;
     for (int i = 0; i < npairs; i++) cells += (double)q_len[i] * (double)c_len[i];
     timed_add_work(ctx, GAT_KERNEL_EDR, cells);
-    GAT_CUDA_TRY(ctx, cudaMemcpyAsync(out, d_out, n4, cudaMemcpyDeviceToHost, s), "edr D2H");
-    GAT_CUDA_TRY(ctx, cudaStreamSynchronize(s), "edr");
     return GAT_OK;
 }
 

@@ -281,6 +281,13 @@ int plain_groups_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, i
                         int* state, unsigned long long* work);
 /* reads and clears the device status word; returns GAT_OK or the code a kernel stored */
 int check_device_flag(gat_ctx* ctx, const char* what);
+/* the same in two parts around a stream wait of the caller's: queue the read, then judge it */
+int queue_device_flag(gat_ctx* ctx, const char* what);
+int judge_device_flag(gat_ctx* ctx, const char* what);
+/* Small host arrays of a call go through pinned staging, all in one copy: a copy from or to pageable
+ * memory costs about 10 us by itself (16 short EDR pairs: six of them in a 92 us call), while staging
+ * costs a memcpy. Beyond the limits the driver's own pipelined staging is as fast. */
+constexpr size_t kStageIn = (size_t)1 << 20, kStageOut = (size_t)4 << 20;
 inline void count_launch(gat_ctx* ctx, int n = 1) { ctx->launches += n; }
 /* brackets one launch of a timed kernel class (no-ops unless timing is on) */
 void timed_begin(gat_ctx* ctx, int cls);

@@ -23,6 +23,7 @@
  */
 #include <algorithm>
 #include <climits>
+#include <cstring>
 
 #include "cells.cuh"
 #include "internal.h"
@@ -1988,7 +1989,15 @@ int gat_range_query(gat_ctx* ctx, const gat_index* ix, const gat_mbb* queries, i
     int st = GAT_OK;
     gat_mbb* dq = (gat_mbb*)scratch(ctx, S_RANGE_Q, (size_t)(nq + 1) * sizeof(gat_mbb), &st);
     if (!dq) return st;
-    if (nq > 0) GAT_CUDA_TRY(ctx, cudaMemcpyAsync(dq, queries, nq * sizeof(gat_mbb), cudaMemcpyHostToDevice, s), "range H2D");
+    const size_t q_bytes = (size_t)nq * sizeof(gat_mbb);
+    const void* from = queries;
+    if (nq > 0 && q_bytes <= kStageIn) {
+        void* stage = host_stage(ctx, q_bytes, &st);
+        if (!stage) return st;
+        memcpy(stage, queries, q_bytes);
+        from = stage;
+    }
+    if (nq > 0) GAT_CUDA_TRY(ctx, cudaMemcpyAsync(dq, from, q_bytes, cudaMemcpyHostToDevice, s), "range H2D");
     /* outputs land in device scratch first, sized to the host capacity */
     int64_t dcap = std::max<int64_t>(capacity, 1);
     int32_t* dt = (int32_t*)scratch(ctx, S_RANGE_OUT_T, (size_t)dcap * 4, &st);
@@ -1998,8 +2007,25 @@ int gat_range_query(gat_ctx* ctx, const gat_index* ix, const gat_mbb* queries, i
     int64_t need = 0;
     st = range_dev(ctx, ix, dq, nq, result_kind, exec, csr, dt, dp, capacity, &need);
     *needed = need;
+    const size_t off_bytes = (size_t)(nq + 1) * sizeof(int64_t), id_bytes = st == GAT_OK ? (size_t)need * 4 : 0;
+    const bool points = result_kind == GAT_RESULT_POINTS;
+    const size_t back_bytes = off_bytes + id_bytes * (points ? 2 : 1);
+    if ((st == GAT_OK || st == GAT_ERR_TRUNCATED) && back_bytes <= kStageOut) {
+        int hs = GAT_OK;
+        char* back = (char*)host_stage(ctx, back_bytes, &hs);
+        if (!back) return hs;
+        GAT_CUDA_TRY(ctx, cudaMemcpyAsync(back, csr, off_bytes, cudaMemcpyDeviceToHost, s), "range D2H");
+        if (id_bytes) GAT_CUDA_TRY(ctx, cudaMemcpyAsync(back + off_bytes, dt, id_bytes, cudaMemcpyDeviceToHost, s), "range D2H");
+        if (id_bytes && points)
+            GAT_CUDA_TRY(ctx, cudaMemcpyAsync(back + off_bytes + id_bytes, dp, id_bytes, cudaMemcpyDeviceToHost, s), "range D2H");
+        GAT_CUDA_TRY(ctx, cudaStreamSynchronize(s), "range");
+        memcpy(offsets, back, off_bytes);
+        if (id_bytes) memcpy(out_tid, back + off_bytes, id_bytes);
+        if (id_bytes && points) memcpy(out_pidx, back + off_bytes + id_bytes, id_bytes);
+        return st;
+    }
     if (st == GAT_OK || st == GAT_ERR_TRUNCATED)
-        GAT_CUDA_TRY(ctx, cudaMemcpyAsync(offsets, csr, (size_t)(nq + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost, s), "range D2H");
+        GAT_CUDA_TRY(ctx, cudaMemcpyAsync(offsets, csr, off_bytes, cudaMemcpyDeviceToHost, s), "range D2H");
     if (st == GAT_OK && need > 0) {
         GAT_CUDA_TRY(ctx, cudaMemcpyAsync(out_tid, dt, (size_t)need * 4, cudaMemcpyDeviceToHost, s), "range D2H");
         if (result_kind == GAT_RESULT_POINTS)

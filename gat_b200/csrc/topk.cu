@@ -19,6 +19,7 @@
  */
 #include <algorithm>
 #include <climits>
+#include <cstring>
 
 #include "edr_kernel.cuh"
 #include "internal.h"
@@ -1363,8 +1364,7 @@ int topk_plain_graph(gat_ctx* ctx, const gat_index* g, int nq, const int32_t* d_
     for (int q = first; q < nq; q++) GAT_CUDA_TRY(ctx, cudaGraphLaunch(L->exec, s), "top-k graph launch");
     GAT_CUDA_TRY(ctx, cudaMemcpyAsync(w->h_pinned + 8, L->acc, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s),
                  "top-k");
-    GAT_CUDA_TRY(ctx, cudaStreamSynchronize(s), "top-k");
-    if ((st = check_device_flag(w, "top-k")) != GAT_OK) return fail(ctx, st, w->err);
+    if ((st = check_device_flag(w, "top-k")) != GAT_OK) return fail(ctx, st, w->err); /* waits for the copies above too */
     const int64_t rounds = w->h_pinned[10];
     ctx->launches += (w->launches - lw0) + (int64_t)(nq - first) * L->launches_fixed + rounds * L->launches_round;
     if (stats) {
@@ -1463,14 +1463,24 @@ int upload_queries(gat_ctx* ctx, int nq, const int32_t* q_len, const float* lon,
     float* dlat = (float*)(p + b_len + b_off + b_f);
     *dxy = (float2*)(p + b_len + b_off + 2 * b_f);
     cudaStream_t s = ctx->stream;
-    GAT_CUDA_TRY(ctx, cudaMemcpyAsync(*dl, q_len, (size_t)nq * 4, cudaMemcpyHostToDevice, s), "top-k H2D");
+    const size_t all = b_len + b_off + 2 * b_f;
+    const bool staged = all <= kStageIn;
     /* the offsets are built here: copied from pinned staging, not from pageable memory */
-    int64_t* hoff = (int64_t*)host_stage(ctx, (size_t)(nq + 1) * 8, &st);
-    if (!hoff) return st;
+    char* stage = (char*)host_stage(ctx, staged ? all : (size_t)(nq + 1) * 8, &st);
+    if (!stage) return st;
+    int64_t* hoff = reinterpret_cast<int64_t*>(staged ? stage + b_len : stage);
     std::copy(h.off.begin(), h.off.begin() + (nq + 1), hoff);
-    GAT_CUDA_TRY(ctx, cudaMemcpyAsync(*doff, hoff, (size_t)(nq + 1) * 8, cudaMemcpyHostToDevice, s), "top-k H2D");
-    GAT_CUDA_TRY(ctx, cudaMemcpyAsync(dlon, lon, (size_t)h.total * 4, cudaMemcpyHostToDevice, s), "top-k H2D");
-    GAT_CUDA_TRY(ctx, cudaMemcpyAsync(dlat, lat, (size_t)h.total * 4, cudaMemcpyHostToDevice, s), "top-k H2D");
+    if (staged) {
+        memcpy(stage, q_len, (size_t)nq * 4);
+        memcpy(stage + b_len + b_off, lon, (size_t)h.total * 4);
+        memcpy(stage + b_len + b_off + b_f, lat, (size_t)h.total * 4);
+        GAT_CUDA_TRY(ctx, cudaMemcpyAsync(p, stage, all, cudaMemcpyHostToDevice, s), "top-k H2D");
+    } else {
+        GAT_CUDA_TRY(ctx, cudaMemcpyAsync(*dl, q_len, (size_t)nq * 4, cudaMemcpyHostToDevice, s), "top-k H2D");
+        GAT_CUDA_TRY(ctx, cudaMemcpyAsync(*doff, hoff, (size_t)(nq + 1) * 8, cudaMemcpyHostToDevice, s), "top-k H2D");
+        GAT_CUDA_TRY(ctx, cudaMemcpyAsync(dlon, lon, (size_t)h.total * 4, cudaMemcpyHostToDevice, s), "top-k H2D");
+        GAT_CUDA_TRY(ctx, cudaMemcpyAsync(dlat, lat, (size_t)h.total * 4, cudaMemcpyHostToDevice, s), "top-k H2D");
+    }
     int grid = (int)std::min<int64_t>(ctx->sm_count * 8, (h.total + 255) / 256 + 1);
     k_interleave<<<grid, 256, 0, s>>>(dlon, dlat, h.total, *dxy);
     count_launch(ctx);
@@ -1520,6 +1530,17 @@ int gat_topk(gat_ctx* ctx, const gat_index* grid, int nq, const int32_t* q_len, 
     int32_t* dres = (int32_t*)scratch(ctx, S_TOPK_OUT, (size_t)nq * k * 8 + 16, &st);
     if (!dres) return st;
     st = topk_dev(ctx, grid, nq, dl, doff, dxy, h.maxlen, k, eps, exec, dres, dres + (size_t)nq * k, stats);
+    const size_t half = (size_t)nq * k * 4;
+    if (st == GAT_OK && 2 * half <= kStageOut) {
+        int hs = GAT_OK;
+        char* back = (char*)host_stage(ctx, 2 * half, &hs);
+        if (!back) return hs;
+        GAT_CUDA_TRY(ctx, cudaMemcpyAsync(back, dres, 2 * half, cudaMemcpyDeviceToHost, ctx->stream), "top-k D2H");
+        GAT_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream), "top-k D2H");
+        memcpy(out_ids, back, half);
+        memcpy(out_dist, back + half, half);
+        return GAT_OK;
+    }
     if (st == GAT_OK) {
         GAT_CUDA_TRY(ctx, cudaMemcpyAsync(out_ids, dres, (size_t)nq * k * 4, cudaMemcpyDeviceToHost, ctx->stream), "top-k D2H");
         GAT_CUDA_TRY(ctx, cudaMemcpyAsync(out_dist, dres + (size_t)nq * k, (size_t)nq * k * 4, cudaMemcpyDeviceToHost, ctx->stream), "top-k D2H");
