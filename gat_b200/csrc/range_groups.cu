@@ -337,7 +337,7 @@ __device__ void walk_fsg(const FsgDev& f, const int32_t* __restrict__ cell_g, co
 /* groups a warp has found to straddle the query's border, tested kOpen / 2 or more at a time */
 constexpr int kOpen = 64;
 struct OpenGroups {
-    int beg[kOpen], end[kOpen], id[kOpen];
+    int at[kOpen], id[kOpen]; /* group and trajectory */
 };
 
 /* Tests the points of `n` open groups whose trajectory is not in the set yet, eight groups at a time with
@@ -347,17 +347,19 @@ struct OpenGroups {
 constexpr int kFly = 6;
 
 template <class T>
-__device__ __forceinline__ void test_open(const OpenGroups& og, int n, const Box& q, const float* __restrict__ X,
-                                          const float* __restrict__ Y, T& t, unsigned& bytes) {
+__device__ __forceinline__ void test_open(const OpenGroups& og, int n, const Box& q, const int32_t* __restrict__ gbeg,
+                                          const float* __restrict__ X, const float* __restrict__ Y, T& t, unsigned& bytes) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     for (int k0 = 0; k0 < n; k0 += 32) {
         const bool on = k0 + lane < n;
         int b = 0, e = 0, id = -1;
         if (on) {
-            b = og.beg[k0 + lane];
-            e = og.end[k0 + lane];
+            const int g = og.at[k0 + lane];
             id = og.id[k0 + lane];
+            b = __ldg(gbeg + g);
+            e = __ldg(gbeg + g + 1);
+            bytes += 8;
         }
         const unsigned m = __ballot_sync(FULL, on && !t.has(id));
         const int total = __popc(m);
@@ -392,8 +394,8 @@ __device__ __forceinline__ void test_open(const OpenGroups& og, int n, const Box
 }
 
 /* One warp takes the `n` <= 32 ranges from items[0]: their ids are dealt to the lanes as one sequence
- * (an owner search over the running lengths), so that short ranges fill the warp. The ids, boxes and
- * extents of the next 32 are loaded before the current 32 are looked at: with a load after each test
+ * (a mask of where ranges begin tells a lane its range), so that short ranges fill the warp. The ids and
+ * boxes of the next 32 are loaded before the current 32 are looked at: with a load after each test
  * a step waited for three trips to L2 (100k rectangles over 1M walks 4.6 ms). Groups that straddle
  * the border gather in `og`. */
 template <class T>
@@ -413,34 +415,28 @@ __device__ __forceinline__ void take_items(const int2* items, int n, const Box& 
     }
     const int total = __shfl_sync(FULL, incl, 31);
     const int shift = it.x - (incl - len); /* position = shift + sequence index */
-    unsigned bytes = 0;
+    unsigned bytes = len * (it.y < 0 ? 20 : 4); /* ids, and boxes of border groups */
     int nopen = 0;
     struct Next {
-        int id, beg, end;
+        int id, pos;
         float4 box;
         bool border;
     };
+    int begun = 0; /* ranges that begin before the current 32 */
     auto load = [&](int e0) {
         Next x;
-        const int e = e0 + lane;
-        int l = 0; /* the owner: the first lane whose running length exceeds e */
-#pragma unroll
-        for (int s = 16; s > 0; s >>= 1)
-            if (__shfl_sync(FULL, incl, l + s - 1) <= e) l += s;
-        const int pos = __shfl_sync(FULL, shift, l) + e;
+        /* the owner: the last range that begins at or before the lane's element */
+        const unsigned at = (unsigned)(incl - len - e0);
+        const unsigned heads = __reduce_or_sync(FULL, lane < n && at < 32u ? 1u << at : 0u);
+        const int l = begun + __popc(heads & ((2u << lane) - 1u)) - 1;
+        begun += __popc(heads);
+        x.pos = __shfl_sync(FULL, shift, l) + e0 + lane;
         x.border = __shfl_sync(FULL, it.y, l) < 0;
         x.id = -1;
-        x.beg = x.end = 0;
         x.box = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (e < total) {
-            x.id = __ldg(ids + pos);
-            bytes += 4;
-            if (x.border) {
-                x.box = __ldg(gbox + pos);
-                x.beg = __ldg(gbeg + pos);
-                x.end = __ldg(gbeg + pos + 1);
-                bytes += 24;
-            }
+        if (e0 + lane < total) {
+            x.id = __ldg(ids + x.pos);
+            if (x.border) x.box = __ldg(gbox + x.pos);
         }
         return x;
     };
@@ -456,18 +452,17 @@ __device__ __forceinline__ void take_items(const int2* items, int n, const Box& 
         const unsigned m = __ballot_sync(FULL, open);
         if (open) {
             const int k = nopen + __popc(m & ((1u << lane) - 1u));
-            og.beg[k] = x.beg;
-            og.end[k] = x.end;
+            og.at[k] = x.pos;
             og.id[k] = x.id;
         }
         nopen += __popc(m);
         __syncwarp();
         if (nopen > kOpen - 32) {
-            test_open(og, nopen, q, X, Y, t, bytes);
+            test_open(og, nopen, q, gbeg, X, Y, t, bytes);
             nopen = 0;
         }
     }
-    if (nopen) test_open(og, nopen, q, X, Y, t, bytes);
+    if (nopen) test_open(og, nopen, q, gbeg, X, Y, t, bytes);
     work += bytes;
 }
 
