@@ -671,14 +671,16 @@ __device__ __forceinline__ bool row_tile(const float2* __restrict__ rows, const 
     const carry_t tag_hi = tag_out << 16;
     const int from = cin ? fr.above : kNever; /* first column whose value above comes from cin */
     float2 nb = make_float2(0.f, 0.f);
-    carry_t nw = 0;
-    bool nw_ok = false;
+    /* The next chunk's carry word as loaded; its tag is looked at when that chunk starts, never beside
+     * the load, where the compare would hold the warp for an L2 round trip in every chunk (two tiles of
+     * 64 rows over 16,384 columns: 95 cycles a step with the compare there, 82 without; chunks without
+     * matches 78 and 64). A load later in the chunk's loop, closer to its use, shortens the lag between
+     * tiles but costs more: the loop waits for it (95 again), and the loop cut in two for it does not
+     * stay in the instruction cache (4,096 pairs of mid length, 4 rows a lane: 0.166 -> 0.193 ms). */
+    carry_t nw = 0; /* no tag is 0: epochs start at 1 */
     if (c0 + lane < len2) {
         nb = cols[c0 + lane];
-        if (c0 + lane >= from) {
-            nw = ld_carry(cin + c0 + lane + 1);
-            nw_ok = (nw >> 16) == tag_in;
-        }
+        if (c0 + lane >= from) nw = ld_carry(cin + c0 + lane + 1);
     }
     float2* pts = reinterpret_cast<float2*>(sh.pts);
     unsigned near = 0; /* bit 0: this chunk holds a near column, bits 1 and 2: the two before */
@@ -689,7 +691,7 @@ __device__ __forceinline__ bool row_tile(const float2* __restrict__ rows, const 
             unsigned cv = s0 < from ? (unsigned)(kBias + unmatched_e(t0, c + 1)) : 0u;
             if (s0 + 31 >= from) {
                 const bool want = c >= from && c < len2;
-                bool ok = !want || nw_ok;
+                bool ok = !want || (nw >> 16) == tag_in;
                 for (int polls = 0;; polls++) {
                     if (!ok) {
                         nw = ld_carry(cin + c + 1);
@@ -709,13 +711,9 @@ __device__ __forceinline__ bool row_tile(const float2* __restrict__ rows, const 
             reinterpret_cast<unsigned*>(sh.in)[lane] = cv << 16;
             __syncwarp();
             const int cn = c + 32;
-            nw_ok = false;
             if (cn < len2) {
                 nb = cols[cn];
-                if (cn >= from) {
-                    nw = ld_carry(cin + cn + 1);
-                    nw_ok = (nw >> 16) == tag_in;
-                }
+                if (cn >= from) nw = ld_carry(cin + cn + 1);
             }
         } else {
             __syncwarp();
