@@ -1643,20 +1643,57 @@ int run_batch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, int
 /* Offsets and gather of a batch (ids, or point keys when pidx_bits >= 0) whose counts are known on the device only: nothing is copied
  * when the ids do not fit the caller's capacity or the arena, or when queries are left for the bitmap
  * scan (ctr as in range_groups_launch); the host then learns it from ctr and off[nq].
- * Up to kGatherScan queries the CTAs sum the counts themselves, so a small batch needs no scan
- * launches; ctr[8] receives the total. */
+ * Up to kGatherScan queries (SCAN) the CTAs sum the counts themselves, a CTA a query, so a small batch
+ * needs no scan launches; ctr[8] receives the total. Beyond, a warp copies a query, four ids a lane in
+ * flight, and knows its next query's place before it copies: the time is the chain of dependent loads
+ * a query costs (place, ids), not the 170 MB that 100k rectangles on 1M walks move (the batch
+ * 1995 us with a CTA a query, 1930 us with a warp). */
 constexpr int kGatherScan = 1024;
 
+template <bool SCAN>
 __global__ void __launch_bounds__(kThreads) k_gather_groups(int nq, const int64_t* __restrict__ segbase,
                                                          const int64_t* __restrict__ segcnt, int64_t* off,
                                                          const uint32_t* __restrict__ arena, int64_t arena_cap, int32_t* out,
-                                                         int64_t capacity, unsigned long long* ctr, bool scan, int pidx_bits,
+                                                         int64_t capacity, unsigned long long* ctr, int pidx_bits,
                                                          int32_t* out_pidx) {
-    __shared__ int64_t wsum[2][kThreads / 32];
-    int64_t total = scan ? 0 : off[nq];
-    for (int qi = blockIdx.x; qi < nq; qi += gridDim.x) {
-        int64_t o = 0;
-        if (scan) {
+    auto put = [&](int64_t at, uint32_t k) {
+        out[at] = pidx_bits < 0 ? (int32_t)k : (int32_t)(k >> pidx_bits);
+        if (pidx_bits >= 0 && out_pidx) out_pidx[at] = (int32_t)(k & ((1u << pidx_bits) - 1u));
+    };
+    if constexpr (!SCAN) {
+        constexpr int kFlight = 4;
+        const int lane = threadIdx.x & 31, warps = gridDim.x * (kThreads / 32);
+        int qi = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+        const int64_t total = off[nq];
+        if (qi == 0 && lane == 0) ctr[8] = (unsigned long long)total;
+        if (total > capacity || (int64_t)ctr[0] > arena_cap || ctr[3] != 0 || qi >= nq) return;
+        int64_t o = off[qi], b = segbase[qi], n = segcnt[qi];
+        for (;;) {
+            const bool more = qi < nq - warps;
+            const int next = more ? qi + warps : 0;
+            int64_t o2 = 0, b2 = 0, n2 = 0;
+            if (more) {
+                o2 = off[next];
+                b2 = segbase[next];
+                n2 = segcnt[next];
+            }
+            for (int64_t i = lane; i < n; i += 32 * kFlight) {
+                uint32_t k[kFlight];
+#pragma unroll
+                for (int f = 0; f < kFlight; f++) k[f] = i + 32 * f < n ? arena[b + i + 32 * f] : 0u;
+#pragma unroll
+                for (int f = 0; f < kFlight; f++)
+                    if (i + 32 * f < n) put(o + i + 32 * f, k[f]);
+            }
+            if (!more) break;
+            qi = next;
+            o = o2;
+            b = b2;
+            n = n2;
+        }
+    } else {
+        __shared__ int64_t wsum[2][kThreads / 32];
+        for (int qi = blockIdx.x; qi < nq; qi += gridDim.x) {
             int64_t before = 0, all = 0;
             for (int j = threadIdx.x; j < nq; j += kThreads) {
                 const int64_t c = segcnt[j];
@@ -1673,7 +1710,7 @@ __global__ void __launch_bounds__(kThreads) k_gather_groups(int nq, const int64_
                 wsum[1][threadIdx.x >> 5] = all;
             }
             __syncthreads();
-            total = 0;
+            int64_t o = 0, total = 0;
             for (int w = 0; w < kThreads / 32; w++) {
                 o += wsum[0][w];
                 total += wsum[1][w];
@@ -1681,21 +1718,11 @@ __global__ void __launch_bounds__(kThreads) k_gather_groups(int nq, const int64_
             if (threadIdx.x == 0) {
                 off[qi] = o;
                 if (qi == nq - 1) off[nq] = total;
+                if (qi == 0) ctr[8] = (unsigned long long)total;
             }
-        } else {
-            o = off[qi];
-        }
-        if (qi == 0 && threadIdx.x == 0) ctr[8] = (unsigned long long)total;
-        if (total > capacity || (int64_t)ctr[0] > arena_cap || ctr[3] != 0) continue;
-        const int64_t b = segbase[qi], n = segcnt[qi];
-        for (int64_t i = threadIdx.x; i < n; i += kThreads) {
-            const uint32_t k = arena[b + i];
-            if (pidx_bits < 0) {
-                out[o + i] = (int32_t)k;
-            } else {
-                out[o + i] = (int32_t)(k >> pidx_bits);
-                if (out_pidx) out_pidx[o + i] = (int32_t)(k & ((1u << pidx_bits) - 1u));
-            }
+            if (total > capacity || (int64_t)ctr[0] > arena_cap || ctr[3] != 0) continue;
+            const int64_t b = segbase[qi], n = segcnt[qi];
+            for (int64_t i = threadIdx.x; i < n; i += kThreads) put(o + i, arena[b + i]);
         }
     }
 }
@@ -1720,8 +1747,12 @@ int run_groups(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, in
         const bool scan = nq <= kGatherScan;
         int rc = GAT_OK;
         if (!scan && (rc = scan_i64(ctx, segcnt, d_off, nq)) != GAT_OK) return rc;
-        k_gather_groups<<<std::max(1, std::min(nq, ctx->sm_count * 8)), kThreads, 0, s>>>(nq, segbase, segcnt, d_off, arena, cap,
-                                                                                    d_tid, capacity, ctr, scan, ids ? -1 : ix->pidx_bits, d_pidx);
+        const int bits = ids ? -1 : ix->pidx_bits;
+        if (scan)
+            k_gather_groups<true><<<nq, kThreads, 0, s>>>(nq, segbase, segcnt, d_off, arena, cap, d_tid, capacity, ctr, bits, d_pidx);
+        else
+            k_gather_groups<false><<<std::min((nq + kThreads / 32 - 1) / (kThreads / 32), ctx->sm_count * 8), kThreads, 0, s>>>(
+                nq, segbase, segcnt, d_off, arena, cap, d_tid, capacity, ctr, bits, d_pidx);
         count_launch(ctx);
         GAT_CUDA_TRY(ctx, cudaGetLastError(), "range gather launch");
         GAT_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_pinned, ctr, 9 * sizeof(int64_t), cudaMemcpyDeviceToHost, s), "range");

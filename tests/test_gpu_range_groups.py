@@ -141,3 +141,15 @@ def test_snapshot_keeps_groups(gpu_ctx, tmp_path):
         assert back.info()["device_bytes"] == ix.info()["device_bytes"]
         a, b = ix.range_query(q), back.range_query(q)
         assert np.array_equal(a.offsets, b.offsets) and np.array_equal(a.tids, b.tids)
+
+
+@pytest.mark.parametrize("nq", [1024, 1025, 1185, 9473])
+def test_point_lists_of_long_batches(gpu_ctx, nq):
+    """Both gathers of a batch's point lists: a CTA a query, and a warp a query in one and in two turns."""
+    t = D.walks(D.lengths(3_000, 0, 0, 0, 20, 200, 36), 36)
+    g = G.Grid(gpu_ctx, G.TrajectorySet(gpu_ctx, t), D.BOX, 0.005, 2, 512)
+    q = D.boxes(nq, 1, 0.001, 0.05, 37)
+    a = _general(gpu_ctx, g, q, "points")
+    b = g.range_query(q, "points", "batched", capacity=4_000_000)
+    assert np.array_equal(a.offsets, b.offsets)
+    assert np.array_equal(a.tids, b.tids) and np.array_equal(a.pidx, b.pidx)
