@@ -31,9 +31,12 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 OPS_PER_CELL = 12  # int32 / fp32 instructions per DP cell of the EDR recurrence (match test, three-way min, carries)
-# ALU-pipe instructions per DP cell of k_edr_tiles (8 rows per lane, row tiles) from an ncu capture of the
-# C4 launch: ALU pipe 76.7% busy over the active cycles at 64 lanes per clock per SM, 2.257 G cells
-ALU_PER_CELL = 10.2
+# ALU-pipe instructions per DP cell of k_edr_rows (8 rows per lane, two cells per word) from an ncu capture of
+# the C4 pairs: 306.5 M warp instructions on the ALU pipe for 2.170 G cells
+ALU_PER_CELL = 4.5
+# of the top-k workloads: their cell rate says nothing about how busy the kernel's lanes are
+TOPK_CELLS_NOTE = ("cells count every evaluated pair, also those whose boxes lie apart and whose distance is known in closed "
+                   "form without a DP cell, so no fraction of the peak is given")
 
 
 def log(*a):
@@ -331,9 +334,9 @@ def roofline_c2(edr, bnd, hbm_gbs, clk):
     achieved = per_launch_cells / per_launch_s / 1e9
     mhz = clk.get("sm_mhz") or 1965.0
     peak = 148 * 128 * mhz * 1e6 / OPS_PER_CELL / 1e9
-    return {"kernel": "k_edr", "bound": "alu", "achieved": round(achieved, 2), "peak": round(peak, 1), "unit": "Gcell/s",
-            "frac": round(achieved / peak, 4), "traffic": None,
-            "note": f"peak = 148 SM x 128 int32 lanes x measured SM clock / {OPS_PER_CELL} ops per cell"}
+    return {"kernel": "k_edr_rows", "bound": "alu", "achieved": round(achieved, 2), "peak": round(peak, 1), "unit": "Gcell/s",
+            "frac": None, "traffic": None,
+            "note": f"peak = 148 SM x 128 int32 lanes x measured SM clock / {OPS_PER_CELL} ops per cell; {TOPK_CELLS_NOTE}"}
 
 
 def cpu_baseline_c2(t, qids, sample=32, reps=1):
@@ -435,11 +438,10 @@ def hbm_peak():
     return float(p.get("hbm_gbs", 6650.0)), ("measured" if "hbm_gbs" in p else "fallback")
 
 
-# DRAM read + write / algorithmic bytes of k_range_hash, from one-pass ncu captures (dram__bytes_read.sum,
-# dram__bytes_write.sum) of the C3 batch on the 1M-walk set in the tuned shape (small queries one per warp):
-# Grid (4.319 + 0.088) GB / 20.79 GB; FSG (block mode) (5.333 + 0.088) GB / 41.29 GB. The locality order serves
-# neighbouring queries' points from L2.
-RANGE_TRAFFIC_RATIO = {"grid": 0.212, "fsg": 0.131}
+# DRAM read + write / algorithmic bytes of k_range_groups, from one-pass ncu captures (dram__bytes_read.sum,
+# dram__bytes_write.sum) of the C3 batch on the 1M-walk set: Grid (1.931 + 0.085) GB / 2.040 GB; FSG
+# (2.462 + 0.085) GB / 3.194 GB. Reads move 32-byte sectors, of which a short list or run uses a part.
+RANGE_TRAFFIC_RATIO = {"grid": 0.988, "fsg": 0.797}
 
 
 def range_roofline(st, name, index="grid"):
@@ -453,12 +455,11 @@ def range_roofline(st, name, index="grid"):
     return {"kernel": name, "bound": "hbm", "achieved": round(ach, 1), "peak": gbs, "unit": "GB/s",
             "frac": round(ach / gbs, 4), "traffic": round(ratio * per_bytes) if ratio else None,
             "work_per_launch": per_bytes,
-            "note": f"algorithmic bytes: 8 B (x, y) per tested point + 4 B per hit + 4 B per point of an all-hit item; "
-                    f"peak of {src}; traffic = "
+            "note": f"algorithmic bytes: 4 B per id of a node inside the rectangle, 20 B (id, box) per point group of a "
+                    f"node on its border, 8 B (x, y) per tested point; peak of {src}; traffic = "
                     + (f"{ratio} x algorithmic, the dram read+write / algorithmic ratio of a one-pass ncu capture of "
-                       f"this index's k_range_hash on the 1M-walk C3 batch" if ratio else "not captured for this index")
-                    + "; DRAM traffic well below the algorithmic bytes means L2 serves most of them (locality order), "
-                      "so the kernel is issue-bound, not HBM-bound"}
+                       f"this index's k_range_groups on the 1M-walk C3 batch" if ratio else "not captured for this index")
+                    + "; the kernel is bound by issue and latency (walk, id set and sort of each query), not by HBM"}
 
 
 def edr_roofline(st, clk):
@@ -470,7 +471,7 @@ def edr_roofline(st, clk):
     mhz = clk.get("sm_mhz") or 1965.0
     peak = 148 * 128 * mhz * 1e6 / OPS_PER_CELL / 1e9
     alu = 148 * 64 * mhz * 1e6 / ALU_PER_CELL / 1e9
-    return {"kernel": "k_edr", "bound": "alu", "achieved": round(ach, 2), "peak": round(peak, 1), "unit": "Gcell/s",
+    return {"kernel": "k_edr_rows", "bound": "alu", "achieved": round(ach, 2), "peak": round(peak, 1), "unit": "Gcell/s",
             "frac": round(ach / peak, 4), "traffic": None, "work_per_launch": per_cells,
             "note": f"peak = 148 SM x 128 int32 lanes x sampled SM clock / {OPS_PER_CELL} ops per cell (nominal issue rate)",
             "alu_pipe": {"peak": round(alu, 1), "frac": round(ach / alu, 4), "alu_instructions_per_cell": ALU_PER_CELL,
@@ -567,7 +568,7 @@ def run_c1(args, world, rank, local, td):
                 "h2d_bytes_per_step": int(q.nbytes), "d2h_bytes_per_step": int((nq + 1) * 8 + total_ids * 4)},
         "gpu_launches": int(launches),
         "batched": {"value": round(nq * world * args.steps / (btot / 1e3), 3), "unit": "queries/s",
-                    "speedup_vs_plain": round(tot / btot, 2), "roofline": range_roofline(bscan, "k_range_hash", None)},
+                    "speedup_vs_plain": round(tot / btot, 2), "roofline": range_roofline(bscan, "k_range_groups", None)},
         "roofline": range_roofline(scan, "k_plain_scan", None),
         "clocks": clk,
         "result_ids": total_ids,
@@ -704,10 +705,10 @@ def run_c3(args, world, rank, local, td):
                 "h2d_bytes_per_step": int(q.nbytes), "d2h_bytes_per_step": int((nq + 1) * 8 + g["ids"] * 4)},
         "gpu_launches": int(g["launches"]),
         "indexes": {k: {"queries_per_s": round(nq * world * args.steps / (v["ms"] / 1e3), 1), "result_ids": v["ids"],
-                        "roofline": range_roofline(v["scan"], "k_range_hash", k)} for k, v in res.items()},
+                        "roofline": range_roofline(v["scan"], "k_range_groups", k)} for k, v in res.items()},
         "plain_sample": {"queries": ns, "queries_per_s": round(plain_qps, 1),
                          "batched_speedup": round(nq * world * args.steps / (g["ms"] / 1e3) / plain_qps, 1)},
-        "roofline": range_roofline(g["scan"], "k_range_hash"),
+        "roofline": range_roofline(g["scan"], "k_range_groups"),
         "clocks": g["clk"],
     })
     ctx.close()
@@ -932,7 +933,7 @@ def run_c4k(args, world, rank, local, td):
         "pruned_fraction": round(1.0 - float(stats[0]) / (nq * t.n), 6),
         "gcups_evaluated": round(cells / (edr["ms"] / 1e3) / 1e9, 2) if edr["ms"] else None,
         "kernels": {"edr": edr, "bounds": bnd},
-        "roofline": edr_roofline(edr, clk),
+        "roofline": dict(edr_roofline(edr, clk) or {}, frac=None, alu_pipe=None, note=TOPK_CELLS_NOTE),
         "exhaustive_check": {"queries": int(len(chk)), "identical": ok},
         "clocks": clk,
     })
@@ -1446,12 +1447,12 @@ def run_suite(args, world, rank, local, td):
                 "h2d_bytes_per_step": int(q.nbytes), "d2h_bytes_per_step": int((nq + 1) * 8 + len(grid_ids) * 4),
                 "call": "gat_range_query (pinned host rectangles in, CSR id sets out), GT-quadtree, batched"},
         "gpu_launches": int(g["launches"]),
-        "roofline": range_roofline(g["scan"], "k_range_hash"),
+        "roofline": range_roofline(g["scan"], "k_range_groups"),
         "clocks": clk,
         "range": {
             "indexes": {k: {"queries_per_s": round(nq * world * args.steps / (v["ms"] / 1e3), 1), "result_ids": v["ids"],
                             "ms_per_step": round(v["ms"] / args.steps, 4),
-                            "roofline": range_roofline(v["scan"], "k_range_hash", k)} for k, v in res.items()},
+                            "roofline": range_roofline(v["scan"], "k_range_groups", k)} for k, v in res.items()},
             "plain": {"queries": ps, "steps": len(pms), "queries_per_s": round(plain_qps, 1),
                       "form": "gat_range_query_dev with GAT_EXEC_PLAIN: one query per launch sequence",
                       "sample": f"every {nq // ps}th of the 100k rectangles"},

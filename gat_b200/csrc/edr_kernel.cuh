@@ -203,8 +203,8 @@ __global__ void __launch_bounds__(kWarps * 32) k_edr(Src src, float u, int* __re
  * accepts a word whose tag is the one it expects, so the hand-over needs neither a progress
  * flag nor a memory fence: a 64-bit store is seen whole or not at all. Values are the
  * column-shifted distances E = D - c, which lie in [-16384, 16384] and fit 16 bits; epochs
- * come from a per-context device counter and only grow (2^40 launches before a repeat), and carry buffers are zeroed when allocated, so a
- * stale word never carries the expected tag. A tile rewrites the buffer its predecessor read
+ * come from a per-context device counter and only grow (2^40 launches before a repeat), and carry
+ * buffers are zeroed when allocated, so a stale word never carries the expected tag. A tile rewrites the buffer its predecessor read
  * (double buffering per pair) only for columns that predecessor has already consumed.
  *
  * Schedule (longest first): a count pass puts every pair in one of kClasses duration classes
@@ -419,7 +419,7 @@ __device__ __forceinline__ int match_mask(float ax, float ay, float2 b, float u)
  * ran at 62 lanes per clock and SM on a B200, float adds at 117 and multiply-adds at 62 beside
  * them). Two cells take 8 ALU and 7 FMA-pipe instructions where a match is possible and 4 + 1 where
  * it is not, against 14 ALU and 4 FMA for two cells held one per word. Measured on 4,096 pairs of
- * log-uniform [16, 4096] lengths: 0.87 ms, 2.5 Tcell/s; one cell per word: 1.62 ms, 1.34 Tcell/s. */
+ * log-uniform [16, 4096] lengths: 0.84 ms, 2.6 Tcell/s; one cell per word: 1.62 ms, 1.34 Tcell/s. */
 constexpr int kBias = 16384;
 constexpr unsigned kHalfOnes = 0x00010001u, kHalfTops = 0x80008000u, kHalfRest = 0x7fff7fffu;
 
@@ -591,8 +591,8 @@ __device__ __forceinline__ void put_words(unsigned addr, const unsigned (&v)[4],
  * carry values come in 128-bit shared loads, their bottom-row words leave in one store. UN groups of
  * four are unrolled: two where the kernel holds the loops of one or two tile heights, one where it
  * holds three, since warps in loops that do not fit the instruction cache together wait for
- * instructions (4,096 pairs of log-uniform [16, 4096] lengths, 8 rows per lane: 0.86 ms with one
- * group, 1.15 ms with two; 4 rows: 0.96 and 0.92 ms). */
+ * instructions (4,096 pairs of log-uniform [16, 4096] lengths, 8 rows per lane: 0.85 ms with one
+ * group, 1.03 ms with two; 4 rows: 0.94 and 0.91 ms). */
 template <int H, int UN, bool MATCH, bool MASKED>
 __device__ __forceinline__ void row_chunk(const float (&ax)[2 * H], const float (&ay)[2 * H], unsigned (&L)[H], unsigned& d0,
                                           RowShared& sh, int s0, int kend, int c0, int len2, bool writer, float u,

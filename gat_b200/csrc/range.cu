@@ -1640,9 +1640,10 @@ int run_batch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, int
     return GAT_OK;
 }
 
-/* Offsets and gather of a batch (ids, or point keys when pidx_bits >= 0) whose counts are known on the device only: nothing is copied
- * when the ids do not fit the caller's capacity or the arena, or when queries are left for the bitmap
- * scan (ctr as in range_groups_launch); the host then learns it from ctr and off[nq].
+/* Offsets and gather of a batch (ids, or point keys when pidx_bits >= 0) whose counts are known on the
+ * device only: nothing is copied when the ids do not fit the caller's capacity or the arena, or when
+ * queries are left for the bitmap scan (ctr as in range_groups_launch); the host then learns it from
+ * ctr and off[nq].
  * Up to kGatherScan queries (SCAN) the CTAs sum the counts themselves, a CTA a query, so a small batch
  * needs no scan launches; ctr[8] receives the total. Beyond, a warp copies a query, four ids a lane in
  * flight, and knows its next query's place before it copies: the time is the chain of dependent loads

@@ -17,7 +17,7 @@
  * pair of warps, or the CTA of 256 threads, each with its share of the CTA's shared memory (an eighth,
  * a quarter, all). Small teams keep more queries in flight and wait less at barriers: 15k rectangles
  * of 0.02 to 0.05 degrees over 1M walks took 2.07 ms by CTAs alone, 1.86 ms with pairs for those of
- * 400 to 1,100 expected ids (1.16 ms less on 100k of 0.001 to 0.05). A query that outgrows its team
+ * 400 to 1,100 expected ids. A query that outgrows its team
  * runs again on the CTA, one that outgrows that goes to the bitmap scan (range.cu).
  *
  * Plain execution (one query per launch): the CTA answers one query and writes it where the query before

@@ -127,9 +127,9 @@ int gat_ctx_kernel_stats(gat_ctx* ctx, int kernel_class, double* ms, int64_t* la
  *   range lane; 0 (default) = 12. Same results.
  * GAT_TUNE_RANGE_SHAPE: how batched range queries find trajectory-id sets. 0 (default): through
  *   the index's point groups (the runs of one trajectory inside one leaf or cell, with their boxes);
- *   on an index whose groups found no memory by the point scan with an autotuned block shape: the first batch of each (index kind, batch size rounded up to a
- *   power of two) class times the shapes on its own queries and keeps the fastest. 1..3: the point
- *   scan on every index with a fixed shape: 1 = 256 threads per CTA with an 8192-slot id set, 2 = 128
+ *   on an index whose groups found no memory by the point scan with an autotuned block shape: the
+ *   first batch of each (index kind, batch size rounded up to a power of two) class times the shapes
+ *   on its own queries and keeps the fastest. 1..3: the point scan on every index with a fixed shape: 1 = 256 threads per CTA with an 8192-slot id set, 2 = 128
  *   threads with a 4096-slot set, 3 = the batch split by size (queries with more than 16 candidate
  *   items on shape 1, the others one per warp with a 1024-slot set and no block barrier, in the same
  *   launch). Same results. Setting the knob clears the tuned table.
