@@ -271,9 +271,9 @@ void index_groups_free(gat_index* ix);
 int range_groups_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, uint32_t* arena, int64_t cap,
                         unsigned long long* ctr, int64_t* segbase, int64_t* segcnt, int* ovf_list, bool timed);
 /* Point lists likewise (Grid, FSG, MortonGrid; keys in the arena), queries of more than 4,096 points left
- * in ovf_list. */
+ * in ovf_list; again: nq ints of its own. */
 int group_points_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, uint32_t* arena, int64_t cap,
-                        unsigned long long* ctr, int64_t* segbase, int64_t* segcnt, int* ovf_list);
+                        unsigned long long* ctr, int64_t* segbase, int64_t* segcnt, int* ovf_list, int* again);
 /* Plain execution of id-set query qi over an index with groups, launched in the order of qi: writes
  * off[qi + 1] (and off[0]) and the ids at off[qi]; state: [0] set when they do not fit, [1] = 1 + the first
  * query that outgrew the kernel (later ones then write nothing), [2..3] the end so far (64-bit). */

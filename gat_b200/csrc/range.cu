@@ -1739,7 +1739,7 @@ int run_groups(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, in
     int64_t* segbase = (int64_t*)scratch(ctx, S_RANGE_SEGBASE, (nq + 1) * sizeof(int64_t), &st);
     int64_t* segcnt = (int64_t*)scratch(ctx, S_RANGE_SEGCNT, (nq + 1) * sizeof(int64_t), &st);
     unsigned long long* ctr = (unsigned long long*)scratch(ctx, S_RANGE_CURSOR, 128, &st);
-    int* ovf_list = (int*)scratch(ctx, S_RANGE_OVF, (size_t)(nq + 1) * sizeof(int), &st);
+    int* ovf_list = (int*)scratch(ctx, S_RANGE_OVF, (ids ? 1 : 2) * (size_t)(nq + 1) * sizeof(int), &st);
     if (!segbase || !segcnt || !ctr || !ovf_list) return st;
     int64_t cap = std::max<int64_t>(1 << 20, (int64_t)nq * 256);
     uint32_t* arena = nullptr;
@@ -1766,7 +1766,7 @@ int run_groups(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, in
         cap = (int64_t)(ctx->slot_bytes[S_RANGE_ARENA] / 4);
         timed_begin(ctx, GAT_KERNEL_RANGE_SCAN);
         st = ids ? range_groups_launch(ctx, ix, d_q, nq, arena, cap, ctr, segbase, segcnt, ovf_list, ctx->timing)
-                 : group_points_launch(ctx, ix, d_q, nq, arena, cap, ctr, segbase, segcnt, ovf_list);
+                 : group_points_launch(ctx, ix, d_q, nq, arena, cap, ctr, segbase, segcnt, ovf_list, ovf_list + nq + 1);
         timed_end(ctx, GAT_KERNEL_RANGE_SCAN, 0.0);
         if (st != GAT_OK || (st = finish()) != GAT_OK) return st;
         const int64_t n_ovf = ctx->h_pinned[3];

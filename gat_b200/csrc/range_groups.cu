@@ -116,6 +116,7 @@ struct Team {
     }
 };
 using BlockTeam = Team<kBlockBits, kBlockIds, kBlockFront, kBlockItems, kNT>;
+using LongTeam = Team<14, 14336, kBlockFront, kBlockItems, kNT>; /* point lists: one CTA per SM */
 using MidTeam = Team<kMidBits, kMidIds, kMidFront, kMidItems, 64>;
 using SmallTeam = Team<kSmallBits, kSmallIds, kSmallFront, kSmallItems, 32>;
 constexpr int kInts = BlockTeam::kInts;
@@ -809,10 +810,15 @@ __global__ void __launch_bounds__(kNT, 2) k_plain_groups(GroupQuery a, int qi) {
 }
 
 /* Point lists: the keys (trajectory << bits | point index) of the points inside, ascending. A query of
- * more than kBlockIds points, or one that outgrows the walk's memory, goes on the overflow list for
- * k_range_points. Keys are held with the top bit flipped, so that signed compares order them. */
-template <int KIND>
-__global__ void __launch_bounds__(kNT, 3) k_group_points(GroupQuery a, const uint32_t* __restrict__ key, int nq) {
+ * more than T::IDS points (known at once when the nodes inside it hold more), or one that outgrows the
+ * walk's memory, is left: by the first pass to the second (AGAIN, the list `again` of ctr[5] queries),
+ * which has 3.5 times the memory and one CTA per SM, by that on the overflow list for k_range_points.
+ * Without the second pass a batch with some long lists paid the items and the host's wait for them: 710
+ * rectangles of 0.0055 to 0.05 degrees on an FSG of 16k walks 303 us, 254 us now (the point scan 267 us). Keys are held with the top bit flipped, so that signed compares order them. */
+template <int KIND, class T, bool AGAIN>
+__global__ void __launch_bounds__(kNT, AGAIN ? 1 : 3) k_group_points(GroupQuery a, const uint32_t* __restrict__ key, int nq,
+                                                                      int* __restrict__ again) {
+    dep_wait();
     extern __shared__ int4 smem4[];
     int* mem = reinterpret_cast<int*>(smem4);
     __shared__ __align__(8) int ctl[kCtl];
@@ -820,14 +826,16 @@ __global__ void __launch_bounds__(kNT, 3) k_group_points(GroupQuery a, const uin
     const int lane = threadIdx.x & 31, me = threadIdx.x;
     const unsigned FULL = 0xffffffffu;
     if (me < kCtl) ctl[me] = 0;
-    BlockTeam t(mem, ctl, 0);
+    T t(mem, ctl, 0);
     const float *X = a.g.X, *Y = a.g.Y;
+    const int todo = AGAIN ? (int)a.ctr[5] : nq;
     for (;;) {
-        if (me == 0) q_sh = (int)atomicAdd(&a.ctr[2], 1ull);
+        if (me == 0) q_sh = (int)atomicAdd(&a.ctr[AGAIN ? 4 : 2], 1ull);
         __syncthreads();
-        const int qi = q_sh;
+        const int turn = q_sh;
         __syncthreads();
-        if (qi >= nq) break;
+        if (turn >= todo) break;
+        const int qi = AGAIN ? again[turn] : turn;
         const Box q = load_box(a.queries, qi);
         if (KIND == GAT_INDEX_GRID)
             walk_grid<true>(a.g, a.grid, q, t, me);
@@ -835,8 +843,16 @@ __global__ void __launch_bounds__(kNT, 3) k_group_points(GroupQuery a, const uin
             walk_morton(a.morton, a.morton.cbeg, q, t, me);
         else
             walk_fsg<true>(a.fsg, nullptr, q, t, me);
-        const int n = min(*t.nitems, BlockTeam::ITEMS);
-        if (!__shfl_sync(FULL, *(volatile int*)t.ovf, 0)) {
+        const int n = min(*t.nitems, T::ITEMS);
+        /* the points of the nodes inside */
+        int inside = 0;
+        for (int i = me; i < n; i += kNT)
+            if (t.items[i].y >= 0) inside += t.items[i].y - t.items[i].x;
+        inside = __reduce_add_sync(FULL, inside);
+        if (lane == 0 && inside) atomicAdd(t.query, inside);
+        __syncthreads();
+        const bool many = *t.query > T::IDS;
+        if (!many && !__shfl_sync(FULL, *(volatile int*)t.ovf, 0)) {
             for (;;) {
                 int k = 0;
                 if (lane == 0) k = atomicAdd(t.next, 1);
@@ -865,18 +881,18 @@ __global__ void __launch_bounds__(kNT, 3) k_group_points(GroupQuery a, const uin
                         int at = 0;
                         if (lane == 0) at = atomicAdd(t.cnt, __popc(m));
                         at = __shfl_sync(FULL, at, 0) + __popc(m & ((1u << lane) - 1u));
-                        if (hit && at < kBlockIds) t.list[at] = (int)(kk[u] ^ 0x80000000u);
+                        if (hit && at < T::IDS) t.list[at] = (int)(kk[u] ^ 0x80000000u);
                     }
                 }
-                if (__shfl_sync(FULL, *(volatile int*)t.cnt, 0) > kBlockIds) break;
+                if (__shfl_sync(FULL, *(volatile int*)t.cnt, 0) > T::IDS) break;
             }
         }
         __syncthreads();
         const int m = *t.cnt;
-        const bool lost = *(volatile int*)t.ovf != 0 || m > kBlockIds;
+        const bool lost = many || *(volatile int*)t.ovf != 0 || m > T::IDS;
         if (me == 0) {
             if (lost) {
-                a.ovf_list[atomicAdd(&a.ctr[3], 1ull)] = qi;
+                (AGAIN ? a.ovf_list : again)[atomicAdd(&a.ctr[AGAIN ? 3 : 5], 1ull)] = qi;
                 a.segcnt[qi] = 0;
                 a.segbase[qi] = 0;
             } else {
@@ -888,10 +904,10 @@ __global__ void __launch_bounds__(kNT, 3) k_group_points(GroupQuery a, const uin
         __syncthreads();
         if (!lost) {
             const int64_t at = (int64_t)*t.base;
-            sort_ids<BlockTeam, 0x80000000u>(t, m, a.arena + at, at + m <= a.cap, me);
+            sort_ids<T, 0x80000000u>(t, m, a.arena + at, at + m <= a.cap, me);
         }
         __syncthreads();
-        if (me == 0) *t.nitems = t.nfront[0] = t.nfront[1] = *t.cnt = *t.ovf = *t.next = 0;
+        if (me == 0) *t.nitems = t.nfront[0] = t.nfront[1] = *t.cnt = *t.ovf = *t.next = *t.query = 0;
         __syncthreads();
     }
 }
@@ -1087,21 +1103,31 @@ int plain_groups_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, i
 }
 
 int group_points_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, uint32_t* arena, int64_t cap,
-                        unsigned long long* ctr, int64_t* segbase, int64_t* segcnt, int* ovf_list) {
+                        unsigned long long* ctr, int64_t* segbase, int64_t* segcnt, int* ovf_list, int* again) {
     cudaStream_t s = ctx->stream;
-    auto kernel = ix->kind == GAT_INDEX_GRID     ? k_group_points<GAT_INDEX_GRID>
-                  : ix->kind == GAT_INDEX_MORTON ? k_group_points<GAT_INDEX_MORTON>
-                                                 : k_group_points<GAT_INDEX_FSG>;
-    allow_smem(kernel, kSmem);
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kNT, kSmem);
-    GAT_CUDA_TRY(ctx, cudaMemsetAsync(ctr, 0, 8 * sizeof(unsigned long long), s), "range");
-    GroupQuery a{d_q, ix->grid, ix->fsg, ix->morton, ix->groups, arena, cap, ctr, segbase, segcnt, nullptr, nullptr, 0, nullptr,
-                 nullptr, ovf_list, nullptr};
-    kernel<<<std::min(nq, std::max(1, per_sm) * ctx->sm_count), kNT, kSmem, s>>>(a, ix->d_key, nq);
-    count_launch(ctx);
-    GAT_CUDA_TRY(ctx, cudaGetLastError(), "range scan launch");
-    return GAT_OK;
+    auto launch = [&](auto kind) -> int {
+        constexpr int KIND = decltype(kind)::value;
+        auto first = k_group_points<KIND, BlockTeam, false>;
+        auto second = k_group_points<KIND, LongTeam, true>;
+        constexpr size_t kLongSmem = (size_t)LongTeam::kInts * sizeof(int);
+        allow_smem(first, kSmem);
+        allow_smem(second, kLongSmem);
+        int per_sm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, first, kNT, kSmem);
+        GAT_CUDA_TRY(ctx, cudaMemsetAsync(ctr, 0, 8 * sizeof(unsigned long long), s), "range");
+        GroupQuery a{d_q, ix->grid, ix->fsg, ix->morton, ix->groups, arena, cap, ctr, segbase, segcnt, nullptr, nullptr, 0,
+                     nullptr, nullptr, ovf_list, nullptr};
+        first<<<std::min(nq, std::max(1, per_sm) * ctx->sm_count), kNT, kSmem, s>>>(a, ix->d_key, nq, again);
+        (void)launch_dep(ctx, second, dim3(std::min(nq, ctx->sm_count)), dim3(kNT), kLongSmem, s, a, (const uint32_t*)ix->d_key, nq,
+                         again);
+        count_launch(ctx);
+        count_launch(ctx);
+        GAT_CUDA_TRY(ctx, cudaGetLastError(), "range scan launch");
+        return GAT_OK;
+    };
+    if (ix->kind == GAT_INDEX_GRID) return launch(std::integral_constant<int, GAT_INDEX_GRID>{});
+    if (ix->kind == GAT_INDEX_MORTON) return launch(std::integral_constant<int, GAT_INDEX_MORTON>{});
+    return launch(std::integral_constant<int, GAT_INDEX_FSG>{});
 }
 
 }  // namespace gat

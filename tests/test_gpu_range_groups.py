@@ -153,3 +153,18 @@ def test_point_lists_of_long_batches(gpu_ctx, nq):
     b = g.range_query(q, "points", "batched", capacity=4_000_000)
     assert np.array_equal(a.offsets, b.offsets)
     assert np.array_equal(a.tids, b.tids) and np.array_equal(a.pidx, b.pidx)
+
+
+@pytest.mark.parametrize("walks", [64, 65, 224, 225])
+def test_long_point_lists(gpu_ctx, walks):
+    """Lists of 64 points a walk on both sides of what the two passes hold (4,096 and 14,336)."""
+    t = D.walks(D.lengths(walks, 0, 0, 0, 64, 64, 38), 38)
+    g = G.Grid(gpu_ctx, G.TrajectorySet(gpu_ctx, t), D.BOX, 0.005, 2, 64)
+    box = np.array([[t.lon.min(), t.lat.min(), t.lon.max(), t.lat.max()]], np.float32)
+    q = np.concatenate([box, D.boxes(30, 1, 0.1, 0.6, 39), box])
+    for ix in (g, G.FSG(gpu_ctx, g.db, D.BOX, 0.005), G.MortonGrid(g)):
+        a = _general(gpu_ctx, ix, q, "points")
+        b = ix.range_query(q, "points", "batched", capacity=4_000_000)
+        assert a.offsets[1] > 0
+        assert np.array_equal(a.offsets, b.offsets)
+        assert np.array_equal(a.tids, b.tids) and np.array_equal(a.pidx, b.pidx)
