@@ -473,7 +473,9 @@ __device__ __forceinline__ void take_items(const int2* items, int n, const Box& 
  * crowd in a few buckets the list is sorted in runs of 32 that are merged in pairs instead. (Sorting
  * runs and searching every id in every run took half of a query's instructions.) `out` may be the list
  * itself. FLIP is xored into what is written (point keys are held with their top bit flipped). */
-constexpr int kCrowd = 32;
+/* Fullest bucket that is ranked: ids, and point keys, which lie in clusters (1,500 rectangles of 0.003 to 0.03
+ * degrees on 100k walks: 1270 us with 32, 1132 us with 512). */
+constexpr int kCrowd = 32, kKeyCrowd = 512;
 
 template <class T, unsigned FLIP = 0>
 __device__ void sort_ids(T& t, int m, uint32_t* out, bool write, int me) {
@@ -540,7 +542,7 @@ __device__ void sort_ids(T& t, int m, uint32_t* out, bool write, int me) {
         most = lo_hi[2];
         for (int w = 0; w < warp; w++) start += lo_hi[4 + w];
     }
-    if (most <= kCrowd) {
+    if (most <= (FLIP ? kKeyCrowd : kCrowd)) {
 #pragma unroll
         for (int k = 0; k < kPer; k++) {
             tab[me * kPer + k] = start;
@@ -810,11 +812,12 @@ __global__ void __launch_bounds__(kNT, 2) k_plain_groups(GroupQuery a, int qi) {
 }
 
 /* Point lists: the keys (trajectory << bits | point index) of the points inside, ascending. A query of
- * more than T::IDS points (known at once when the nodes inside it hold more), or one that outgrows the
+ * more than T::IDS points, or with far more candidates than that, or one that outgrows the
  * walk's memory, is left: by the first pass to the second (AGAIN, the list `again` of ctr[5] queries),
  * which has 3.5 times the memory and one CTA per SM, by that on the overflow list for k_range_points.
  * Without the second pass a batch with some long lists paid the items and the host's wait for them: 710
- * rectangles of 0.0055 to 0.05 degrees on an FSG of 16k walks 303 us, 254 us now (the point scan 267 us). Keys are held with the top bit flipped, so that signed compares order them. */
+ * rectangles of 0.0055 to 0.05 degrees on an FSG of 16k walks 303 us, 254 us now (the point scan 267 us).
+ * Keys are held with the top bit flipped, so that signed compares order them. */
 template <int KIND, class T, bool AGAIN>
 __global__ void __launch_bounds__(kNT, AGAIN ? 1 : 3) k_group_points(GroupQuery a, const uint32_t* __restrict__ key, int nq,
                                                                       int* __restrict__ again) {
@@ -844,14 +847,16 @@ __global__ void __launch_bounds__(kNT, AGAIN ? 1 : 3) k_group_points(GroupQuery 
         else
             walk_fsg<true>(a.fsg, nullptr, q, t, me);
         const int n = min(*t.nitems, T::ITEMS);
-        /* the points of the nodes inside */
-        int inside = 0;
-        for (int i = me; i < n; i += kNT)
-            if (t.items[i].y >= 0) inside += t.items[i].y - t.items[i].x;
-        inside = __reduce_add_sync(FULL, inside);
-        if (lane == 0 && inside) atomicAdd(t.query, inside);
+        /* the candidate points: far more than the list holds go on unread, past the second pass where they
+         * are far more than it holds */
+        int all = 0;
+        for (int i = me; i < n; i += kNT) all += (t.items[i].y & ~kBorder) - t.items[i].x;
+        all = __reduce_add_sync(FULL, all);
+        if (lane == 0 && all) atomicAdd(t.query, all);
         __syncthreads();
-        const bool many = *t.query > T::IDS;
+        const int points = *t.query;
+        const bool last = AGAIN || points > LongTeam::IDS + LongTeam::IDS / 4;
+        const bool many = points > 2 * kBlockIds && (!AGAIN || points > 2 * T::IDS);
         if (!many && !__shfl_sync(FULL, *(volatile int*)t.ovf, 0)) {
             for (;;) {
                 int k = 0;
@@ -892,7 +897,7 @@ __global__ void __launch_bounds__(kNT, AGAIN ? 1 : 3) k_group_points(GroupQuery 
         const bool lost = many || *(volatile int*)t.ovf != 0 || m > T::IDS;
         if (me == 0) {
             if (lost) {
-                (AGAIN ? a.ovf_list : again)[atomicAdd(&a.ctr[AGAIN ? 3 : 5], 1ull)] = qi;
+                (last ? a.ovf_list : again)[atomicAdd(&a.ctr[last ? 3 : 5], 1ull)] = qi;
                 a.segcnt[qi] = 0;
                 a.segbase[qi] = 0;
             } else {
