@@ -24,7 +24,7 @@
  * it ended. Each launch lets the next start at once; a query waits for the one before only to read its
  * end, so the walks, scans and sorts of neighbouring launches overlap.
  *
- * Point lists (Grid, FSG, MortonGrid): the same walk gives ranges of points, the CTA collects the keys of
+ * Point lists (Grid, MortonGrid): the same walk gives ranges of points, the CTA collects the keys of
  * those inside, sorts and writes them.
  */
 #include <algorithm>
@@ -302,10 +302,9 @@ __device__ void walk_morton(const MortonDev& m, const int32_t* __restrict__ cell
  * arithmetic, so a point in a column strictly between g1 and g2 and a row strictly between g3 and g4
  * lies inside the query: those cells are taken whole, the rest by their groups' boxes. (A NaN
  * coordinate would break the ordering: no cell is then taken whole.) */
-template <bool PTS, class T>
+template <class T>
 __device__ void walk_fsg(const FsgDev& f, const int32_t* __restrict__ cell_g, const Box& q, T& t, int me) {
-    /* where cell c begins: its first group, or PTS its first point */
-    auto begin = [&](int c) { return PTS ? (c < f.cellnum ? f.cbeg[c] : f.cend[f.cellnum - 1]) : cell_g[c]; };
+    auto begin = [&](int c) { return cell_g[c]; }; /* the cell's first group */
     const int g1 = (int)__fdiv_rn(__fsub_rn(q.xmin, f.rxmin), f.cell), g2 = (int)__fdiv_rn(__fsub_rn(q.xmax, f.rxmin), f.cell);
     const int g3 = (int)__fdiv_rn(__fsub_rn(f.rymax, q.ymax), f.cell), g4 = (int)__fdiv_rn(__fsub_rn(f.rymax, q.ymin), f.cell);
     if (max(max(g1, g2), max(g3, g4)) > kFarCell || min(min(g1, g2), min(g3, g4)) < -kFarCell || g4 - g3 > 4 * T::ITEMS) {
@@ -644,7 +643,7 @@ __device__ bool answer(const GroupQuery& a, int qi, T& t, OpenGroups& og, int me
     else if (KIND == GAT_INDEX_MORTON)
         walk_morton(a.morton, a.g.cell_g, q, t, me);
     else
-        walk_fsg<false>(a.fsg, a.g.cell_g, q, t, me);
+        walk_fsg(a.fsg, a.g.cell_g, q, t, me);
     const int n = min(*t.nitems, T::ITEMS);
     if (!__shfl_sync(0xffffffffu, *(volatile int*)t.ovf, 0)) {
         /* ranges per turn: enough turns for every warp, up to 32 a turn */
@@ -815,8 +814,8 @@ __global__ void __launch_bounds__(kNT, 2) k_plain_groups(GroupQuery a, int qi) {
  * more than T::IDS points, or with far more candidates than that, or one that outgrows the
  * walk's memory, is left: by the first pass to the second (AGAIN, the list `again` of ctr[5] queries),
  * which has 3.5 times the memory and one CTA per SM, by that on the overflow list for k_range_points.
- * Without the second pass a batch with some long lists paid the items and the host's wait for them: 710
- * rectangles of 0.0055 to 0.05 degrees on an FSG of 16k walks 303 us, 254 us now (the point scan 267 us).
+ * Without the second pass a batch with some long lists paid the items and the host's wait for them (710
+ * rectangles of 0.0055 to 0.05 degrees on 16k walks: 303 us and 254 us with it).
  * Keys are held with the top bit flipped, so that signed compares order them. */
 template <int KIND, class T, bool AGAIN>
 __global__ void __launch_bounds__(kNT, AGAIN ? 1 : 3) k_group_points(GroupQuery a, const uint32_t* __restrict__ key, int nq,
@@ -842,10 +841,8 @@ __global__ void __launch_bounds__(kNT, AGAIN ? 1 : 3) k_group_points(GroupQuery 
         const Box q = load_box(a.queries, qi);
         if (KIND == GAT_INDEX_GRID)
             walk_grid<true>(a.g, a.grid, q, t, me);
-        else if (KIND == GAT_INDEX_MORTON)
-            walk_morton(a.morton, a.morton.cbeg, q, t, me);
         else
-            walk_fsg<true>(a.fsg, nullptr, q, t, me);
+            walk_morton(a.morton, a.morton.cbeg, q, t, me);
         const int n = min(*t.nitems, T::ITEMS);
         /* the candidate points: far more than the list holds go on unread, past the second pass where they
          * are far more than it holds */
@@ -1131,8 +1128,7 @@ int group_points_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, i
         return GAT_OK;
     };
     if (ix->kind == GAT_INDEX_GRID) return launch(std::integral_constant<int, GAT_INDEX_GRID>{});
-    if (ix->kind == GAT_INDEX_MORTON) return launch(std::integral_constant<int, GAT_INDEX_MORTON>{});
-    return launch(std::integral_constant<int, GAT_INDEX_FSG>{});
+    return launch(std::integral_constant<int, GAT_INDEX_MORTON>{});
 }
 
 }  // namespace gat
