@@ -270,7 +270,7 @@ int gat_ctx_create(int device, gat_ctx** out) {
         (e = cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaMalloc(&c->d_flag, 16 * sizeof(int32_t))) != cudaSuccess ||
-        (e = cudaMemset(c->d_flag, 0, 16 * sizeof(int32_t))) != cudaSuccess ||
+        (e = cudaMemsetAsync(c->d_flag, 0, 16 * sizeof(int32_t), c->stream)) != cudaSuccess ||
         (e = cudaMallocHost(&c->h_pinned, kPinnedWords * sizeof(int64_t) + kFirstStage)) != cudaSuccess) {
         cudaGetLastError();
         gat_ctx_destroy(c);
@@ -502,8 +502,8 @@ int gat_db_create(gat_ctx* ctx, int n, const int32_t* lengths, const float* lon,
         (e = cudaMalloc(&db->d_off, (n + 2) * sizeof(int64_t))) != cudaSuccess ||
         (e = cudaMalloc(&db->d_xy, (db->npoints + 1) * sizeof(float2))) != cudaSuccess ||
         (e = cudaMalloc(&db->d_box, (n + 1) * sizeof(float4))) != cudaSuccess ||
-        (e = cudaMemcpy(db->d_len, db->h_len.data(), (n + 1) * sizeof(int32_t), cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = cudaMemcpy(db->d_off, db->h_off.data(), (n + 2) * sizeof(int64_t), cudaMemcpyHostToDevice)) != cudaSuccess) {
+        (e = cudaMemcpyAsync(db->d_len, db->h_len.data(), (n + 1) * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(db->d_off, db->h_off.data(), (n + 2) * sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream)) != cudaSuccess) {
         int rc = cuda_fail(ctx, e, "gat_db_create");
         gat_db_destroy(db);
         return rc;

@@ -245,8 +245,12 @@ template <class T>
 T* index_upload(gat_index* ix, const std::vector<T>& v, int* status) {
     T* p = (T*)index_alloc(ix, v.size() * sizeof(T) + sizeof(T), status);
     if (!p) return nullptr;
-    cudaError_t e = v.empty() ? cudaSuccess : cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(p + v.size(), 0, sizeof(T)); /* the padding element */
+    /* on the context's stream: kernels that derive other arrays from this one follow there, and that stream is
+     * not ordered with the legacy default stream, whose copies may return before their data has arrived */
+    cudaStream_t s = ix->ctx->stream;
+    cudaError_t e = v.empty() ? cudaSuccess : cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(p + v.size(), 0, sizeof(T), s); /* the padding element */
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s); /* v is the caller's to release */
     if (e != cudaSuccess) {
         *status = cuda_fail(ix->ctx, e, "upload");
         return nullptr;

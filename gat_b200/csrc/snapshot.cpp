@@ -251,14 +251,16 @@ int gat_index_load(gat_ctx* ctx, const gat_db* db, const char* path, gat_index**
                 gat_index_destroy(ix);
                 return st;
             }
-            cudaError_t e = cudaMemcpy(p, host[i].data(), host[i].size(), cudaMemcpyHostToDevice);
+            cudaError_t e = cudaMemcpyAsync(p, host[i].data(), host[i].size(), cudaMemcpyHostToDevice, ctx->stream);
             if (e != cudaSuccess) {
                 gat_index_destroy(ix);
                 return cuda_fail(ctx, e, "gat_index_load");
             }
             *fl[i] = p;
         }
-        int st = index_groups(ix);
+        /* the copies, and what is derived from them, in the order of the context's stream */
+        const cudaError_t arrived = cudaStreamSynchronize(ctx->stream);
+        int st = arrived == cudaSuccess ? index_groups(ix) : cuda_fail(ctx, arrived, "gat_index_load");
         if (st == GAT_OK) st = index_point_boxes(ix);
         if (st != GAT_OK) {
             gat_index_destroy(ix);
