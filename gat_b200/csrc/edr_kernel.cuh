@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "edr_words.h"
 #include "internal.h"
 #include "launch.cuh"
 
@@ -408,7 +409,8 @@ __device__ __forceinline__ int match_mask(float ax, float ay, float2 b, float u)
  * mml = min(m, l) or +inf when m == l, is taken on shifted values unchanged.
  *
  * |E[r][c]| <= r (D <= c + r along the column boundary; D >= |r - c|), so with a bias of 16384 every
- * value of a supported pair lies in [0, 0x8000] and two of them share a 32-bit word. A lane owns
+ * value of a supported pair lies in [0, 0x8000] and two of them share a 32-bit word (edr_words.h; the
+ * last of 16,384 rows, where 0x8000 occurs, by row_tile_top). A lane owns
  * 2H consecutive rows: word i holds row i of the lane (low half) and row H + i (high half). The
  * high half runs one column behind the low half, and the next lane's low half one column behind
  * that, so the value above a half's first row is always one step old: the lane's own low bottom
@@ -421,18 +423,9 @@ __device__ __forceinline__ int match_mask(float ax, float ay, float2 b, float u)
  * it is not, against 14 ALU and 4 FMA for two cells held one per word. Measured on 4,096 pairs of
  * log-uniform [16, 4096] lengths: 0.84 ms, 2.6 Tcell/s; one cell per word: 1.62 ms, 1.34 Tcell/s. */
 constexpr int kBias = 16384;
-constexpr unsigned kHalfOnes = 0x00010001u, kHalfTops = 0x80008000u, kHalfRest = 0x7fff7fffu;
+constexpr unsigned kTop = 0x8000u; /* E + kBias of row kBias at column 0, and where its fall restarts */
+static_assert(kBias == GAT_EDR_MAX_LEN && kTop == 2u * kBias && kBias % 256 == 0, "the last row of the longest side ends a tile");
 
-__device__ __forceinline__ unsigned add_u16x2(unsigned a, unsigned b) {
-    unsigned d;
-    asm("add.u16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-}
-__device__ __forceinline__ unsigned min_u16x2(unsigned a, unsigned b) {
-    unsigned d;
-    asm("min.u16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-}
 /* Negative exactly when |dx| < u and |dy| < u: max propagates a NaN (no match, as the compares
  * have it), and a difference of unequal floats is never zero. */
 __device__ __forceinline__ float match_sign(float dx, float dy, float u) {
@@ -541,10 +534,9 @@ __device__ __forceinline__ Front row_front(const float2* __restrict__ rows, cons
 
 /* One step of a lane: up0 holds the values above its two halves' first rows, d0 the same one
  * column earlier. L[i] goes from column c - 1 to column c of its half, where `keep` (MASKED: the
- * halves whose column lies inside the pair) allows it. m == l is found by (m ^ l) + 0x7fff, whose
- * top bit is clear only for zero; it then sets the top bit of min(m, l), which no value below
- * exceeds. */
-template <int H, bool MATCH, bool MASKED>
+ * halves whose column lies inside the pair) allows it. The choice is min_or_top's; EXACT for the tile
+ * that holds row kBias. */
+template <int H, bool MATCH, bool MASKED, bool EXACT>
 __device__ __forceinline__ void row_step(const float (&ax)[2 * H], const float (&ay)[2 * H], unsigned (&L)[H], unsigned& d0,
                                          float2 blo, float2 bhi, unsigned up0, float u, unsigned one, unsigned keep) {
     unsigned mml[H];
@@ -556,13 +548,12 @@ __device__ __forceinline__ void row_step(const float (&ax)[2 * H], const float (
             const float shi = match_sign(__fsub_rn(ax[H + i], bhi.x), __fsub_rn(ay[H + i], bhi.y), u);
             m = add_u16x2(m, sign_halves(slo, shi));
         }
-        const unsigned y = (m ^ L[i]) * one + kHalfRest;
-        mml[i] = min_u16x2(m, L[i]) | (~y & kHalfTops);
+        mml[i] = min_or_top<kTop, EXACT>(m, L[i], one);
     }
     unsigned up = up0;
 #pragma unroll
     for (int i = 0; i < H; i++) {
-        up = __viaddmin_u16x2(up, kHalfOnes, mml[i]);
+        up = inc_min_u16x2(up, mml[i]);
         if (MASKED)
             L[i] = (up & keep) | (L[i] & ~keep);
         else
@@ -593,7 +584,7 @@ __device__ __forceinline__ void put_words(unsigned addr, const unsigned (&v)[4],
  * holds three, since warps in loops that do not fit the instruction cache together wait for
  * instructions (4,096 pairs of log-uniform [16, 4096] lengths, 8 rows per lane: 0.85 ms with one
  * group, 1.03 ms with two; 4 rows: 0.94 and 0.91 ms). */
-template <int H, int UN, bool MATCH, bool MASKED>
+template <int H, int UN, bool MATCH, bool MASKED, bool EXACT>
 __device__ __forceinline__ void row_chunk(const float (&ax)[2 * H], const float (&ay)[2 * H], unsigned (&L)[H], unsigned& d0,
                                           RowShared& sh, int s0, int kend, int c0, int len2, bool writer, float u,
                                           unsigned one) {
@@ -624,7 +615,7 @@ __device__ __forceinline__ void row_chunk(const float (&ax)[2 * H], const float 
                 const int j = s0 + 4 * g + k - 2 * lane;
                 keep = (j >= c0 && j < len2 ? 0xffffu : 0u) | (j > c0 && j <= len2 ? 0xffff0000u : 0u);
             }
-            row_step<H, MATCH, MASKED>(ax, ay, L, d0, b[k], bhi, up0, u, one, keep);
+            row_step<H, MATCH, MASKED, EXACT>(ax, ay, L, d0, b[k], bhi, up0, u, one, keep);
             bhi = b[k];
             o[k] = L[H - 1];
         }
@@ -640,7 +631,7 @@ __device__ __forceinline__ void row_chunk(const float (&ax)[2 * H], const float 
  * chunk early. A chunk none of whose columns is near the tile's rows (their box) takes the steps
  * without the match test: 29% of the chunks over pairs of log-uniform [16, 4096] lengths that follow
  * one another, nearly all over a top-k walk's candidates. */
-template <int H, int UN>
+template <int H, int UN, bool EXACT>
 __device__ __forceinline__ bool row_tile(const float2* __restrict__ rows, const float2* __restrict__ cols, int len1, int len2,
                                       int t0, Front fr, const carry_t* cin, carry_t* cout, carry_t tag_in, carry_t tag_out,
                                       float u, RowShared& sh, int& result, int spin_limit, unsigned one) {
@@ -723,13 +714,13 @@ __device__ __forceinline__ bool row_tile(const float2* __restrict__ rows, const 
         }
         if (s0 >= c0 + 64 && s0 + 32 <= len2) {
             /* both columns of every lane lie in [c0, len2) throughout */
-            if (near)
-                row_chunk<H, UN, true, false>(ax, ay, L, d0, sh, s0, 32, c0, len2, writer, u, one);
+            if (EXACT || near)
+                row_chunk<H, UN, true, false, EXACT>(ax, ay, L, d0, sh, s0, 32, c0, len2, writer, u, one);
             else
-                row_chunk<H, UN, false, false>(ax, ay, L, d0, sh, s0, 32, c0, len2, writer, u, one);
+                row_chunk<H, UN, false, false, EXACT>(ax, ay, L, d0, sh, s0, 32, c0, len2, writer, u, one);
         } else {
             const int kend = min(32, steps - s0);
-            row_chunk<H, UN, true, true>(ax, ay, L, d0, sh, s0, kend, c0, len2, writer, u, one);
+            row_chunk<H, UN, true, true, EXACT>(ax, ay, L, d0, sh, s0, kend, c0, len2, writer, u, one);
         }
         if (cout) {
             /* lane 31's high half was at column s0 + k - 63 in step k */
@@ -746,6 +737,23 @@ __device__ __forceinline__ bool row_tile(const float2* __restrict__ rows, const 
     }
     __syncwarp();
     return true;
+}
+
+/* The tile that holds row kBias (the last one of a pair whose shorter side has that many points): a
+ * function of its own, so that its loops stay out of the kernel's. One chunk form less: it always
+ * tests for matches. */
+struct TileEnd {
+    bool ok;
+    int result;
+};
+template <int H>
+__device__ __noinline__ TileEnd row_tile_top(const float2* rows, const float2* cols, int len1, int len2, int t0, int above,
+                                             int mine, const carry_t* cin, carry_t tag_in, float u, RowShared* sh,
+                                             int spin_limit) {
+    TileEnd e{false, 0};
+    e.ok = row_tile<H, 1, true>(rows, cols, len1, len2, t0, Front{above, mine}, cin, nullptr, tag_in, 0, u, *sh, e.result,
+                                spin_limit, 1u);
+    return e;
 }
 
 /* Column-tile form of the same recurrence: a lane owns R consecutive DP columns and a step
@@ -986,11 +994,17 @@ __global__ void __launch_bounds__(kRowWarps * 32, 1) k_edr_rows(Src src, float u
             auto tile = [&](auto half) {
                 constexpr int H = decltype(half)::value;
                 if constexpr (2 * H <= R) {
-                    ok = row_tile<H, kGroups>(rows, cols, len1, len2, t0, fr, cin, cout, tin, tout, u, sh, result, ctl.spin_limit, ctl.one);
+                    ok = row_tile<H, kGroups, false>(rows, cols, len1, len2, t0, fr, cin, cout, tin, tout, u, sh, result, ctl.spin_limit, ctl.one);
                     owner = (left - 1) / (2 * H); /* the last tile's */
                 }
             };
-            if (left <= 64 || R == 2)
+            if (len1 == kBias && t == T - 1) {
+                /* full: kBias is a multiple of every tile height */
+                const TileEnd e = row_tile_top<R / 2>(rows, cols, len1, len2, t0, fr.above, fr.mine, cin, tin, u, &sh, ctl.spin_limit);
+                ok = e.ok;
+                result = e.result;
+                owner = 31;
+            } else if (left <= 64 || R == 2)
                 tile(std::integral_constant<int, 1>{});
             else if (left <= 128 || R == 4)
                 tile(std::integral_constant<int, 2>{});

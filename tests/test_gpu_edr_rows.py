@@ -90,3 +90,40 @@ def test_not_finite(gpu_ctx):
     B[4][3] = -np.inf
     _check(gpu_ctx, A, B, 0)
     _check(gpu_ctx, B, A, 8)
+
+
+def _restart_at_the_end():
+    """16,384 points a side (eps = 1): the last row's fall restarts on the last column but one, and the last
+    row meets the last column there."""
+    n = 16384
+    cols = np.full((n, 2), 1000.0)
+    cols[n - 5:n - 1] = [(0.25 * k, -0.25 * k) for k in range(4)]
+    cols[n - 1] = (-0.375, 1.3)
+    # row r meets columns n - 4 + s .. n - 4 + e, by r mod 8; 4 and 7 meet none
+    meets = {1: (2, 2), 2: (0, 0), 3: (0, 0), 5: (0, 0), 6: (0, 1), 0: (0, 2)}
+    rows = np.array([(0.25 * meets[r % 8][1] - 0.875, -0.875 - 0.25 * meets[r % 8][0]) if r % 8 in meets else (-1000.0, -1000.0)
+                     for r in range(1, n + 1)])
+    rows[0] = (0.25 * 3 - 0.875, -0.875 - 0.25 * 2)
+    rows[n - 1] = (-0.375, 0.4)
+    return rows.astype(np.float32), cols.astype(np.float32)
+
+
+@pytest.mark.parametrize("rows", [2, 4, 8])
+def test_last_row_of_the_longest_side(gpu_ctx, rows):
+    """Row 16,384 holds the one value that fills its half word to the top: at column 0 (the last point against the
+    first ones), where its fall restarts at the end, and beside pairs of 16,383 points."""
+    a, b = _restart_at_the_end()
+    (x,) = _walks([16384], 17)
+    far = x + np.float32(4)
+    corner = far.copy()
+    corner[[0, 1, 2, 31, 32, 16380, 16383]] = x[[-1, -1, -2, -1, -3, -1, -2]]
+    A = [a, b, x, corner, a[1:], x[1:]]
+    B = [b, a, corner, x, b[1:], corner[:-1]]
+    _check(gpu_ctx, A[:2] + A[4:5], B[:2] + B[4:5], rows, 1.0)
+    _check(gpu_ctx, A[2:4] + A[5:], B[2:4] + B[5:], rows)
+    la = np.array([16384], np.int32)
+    gpu_ctx.set_edr_rows(rows)
+    try:
+        assert G.edr_pairs(gpu_ctx, la, a, la, b, 1.0)[0] == 32766
+    finally:
+        gpu_ctx.set_edr_rows(0)
