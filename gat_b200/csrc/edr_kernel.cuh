@@ -28,7 +28,8 @@ namespace edr {
 
 constexpr int kWarps = 8; /* k_edr (one warp per pair) */
 constexpr int kRowWarps = 16; /* k_edr_rows: one CTA per SM, 128 registers per thread */
-constexpr int kColWarps = 8;  /* k_edr_cols */
+template <int R>
+constexpr int kColWarps = R == 8 ? 10 : 8; /* k_edr_cols */
 constexpr int kBig = 1 << 29; /* above any distance; up + 1 never overflows against it */
 
 /* Pair source over (a_off, a_len, b_off, b_len) arrays; results to out[p]. A pair with a side
@@ -1016,18 +1017,19 @@ __global__ void __launch_bounds__(kRowWarps * 32, 1) k_edr_rows(Src src, float u
     });
 }
 
-/* Column tiles of 32 R columns. What bounds few pairs is the chain of a step's cells: with 8 columns a lane and three
- * CTAs per SM (80 registers) values of the chain spilled, 64 x 16,384 points took 0.82 ms; with two CTAs (93
- * registers) 0.68 ms, and 4,096 pairs of log-uniform [16, 4096] lengths 1.62 instead of 1.69 ms. */
+/* Column tiles of 32 R columns. What bounds few pairs is the chain of a step's cells: with 8 columns a lane and 24
+ * warps per SM (80 registers) values of the chain spilled, 64 x 16,384 points took 0.82 ms. Two CTAs of ten warps
+ * (92 registers) take 0.68 ms, 64 pairs of 1 x 16,384 points 0.49 (two of eight warps: 0.56), and 4,096 pairs of
+ * log-uniform [16, 4096] lengths 1.56 ms (24 warps: 1.69). */
 template <int R, class Src>
-__global__ void __launch_bounds__(kColWarps * 32, R == 2 ? 4 : R == 4 ? 3 : 2) k_edr_cols(Src src, float u, TileCtl ctl,
+__global__ void __launch_bounds__(kColWarps<R> * 32, R == 2 ? 4 : R == 4 ? 3 : 2) k_edr_cols(Src src, float u, TileCtl ctl,
                                                                               unsigned* __restrict__ work,
                                                                               unsigned long long* __restrict__ cells) {
     dep_wait();
-    __shared__ float2 bring[kColWarps][64];
-    __shared__ int cring[kColWarps][32];
+    __shared__ float2 bring[kColWarps<R>][64];
+    __shared__ int cring[kColWarps<R>][32];
     const int wib = threadIdx.x >> 5;
-    carry_t* wc0 = ctl.warp_carry + (size_t)(blockIdx.x * kColWarps + wib) * 2 * ctl.stride;
+    carry_t* wc0 = ctl.warp_carry + (size_t)(blockIdx.x * kColWarps<R> + wib) * 2 * ctl.stride;
     const carry_t ep = *ctl.epoch << 8;
     walk_tiles(src, ctl, work, cells, [&](const int4& it, const float2* rows, const float2* cols, int len1, int len2,
                                           int& result, int& owner, bool& finished) {
@@ -1054,7 +1056,7 @@ struct TileKernel {
 };
 template <int R, class Src>
 struct TileKernel<R, true, Src> {
-    static constexpr int kWarps = kColWarps;
+    static constexpr int kWarps = kColWarps<R>;
     static constexpr auto get() { return k_edr_cols<R, Src>; }
 };
 
@@ -1152,6 +1154,13 @@ inline uint64_t ceil_log2(int64_t v) {
     return e;
 }
 
+/* Column tiles pay for a few pairs with a side of a handful of points: a row tile then walks the longer side on
+ * one warp whatever it holds (16,384 columns 0.50 ms), while the longer side's 64 column tiles are short. One
+ * pair of 1, 8, 16 and 64 x 16,384 points: 0.35, 0.43, 0.51 and 0.68 ms by columns of 8 a lane; 64 pairs of
+ * 1 x 16,384: 0.49 ms and 0.51 ms by rows, and beyond kColPairs pairs their tiles no longer run at one time
+ * (256 pairs of 16 x 16,384: 1.7 ms, rows 0.55). They are timed when no pair has a second tile of 64 rows. */
+constexpr int kColPairs = 64;
+
 /* EDR over a pair source with the context's tile shape. Rows per lane (GAT_TUNE_EDR_ROWS) and
  * form (GAT_TUNE_EDR_FORM) are fixed by the knobs or autotuned: the first launch of a shape
  * class times the open candidates on this launch's own pairs (every candidate writes the same
@@ -1161,14 +1170,13 @@ template <class Src>
 int edr_launch(gat_ctx* ctx, const Src& src, int64_t cap, int max_rows, int max_cols, float u,
                unsigned long long* cells) {
     if (cap <= 0) return GAT_OK;
-    int cand[6], nc = 0;
-    for (int form = 0; form < 2; form++) {
-        if ((ctx->edr_form ? ctx->edr_form : 1) != form + 1) continue; /* column tiles only when asked for */
-        for (int r : {8, 4, 2}) {
-            if (ctx->edr_rows && ctx->edr_rows != r) continue;
-            cand[nc++] = r | (form ? kShapeCol : 0);
-        }
+    int cand[4], nc = 0;
+    for (int r : {8, 4, 2}) {
+        if (ctx->edr_rows && ctx->edr_rows != r) continue;
+        cand[nc++] = r | (ctx->edr_form == 2 ? kShapeCol : 0);
     }
+    const bool columns = ctx->edr_form == 0 && ctx->edr_rows == 0 && cap <= kColPairs;
+    if (columns) cand[nc++] = 8 | kShapeCol;
     if (nc == 1) return launch_shape(ctx, cand[0], src, cap, max_rows, max_cols, u, cells);
     const uint64_t key = ((uint64_t)Src::kKind << 60) | ((uint64_t)(ctx->edr_rows | ctx->edr_form << 4) << 52) |
                          (ceil_log2(cap) << 40) | (ceil_log2(max_rows) << 20) | ceil_log2(max_cols);
@@ -1191,6 +1199,17 @@ int edr_launch(gat_ctx* ctx, const Src& src, int64_t cap, int max_rows, int max_
     int best = cand[0], st = GAT_OK;
     float best_ms = 0.f;
     for (int i = 0; i < nc && st == GAT_OK; i++) {
+        if (columns && i == nc - 1) {
+            /* the items of the launch before, in tiles of 64 rows */
+            int* items = reinterpret_cast<int*>(ctx->h_pinned + 20);
+            if (cudaMemcpyAsync(items, (const int*)ctx->slot_ptr[S_EDR_COUNTERS] + 2, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream) !=
+                    cudaSuccess ||
+                cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
+                st = cuda_fail(ctx, cudaGetLastError(), "edr autotune");
+                break;
+            }
+            if (*items > cap) break;
+        }
         st = launch_shape(ctx, cand[i], src, cap, max_rows, max_cols, u, i == 0 ? cells : nullptr, e0, e1);
         if (st != GAT_OK) break;
         float ms = 0.f;

@@ -98,14 +98,17 @@ int gat_ctx_kernel_stats(gat_ctx* ctx, int kernel_class, double* ms, int64_t* la
  * GAT_TUNE_EDR_ROWS: rows each lane of the EDR wavefront owns (tile height = 32 x rows; the last
  *   tile of a pair may be lower). 0 (default) = autotune: the first launch of each shape class
  *   (pair count, longest shorter side and longest longer side, each rounded up to a power of two)
- *   times 2, 4 and 8 rows per lane on the caller's own data and keeps the fastest for that class;
+ *   times 2, 4 and 8 rows per lane on the caller's own data and keeps the fastest for that class
+ *   (gat_edr_pairs_dev does not know the sides: its classes go by the pair count alone);
  *   results are the same for every choice. 2, 4 or 8 fixes the value. Setting the knob clears the
  *   tuned table.
  * gat_ctx_get_tuning(GAT_TUNE_EDR_ROWS) returns the knob; GAT_TUNE_EDR_TUNED returns the
  * number of tuned shape classes.
- * GAT_TUNE_EDR_FORM: 0 (default) and 1 = row tiles (lanes own rows of the shorter side, steps walk
- *   the longer side), 2 = column tiles (lanes own columns, steps walk the shorter side: a shorter
- *   critical path for pairs of uneven length, at a fraction of the row tiles' rate). Same results.
+ * GAT_TUNE_EDR_FORM: 1 = row tiles (lanes own rows of the shorter side, steps walk the longer side),
+ *   2 = column tiles (lanes own columns, steps walk the shorter side: a shorter critical path for pairs
+ *   with a side of a few points, at a fraction of the row tiles' rate), 0 (default) = row tiles, and
+ *   column tiles where the autotune finds them faster: it times them (8 columns per lane) for at most 64
+ *   pairs whose shorter sides have at most 64 points. Same results.
  * GAT_TUNE_TOPK_CHUNK / GAT_TUNE_TOPK_GROWTH: candidates a query evaluates in the first round
  *   of the top-k walk, and the factor each later round grows by (0 = defaults: a first round of
  *   1280 for up to 4 queries per batch and 1024 for larger batches, never below 8k or 4k;

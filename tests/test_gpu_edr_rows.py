@@ -127,3 +127,18 @@ def test_last_row_of_the_longest_side(gpu_ctx, rows):
         assert G.edr_pairs(gpu_ctx, la, a, la, b, 1.0)[0] == 32766
     finally:
         gpu_ctx.set_edr_rows(0)
+
+
+@pytest.mark.parametrize("n", [1, 64, 65])
+def test_few_pairs_of_a_short_side(gpu_ctx, n):
+    """Sides of up to 16 points against long ones: the tuner may take column tiles up to 64 pairs. The same pairs again
+    take what it chose."""
+    rng = np.random.default_rng(n)
+    short = rng.integers(1, 17, n).astype(np.int32)
+    long = np.maximum(short, np.exp(rng.uniform(0, np.log(16384), n)).astype(np.int32))
+    long[0] = 16384
+    a, b = D.pairs(short, long, 19)
+    want = po.edr_batch(short, a, long, b, 5e-3)
+    for _ in range(2):
+        assert np.array_equal(G.edr_pairs(gpu_ctx, short, a, long, b, 5e-3), want)
+        assert np.array_equal(G.edr_pairs(gpu_ctx, long, b, short, a, 5e-3), po.edr_batch(long, b, short, a, 5e-3))
