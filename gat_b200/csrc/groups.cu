@@ -180,23 +180,42 @@ __device__ __forceinline__ float4 join_boxes(const float4& a, const float4& b) {
     return make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fmaxf(a.z, b.z), fmaxf(a.w, b.w));
 }
 
-/* records of all nodes; a leaf's ids and point box are final, an inner node's follow by level */
-__global__ void k_node_records(GridDev t, int G, const int32_t* __restrict__ gbeg, const float4* __restrict__ gbox,
-                               NodeRec* rec, float4* pbox) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < t.nnodes; j += gridDim.x * blockDim.x) {
-        NodeRec r;
-        r.mbb = t.node_mbb[j];
-        r.child = t.node_child[j];
-        r.ib = r.ie = 0;
-        r.pbox = no_points();
-        r.aux = 0;
-        if (r.child < 0 && t.node_pbeg[j] < t.node_pend[j]) {
-            r.ib = group_at(gbeg, G, t.node_pbeg[j]);
-            r.ie = group_at(gbeg, G, t.node_pend[j]);
-            for (int g = r.ib; g < r.ie; g++) r.pbox = join_boxes(r.pbox, gbox[g]);
+/* Records of all nodes, a warp each; a leaf's ids and point box are final, an inner node's follow by level. (One
+ * thread per node walked a crowded cell's groups in sequence: a Grid over 1M walks of which 30% of the points
+ * stand at one place took HOT0 ms, now HOT1.) */
+__global__ void __launch_bounds__(256) k_node_records(GridDev t, int G, const int32_t* __restrict__ gbeg,
+                                                      const float4* __restrict__ gbox, NodeRec* rec, float4* pbox) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    for (int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < t.nnodes; j += (gridDim.x * blockDim.x) >> 5) {
+        const int child = t.node_child[j], pb = t.node_pbeg[j], pe = t.node_pend[j];
+        int ib = 0, ie = 0;
+        float4 box = no_points();
+        if (child < 0 && pb < pe) {
+            ib = group_at(gbeg, G, pb);
+            ie = group_at(gbeg, G, pe);
+#pragma unroll 4
+            for (int g = ib + lane; g < ie; g += 32) box = join_boxes(box, gbox[g]);
+            for (int o = 16; o > 0; o >>= 1) {
+                float4 b;
+                b.x = __shfl_xor_sync(FULL, box.x, o);
+                b.y = __shfl_xor_sync(FULL, box.y, o);
+                b.z = __shfl_xor_sync(FULL, box.z, o);
+                b.w = __shfl_xor_sync(FULL, box.w, o);
+                box = join_boxes(box, b);
+            }
         }
-        rec[j] = r;
-        pbox[j] = r.pbox;
+        if (lane == 0) {
+            NodeRec r;
+            r.mbb = t.node_mbb[j];
+            r.pbox = box;
+            r.child = child;
+            r.ib = ib;
+            r.ie = ie;
+            r.aux = 0;
+            rec[j] = r;
+            pbox[j] = box;
+        }
     }
 }
 
@@ -559,7 +578,7 @@ int index_groups(gat_index* ix) {
             GAT_CUDA_TRY(ctx, cudaMalloc(&ix->d_pbox, (size_t)n * sizeof(float4)), "point boxes");
             ix->device_bytes += (size_t)n * sizeof(float4);
         }
-        k_node_records<<<blocks_for(ctx, n), 256, 0, s>>>(ix->grid, G, gbeg, gbox, rec, ix->d_pbox);
+        k_node_records<<<blocks_for(ctx, (int64_t)n * 32), 256, 0, s>>>(ix->grid, G, gbeg, gbox, rec, ix->d_pbox);
         /* level l is [level[l], level[l + 1]); the root is level 0 */
         ctx->h_pinned[3] = 1;
         ctx->h_pinned[4] = total;
