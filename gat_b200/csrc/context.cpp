@@ -113,6 +113,16 @@ void* host_stage(gat_ctx* ctx, size_t bytes, int* status) {
     return p;
 }
 
+void raise_smem_limit(const void* kernel, size_t bytes) {
+    static std::mutex mu;
+    static std::map<std::pair<const void*, int>, size_t> limit;
+    int device = 0;
+    cudaGetDevice(&device);
+    std::lock_guard<std::mutex> lk(mu);
+    size_t& now = limit[{kernel, device}];
+    if (bytes > now && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess) now = bytes;
+}
+
 void* scratch_zeroed(gat_ctx* ctx, int slot, size_t bytes, int* status) {
     void* p = scratch(ctx, slot, bytes, status);
     if (p && ctx->slot_fresh[slot]) {

@@ -309,10 +309,12 @@ int ctx_use_priority_stream(gat_ctx* ctx);
 /* GAT_ERR_STATE for a host-only context (device -1) */
 int require_device(gat_ctx* ctx, const char* what);
 /* Opts a kernel into `bytes` of dynamic shared memory when that (plus the kernel's few KB of
- * static shared memory) could exceed the 48 KB default. */
+ * static shared memory) could exceed the 48 KB default. The limit belongs to the kernel on the current
+ * device, which other contexts may be launching from other threads: it is only ever raised. */
+void raise_smem_limit(const void* kernel, size_t bytes);
 template <class K>
 inline void allow_smem(K kernel, size_t bytes) {
-    if (bytes > 40 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (bytes > 40 * 1024) raise_smem_limit(reinterpret_cast<const void*>(kernel), bytes);
 }
 /* true when `user` may run queries on objects created through `owner` (the same context, or
  * worker contexts of one parent) */
