@@ -93,21 +93,16 @@ constexpr size_t kPinnedWords = 64, kFirstStage = (size_t)64 << 10;
 
 void* host_stage(gat_ctx* ctx, size_t bytes, int* status) {
     if (bytes <= ctx->h_stage_bytes) return ctx->h_stage;
-    const size_t had = ctx->h_stage_bytes;
-    if (ctx->h_stage) {
-        /* an earlier copy may still read it */
-        cudaStreamSynchronize(ctx->stream);
-        if (ctx->h_stage != ctx->h_pinned + kPinnedWords) cudaFreeHost(ctx->h_stage);
-        ctx->h_stage = nullptr;
-        ctx->h_stage_bytes = 0;
-    }
-    const size_t nb = std::max<size_t>(std::max<size_t>(bytes, 2 * had), (size_t)64 << 10); /* grows by doubling */
+    const size_t nb = std::max<size_t>(bytes, 2 * ctx->h_stage_bytes); /* grows by doubling */
     void* p = nullptr;
     cudaError_t e = cudaMallocHost(&p, nb);
     if (e != cudaSuccess) {
         *status = cuda_fail(ctx, e, "pinned staging");
-        return nullptr;
+        return nullptr; /* the area so far stays */
     }
+    /* an earlier copy may still read it */
+    cudaStreamSynchronize(ctx->stream);
+    if (ctx->h_stage != ctx->h_pinned + kPinnedWords) cudaFreeHost(ctx->h_stage);
     ctx->h_stage = p;
     ctx->h_stage_bytes = nb;
     return p;

@@ -78,9 +78,9 @@ int gat_edr_pairs(gat_ctx* ctx, int npairs, const int32_t* q_len, const int64_t*
         size_t bytes;
     } in[6] = {{d_aoff, q_off, n8}, {d_boff, c_off, n8}, {d_alen, q_len, n4}, {d_blen, c_len, n4}, {d_a, q_xy, a_bytes},
                {d_b, c_xy, b_bytes}};
-    if (total <= kStageIn) {
-        char* stage = (char*)host_stage(ctx, total, &st);
-        if (!stage) return st;
+    int hs = GAT_OK;
+    char* stage = total <= kStageIn ? (char*)host_stage(ctx, total, &hs) : nullptr;
+    if (stage) {
         for (const auto& c : in)
             if (c.bytes) memcpy(stage + ((char*)c.d - buf), c.h, c.bytes);
         GAT_CUDA_TRY(ctx, cudaMemcpyAsync(buf, stage, total, cudaMemcpyHostToDevice, s), "edr H2D");
@@ -92,8 +92,7 @@ int gat_edr_pairs(gat_ctx* ctx, int npairs, const int32_t* q_len, const int64_t*
                              match_threshold(eps), d_out, nullptr)) != GAT_OK)
         return st;
     /* the distances come back with the status word, in one wait; they are handed over when it is clear */
-    int32_t* back = n4 <= kStageOut ? (int32_t*)host_stage(ctx, n4, &st) : nullptr;
-    if (n4 <= kStageOut && !back) return st;
+    int32_t* back = n4 <= kStageOut ? (int32_t*)host_stage(ctx, n4, &hs) : nullptr;
     if (back) GAT_CUDA_TRY(ctx, cudaMemcpyAsync(back, d_out, n4, cudaMemcpyDeviceToHost, s), "edr D2H");
     if ((st = check_device_flag(ctx, "edr")) != GAT_OK) return st;
     if (back) {

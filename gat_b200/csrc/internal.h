@@ -258,7 +258,8 @@ T* index_upload(gat_index* ix, const std::vector<T>& v, int* status) {
     return p;
 }
 /* pinned host staging of at least `bytes` bytes, owned by the context (one user at a time: the
- * caller's copies from it must finish before the next call) */
+ * caller's copies from it must finish before the next call). Null, with *status set, when there is no such
+ * memory: callers that stage for speed alone then copy directly. */
 void* host_stage(gat_ctx* ctx, size_t bytes, int* status);
 /* Derives the exact box of the points under every quadtree node (Grid) or STIG leaf, so that the
  * range walks can mark candidate ranges whose every point is a hit (pbox.cu). Called after a

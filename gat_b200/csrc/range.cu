@@ -2027,10 +2027,11 @@ int gat_range_query(gat_ctx* ctx, const gat_index* ix, const gat_mbb* queries, i
     const size_t q_bytes = (size_t)nq * sizeof(gat_mbb);
     const void* from = queries;
     if (nq > 0 && q_bytes <= kStageIn) {
-        void* stage = host_stage(ctx, q_bytes, &st);
-        if (!stage) return st;
-        memcpy(stage, queries, q_bytes);
-        from = stage;
+        int hs = GAT_OK;
+        if (void* stage = host_stage(ctx, q_bytes, &hs)) {
+            memcpy(stage, queries, q_bytes);
+            from = stage;
+        }
     }
     if (nq > 0) GAT_CUDA_TRY(ctx, cudaMemcpyAsync(dq, from, q_bytes, cudaMemcpyHostToDevice, s), "range H2D");
     /* outputs land in device scratch first, sized to the host capacity */
@@ -2045,10 +2046,9 @@ int gat_range_query(gat_ctx* ctx, const gat_index* ix, const gat_mbb* queries, i
     const size_t off_bytes = (size_t)(nq + 1) * sizeof(int64_t), id_bytes = st == GAT_OK ? (size_t)need * 4 : 0;
     const bool points = result_kind == GAT_RESULT_POINTS;
     const size_t back_bytes = off_bytes + id_bytes * (points ? 2 : 1);
-    if ((st == GAT_OK || st == GAT_ERR_TRUNCATED) && back_bytes <= kStageOut) {
-        int hs = GAT_OK;
-        char* back = (char*)host_stage(ctx, back_bytes, &hs);
-        if (!back) return hs;
+    int hs = GAT_OK;
+    char* back = (st == GAT_OK || st == GAT_ERR_TRUNCATED) && back_bytes <= kStageOut ? (char*)host_stage(ctx, back_bytes, &hs) : nullptr;
+    if (back) {
         GAT_CUDA_TRY(ctx, cudaMemcpyAsync(back, csr, off_bytes, cudaMemcpyDeviceToHost, s), "range D2H");
         if (id_bytes) GAT_CUDA_TRY(ctx, cudaMemcpyAsync(back + off_bytes, dt, id_bytes, cudaMemcpyDeviceToHost, s), "range D2H");
         if (id_bytes && points)

@@ -1464,9 +1464,11 @@ int upload_queries(gat_ctx* ctx, int nq, const int32_t* q_len, const float* lon,
     *dxy = (float2*)(p + b_len + b_off + 2 * b_f);
     cudaStream_t s = ctx->stream;
     const size_t all = b_len + b_off + 2 * b_f;
-    const bool staged = all <= kStageIn;
+    char* stage = all <= kStageIn ? (char*)host_stage(ctx, all, &st) : nullptr;
+    const bool staged = stage != nullptr;
+    st = GAT_OK;
     /* the offsets are built here: copied from pinned staging, not from pageable memory */
-    char* stage = (char*)host_stage(ctx, staged ? all : (size_t)(nq + 1) * 8, &st);
+    if (!staged) stage = (char*)host_stage(ctx, (size_t)(nq + 1) * 8, &st);
     if (!stage) return st;
     int64_t* hoff = reinterpret_cast<int64_t*>(staged ? stage + b_len : stage);
     std::copy(h.off.begin(), h.off.begin() + (nq + 1), hoff);
@@ -1531,10 +1533,8 @@ int gat_topk(gat_ctx* ctx, const gat_index* grid, int nq, const int32_t* q_len, 
     if (!dres) return st;
     st = topk_dev(ctx, grid, nq, dl, doff, dxy, h.maxlen, k, eps, exec, dres, dres + (size_t)nq * k, stats);
     const size_t half = (size_t)nq * k * 4;
-    if (st == GAT_OK && 2 * half <= kStageOut) {
-        int hs = GAT_OK;
-        char* back = (char*)host_stage(ctx, 2 * half, &hs);
-        if (!back) return hs;
+    int hs = GAT_OK;
+    if (char* back = st == GAT_OK && 2 * half <= kStageOut ? (char*)host_stage(ctx, 2 * half, &hs) : nullptr) {
         GAT_CUDA_TRY(ctx, cudaMemcpyAsync(back, dres, 2 * half, cudaMemcpyDeviceToHost, ctx->stream), "top-k D2H");
         GAT_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream), "top-k D2H");
         memcpy(out_ids, back, half);

@@ -1,0 +1,75 @@
+"""Calls with host arrays when no more pinned memory can be had: they copy directly and answer the same."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+CHILD = r"""
+import ctypes as C, resource, sys
+import numpy as np
+import gat_b200 as G
+from gat_b200 import _lib as L, data as D
+
+ctx = G.Context(0)
+t = D.walks(D.lengths(20_000, 0, 0, 0, 20, 200, 1), 1)
+grid = G.Grid(ctx, G.TrajectorySet(ctx, t), D.BOX, 0.005, 2, 512)
+
+def ranges(nq, off, tid):
+    need = C.c_int64(0)
+    q = boxes[:nq]
+    rc = L.lib.gat_range_query(ctx.h, grid.h, q.ctypes.data, nq, L.GAT_RESULT_IDS, L.GAT_EXEC_BATCHED,
+                               off.ctypes.data_as(L.P_i64), tid.ctypes.data_as(L.P_i32), None, len(tid), C.byref(need))
+    return rc, need.value
+
+# wide rectangles of 3,500 ids or so: 440 of them are too many to be staged, 150 are 2 MB
+boxes = D.boxes(440, L.GAT_SIDE_FIXED, 0.4, 0.4, 2)
+off, tid = np.zeros(441, np.int64), np.zeros(8_000_000, np.int32)
+off2, tid2 = np.zeros(441, np.int64), np.zeros(8_000_000, np.int32)
+rc, need = ranges(440, off, tid)   # sizes every device buffer
+assert rc == 0 and need * 4 > 4 << 20, (rc, need)
+part = int(off[150])
+assert 1 << 20 < part * 4 < 3 << 20, part
+la = D.lengths(9_000, 0, 0, 0, 2, 6, 3)  # staged: 0.8 MB in
+a, b = D.pairs(la, la, 4)
+starts = np.zeros(len(la) + 1, np.int64)
+np.cumsum(la, out=starts[1:])
+out, out2 = np.zeros(len(la), np.int32), np.zeros(len(la), np.int32)
+
+def edr(o):
+    return L.lib.gat_edr_pairs(ctx.h, len(la), la.ctypes.data_as(L.P_i32), starts.ctypes.data_as(L.P_i64), a.ctypes.data_as(L.P_f32),
+                               int(starts[-1]), la.ctypes.data_as(L.P_i32), starts.ctypes.data_as(L.P_i64),
+                               b.ctypes.data_as(L.P_f32), int(starts[-1]), 5e-4, o.ctypes.data_as(L.P_i32))
+
+if sys.argv[1] == "edr":
+    two = np.concatenate([la, la])  # beyond the staged size, and sizes every device buffer
+    want = G.edr_pairs(ctx, two, np.concatenate([a, a]), two, np.concatenate([b, b]), 5e-4)
+
+size = int(open("/proc/self/statm").read().split()[0]) * resource.getpagesize()
+resource.setrlimit(resource.RLIMIT_AS, (size, resource.RLIM_INFINITY))
+# what the driver still holds of pinned memory, in pieces; at most 64 MB
+pinned = C.CDLL("libcuda.so.1").cuMemAllocHost_v2
+for piece in (1 << 20, 256 << 10):
+    for _ in range(32):
+        if pinned(C.byref(C.c_void_p()), C.c_size_t(piece)) != 0:
+            break
+    else:
+        sys.exit("pinned memory does not run out under the limit")
+rc = edr(out) if sys.argv[1] == "edr" else ranges(150, off2, tid2)[0]
+resource.setrlimit(resource.RLIMIT_AS, (resource.RLIM_INFINITY, resource.RLIM_INFINITY))
+assert rc == 0, (rc, L.lib.gat_last_error(ctx.h))
+if sys.argv[1] == "edr":
+    assert np.array_equal(out, want[:len(la)])
+else:
+    assert np.array_equal(off[:151], off2[:151]) and np.array_equal(tid[:part], tid2[:part])
+print("same")
+"""
+
+
+@pytest.mark.parametrize("call", ["range", "edr"])
+def test_no_pinned_memory(call):
+    r = subprocess.run([sys.executable, "-c", CHILD, call], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "same" in r.stdout, r.stdout + r.stderr
