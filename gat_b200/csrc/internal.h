@@ -275,8 +275,8 @@ void index_groups_free(gat_index* ix);
  * used, [1] work bytes when `timed`, [3] queries left in ovf_list for the bitmap scan. */
 int range_groups_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, uint32_t* arena, int64_t cap,
                         unsigned long long* ctr, int64_t* segbase, int64_t* segcnt, int* ovf_list, bool timed);
-/* Point lists likewise (Grid, FSG, MortonGrid; keys in the arena), queries of more than 4,096 points left
- * in ovf_list; again: nq ints of its own. */
+/* Point lists likewise (Grid, MortonGrid; keys in the arena); the queries left in ovf_list are those of more
+ * than 14,336 points, or whose walk or candidates outgrow the kernel; again: nq ints of its own. */
 int group_points_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, uint32_t* arena, int64_t cap,
                         unsigned long long* ctr, int64_t* segbase, int64_t* segcnt, int* ovf_list, int* again);
 /* Plain execution of id-set query qi over an index with groups, launched in the order of qi: writes

@@ -49,7 +49,6 @@ constexpr int kCtl = 24; /* control words of a team */
 constexpr float kSmallMax = 400.f, kMidMax = 1100.f;
 constexpr int kFarCell = 1 << 20; /* FSG cell coordinates beyond this take the general scan */
 constexpr int kBorder = (int)0x80000000; /* item end flag: groups to be tested by box */
-constexpr int kDirectMax = 444; /* batches up to this size: every query in block mode */
 
 /* shared memory of one query's team */
 template <int HB_, int IDS_, int FRONT_, int ITEMS_, int NTHREADS_>
@@ -811,9 +810,11 @@ __global__ void __launch_bounds__(kNT, 2) k_plain_groups(GroupQuery a, int qi) {
 }
 
 /* Point lists: the keys (trajectory << bits | point index) of the points inside, ascending. A query of
- * more than T::IDS points, or with far more candidates than that, or one that outgrows the
- * walk's memory, is left: by the first pass to the second (AGAIN, the list `again` of ctr[5] queries),
- * which has 3.5 times the memory and one CTA per SM, by that on the overflow list for k_range_points.
+ * more than T::IDS points, or with more than twice as many candidates, is left by the first pass to the second
+ * (AGAIN, the list `again` of ctr[5] queries), which has 3.5 times the list and one CTA per SM. What outgrows
+ * that too goes on the overflow list for k_range_points, and so do at once the queries with far more candidates
+ * than the second pass holds and those whose walk outgrows its frontier or its ranges, of which both passes
+ * have the same.
  * Without the second pass a batch with some long lists paid the items and the host's wait for them (710
  * rectangles of 0.0055 to 0.05 degrees on 16k walks: 303 us and 254 us with it).
  * Keys are held with the top bit flipped, so that signed compares order them. */
@@ -852,9 +853,10 @@ __global__ void __launch_bounds__(kNT, AGAIN ? 1 : 3) k_group_points(GroupQuery 
         if (lane == 0 && all) atomicAdd(t.query, all);
         __syncthreads();
         const int points = *t.query;
-        const bool last = AGAIN || points > LongTeam::IDS + LongTeam::IDS / 4;
-        const bool many = points > 2 * kBlockIds && (!AGAIN || points > 2 * T::IDS);
-        if (!many && !__shfl_sync(FULL, *(volatile int*)t.ovf, 0)) {
+        const bool outgrown = *(volatile int*)t.ovf != 0; /* by the walk, which has no more room in the second pass */
+        const bool last = AGAIN || outgrown || points > LongTeam::IDS + LongTeam::IDS / 4;
+        const bool many = !AGAIN && points > 2 * kBlockIds;
+        if (!many && !outgrown) {
             for (;;) {
                 int k = 0;
                 if (lane == 0) k = atomicAdd(t.next, 1);
@@ -891,7 +893,7 @@ __global__ void __launch_bounds__(kNT, AGAIN ? 1 : 3) k_group_points(GroupQuery 
         }
         __syncthreads();
         const int m = *t.cnt;
-        const bool lost = many || *(volatile int*)t.ovf != 0 || m > T::IDS;
+        const bool lost = many || outgrown || m > T::IDS;
         if (me == 0) {
             if (lost) {
                 (last ? a.ovf_list : again)[atomicAdd(&a.ctr[last ? 3 : 5], 1ull)] = qi;
@@ -1056,8 +1058,8 @@ int range_groups_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, i
     GAT_CUDA_TRY(ctx, cudaMemsetAsync(ctr, 0, 8 * sizeof(unsigned long long), s), "range");
     GroupQuery a{d_q, ix->grid, ix->fsg, ix->morton, ix->groups, arena, cap, ctr, segbase, segcnt, nullptr, nullptr, 0, nullptr, nullptr,
                  ovf_list, timed ? ctr + 1 : nullptr};
-    if (nq <= std::min(full, kDirectMax)) {
-        /* no more queries than resident CTAs: one each */
+    if (nq <= full) {
+        /* no more queries than resident CTAs: one each, in block mode */
         kernel<<<nq, kNT, kSmem, s>>>(a, nullptr, nullptr, nq);
         count_launch(ctx);
         GAT_CUDA_TRY(ctx, cudaGetLastError(), "range scan launch");

@@ -168,3 +168,18 @@ def test_long_point_lists(gpu_ctx, walks):
         assert a.offsets[1] > 0
         assert np.array_equal(a.offsets, b.offsets)
         assert np.array_equal(a.tids, b.tids) and np.array_equal(a.pidx, b.pidx)
+
+
+def test_point_lists_of_walks_that_outgrow(gpu_ctx):
+    """Rectangles whose border crosses more leaves than the walk's ranges hold, and more nodes than its frontier,
+    with few points and with many; beside ordinary ones."""
+    t = D.walks(D.lengths(2_000, 0, 0, 0, 20, 200, 61), 61)
+    g = G.Grid(gpu_ctx, G.TrajectorySet(gpu_ctx, t), D.BOX, 0.0005, 2, 1)
+    x0, y0, x1, y1 = D.BOX
+    wide = [[x0 - 1, y0 + 0.001 * k, x1 + 1, y0 + 0.001 * k + 0.0007] for k in range(0, 900, 30)]
+    large = [[x0 + 0.01 * k, y0 + 0.01 * k, x1 - 0.01 * k, y1 - 0.01 * k] for k in range(1, 25)]
+    q = np.concatenate([np.array(wide + large, np.float32), D.boxes(100, 1, 0.001, 0.1, 62)])
+    off, tid, pidx = po.OracleGrid(t, D.BOX, 0.0005, 2, 1).range(q, 1)
+    for ix in (g, G.MortonGrid(g)):
+        r = ix.range_query(q, "points", "batched", capacity=4_000_000)
+        assert np.array_equal(r.offsets, off) and np.array_equal(r.tids, tid) and np.array_equal(r.pidx, pidx)
