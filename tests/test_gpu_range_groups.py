@@ -183,3 +183,23 @@ def test_point_lists_of_walks_that_outgrow(gpu_ctx):
     for ix in (g, G.MortonGrid(g)):
         r = ix.range_query(q, "points", "batched", capacity=4_000_000)
         assert np.array_equal(r.offsets, off) and np.array_equal(r.tids, tid) and np.array_equal(r.pidx, pidx)
+
+
+@pytest.mark.parametrize("walks,cell,block", [(3000, 0.01, 64), (225, 0.005, 5000), (1, 0.5, 2)])
+def test_point_lists_of_every_index(gpu_ctx, walks, cell, block):
+    """Point lists against the oracle: those of an FSG and a STIG take the point scan whatever the knob says, so one
+    path cannot be held against the other there."""
+    t = D.walks(D.lengths(walks, 0, 0, 0, 1, 200, 63), 63)
+    q = _odd_rectangles(t, cell, 64)
+    q = np.concatenate([q[np.isfinite(q).all(1)][::3], D.boxes(40, 1, 0.001, 0.4, 65)])
+    db = G.TrajectorySet(gpu_ctx, t)
+    g = G.Grid(gpu_ctx, db, D.BOX, cell, 2, 64)
+    grid = po.OracleGrid(t, D.BOX, cell, 2, 64)
+    for ix, o in ((g, grid), (G.MortonGrid(g), grid), (G.FSG(gpu_ctx, db, D.BOX, cell), po.OracleFSG(t, D.BOX, cell)),
+                  (G.STIG(gpu_ctx, db, block), po.OracleSTIG(t, block))):
+        off, tid, pidx = o.range(q, 1)
+        for execution, part in (("batched", len(q)), ("plain", 20)):
+            r = ix.range_query(q[:part], "points", execution, capacity=8_000_000)
+            e = off[part]
+            assert np.array_equal(r.offsets, off[:part + 1])
+            assert np.array_equal(r.tids, tid[:e]) and np.array_equal(r.pidx, pidx[:e])
