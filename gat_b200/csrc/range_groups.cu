@@ -472,8 +472,74 @@ __device__ __forceinline__ void take_items(const int2* items, int n, const Box& 
  * runs and searching every id in every run took half of a query's instructions.) `out` may be the list
  * itself. FLIP is xored into what is written (point keys are held with their top bit flipped). */
 /* Fullest bucket that is ranked: ids, and point keys, which lie in clusters (1,500 rectangles of 0.003 to 0.03
- * degrees on 100k walks: 1270 us with 32, 1132 us with 512). */
-constexpr int kCrowd = 32, kKeyCrowd = 512;
+ * degrees on 100k walks: 1270 us with 32, 1132 us with 512). Lists of more than kRadixMin keys are sorted by digits
+ * instead as soon as a bucket holds more than kCrowd: a key is compared with every other of its bucket, a walk's
+ * hundred or more points (148 lists of 10k points 248 us by ranks, 139 by digits; a thousand 1409 and 912). */
+constexpr int kCrowd = 32, kKeyCrowd = 512, kRadixMin = 1024;
+
+/* The m keys of the team's list by a stable radix sort in shared memory, 8 bits of (key - lo) a pass, between the
+ * list and the set's slots: each warp counts the digits of its share, a scan over digits and warps gives it
+ * its places, and it puts its keys there in order. */
+template <class T, unsigned FLIP>
+__device__ void radix_keys(T& t, int m, unsigned range, unsigned lo, uint32_t* out, bool write, int me) {
+    constexpr int W = T::NTHREADS / 32;
+    static_assert(T::NTHREADS != kNT || T::IDS + W * 256 <= (1 << T::HB), "the keys and the counters share the set's slots");
+    const unsigned FULL = 0xffffffffu;
+    const int lane = me & 31, warp = me >> 5;
+    int* const hist = t.tab + (1 << T::HB) - W * 256;
+    const int share = ((m + W - 1) / W + 31) & ~31, begin = min(m, warp * share), end = min(m, begin + share);
+    int *src = t.list, *dst = t.tab;
+    t.sync(); /* the counts in the slots have been read */
+    for (int shift = 0; shift < 32 && (range >> shift) != 0; shift += 8) {
+        for (int i = me; i < W * 256; i += T::NTHREADS) hist[i] = 0;
+        t.sync();
+        for (int i = begin + lane; i < end; i += 32) atomicAdd(&hist[warp * 256 + ((((unsigned)src[i] - lo) >> shift) & 255u)], 1);
+        t.sync();
+        int c[W], sum = 0;
+#pragma unroll
+        for (int w = 0; w < W; w++) {
+            c[w] = hist[w * 256 + me];
+            sum += c[w];
+        }
+        int incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(FULL, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) t.sort[4 + warp] = incl;
+        t.sync();
+        int at = incl - sum;
+        for (int w = 0; w < warp; w++) at += t.sort[4 + w];
+#pragma unroll
+        for (int w = 0; w < W; w++) {
+            hist[w * 256 + me] = at;
+            at += c[w];
+        }
+        t.sync();
+        for (int i0 = begin; i0 < end; i0 += 32) {
+            const int i = i0 + lane;
+            const int x = i < end ? src[i] : 0;
+            const int d = i < end ? (int)((((unsigned)x - lo) >> shift) & 255u) : -1;
+            const unsigned peers = __match_any_sync(FULL, d);
+            const int rank = __popc(peers & ((1u << lane) - 1u));
+            int at0 = 0;
+            if (d >= 0) at0 = hist[warp * 256 + d];
+            __syncwarp();
+            if (d >= 0) {
+                if (rank == 0) hist[warp * 256 + d] = at0 + __popc(peers);
+                dst[at0 + rank] = x;
+            }
+            __syncwarp();
+        }
+        t.sync();
+        int* s = src;
+        src = dst;
+        dst = s;
+    }
+    if (write)
+        for (int i = me; i < m; i += T::NTHREADS) out[i] = (uint32_t)src[i] ^ FLIP;
+}
 
 template <class T, unsigned FLIP = 0>
 __device__ void sort_ids(T& t, int m, uint32_t* out, bool write, int me) {
@@ -540,7 +606,9 @@ __device__ void sort_ids(T& t, int m, uint32_t* out, bool write, int me) {
         most = lo_hi[2];
         for (int w = 0; w < warp; w++) start += lo_hi[4 + w];
     }
-    if (most <= (FLIP ? kKeyCrowd : kCrowd)) {
+    if (FLIP && (most > kKeyCrowd || (most > kCrowd && m > kRadixMin))) {
+        radix_keys<T, FLIP>(t, m, (unsigned)hi - (unsigned)lo, (unsigned)lo, out, write, me);
+    } else if (most <= (FLIP ? kKeyCrowd : kCrowd)) {
 #pragma unroll
         for (int k = 0; k < kPer; k++) {
             tab[me * kPer + k] = start;

@@ -203,3 +203,27 @@ def test_point_lists_of_every_index(gpu_ctx, walks, cell, block):
             e = off[part]
             assert np.array_equal(r.offsets, off[:part + 1])
             assert np.array_equal(r.tids, tid[:e]) and np.array_equal(r.pidx, pidx[:e])
+
+
+@pytest.mark.parametrize("walks,points", [(3, 1000), (20, 400), (33, 130), (1100, 4)])
+def test_clustered_point_keys(gpu_ctx, walks, points):
+    """Lists around 1,024 points and above whose keys crowd in few buckets (walks of many points, ids far apart) or
+    in none, in both passes."""
+    rng = np.random.default_rng(69)
+    lens = np.full(9000, 1, np.int32)
+    ids = np.sort(rng.choice(9000, walks, replace=False))
+    lens[ids] = points
+    t = D.walks(lens, 69)
+    off = t.offsets
+    for i in ids:  # inside one square
+        s, e = off[i], off[i + 1]
+        t.lon[s:e] = rng.uniform(121.3, 121.34, e - s)
+        t.lat[s:e] = rng.uniform(31.1, 31.14, e - s)
+    g = G.Grid(gpu_ctx, G.TrajectorySet(gpu_ctx, t), D.BOX, 0.005, 2, 64)
+    k = rng.uniform(0, 0.02, (40, 2))
+    q = np.concatenate([121.3 + k[:, :1], 31.1 + k[:, 1:], 121.34 - k[:, 1:], 31.14 - k[:, :1]], 1).astype(np.float32)
+    q = np.concatenate([q, np.array([[121.3, 31.1, 121.34, 31.14], [121.0, 30.7, 122.0, 31.7]], np.float32)])
+    off, tid, pidx = po.OracleGrid(t, D.BOX, 0.005, 2, 64).range(q, 1)
+    for ix in (g, G.MortonGrid(g)):
+        r = ix.range_query(q, "points", "batched", capacity=4_000_000)
+        assert np.array_equal(r.offsets, off) and np.array_equal(r.tids, tid) and np.array_equal(r.pidx, pidx)
