@@ -272,7 +272,8 @@ int index_groups(gat_index* ix);
 void index_groups_free(gat_index* ix);
 /* Batched id-set queries over an index with groups (range_groups.cu): per-query segments of `arena`
  * (cap entries) in segbase / segcnt, the counters in ctr[0..8) (device, 8 words): [0] arena entries
- * used, [1] work bytes when `timed`, [3] queries left in ovf_list for the bitmap scan. */
+ * used, [1] work bytes when `timed`, [3] queries left at the front of ovf_list (nq entries) for the bitmap scan,
+ * [6] queries left at its end for the point scan. */
 int range_groups_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, uint32_t* arena, int64_t cap,
                         unsigned long long* ctr, int64_t* segbase, int64_t* segcnt, int* ovf_list, bool timed);
 /* Point lists likewise (Grid, MortonGrid; keys in the arena); the queries left in ovf_list are those of more
@@ -347,6 +348,7 @@ enum Slot {
     S_RANGE_TPOS,
     S_RANGE_TASK,
     S_RANGE_SPLIT,
+    S_RANGE_LEFT,
     S_EDR_PAIRS,
     S_EDR_CARRY,
     S_EDR_COUNTERS,

@@ -1661,13 +1661,15 @@ __global__ void __launch_bounds__(kThreads) k_gather_groups(int nq, const int64_
         out[at] = pidx_bits < 0 ? (int32_t)k : (int32_t)(k >> pidx_bits);
         if (pidx_bits >= 0 && out_pidx) out_pidx[at] = (int32_t)(k & ((1u << pidx_bits) - 1u));
     };
+    /* read before the counts are summed, not one after the other behind them */
+    const bool spilled = (int64_t)ctr[0] > arena_cap, left = (ctr[3] | ctr[6]) != 0;
     if constexpr (!SCAN) {
         constexpr int kFlight = 4;
         const int lane = threadIdx.x & 31, warps = gridDim.x * (kThreads / 32);
         int qi = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
         const int64_t total = off[nq];
         if (qi == 0 && lane == 0) ctr[8] = (unsigned long long)total;
-        if (total > capacity || (int64_t)ctr[0] > arena_cap || ctr[3] != 0 || qi >= nq) return;
+        if (total > capacity || spilled || left || qi >= nq) return;
         int64_t o = off[qi], b = segbase[qi], n = segcnt[qi];
         for (;;) {
             const bool more = qi < nq - warps;
@@ -1721,15 +1723,28 @@ __global__ void __launch_bounds__(kThreads) k_gather_groups(int nq, const int64_
                 if (qi == nq - 1) off[nq] = total;
                 if (qi == 0) ctr[8] = (unsigned long long)total;
             }
-            if (total > capacity || (int64_t)ctr[0] > arena_cap || ctr[3] != 0) continue;
+            if (total > capacity || spilled || left) continue;
             const int64_t b = segbase[qi], n = segcnt[qi];
             for (int64_t i = threadIdx.x; i < n; i += kThreads) put(o + i, arena[b + i]);
         }
     }
 }
 
+/* the queries of a list as a batch of their own, and its segments back at their places */
+__global__ void k_take_left(int n, const int* __restrict__ list, const gat_mbb* __restrict__ queries, gat_mbb* __restrict__ out) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < n) out[j] = queries[list[j]];
+}
+__global__ void k_put_left(int n, const int* __restrict__ list, const int64_t* __restrict__ base, const int64_t* __restrict__ cnt,
+                           int64_t* __restrict__ segbase, int64_t* __restrict__ segcnt) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= n) return;
+    segbase[list[j]] = base[j];
+    segcnt[list[j]] = cnt[j];
+}
+
 /* A batch over an index with point groups (range_groups.cu), offsets and results in the caller's device
- * arrays. Queries whose results outgrow the kernel's memory get their items built and take the bitmap
+ * arrays. Queries that outgrow the kernel's memory get their items built and take the point scan, the bitmap
  * or the point-list kernel. The host waits once, after the gather. */
 int run_groups(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, int mode, int64_t* d_off, int32_t* d_tid,
                int32_t* d_pidx, int64_t capacity, int64_t* total) {
@@ -1760,6 +1775,58 @@ int run_groups(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, in
         GAT_CUDA_TRY(ctx, cudaStreamSynchronize(s), "range scan");
         return GAT_OK;
     };
+    /* id sets of more ids than a hash set holds: the `n` queries of `list` (items by list position when by_pos) */
+    auto bitmap_scan = [&](const gat_mbb* q, int n, const int64_t* ioff, const int2* items, int64_t* base, int64_t* cnt,
+                           const int* list, int by_pos) -> int {
+        const int words = (ix->db->n + 1 + 31) / 32;
+        const size_t smem = (size_t)words * 4;
+        const bool in_smem = smem <= 200 * 1024;
+        int per_sm = 0, rc = GAT_OK;
+        if (in_smem) allow_smem(k_range_ids, smem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_range_ids, kThreads, in_smem ? smem : 0);
+        const int g = std::min(n, std::max(1, per_sm) * ctx->sm_count);
+        uint32_t* gbm = in_smem ? nullptr : (uint32_t*)scratch(ctx, S_RANGE_ARENA2, (size_t)g * words * 4, &rc);
+        if (!in_smem && !gbm) return rc;
+        k_range_ids<<<g, kThreads, in_smem ? smem : 0, s>>>(q, n, ioff, items, ix->d_x, ix->d_y, ix->d_tid, words, gbm, arena, cap, ctr,
+                                                           base, cnt, ctx->timing ? ctr + 1 : nullptr, list, by_pos);
+        return GAT_OK;
+    };
+    /* queries whose walk outgrew the groups' kernel: as a batch of their own by the point scan, the ones with too
+     * many ids for its hash set by the bitmap */
+    auto point_scan = [&](int n, const int* list) -> int {
+        int rc = GAT_OK;
+        char* p = (char*)scratch(ctx, S_RANGE_LEFT, (size_t)n * (sizeof(gat_mbb) + 2 * sizeof(int64_t) + sizeof(int)), &rc);
+        if (!p) return rc;
+        gat_mbb* q = reinterpret_cast<gat_mbb*>(p);
+        int64_t* base = reinterpret_cast<int64_t*>(q + n);
+        int64_t* cnt = base + n;
+        int* many = reinterpret_cast<int*>(cnt + n);
+        k_take_left<<<(n + 255) / 256, 256, 0, s>>>(n, list, d_q, q);
+        int64_t* ioff = nullptr;
+        int2* items = nullptr;
+        if ((rc = build_items(ctx, ix, q, n, nullptr, &ioff, &items)) != GAT_OK) return rc;
+        if ((rc = check_device_flag(ctx, "range candidates")) != GAT_OK) return rc;
+        constexpr size_t kHashSmem = (size_t)(8192 + 4096) * sizeof(int);
+        allow_smem(k_range_hash<256, 13>, kHashSmem);
+        int per_sm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_range_hash<256, 13>, 256, kHashSmem);
+        GAT_CUDA_TRY(ctx, cudaMemsetAsync(ctr + 2, 0, 2 * sizeof(int64_t), s), "range"); /* its query and overflow counters */
+        timed_begin(ctx, GAT_KERNEL_RANGE_SCAN);
+        k_range_hash<256, 13><<<std::min(n, std::max(1, per_sm) * ctx->sm_count), 256, kHashSmem, s>>>(
+            q, n, ioff, items, ix->d_x, ix->d_y, ix->d_tid, arena, cap, ctr, base, cnt, many, ctx->timing ? ctr + 1 : nullptr, nullptr,
+            nullptr, 0);
+        GAT_CUDA_TRY(ctx, cudaGetLastError(), "range scan launch");
+        GAT_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_pinned, ctr, 4 * sizeof(int64_t), cudaMemcpyDeviceToHost, s), "range");
+        GAT_CUDA_TRY(ctx, cudaStreamSynchronize(s), "range scan");
+        const int n_many = (int)ctx->h_pinned[3];
+        if (n_many > 0) rc = bitmap_scan(q, n_many, ioff, items, base, cnt, many, 0);
+        timed_end(ctx, GAT_KERNEL_RANGE_SCAN, 0.0);
+        if (rc != GAT_OK) return rc;
+        k_put_left<<<(n + 255) / 256, 256, 0, s>>>(n, list, base, cnt, segbase, segcnt);
+        count_launch(ctx, n_many > 0 ? 4 : 3);
+        GAT_CUDA_TRY(ctx, cudaGetLastError(), "range scan launch");
+        return GAT_OK;
+    };
     for (int attempt = 0; attempt < 2; attempt++) {
         arena = (uint32_t*)scratch(ctx, S_RANGE_ARENA, (size_t)cap * 4, &st);
         if (!arena) return st;
@@ -1769,36 +1836,30 @@ int run_groups(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, int nq, in
                  : group_points_launch(ctx, ix, d_q, nq, arena, cap, ctr, segbase, segcnt, ovf_list, ovf_list + nq + 1);
         timed_end(ctx, GAT_KERNEL_RANGE_SCAN, 0.0);
         if (st != GAT_OK || (st = finish()) != GAT_OK) return st;
-        const int64_t n_ovf = ctx->h_pinned[3];
-        if (n_ovf > 0) {
-            int64_t* ioff = nullptr;
-            int2* items = nullptr;
-            if ((st = build_items(ctx, ix, d_q, (int)n_ovf, ovf_list, &ioff, &items)) != GAT_OK) return st;
-            if ((st = check_device_flag(ctx, "range candidates")) != GAT_OK) return st;
-            const int words = (ix->db->n + 1 + 31) / 32;
-            const size_t smem_bm = (size_t)words * 4;
-            const bool in_smem = smem_bm <= 200 * 1024;
-            int per_sm = 0;
-            if (ids && in_smem) allow_smem(k_range_ids, smem_bm);
-            if (ids)
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_range_ids, kThreads, in_smem ? smem_bm : 0);
-            else
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_range_points, kThreads, 0);
-            const int g = (int)std::max<int64_t>(1, std::min<int64_t>(n_ovf, (int64_t)std::max(1, per_sm) * ctx->sm_count));
-            uint32_t* gbm = !ids || in_smem ? nullptr : (uint32_t*)scratch(ctx, S_RANGE_ARENA2, (size_t)g * words * 4, &st);
-            if (ids && !in_smem && !gbm) return st;
-            timed_begin(ctx, GAT_KERNEL_RANGE_SCAN);
-            if (ids)
-                k_range_ids<<<g, kThreads, in_smem ? smem_bm : 0, s>>>(d_q, (int)n_ovf, ioff, items, ix->d_x, ix->d_y, ix->d_tid,
-                                                                      words, gbm, arena, cap, ctr, segbase, segcnt,
-                                                                      ctx->timing ? ctr + 1 : nullptr, ovf_list, 1);
-            else
-                k_range_points<<<g, kThreads, 0, s>>>(d_q, (int)n_ovf, ioff, items, ix->d_x, ix->d_y, ix->d_key, key_bits_of(ix),
-                                                      arena, cap, ctr, segbase, segcnt, ovf_list);
-            timed_end(ctx, GAT_KERNEL_RANGE_SCAN, 0.0);
-            count_launch(ctx);
-            GAT_CUDA_TRY(ctx, cudaGetLastError(), "range scan launch");
-            GAT_CUDA_TRY(ctx, cudaMemsetAsync(ctr + 3, 0, sizeof(int64_t), s), "range");
+        const int n_many = (int)ctx->h_pinned[3], n_long = (int)ctx->h_pinned[6];
+        if (n_many > 0 || n_long > 0) {
+            if (n_long > 0 && (st = point_scan(n_long, ovf_list + nq - n_long)) != GAT_OK) return st;
+            if (n_many > 0) {
+                int64_t* ioff = nullptr;
+                int2* items = nullptr;
+                if ((st = build_items(ctx, ix, d_q, n_many, ovf_list, &ioff, &items)) != GAT_OK) return st;
+                if ((st = check_device_flag(ctx, "range candidates")) != GAT_OK) return st;
+                timed_begin(ctx, GAT_KERNEL_RANGE_SCAN);
+                if (ids) {
+                    st = bitmap_scan(d_q, n_many, ioff, items, segbase, segcnt, ovf_list, 1);
+                } else {
+                    int per_sm = 0;
+                    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_range_points, kThreads, 0);
+                    k_range_points<<<std::min(n_many, std::max(1, per_sm) * ctx->sm_count), kThreads, 0, s>>>(
+                        d_q, n_many, ioff, items, ix->d_x, ix->d_y, ix->d_key, key_bits_of(ix), arena, cap, ctr, segbase, segcnt,
+                        ovf_list);
+                }
+                timed_end(ctx, GAT_KERNEL_RANGE_SCAN, 0.0);
+                count_launch(ctx);
+                if (st != GAT_OK) return st;
+                GAT_CUDA_TRY(ctx, cudaGetLastError(), "range scan launch");
+            }
+            GAT_CUDA_TRY(ctx, cudaMemsetAsync(ctr + 3, 0, 4 * sizeof(int64_t), s), "range");
             if ((st = finish()) != GAT_OK) return st;
         }
         const int64_t used = ctx->h_pinned[0];

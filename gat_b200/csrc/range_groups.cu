@@ -18,7 +18,9 @@
  * a quarter, all). Small teams keep more queries in flight and wait less at barriers: 15k rectangles
  * of 0.02 to 0.05 degrees over 1M walks took 2.07 ms by CTAs alone, 1.86 ms with pairs for those of
  * 400 to 1,100 expected ids. A query that outgrows its team
- * runs again on the CTA, one that outgrows that goes to the bitmap scan (range.cu).
+ * runs again on the CTA; one with more ids than that holds goes to the bitmap scan, one whose walk outgrows it to
+ * the point scan (range.cu; a rectangle over the whole of an FSG of 1,000 rows and 300 long walks: 1.16 ms by
+ * the point scan, 3.57 ms by the bitmap).
  *
  * Plain execution (one query per launch): the CTA answers one query and writes it where the query before
  * it ended. Each launch lets the next start at once; a query waits for the one before only to read its
@@ -47,6 +49,8 @@ constexpr int kMidTeams = kW / 2; /* pairs of warps */
 constexpr int kCtl = 24; /* control words of a team */
 /* expected ids up to which a query is small or mid: short of the set, since the estimate is not exact */
 constexpr float kSmallMax = 400.f, kMidMax = 1100.f;
+constexpr int kSmallScan = 4096, kMidScan = 8192; /* groups a small or a mid team takes on */
+constexpr float kBoundToOutgrow = 1.2f; /* plain execution: expected ids, as a multiple of the set's, that are not tried */
 constexpr int kFarCell = 1 << 20; /* FSG cell coordinates beyond this take the general scan */
 constexpr int kBorder = (int)0x80000000; /* item end flag: groups to be tested by box */
 
@@ -472,10 +476,11 @@ __device__ __forceinline__ void take_items(const int2* items, int n, const Box& 
  * runs and searching every id in every run took half of a query's instructions.) `out` may be the list
  * itself. FLIP is xored into what is written (point keys are held with their top bit flipped). */
 /* Fullest bucket that is ranked: ids, and point keys, which lie in clusters (1,500 rectangles of 0.003 to 0.03
- * degrees on 100k walks: 1270 us with 32, 1132 us with 512). Lists of more than kRadixMin keys are sorted by digits
- * instead as soon as a bucket holds more than kCrowd: a key is compared with every other of its bucket, a walk's
- * hundred or more points (148 lists of 10k points 248 us by ranks, 139 by digits; a thousand 1409 and 912). */
-constexpr int kCrowd = 32, kKeyCrowd = 512, kRadixMin = 1024;
+ * degrees on 100k walks: 1270 us with 32, 1132 us with 512). The second pass of point lists sorts by
+ * digits instead as soon as a bucket holds more than kCrowd: a key is compared with every other of its bucket, a
+ * walk's hundred or more points (148 lists of 10k points 248 us by ranks, 139 by digits; a thousand 1409 and 912). The
+ * first pass keeps to ranks: the digits' code in it cost 1,000 lists of about 110 points 5 us of 38. */
+constexpr int kCrowd = 32, kKeyCrowd = 512;
 
 /* The m keys of the team's list by a stable radix sort in shared memory, 8 bits of (key - lo) a pass, between the
  * list and the set's slots: each warp counts the digits of its share, a scan over digits and warps gives it
@@ -483,7 +488,7 @@ constexpr int kCrowd = 32, kKeyCrowd = 512, kRadixMin = 1024;
 template <class T, unsigned FLIP>
 __device__ void radix_keys(T& t, int m, unsigned range, unsigned lo, uint32_t* out, bool write, int me) {
     constexpr int W = T::NTHREADS / 32;
-    static_assert(T::NTHREADS != kNT || T::IDS + W * 256 <= (1 << T::HB), "the keys and the counters share the set's slots");
+    static_assert(T::NTHREADS == 256 && T::IDS + W * 256 <= (1 << T::HB), "the keys and the counters share the set's slots");
     const unsigned FULL = 0xffffffffu;
     const int lane = me & 31, warp = me >> 5;
     int* const hist = t.tab + (1 << T::HB) - W * 256;
@@ -606,8 +611,12 @@ __device__ void sort_ids(T& t, int m, uint32_t* out, bool write, int me) {
         most = lo_hi[2];
         for (int w = 0; w < warp; w++) start += lo_hi[4 + w];
     }
-    if (FLIP && (most > kKeyCrowd || (most > kCrowd && m > kRadixMin))) {
-        radix_keys<T, FLIP>(t, m, (unsigned)hi - (unsigned)lo, (unsigned)lo, out, write, me);
+    bool placed = false;
+    if constexpr (FLIP != 0 && T::IDS > kBlockIds) {
+        placed = most > kCrowd;
+        if (placed) radix_keys<T, FLIP>(t, m, (unsigned)hi - (unsigned)lo, (unsigned)lo, out, write, me);
+    }
+    if (placed) {
     } else if (most <= (FLIP ? kKeyCrowd : kCrowd)) {
 #pragma unroll
         for (int k = 0; k < kPer; k++) {
@@ -684,7 +693,7 @@ struct GroupQuery {
     uint32_t* arena;
     int64_t cap;
     /* [0] arena cursor, [1] work bytes, [2] big queries taken, [3] queries for the bitmap scan, [4] small
-     * queries taken, [5] queries that outgrew their team, [7] mid queries taken */
+     * queries taken, [5] queries that outgrew their team, [6] queries for the point scan, [7] mid queries taken */
     unsigned long long* ctr;
     int64_t* segbase;
     int64_t* segcnt;
@@ -694,15 +703,47 @@ struct GroupQuery {
     int64_t p_cap;
     int* p_state;
     int2* retry;   /* queries that outgrew their team, chained per CTA: (query, next or -1) */
-    int* ovf_list; /* queries for the bitmap scan */
+    int* ovf_list; /* queries for the bitmap scan from its front, for the point scan from its end */
     unsigned long long* work;
+    float share_border, share_inside; /* plain execution: new ids per group of a border item, per id of an inside one */
+    float points;                     /* points per group of the index */
 };
 
-/* one query of a team: walk, scan, sort, write; false when it outgrew the team's memory (which is
- * then empty again) */
+/* How a query ended: answered; more ids than the team's set holds; a walk beyond its frontier or ranges (nothing is
+ * scanned then). */
+enum Ending { kAnswered, kManyIds, kLongWalk };
+
+/* Whether a walk's candidates are left unscanned, by the groups to be tested by their boxes and the ids and groups
+ * inside (small and mid teams scan what they get: their class goes by the expected length too, k_order_class):
+ *   - by the CTA to the point scan when there are very many and they hold few points each: a group costs about as much
+ *     as four points of that scan when its box is looked at and two when it is inside (16 rectangles of 0.3 degrees on a
+ *     MortonGrid with 1.2 points a group, 450k groups each: 5.2 times the point scan's time by groups, the same now). That
+ *     scan begins when the batch is done, which a shorter query does not make up for (20k rectangles of up to 0.05 degrees
+ *     there: 1.2 times the point scan's time, 1.8 when those of 12k groups are left too);
+ *   - by plain execution, where one CTA stands against a grid that scans a long query's points (16k groups take it 50
+ *     us, about what it costs to change over), and which fills the set in vain when the query is bound to hold more ids
+ *     (a rectangle of 0.3 degrees on a MortonGrid of 100k walks: 528 us, 146 now, 120 by the point scan's three launches
+ *     alone). Candidates that count groups twice are kept: an FSG's rows overlap when the rectangle is wider than the
+ *     FSG, and the plain point scan has room for every point once.
+ * A Grid's batches are not weighed: its nodes' lists stand for many points each. */
+constexpr int kPlainScan = 16384, kBatchScan = 24576;
+template <int KIND, bool PLAIN>
+constexpr bool kWeighed = PLAIN || KIND != GAT_INDEX_GRID;
+
+template <bool PLAIN, class T>
+__device__ __forceinline__ bool too_long(const GroupQuery& a, int border, int inside) {
+    const float b = (float)border, i = (float)inside;
+    if (PLAIN)
+        return (b + 0.25f * i > (float)kPlainScan || b * a.share_border + i * a.share_inside > kBoundToOutgrow * (float)T::IDS) &&
+               border + inside <= a.g.n;
+    return b + i > (float)kBatchScan && 4.f * b + 2.f * i > (b + i) * a.points;
+}
+
+/* one query of a team: walk, scan, sort, write; the team's memory is empty again when it could not answer */
 template <int KIND, bool PLAIN = false, class T>
-__device__ bool answer(const GroupQuery& a, int qi, T& t, OpenGroups& og, int me, unsigned long long& bytes) {
+__device__ Ending answer(const GroupQuery& a, int qi, T& t, OpenGroups& og, int me, unsigned long long& bytes) {
     const Box q = load_box(a.queries, qi);
+    if (kWeighed<KIND, PLAIN> && T::NTHREADS == kNT && me == 0) *t.base = 0; /* the sums below, after the walk's barriers */
     if (KIND == GAT_INDEX_GRID)
         walk_grid<false>(a.g, a.grid, q, t, me);
     else if (KIND == GAT_INDEX_STIG)
@@ -712,6 +753,24 @@ __device__ bool answer(const GroupQuery& a, int qi, T& t, OpenGroups& og, int me
     else
         walk_fsg(a.fsg, a.g.cell_g, q, t, me);
     const int n = min(*t.nitems, T::ITEMS);
+    if constexpr (kWeighed<KIND, PLAIN> && T::NTHREADS == kNT) {
+        /* groups to be tested by their boxes, and ids and groups inside */
+        int border = 0, inside = 0;
+        for (int i = me; i < n; i += T::NTHREADS) {
+            const int2 it = t.items[i];
+            const int len = (it.y & ~kBorder) - it.x;
+            border += it.y < 0 ? len : 0;
+            inside += it.y < 0 ? 0 : len;
+        }
+        border = __reduce_add_sync(0xffffffffu, border);
+        inside = __reduce_add_sync(0xffffffffu, inside);
+        if ((me & 31) == 0) atomicAdd(t.base, (unsigned long long)border << 32 | (unsigned)inside);
+        t.sync();
+        border = (int)(*t.base >> 32);
+        inside = (int)(*t.base & 0xffffffffull);
+        if (me == 0 && too_long<PLAIN, T>(a, border, inside)) *t.ovf = 1;
+        t.sync();
+    }
     if (!__shfl_sync(0xffffffffu, *(volatile int*)t.ovf, 0)) {
         /* ranges per turn: enough turns for every warp, up to 32 a turn */
         constexpr int kWarps = T::NTHREADS / 32;
@@ -750,7 +809,7 @@ __device__ bool answer(const GroupQuery& a, int qi, T& t, OpenGroups& og, int me
         }
         if (go && at + m <= a.p_cap)
             for (int i = me; i < m; i += T::NTHREADS) a.p_out[at + i] = t.list[i];
-        return go;
+        return go ? kAnswered : kManyIds;
     }
     if (me == 0 && !lost) {
         *t.base = atomicAdd(&a.ctr[0], (unsigned long long)m);
@@ -766,7 +825,7 @@ __device__ bool answer(const GroupQuery& a, int qi, T& t, OpenGroups& og, int me
     }
     t.sync();
     if (me == 0) *t.nitems = t.nfront[0] = t.nfront[1] = *t.cnt = *t.ovf = *t.next = 0;
-    return !lost;
+    return !lost ? kAnswered : m > 0 ? kManyIds : kLongWalk;
 }
 
 /* A team's share of the queries list[0..n), taken from *ctr; the ones that outgrow it go on the CTA's chain. */
@@ -781,7 +840,7 @@ __device__ void answer_list(const GroupQuery& a, const int* __restrict__ list, i
         t.sync();
         if (j >= n) break;
         const int qi = list[j];
-        if (!answer<KIND>(a, qi, t, og, me, bytes) && me == 0) {
+        if (answer<KIND>(a, qi, t, og, me, bytes) != kAnswered && me == 0) {
             const int k = (int)atomicAdd(&a.ctr[5], 1ull);
             a.retry[k] = make_int2(qi, atomicExch(chain, k));
         }
@@ -812,8 +871,12 @@ __global__ void __launch_bounds__(kNT, 3) k_range_groups(GroupQuery a, const int
     int first_big = 0;
     BlockTeam t(mem, ctl[0], 0);
     auto block_query = [&](int qi) {
-        if (!answer<KIND>(a, qi, t, open[warp], threadIdx.x, bytes) && threadIdx.x == 0) {
-            a.ovf_list[atomicAdd(&a.ctr[3], 1ull)] = qi;
+        const Ending e = answer<KIND>(a, qi, t, open[warp], threadIdx.x, bytes);
+        if (e != kAnswered && threadIdx.x == 0) {
+            if (e == kManyIds)
+                a.ovf_list[atomicAdd(&a.ctr[3], 1ull)] = qi;
+            else
+                a.ovf_list[nq - 1 - (int)atomicAdd(&a.ctr[6], 1ull)] = qi;
             a.segcnt[qi] = 0;
             a.segbase[qi] = 0;
         }
@@ -921,10 +984,8 @@ __global__ void __launch_bounds__(kNT, AGAIN ? 1 : 3) k_group_points(GroupQuery 
         if (lane == 0 && all) atomicAdd(t.query, all);
         __syncthreads();
         const int points = *t.query;
-        const bool outgrown = *(volatile int*)t.ovf != 0; /* by the walk, which has no more room in the second pass */
-        const bool last = AGAIN || outgrown || points > LongTeam::IDS + LongTeam::IDS / 4;
         const bool many = !AGAIN && points > 2 * kBlockIds;
-        if (!many && !outgrown) {
+        if (!many && !__shfl_sync(FULL, *(volatile int*)t.ovf, 0)) {
             for (;;) {
                 int k = 0;
                 if (lane == 0) k = atomicAdd(t.next, 1);
@@ -961,9 +1022,11 @@ __global__ void __launch_bounds__(kNT, AGAIN ? 1 : 3) k_group_points(GroupQuery 
         }
         __syncthreads();
         const int m = *t.cnt;
-        const bool lost = many || outgrown || m > T::IDS;
+        const bool lost = many || *(volatile int*)t.ovf != 0 || m > T::IDS;
         if (me == 0) {
             if (lost) {
+                /* a walk that outgrew its memory would do so in the second pass too */
+                const bool last = AGAIN || *(volatile int*)t.ovf != 0 || points > LongTeam::IDS + LongTeam::IDS / 4;
                 (last ? a.ovf_list : again)[atomicAdd(&a.ctr[last ? 3 : 5], 1ull)] = qi;
                 a.segcnt[qi] = 0;
                 a.segbase[qi] = 0;
@@ -1008,6 +1071,7 @@ __global__ void k_order_class(const gat_mbb* queries, int nq, GroupsDev g, GridD
     const float w = q.xmax - q.xmin, h = q.ymax - q.ymin;
     float density = 0.f; /* walks per unit area */
     float est = -1.f;
+    float scan = 0.f;    /* groups of the candidates */
     int at = 0;          /* a group near the query's first one */
     if (KIND == GAT_INDEX_GRID) {
         const float cx = q.xmin + 0.5f * w, cy = q.ymin + 0.5f * h;
@@ -1046,7 +1110,9 @@ __global__ void k_order_class(const gat_mbb* queries, int nq, GroupsDev g, GridD
         const uint32_t id = spread_bits((uint32_t)x) | (spread_bits((uint32_t)y) << 1), span = (uint32_t)cells * (uint32_t)cells;
         const float c = tree.cell + reach;
         at = g.cell_g[id * span];
-        density = (float)(g.cell_g[id * span + span] - at) / ((float)span * c * c);
+        const float groups = (float)(g.cell_g[id * span + span] - at) / (float)span; /* per cell */
+        density = groups / (c * c);
+        scan = groups * (w / tree.cell) * (h / tree.cell);
     } else {
         const int g1 = max((int)__fdiv_rn(__fsub_rn(q.xmin, f.rxmin), f.cell), 0);
         const int g2 = min((int)__fdiv_rn(__fsub_rn(q.xmax, f.rxmin), f.cell), f.nx - 1);
@@ -1056,11 +1122,15 @@ __global__ void k_order_class(const gat_mbb* queries, int nq, GroupsDev g, GridD
             const int row = ((g3 + g4) >> 1) * f.nx;
             const float c = f.cell + reach;
             at = g.cell_g[row + g1];
-            density = (float)(g.cell_g[row + g2 + 1] - at) / ((float)(g2 - g1 + 1) * c * c);
+            const float groups = (float)(g.cell_g[row + g2 + 1] - at); /* of one row */
+            density = groups / ((float)(g2 - g1 + 1) * c * c);
+            scan = groups * (float)(g4 - g3 + 1);
         }
     }
+    if (KIND == GAT_INDEX_STIG) scan = est;
     if (KIND != GAT_INDEX_STIG) est = density * (w + reach) * (h + reach);
-    const int cls = est <= kSmallMax ? 0 : est <= kMidMax ? 1 : 2; /* NaN: big */
+    int cls = est <= kSmallMax ? 0 : est <= kMidMax ? 1 : 2; /* NaN: big */
+    if (scan > (float)kSmallScan) cls = max(cls, scan <= (float)kMidScan ? 1 : 2);
     const int b = cls * kBuckets + (int)min((long long)kBuckets - 1, (long long)at * kBuckets / (g.n + 1));
     bin[qi] = b;
     atomicAdd(&hist[b], 1);
@@ -1125,7 +1195,8 @@ int range_groups_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, i
     const int full = std::max(1, per_sm) * ctx->sm_count;
     GAT_CUDA_TRY(ctx, cudaMemsetAsync(ctr, 0, 8 * sizeof(unsigned long long), s), "range");
     GroupQuery a{d_q, ix->grid, ix->fsg, ix->morton, ix->groups, arena, cap, ctr, segbase, segcnt, nullptr, nullptr, 0, nullptr, nullptr,
-                 ovf_list, timed ? ctr + 1 : nullptr};
+                 ovf_list, timed ? ctr + 1 : nullptr, 0.f, 0.f,
+                 (float)ix->npoints / (float)std::max(1, ix->groups.n)};
     if (nq <= full) {
         /* no more queries than resident CTAs: one each, in block mode */
         kernel<<<nq, kNT, kSmem, s>>>(a, nullptr, nullptr, nq);
@@ -1162,8 +1233,11 @@ int plain_groups_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, i
                   : ix->kind == GAT_INDEX_MORTON ? k_plain_groups<GAT_INDEX_MORTON>
                                                  : k_plain_groups<GAT_INDEX_FSG>;
     if (qi == 0) allow_smem(kernel, kSmem);
+    /* a walk has about G / n groups in all and no more of them in a rectangle; it is in one or two of a Grid's lists */
+    const bool may_outgrow = ix->db->n > kBlockIds;
+    const float share = may_outgrow ? std::min(1.f, (float)ix->db->n / (float)std::max(1, ix->groups.n)) : 0.f;
     GroupQuery a{d_q, ix->grid, ix->fsg, ix->morton, ix->groups, nullptr, 0, nullptr, nullptr, nullptr, off, out, capacity, state,
-                 nullptr, nullptr, work};
+                 nullptr, nullptr, work, share, ix->kind == GAT_INDEX_GRID && may_outgrow ? 0.75f : share, 0.f};
     /* the first launch of a call waits for all before it: the queries may come from a kernel */
     if (qi == 0)
         kernel<<<1, kNT, kSmem, ctx->stream>>>(a, qi);
@@ -1188,7 +1262,7 @@ int group_points_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, i
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, first, kNT, kSmem);
         GAT_CUDA_TRY(ctx, cudaMemsetAsync(ctr, 0, 8 * sizeof(unsigned long long), s), "range");
         GroupQuery a{d_q, ix->grid, ix->fsg, ix->morton, ix->groups, arena, cap, ctr, segbase, segcnt, nullptr, nullptr, 0,
-                     nullptr, nullptr, ovf_list, nullptr};
+                     nullptr, nullptr, ovf_list, nullptr, 0.f, 0.f, 0.f};
         first<<<std::min(nq, std::max(1, per_sm) * ctx->sm_count), kNT, kSmem, s>>>(a, ix->d_key, nq, again);
         (void)launch_dep(ctx, second, dim3(std::min(nq, ctx->sm_count)), dim3(kNT), kLongSmem, s, a, (const uint32_t*)ix->d_key, nq,
                          again);

@@ -227,3 +227,45 @@ def test_clustered_point_keys(gpu_ctx, walks, points):
     for ix in (g, G.MortonGrid(g)):
         r = ix.range_query(q, "points", "batched", capacity=4_000_000)
         assert np.array_equal(r.offsets, off) and np.array_equal(r.tids, tid) and np.array_equal(r.pidx, pidx)
+
+
+@pytest.mark.parametrize("walks", [300, 6000])
+def test_scattered_points(gpu_ctx, walks):
+    """Points far from one another, most of them a group of its own: long candidate lists are handed to the CTA and
+    to the point scan, in batches on both sides of the one-CTA-each size and in plain execution."""
+    rng = np.random.default_rng(66)
+    t = D.walks(D.lengths(walks, 0, 0, 0, 20, 80, 66), 66)
+    t.lon[:] = rng.uniform(121.01, 121.99, t.lon.size)
+    t.lat[:] = rng.uniform(30.71, 31.69, t.lat.size)
+    db = G.TrajectorySet(gpu_ctx, t)
+    c = rng.uniform([121.05, 30.75], [121.95, 31.65], (500, 2))
+    h = np.exp(rng.uniform(np.log(0.002), np.log(0.45), (500, 1)))
+    q = np.concatenate([c - h, c + h], 1).astype(np.float32)
+    q[::50] = [121.0, 30.7, 122.0, 31.7]
+    g = G.Grid(gpu_ctx, db, D.BOX, 0.001, 2, 16)
+    for ix in (g, G.FSG(gpu_ctx, db, D.BOX, 0.001), G.MortonGrid(g), G.STIG(gpu_ctx, db, 32)):
+        a = _same(gpu_ctx, ix, q)
+        _same(gpu_ctx, ix, q[:16])
+        for lo, hi in ((0, 1), (1, 2), (5, 25), (40, 60)):
+            b = ix.range_query(q[lo:hi], "ids", "plain", capacity=4_000_000)
+            assert np.array_equal(b.offsets, a.offsets[lo:hi + 1] - a.offsets[lo])
+            assert np.array_equal(b.tids, a.tids[a.offsets[lo]:a.offsets[hi]])
+
+
+def test_walks_that_outgrow(gpu_ctx):
+    """Id sets of rectangles over more rows of cells, blocks and nodes than a team has room for, of few ids and of
+    more than a set holds, beside ordinary ones."""
+    t = D.walks(D.lengths(9_000, 0, 0, 0, 20, 60, 67), 67)
+    db = G.TrajectorySet(gpu_ctx, t)
+    x0, y0, x1, y1 = D.BOX
+    tall = [[x0 + 0.009 * k, y0 - 1, x0 + 0.009 * k + 0.004, y1 + 1] for k in range(100)]
+    wide = [[x0 - 1, y0 + 0.009 * k, x1 + 1, y0 + 0.009 * k + 0.004] for k in range(100)]
+    large = [[x0 + 0.01 * k, y0 + 0.01 * k, x1 - 0.01 * k, y1 - 0.01 * k] for k in range(20)]
+    q = np.concatenate([np.array(tall + wide + large, np.float32), D.boxes(300, 1, 0.001, 0.05, 68)])
+    g = G.Grid(gpu_ctx, db, D.BOX, 0.0004, 2, 1)
+    for ix in (g, G.FSG(gpu_ctx, db, D.BOX, 0.0004), G.MortonGrid(g), G.STIG(gpu_ctx, db, 16)):
+        a = _same(gpu_ctx, ix, q)
+        assert int(np.diff(a.offsets).max()) > 4096
+        _same(gpu_ctx, ix, q[95:105])
+        b = ix.range_query(q[98:102], "ids", "plain", capacity=4_000_000)
+        assert np.array_equal(b.tids, a.tids[a.offsets[98]:a.offsets[102]])
