@@ -1069,13 +1069,13 @@ int launch_tiles(gat_ctx* ctx, const Src& src, int64_t cap, int max_rows, int ma
     int st = GAT_OK;
     cudaStream_t s = ctx->stream;
     int per_sm = 0;
-    /* An SM's split between L1 and shared memory changes only while no block is resident on it.
-     * With the default (no preference) the persistent grid's blocks, which need 5 to 8 KB, leave their
-     * SMs at a small shared-memory split for the whole launch, and a kernel of another stream that
-     * needs more (the range scan's 48 KB blocks) could not start on any of them until the grid
-     * ended: range batches beside a long top-k round waited for it (16 rectangles, 1.1 ms alone:
-     * 10.5 ms median beside 18 ms EDR launches that left half the SMs free; 2.5 ms with the
-     * largest split). The tile kernel reads its points once and uses little L1. */
+    /* An SM's split between L1 and shared memory changes only while no block is resident on it, so a
+     * persistent grid that leaves room on its SMs and asks for no split keeps out the blocks of other streams
+     * that need more shared memory, until it ends: range batches beside a long top-k round waited for it (16
+     * rectangles, 1.1 ms alone: 10.5 ms median beside 18 ms EDR launches that left half the SMs free; 2.5 ms with
+     * the largest split; measured with CTAs of 256 threads, 5 KB each, and range blocks of 48 KB). It holds for
+     * the column kernel. A CTA of the row kernel takes all 65,536 registers of its SM: beside it only the SMs
+     * that the grid leaves (sm_reserve) are free. The tile kernels read their points once and use little L1. */
     constexpr auto kernel = TileKernel<R, COL, Src>::get();
     constexpr int kWarps = TileKernel<R, COL, Src>::kWarps;
     prefer_split(reinterpret_cast<const void*>(kernel), ctx->device, kEdrCarveoutPct);

@@ -2,12 +2,20 @@
  *
  * launch_dep launches a kernel with cudaLaunchAttributeProgrammaticStreamSerialization when the
  * context allows it (GAT_TUNE_DEP_LAUNCH, on by default): the GPU may then set the kernel up
- * while the previous kernel of the stream finishes. No kernel here triggers its dependents
- * early, so a dependent grid starts only after every block of the previous grid has exited.
- * Every kernel launched this way calls dep_wait() first, which returns once the previous grid
- * has completed and its writes are visible; ordering in the stream is therefore the same as
- * without the attribute, minus the launch gap. dep_wait() is a no-op for a kernel launched
- * without the attribute. */
+ * while the previous kernel of the stream finishes. Every kernel launched this way calls dep_wait(), which
+ * returns once the previous grid has completed and its writes are visible. All but one call it first
+ * and none of them triggers its dependents early, so such a grid starts only after every block of the
+ * previous one has exited, and ordering in the stream is the same as without the attribute, minus the
+ * launch gap. dep_wait() is a no-op for a kernel launched without the attribute.
+ *
+ * The exception is k_plain_groups (range_groups.cu), which lets the next query's launch of itself start at
+ * once and waits late. What keeps it safe:
+ *   - before its wait it reads only the index and the queries, both complete before the call's first launch
+ *     (which goes without the attribute), and writes only its own shared memory;
+ *   - every block of every instance reaches the wait, so that an instance completes after the one before and
+ *     its completion stands for all earlier ones;
+ *   - only instances of itself follow it with the attribute: a kernel behind it that took the attribute and
+ *     touched memory before its own wait would run beside it. The host waits for the stream after each lot. */
 #pragma once
 
 #include <mutex>

@@ -18,8 +18,9 @@
  *                  de-duplicates.
  *   3. offsets     scan of per-query result counts; one CTA per query copies its segment.
  * Plain execution runs the same pipeline once per query.
- * Batched id sets of an index with point groups take range_groups.cu instead; this pipeline serves
- * point lists, indexes without groups and the queries that outgrow that kernel's sets.
+ * An index with point groups takes range_groups.cu instead for id sets, and the Grid and the MortonGrid for
+ * point lists; this pipeline serves the point lists of STIG and the FSG, indexes without groups, the fixed shapes
+ * of GAT_TUNE_RANGE_SHAPE and the queries that outgrow those kernels.
  */
 #include <algorithm>
 #include <climits>

@@ -920,7 +920,9 @@ __global__ void __launch_bounds__(kNT, 3) k_range_groups(GroupQuery a, const int
     }
 }
 
-/* Plain execution: query qi of the call. */
+/* Plain execution: query qi of the call. The next query's instance starts at once; until dep_wait (in answer) an
+ * instance may read nothing that an earlier one writes (offsets, ids, state) and write nothing outside its
+ * shared memory, and none may return before it (launch.cuh). */
 template <int KIND>
 __global__ void __launch_bounds__(kNT, 2) k_plain_groups(GroupQuery a, int qi) {
     asm volatile("griddepcontrol.launch_dependents;");

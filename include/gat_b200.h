@@ -128,11 +128,15 @@ int gat_ctx_kernel_stats(gat_ctx* ctx, int kernel_class, double* ms, int64_t* la
  * GAT_TUNE_SERVE_RESERVE: read by gat_server_create from the context it is given: the percent of
  *   the SMs (1..90) that the persistent EDR grids of the server's top-k lanes leave free for its
  *   range lane; 0 (default) = 12. Same results.
- * GAT_TUNE_RANGE_SHAPE: how batched range queries find trajectory-id sets. 0 (default): through
- *   the index's point groups (the runs of one trajectory inside one leaf or cell, with their boxes);
- *   on an index whose groups found no memory by the point scan with an autotuned block shape: the
- *   first batch of each (index kind, batch size rounded up to a power of two) class times the shapes
- *   on its own queries and keeps the fastest. 1..3: the point scan on every index with a fixed shape: 1 = 256 threads per CTA with an 8192-slot id set, 2 = 128
+ * GAT_TUNE_RANGE_SHAPE: how range queries are answered. 0 (default): through the index's point groups
+ *   (the runs of one trajectory inside one leaf or cell, with their boxes), which take id sets on every
+ *   index and point lists on a Grid and a MortonGrid, batched and plain, and hand on queries that outgrow
+ *   them; everything else by the point scan. An index whose groups found no memory when it was built or
+ *   loaded has none and is answered by the point scan, several times slower (its device bytes in
+ *   gat_index_info are then fewer than those of a like one). Batches of id sets by the point scan take an
+ *   autotuned block shape: the first batch of each (index kind, batch size rounded up to a power of two)
+ *   class times the shapes on its own queries and keeps the fastest. 1..3: the point scan for every call,
+ *   with a fixed shape for batches of id sets: 1 = 256 threads per CTA with an 8192-slot id set, 2 = 128
  *   threads with a 4096-slot set, 3 = the batch split by size (queries with more than 16 candidate
  *   items on shape 1, the others one per warp with a 1024-slot set and no block barrier, in the same
  *   launch). Same results. Setting the knob clears the tuned table.
