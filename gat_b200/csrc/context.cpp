@@ -114,8 +114,11 @@ void raise_smem_limit(const void* kernel, size_t bytes) {
     int device = 0;
     cudaGetDevice(&device);
     std::lock_guard<std::mutex> lk(mu);
-    size_t& now = limit[{kernel, device}];
-    if (bytes > now && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess) now = bytes;
+    size_t& most = limit[{kernel, device}];
+    const size_t had = most;
+    most = std::max(most, bytes);
+    /* set on every call: the attribute does not outlast a cudaDeviceReset, this table does */
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) most = had;
 }
 
 void* scratch_zeroed(gat_ctx* ctx, int slot, size_t bytes, int* status) {
