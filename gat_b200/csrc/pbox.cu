@@ -112,6 +112,7 @@ int index_point_boxes(gat_index* ix) {
         cudaStreamSynchronize(s);
         cudaFree(ix->d_pbox);
         ix->d_pbox = nullptr;
+        ix->device_bytes -= (size_t)nn * sizeof(float4);
     }
     GAT_CUDA_TRY(ctx, cudaMalloc(&ix->d_pbox, (size_t)nn * sizeof(float4)), "point boxes");
     ix->device_bytes += (size_t)nn * sizeof(float4);
