@@ -691,7 +691,12 @@ struct GroupQuery {
     MortonDev morton;
     GroupsDev g;
     uint32_t* arena;
-    int64_t cap;
+    /* Fields of one mode share their place with the other's: 16 bytes more of parameters cost every plain launch 0.3
+     * us (24 plain rectangles on an FSG 128 -> 136 us). */
+    union {
+        int64_t cap;
+        float share[2]; /* plain execution: new ids per group of a border item, per id of an inside one */
+    };
     /* [0] arena cursor, [1] work bytes, [2] big queries taken, [3] queries for the bitmap scan, [4] small
      * queries taken, [5] queries that outgrew their team, [6] queries for the point scan, [7] mid queries taken */
     unsigned long long* ctr;
@@ -700,13 +705,14 @@ struct GroupQuery {
     /* plain execution: offsets, ids, their capacity, and the state of the call (answer) */
     int64_t* p_off;
     int32_t* p_out;
-    int64_t p_cap;
+    union {
+        int64_t p_cap;
+        float points; /* batches: points per group of the index */
+    };
     int* p_state;
     int2* retry;   /* queries that outgrew their team, chained per CTA: (query, next or -1) */
     int* ovf_list; /* queries for the bitmap scan from its front, for the point scan from its end */
     unsigned long long* work;
-    float share_border, share_inside; /* plain execution: new ids per group of a border item, per id of an inside one */
-    float points;                     /* points per group of the index */
 };
 
 /* How a query ended: answered; more ids than the team's set holds; a walk beyond its frontier or ranges (nothing is
@@ -734,7 +740,7 @@ template <bool PLAIN, class T>
 __device__ __forceinline__ bool too_long(const GroupQuery& a, int border, int inside) {
     const float b = (float)border, i = (float)inside;
     if (PLAIN)
-        return (b + 0.25f * i > (float)kPlainScan || b * a.share_border + i * a.share_inside > kBoundToOutgrow * (float)T::IDS) &&
+        return (b + 0.25f * i > (float)kPlainScan || b * a.share[0] + i * a.share[1] > kBoundToOutgrow * (float)T::IDS) &&
                border + inside <= a.g.n;
     return b + i > (float)kBatchScan && 4.f * b + 2.f * i > (b + i) * a.points;
 }
@@ -743,7 +749,6 @@ __device__ __forceinline__ bool too_long(const GroupQuery& a, int border, int in
 template <int KIND, bool PLAIN = false, class T>
 __device__ Ending answer(const GroupQuery& a, int qi, T& t, OpenGroups& og, int me, unsigned long long& bytes) {
     const Box q = load_box(a.queries, qi);
-    if (kWeighed<KIND, PLAIN> && T::NTHREADS == kNT && me == 0) *t.base = 0; /* the sums below, after the walk's barriers */
     if (KIND == GAT_INDEX_GRID)
         walk_grid<false>(a.g, a.grid, q, t, me);
     else if (KIND == GAT_INDEX_STIG)
@@ -754,9 +759,10 @@ __device__ Ending answer(const GroupQuery& a, int qi, T& t, OpenGroups& og, int 
         walk_fsg(a.fsg, a.g.cell_g, q, t, me);
     const int n = min(*t.nitems, T::ITEMS);
     if constexpr (kWeighed<KIND, PLAIN> && T::NTHREADS == kNT) {
-        /* groups to be tested by their boxes, and ids and groups inside */
+        /* groups to be tested by their boxes, and ids and groups inside: every warp adds them up for itself, which
+         * for a few dozen ranges is shorter than barriers */
         int border = 0, inside = 0;
-        for (int i = me; i < n; i += T::NTHREADS) {
+        for (int i = me & 31; i < n; i += 32) {
             const int2 it = t.items[i];
             const int len = (it.y & ~kBorder) - it.x;
             border += it.y < 0 ? len : 0;
@@ -764,12 +770,8 @@ __device__ Ending answer(const GroupQuery& a, int qi, T& t, OpenGroups& og, int 
         }
         border = __reduce_add_sync(0xffffffffu, border);
         inside = __reduce_add_sync(0xffffffffu, inside);
-        if ((me & 31) == 0) atomicAdd(t.base, (unsigned long long)border << 32 | (unsigned)inside);
-        t.sync();
-        border = (int)(*t.base >> 32);
-        inside = (int)(*t.base & 0xffffffffull);
-        if (me == 0 && too_long<PLAIN, T>(a, border, inside)) *t.ovf = 1;
-        t.sync();
+        if ((me & 31) == 0 && too_long<PLAIN, T>(a, border, inside)) *t.ovf = 1; /* the same in every warp */
+        __syncwarp();
     }
     if (!__shfl_sync(0xffffffffu, *(volatile int*)t.ovf, 0)) {
         /* ranges per turn: enough turns for every warp, up to 32 a turn */
@@ -1197,8 +1199,8 @@ int range_groups_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, i
     const int full = std::max(1, per_sm) * ctx->sm_count;
     GAT_CUDA_TRY(ctx, cudaMemsetAsync(ctr, 0, 8 * sizeof(unsigned long long), s), "range");
     GroupQuery a{d_q, ix->grid, ix->fsg, ix->morton, ix->groups, arena, cap, ctr, segbase, segcnt, nullptr, nullptr, 0, nullptr, nullptr,
-                 ovf_list, timed ? ctr + 1 : nullptr, 0.f, 0.f,
-                 (float)ix->npoints / (float)std::max(1, ix->groups.n)};
+                 ovf_list, timed ? ctr + 1 : nullptr};
+    a.points = (float)ix->npoints / (float)std::max(1, ix->groups.n);
     if (nq <= full) {
         /* no more queries than resident CTAs: one each, in block mode */
         kernel<<<nq, kNT, kSmem, s>>>(a, nullptr, nullptr, nq);
@@ -1239,7 +1241,9 @@ int plain_groups_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, i
     const bool may_outgrow = ix->db->n > kBlockIds;
     const float share = may_outgrow ? std::min(1.f, (float)ix->db->n / (float)std::max(1, ix->groups.n)) : 0.f;
     GroupQuery a{d_q, ix->grid, ix->fsg, ix->morton, ix->groups, nullptr, 0, nullptr, nullptr, nullptr, off, out, capacity, state,
-                 nullptr, nullptr, work, share, ix->kind == GAT_INDEX_GRID && may_outgrow ? 0.75f : share, 0.f};
+                 nullptr, nullptr, work};
+    a.share[0] = share;
+    a.share[1] = ix->kind == GAT_INDEX_GRID && may_outgrow ? 0.75f : share;
     /* the first launch of a call waits for all before it: the queries may come from a kernel */
     if (qi == 0)
         kernel<<<1, kNT, kSmem, ctx->stream>>>(a, qi);
@@ -1264,7 +1268,7 @@ int group_points_launch(gat_ctx* ctx, const gat_index* ix, const gat_mbb* d_q, i
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, first, kNT, kSmem);
         GAT_CUDA_TRY(ctx, cudaMemsetAsync(ctr, 0, 8 * sizeof(unsigned long long), s), "range");
         GroupQuery a{d_q, ix->grid, ix->fsg, ix->morton, ix->groups, arena, cap, ctr, segbase, segcnt, nullptr, nullptr, 0,
-                     nullptr, nullptr, ovf_list, nullptr, 0.f, 0.f, 0.f};
+                     nullptr, nullptr, ovf_list, nullptr};
         first<<<std::min(nq, std::max(1, per_sm) * ctx->sm_count), kNT, kSmem, s>>>(a, ix->d_key, nq, again);
         (void)launch_dep(ctx, second, dim3(std::min(nq, ctx->sm_count)), dim3(kNT), kLongSmem, s, a, (const uint32_t*)ix->d_key, nq,
                          again);
