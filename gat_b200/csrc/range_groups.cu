@@ -761,12 +761,13 @@ __device__ Ending answer(const GroupQuery& a, int qi, T& t, OpenGroups& og, int 
     if constexpr (kWeighed<KIND, PLAIN> && T::NTHREADS == kNT) {
         /* groups to be tested by their boxes, and ids and groups inside: every warp adds them up for itself, which
          * for a few dozen ranges is shorter than barriers */
+        constexpr int kEnough = 1 << 24; /* a lane's share: the sums stay below 2^31 */
         int border = 0, inside = 0;
         for (int i = me & 31; i < n; i += 32) {
             const int2 it = t.items[i];
-            const int len = (it.y & ~kBorder) - it.x;
-            border += it.y < 0 ? len : 0;
-            inside += it.y < 0 ? 0 : len;
+            const int len = min((it.y & ~kBorder) - it.x, kEnough);
+            border = min(border + (it.y < 0 ? len : 0), kEnough);
+            inside = min(inside + (it.y < 0 ? 0 : len), kEnough);
         }
         border = __reduce_add_sync(0xffffffffu, border);
         inside = __reduce_add_sync(0xffffffffu, inside);
