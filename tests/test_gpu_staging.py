@@ -50,14 +50,14 @@ if sys.argv[1] == "edr":
 
 size = int(open("/proc/self/statm").read().split()[0]) * resource.getpagesize()
 resource.setrlimit(resource.RLIMIT_AS, (size, resource.RLIM_INFINITY))
-# what the driver still holds of pinned memory, in pieces; at most 64 MB
+# what the driver still holds of pinned memory, in pieces; at most 320 MB
 pinned = C.CDLL("libcuda.so.1").cuMemAllocHost_v2
 for piece in (1 << 20, 256 << 10):
-    for _ in range(32):
+    for _ in range(256):
         if pinned(C.byref(C.c_void_p()), C.c_size_t(piece)) != 0:
             break
     else:
-        sys.exit("pinned memory does not run out under the limit")
+        sys.exit(77)
 rc = edr(out) if sys.argv[1] == "edr" else ranges(150, off2, tid2)[0]
 resource.setrlimit(resource.RLIMIT_AS, (resource.RLIM_INFINITY, resource.RLIM_INFINITY))
 assert rc == 0, (rc, L.lib.gat_last_error(ctx.h))
@@ -72,4 +72,6 @@ print("same")
 @pytest.mark.parametrize("call", ["range", "edr"])
 def test_no_pinned_memory(call):
     r = subprocess.run([sys.executable, "-c", CHILD, call], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    if r.returncode == 77:
+        pytest.skip("pinned memory does not run out under an address space limit here")
     assert r.returncode == 0 and "same" in r.stdout, r.stdout + r.stderr
